@@ -14,10 +14,10 @@
 // Values travel as 64-bit words: i32 sign-extended, u8 and bool zero-extended, f32 as its 32
 // bits. Every fold except the canonical float sum and product is order-free (wrapping integer
 // arithmetic, the 754-2019 minimum/maximum, bit operations), so those reductions are a plain
-// grid fold and the scans a reduce-then-scan over 4096-row tiles. The canonical float order
-// (f32 sums, every float product) is sixteen chains of dependent IEEE operations: one block
-// stages the rows in shared memory while sixteen threads run the chains (fast enough for these
-// secondary entries; the f64 sums have their own exact parallel path in k_canon.cu).
+// grid fold and the scans a reduce-then-scan over 4096-row tiles. The canonical order of a float
+// product is sixteen chains of dependent IEEE multiplies: one block stages the rows in shared
+// memory while sixteen threads run the chains (the float sums have exact parallel paths, in
+// k_canon.cu and k_canon32.cu).
 #include <climits>
 #include <cstring>
 
@@ -27,6 +27,11 @@
 namespace vkc {
 
 vkc_status bucket_key_error(vkc_ctx *ctx, const long long *k, int64_t n, int64_t nb, bool *found);
+// The canonical f32 sums (k_canon32.cu).
+ReducerImpl *make_canon32_sum(vkc_ctx *ctx);
+ReducerImpl *make_canon32_dot(vkc_ctx *ctx);
+ReducerImpl *make_canon32_sumsq(vkc_ctx *ctx);
+ReducerImpl *make_canon32_cond(vkc_ctx *ctx, int cmp);
 
 namespace {
 
@@ -401,31 +406,21 @@ template <vkc_type T, bool MAX> ReducerImpl *make_arg(vkc_ctx *ctx) {
     return r;
 }
 
-// ------------------------------------------------------------------ canonical float chains
+// ------------------------------------------------------------------ canonical float products
 //
-// reduce.rs:45-91: lane j adds (multiplies) rows 16b + j in order from the identity; then +8,
-// +4, +2, +1; then the tail. One block: warps 1..7 stage chunk k + 1 (FC_ROWS rows, as row values)
+// reduce.rs:45-91: lane j multiplies rows 16b + j in order from 1; then the lanes 8, 4, 2 and 1
+// apart; then the tail. One block: warps 1..7 stage chunk k + 1 (FC_ROWS rows, as row values)
 // in shared memory while the first sixteen threads of warp 0 run their lane chains over chunk k.
 constexpr int FC_BLOCKS = 128;               // 16-row blocks per chunk
 constexpr int FC_ROWS = FC_BLOCKS * 16;      // rows per chunk
 
-template <vkc_type T> __device__ __forceinline__ u64 fop(u64 a, u64 b, bool mul) {
-    if (T == VKC_F64) {
-        const double x = __longlong_as_double(static_cast<long long>(a)), y = __longlong_as_double(static_cast<long long>(b));
-        return static_cast<u64>(__double_as_longlong(mul ? __dmul_rn(x, y) : __dadd_rn(x, y)));
-    }
-    const float x = __uint_as_float(static_cast<unsigned>(a)), y = __uint_as_float(static_cast<unsigned>(b));
-    return __float_as_uint(mul ? __fmul_rn(x, y) : __fadd_rn(x, y));
-}
-
-template <vkc_type T, int ROW, bool MUL>
-__global__ void __launch_bounds__(256) fam_chain_kernel(RowArgs a, int64_t nb, u64 *lanes) {
+template <vkc_type T> __global__ void __launch_bounds__(256) fam_chain_kernel(const void *x, int64_t nb, u64 *lanes) {
     __shared__ u64 buf[2][FC_ROWS];
     const int t = threadIdx.x;
     const int64_t chunks = (nb + FC_BLOCKS - 1) / FC_BLOCKS;
     auto stage = [&](int64_t k, int first, int step) {
         const int64_t r0 = k * FC_ROWS, rows = min(static_cast<int64_t>(FC_ROWS), nb * 16 - r0);
-        for (int i = first; i < rows; i += step) buf[k & 1][i] = row_value<T, ROW>(a, r0 + i);
+        for (int i = first; i < rows; i += step) buf[k & 1][i] = ld_word<T>(x, r0 + i);
     };
     u64 s = t < 16 ? lanes[t] : 0ull;
     if (chunks > 0) stage(0, t, 256);
@@ -436,104 +431,70 @@ __global__ void __launch_bounds__(256) fam_chain_kernel(RowArgs a, int64_t nb, u
         } else if (t < 16) {
             const int blocks = static_cast<int>(min(static_cast<int64_t>(FC_BLOCKS), nb - k * FC_BLOCKS));
             const u64 *b = buf[k & 1];
-            for (int i = 0; i < blocks; ++i) s = fop<T>(s, b[i * 16 + t], MUL);
+            for (int i = 0; i < blocks; ++i) s = mul_t<T>(s, b[i * 16 + t]);
         }
         __syncthreads();
     }
     if (t < 16) lanes[t] = s;
 }
 
-// The tail rows (fewer than 16) as row values, kept until finish.
-template <vkc_type T, int ROW>
-__global__ void fam_chain_tail(RowArgs a, int64_t first, int rest, u64 *tail) {
-    if (static_cast<int>(threadIdx.x) < rest) tail[threadIdx.x] = row_value<T, ROW>(a, first + threadIdx.x);
+// The tail rows (fewer than 16), kept until finish.
+template <vkc_type T> __global__ void fam_chain_tail(const void *x, int64_t first, int rest, u64 *tail) {
+    if (static_cast<int>(threadIdx.x) < rest) tail[threadIdx.x] = ld_word<T>(x, first + threadIdx.x);
 }
 
 // reduce.rs:77-91 (finish_lanes).
-template <vkc_type T, bool MUL> __global__ void fam_chain_finish(u64 *st, int tail_len) {
+template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len) {
     u64 acc[16];
     for (int j = 0; j < 16; ++j) acc[j] = st[j];
     for (int s = 8; s > 0; s >>= 1)
-        for (int j = 0; j < s; ++j) acc[j] = fop<T>(acc[j], acc[j + s], MUL);
+        for (int j = 0; j < s; ++j) acc[j] = mul_t<T>(acc[j], acc[j + s]);
     u64 r = acc[0];
-    for (int j = 0; j < tail_len; ++j) r = fop<T>(r, st[16 + j], MUL);
+    for (int j = 0; j < tail_len; ++j) r = mul_t<T>(r, st[16 + j]);
     st[32] = r;
 }
 
 // CanonicalAcc (reduce.rs:253-323) on the device. State: [0..15] lanes, [16..31] tail, [32] result.
-struct ChainReducer : DevReducer {
-    vkc_type in;
-    int row, nargs_want, cmp = 0;
+template <vkc_type T> struct ChainReducer : DevReducer {
     int tail_len = 0;
-    using Launch = void (*)(vkc_ctx *, const RowArgs &, int64_t nb, int64_t first, int rest, u64 *state);
-    Launch launch = nullptr;
-    using Fin = void (*)(vkc_ctx *, u64 *, int);
-    Fin fin = nullptr;
 
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
-        if (nargs != nargs_want) return fail(ctx, VKC_RUNTIME, arity_error(nargs_want, nargs));
-        if (!rows_arg(ctx, args[0], in, &st)) return st;
-        RowArgs a{args[0].a->data(), nullptr, cmp, 0, 0};
-        if (row == R_DOT) {
-            if (!rows_arg(ctx, args[1], in, &st)) return st;
-            if (args[0].len() != args[1].len())
-                return fail(ctx, VKC_RUNTIME, "length mismatch: " + std::to_string(args[0].len()) + " vs " +
-                                                  std::to_string(args[1].len()));
-            a.y = args[1].a->data();
-        } else if (row == R_COND) {
-            if (!splat_arg(ctx, args[1], in, &st) || !splat_arg(ctx, args[2], in, &st)) return st;
-            a.c = scalar_word(in, args[1].s);
-            a.e = scalar_word(in, args[2].s);
-        }
+        if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));
+        if (!rows_arg(ctx, args[0], T, &st)) return st;
         const int64_t n = args[0].len();
         if (tail_len != 0) return fail(ctx, VKC_RUNTIME, "canonical update after a partial block");
+        const void *x = args[0].a->data();
+        auto *s = static_cast<u64 *>(state);
         const int64_t nb = n / 16;
         const int rest = static_cast<int>(n % 16);
-        launch(ctx, a, nb, nb * 16, rest, static_cast<u64 *>(state));
+        if (nb > 0) fam_chain_kernel<T><<<1, 256, 0, ctx->stream>>>(x, nb, s);
+        if (rest > 0) fam_chain_tail<T><<<1, 16, 0, ctx->stream>>>(x, nb * 16, rest, s + 16);
         tail_len = rest;
         return launched(ctx, "family_chain");
     }
+    vkc_status result(vkc_ctx *ctx) {
+        fam_chain_finish<T><<<1, 1, 0, ctx->stream>>>(static_cast<u64 *>(state), tail_len);
+        return launched(ctx, "family_chain_finish");
+    }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
-        fin(ctx, static_cast<u64 *>(state), tail_len);
-        vkc_status st = launched(ctx, "family_chain_finish");
+        vkc_status st = result(ctx);
         if (st) return st;
         u64 r = 0;
         if ((st = download(ctx, &r, 8, 32 * 8))) return st;
-        *out = word_scalar(in, r);
+        *out = word_scalar(T, r);
         return VKC_OK;
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        fin(ctx, static_cast<u64 *>(state), tail_len);
-        vkc_status st = launched(ctx, "family_chain_finish");
-        return st ? st : copy_out(ctx, dst, static_cast<size_t>(width_of(in)), 32 * 8);
+        const vkc_status st = result(ctx);
+        return st ? st : copy_out(ctx, dst, static_cast<size_t>(width_of(T)), 32 * 8);
     }
 };
 
-template <vkc_type T, int ROW, bool MUL>
-void launch_chain(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int64_t first, int rest, u64 *state) {
-    if (nb > 0) fam_chain_kernel<T, ROW, MUL><<<1, 256, 0, ctx->stream>>>(a, nb, state);
-    if (rest > 0) fam_chain_tail<T, ROW><<<1, 16, 0, ctx->stream>>>(a, first, rest, state + 16);
-}
-template <vkc_type T, bool MUL> void finish_chain(vkc_ctx *ctx, u64 *state, int tail_len) {
-    fam_chain_finish<T, MUL><<<1, 1, 0, ctx->stream>>>(state, tail_len);
-}
-
-template <vkc_type T, int ROW, bool MUL, int NARGS> ReducerImpl *make_chain(vkc_ctx *ctx, int cmp) {
-    auto *r = new ChainReducer;
-    if (r->alloc(ctx, 33 * 8)) {
-        delete r;
-        return nullptr;
-    }
-    r->in = T;
-    r->row = ROW;
-    r->nargs_want = NARGS;
-    r->cmp = cmp;
-    r->launch = launch_chain<T, ROW, MUL>;
-    r->fin = finish_chain<T, MUL>;
+template <vkc_type T> ReducerImpl *make_product(vkc_ctx *ctx) {
+    auto *r = new ChainReducer<T>;
     const u64 one = T == VKC_F64 ? 0x3ff0000000000000ull : 0x3f800000ull;
-    const u64 v = MUL ? one : 0ull;
-    if (r->fill(ctx, 33, v, v, v, v)) {
+    if (r->alloc(ctx, 33 * 8) || r->fill(ctx, 33, one, one, one, one)) {
         delete r;
         return nullptr;
     }
@@ -1132,9 +1093,9 @@ bool has(const std::vector<KernelDef> &t, const std::string &name) {
 template <vkc_type T> void reg_numeric(std::vector<KernelDef> &t) {
     const std::string n = type_name(T);
     const uint64_t w = width_of(T);
-    if (is_float(T)) {
-        add_red(t, "reduce_add_" + n, {arr(T)}, T, w, [](vkc_ctx *c) { return make_chain<T, R_PLAIN, false, 1>(c, 0); });
-        add_red(t, "reduce_mul_" + n, {arr(T)}, T, w, [](vkc_ctx *c) { return make_chain<T, R_PLAIN, true, 1>(c, 0); });
+    if (T == VKC_F32) {
+        add_red(t, "reduce_add_" + n, {arr(T)}, T, w, make_canon32_sum);
+        add_red(t, "reduce_mul_" + n, {arr(T)}, T, w, make_product<VKC_F32>);
     } else {
         add_red(t, "reduce_add_" + n, {arr(T)}, sum_type(T), w,
                 [](vkc_ctx *c) { return make_fold<T, F_ADD, R_PLAIN, 1>(c, sum_type(T), 0, false, ""); });
@@ -1163,14 +1124,15 @@ template <vkc_type T> void reg_bits(std::vector<KernelDef> &t) {
 template <vkc_type T, int C> void reg_cmp(std::vector<KernelDef> &t) {
     const std::string n = type_name(T), c = CMP_NAME[C];
     const uint64_t w = width_of(T);
+    static_assert(T != VKC_F64, "the f64 entries are k_reduce.cu's, k_select.cu's and k_canon.cu's");
     add_red(t, "count_" + c + "_" + n, {arr(T), sca(T)}, VKC_I64, w,
             [](vkc_ctx *x) { return make_fold<T, F_ADD, R_PRED, 2>(x, VKC_I64, C, false, ""); });
     KernelDef f{"filter_" + c + "_" + n, VKC_SELECTION, {arr(T), sca(T)}, true, T, 2 * w};
     f.sel = filter_fam<T, C>;
     t.push_back(f);
-    if (is_float(T))
+    if (T == VKC_F32)
         add_red(t, "condsum_" + c + "_" + n, {arr(T), sca(T), sca(T)}, T, w,
-                [](vkc_ctx *x) { return make_chain<T, R_COND, false, 3>(x, C); });
+                [](vkc_ctx *x) { return make_canon32_cond(x, C); });
     else
         add_red(t, "condsum_" + c + "_" + n, {arr(T), sca(T), sca(T)}, sum_type(T), w,
                 [](vkc_ctx *x) { return make_fold<T, F_ADD, R_COND, 3>(x, sum_type(T), C, false, ""); });
@@ -1179,9 +1141,9 @@ template <vkc_type T, int C> void reg_cmp(std::vector<KernelDef> &t) {
 template <vkc_type T> void reg_fused(std::vector<KernelDef> &t) {
     const std::string n = type_name(T);
     const uint64_t w = width_of(T);
-    if (is_float(T)) {
-        add_red(t, "dot_" + n, {arr(T), arr(T)}, T, 2 * w, [](vkc_ctx *c) { return make_chain<T, R_DOT, false, 2>(c, 0); });
-        add_red(t, "sumsq_" + n, {arr(T)}, T, w, [](vkc_ctx *c) { return make_chain<T, R_SUMSQ, false, 1>(c, 0); });
+    if (T == VKC_F32) {
+        add_red(t, "dot_" + n, {arr(T), arr(T)}, T, 2 * w, make_canon32_dot);
+        add_red(t, "sumsq_" + n, {arr(T)}, T, w, make_canon32_sumsq);
     } else {
         add_red(t, "dot_" + n, {arr(T), arr(T)}, sum_type(T), 2 * w,
                 [](vkc_ctx *c) { return make_fold<T, F_ADD, R_DOT, 2>(c, sum_type(T), 0, false, ""); });
@@ -1251,7 +1213,7 @@ void register_families(std::vector<KernelDef> &t) {
     reg_numeric<VKC_U8>(t);
     reg_numeric<VKC_U64>(t);
     add_red(t, "reduce_mul_f64", {arr(VKC_F64)}, VKC_F64, 8,
-            [](vkc_ctx *c) { return make_chain<VKC_F64, R_PLAIN, true, 1>(c, 0); });
+            make_product<VKC_F64>);
     add_red(t, "reduce_mul_i64", {arr(VKC_I64)}, VKC_I64, 8,
             [](vkc_ctx *c) { return make_fold<VKC_I64, F_MUL, R_PLAIN, 1>(c, VKC_I64, 0, false, ""); });
     reg_bits<VKC_I64>(t);
