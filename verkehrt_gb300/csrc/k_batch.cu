@@ -14,11 +14,12 @@
 //    reference's 16 lanes (lane j takes survivors j, j+16, ... below the last whole block of 16,
 //    with IEEE adds in that order), combines the lanes +8, +4, +2, +1 and adds the tail
 //    (src/kernels/scalar/reduce.rs:45-91): the bits of filter then reduce_add_f64.
-//  * argsort (vkc_batch_argsort_i64): the keys of every array, as their sign-flipped images, are
-//    copied into one run with their positions in the run; stable radix passes over the key
-//    digits given (all eight when none are), then over the digits of the array index, sort the
-//    run by (array, key); each array's positions are written to its output relative to its first
-//    row. Stability makes every output the array's own argsort.
+//  * argsort (vkc_batch_argsort_i64): every row of every array gets one image, its array's number
+//    above the key digits given (all eight when none are), in 32 bits where they fit; stable radix
+//    passes over the image sort all rows by (array, key), and the last one writes each array's
+//    positions to its output relative to its first row. Stability makes every output the array's
+//    own argsort. (Key digits and number beyond 64 bits: the order by the keys first, then by the
+//    arrays' numbers, found again from the positions.)
 #include <algorithm>
 #include <cstring>
 #include <numeric>
@@ -26,13 +27,10 @@
 #include <vector>
 
 #include "lookback.cuh"
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
-
-vkc_status radix_pairs(vkc_ctx *ctx, unsigned long long *img[2], unsigned *pos[2], int64_t n, const int *shifts,
-                       int npasses, unsigned *counts, unsigned *offs, unsigned *sums, int *which);
-void radix_pairs_scratch(int64_t n, int64_t *count_words, int64_t *sum_words);
 
 struct BSeg {
     const void *ptr;
@@ -55,7 +53,7 @@ struct vkc_batch {
     vkc::DeviceMem chunks;            // int64 [n + 1]: first concat chunk of each array, table order
     // Argsort scratch, made on first use.
     std::vector<vkc_array *> scratch;
-    unsigned long long *img[2] = {nullptr, nullptr};
+    void *img[2] = {nullptr, nullptr};  // 64-bit images of `total` rows each
     unsigned *pos[2] = {nullptr, nullptr};
     unsigned *counts = nullptr, *offs = nullptr, *sums = nullptr;
     const vkc_batch *out_batch = nullptr;  // the batch whose pointers `outs` holds
@@ -232,25 +230,53 @@ __global__ void __launch_bounds__(BF_THREADS) batch_dot_kernel(const BSeg *__res
 
 // ------------------------------------------------------------------ argsort
 
-// Images and positions of every array, in index order (array i at rows bases[i]..).
-__global__ void __launch_bounds__(256) batch_keys_kernel(const BSeg *__restrict__ segs, int nseg,
-                                                         unsigned long long *__restrict__ img,
-                                                         unsigned *__restrict__ pos) {
-    for (int sg = blockIdx.y; sg < nseg; sg += gridDim.y) {
-        const BSeg seg = segs[sg];
-        const auto *k = static_cast<const long long *>(seg.ptr);
-        for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < seg.n;
-             i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-            img[seg.base + i] = static_cast<unsigned long long>(__ldg(k + i)) ^ 0x8000000000000000ull;
-            pos[seg.base + i] = static_cast<unsigned>(seg.base + i);
-        }
+// Rows of one array per block of the image and concatenation kernels; chunks[] gives each array's
+// first block, table order.
+constexpr int BC_ROWS = 8192;
+
+// The array (table order) that block c works on: the last one whose first block is <= c (an empty
+// array has no block).
+__device__ __forceinline__ int batch_chunk_array(const int64_t *__restrict__ chunks, int nseg, int64_t c) {
+    int lo = 0, hi = nseg - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (chunks[mid] <= c) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The sort images: row i of array a gets (a << 8 digits) + the chosen digits of its key's
+// sign-flipped image (NUMBER = false: the digits alone). One block per chunk: a search a block, not
+// one a row, and 12 bytes moved a row (the former pass wrote 64-bit images and positions from a grid
+// over the arrays: 326 us for 63 M rows).
+struct BatchDigits {
+    int n;
+    int shift[8];
+};
+template <class IMG, bool NUMBER>
+__global__ void __launch_bounds__(256) batch_images_kernel(const BSeg *__restrict__ segs, int nseg,
+                                                           const int64_t *__restrict__ chunks, BatchDigits d,
+                                                           IMG *__restrict__ img) {
+    const int64_t c = blockIdx.x;
+    const int lo = batch_chunk_array(chunks, nseg, c);
+    const BSeg seg = segs[lo];
+    const int64_t r0 = (c - chunks[lo]) * BC_ROWS, r1 = min(seg.n, r0 + BC_ROWS);
+    const auto *k = static_cast<const unsigned long long *>(seg.ptr);
+    const IMG number = NUMBER ? static_cast<IMG>(static_cast<unsigned long long>(seg.index) << (8 * d.n)) : IMG(0);
+#pragma unroll 8
+    for (int64_t r = r0 + threadIdx.x; r < r1; r += 256) {
+        const unsigned long long key = __ldcs(k + r) ^ 0x8000000000000000ull;
+        unsigned long long im = 0;
+        for (int j = 0; j < d.n; ++j) im |= ((key >> d.shift[j]) & 0xffull) << (8 * j);
+        img[seg.base + r] = static_cast<IMG>(im) | number;
     }
 }
 
-// Replaces every image by the index of the array its position belongs to (bases[nseg] = total).
+// The number of the array each position belongs to (bases[nseg] = total).
 __global__ void __launch_bounds__(256) batch_owner_kernel(const int64_t *__restrict__ bases, int nseg,
                                                           const unsigned *__restrict__ pos,
-                                                          unsigned long long *__restrict__ img, int64_t total) {
+                                                          unsigned *__restrict__ number, int64_t total) {
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
          i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
         const int64_t p = pos[i];
@@ -260,24 +286,7 @@ __global__ void __launch_bounds__(256) batch_owner_kernel(const int64_t *__restr
             if (bases[mid] <= p) lo = mid;
             else hi = mid - 1;
         }
-        img[i] = static_cast<unsigned long long>(lo);
-    }
-}
-
-// Row i of the sorted run belongs to the array whose rows cover i; its position relative to that
-// array's first row goes to that array's output at i - first row.
-__global__ void __launch_bounds__(256) batch_split_kernel(const int64_t *__restrict__ bases, int nseg,
-                                                          const unsigned *__restrict__ pos,
-                                                          long long *const *__restrict__ outs, int64_t total) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
-         i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-        int lo = 0, hi = nseg - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (bases[mid] <= i) lo = mid;
-            else hi = mid - 1;
-        }
-        outs[lo][i - bases[lo]] = static_cast<long long>(pos[i]) - bases[lo];
+        number[i] = static_cast<unsigned>(lo);
     }
 }
 
@@ -285,10 +294,7 @@ __global__ void __launch_bounds__(256) batch_split_kernel(const int64_t *__restr
 
 // Batched statements whose kernel has no batched form (group_id, reduce_into, scans) run once
 // over the concatenation of the batch's arrays, with an index column naming each row's array:
-// a segmented statement keyed by that column gives every array's own result. One block per
-// 8192-row chunk of one array (chunks[] gives each array's first chunk, table order).
-constexpr int BC_ROWS = 8192;
-
+// a segmented statement keyed by that column gives every array's own result. One block per chunk.
 template <int W>
 __global__ void __launch_bounds__(256) batch_concat_kernel(const BSeg *__restrict__ segs, int nseg,
                                                            const int64_t *__restrict__ chunks, void *rows,
@@ -296,12 +302,7 @@ __global__ void __launch_bounds__(256) batch_concat_kernel(const BSeg *__restric
     using U = typename std::conditional<W == 8, unsigned long long,
                                         typename std::conditional<W == 4, unsigned, unsigned char>::type>::type;
     const int64_t c = blockIdx.x;
-    int lo = 0, hi = nseg - 1;  // the last array whose first chunk is <= c (no chunk: empty array)
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (chunks[mid] <= c) lo = mid;
-        else hi = mid - 1;
-    }
+    const int lo = batch_chunk_array(chunks, nseg, c);
     const BSeg seg = segs[lo];
     const int64_t r0 = (c - chunks[lo]) * BC_ROWS;
     const int64_t r1 = min(seg.n, r0 + BC_ROWS);
@@ -469,7 +470,7 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
         for (vkc_array *a : keys->scratch) vkc_array_release(a);
         keys->scratch.clear();
         int64_t cw, sw;
-        radix_pairs_scratch(total, &cw, &sw);
+        radix_table_words(total, &cw, &sw);
         vkc_array *a[7];
         const vkc_type ty[7] = {VKC_U64, VKC_U64, VKC_I32, VKC_I32, VKC_I32, VKC_I32, VKC_I32};
         const int64_t len[7] = {total, total, total, total, cw, cw, sw};
@@ -477,8 +478,8 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
             if ((st = new_array(ctx, ty[i], len[i], false, &a[i]))) return st;
             keys->scratch.push_back(a[i]);
         }
-        keys->img[0] = static_cast<unsigned long long *>(a[0]->data());
-        keys->img[1] = static_cast<unsigned long long *>(a[1]->data());
+        keys->img[0] = a[0]->data();
+        keys->img[1] = a[1]->data();
         keys->pos[0] = static_cast<unsigned *>(a[2]->data());
         keys->pos[1] = static_cast<unsigned *>(a[3]->data());
         keys->counts = static_cast<unsigned *>(a[4]->data());
@@ -498,34 +499,45 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
         VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         keys->out_batch = outs;
     }
+    if (n > 65536) return fail(ctx, VKC_USAGE, "batch argsort of more than 65536 arrays");
     const auto *tab = static_cast<const BSeg *>(keys->table.ptr);
     const auto *bases = static_cast<const int64_t *>(keys->bases.ptr);
-    dim3 kg(std::max(1, std::min(64, static_cast<int>((total / n + 255) / 256))), std::min(n, 65535));
-    batch_keys_kernel<<<kg, 256, 0, ctx->stream>>>(tab, n, keys->img[0], keys->pos[0]);
-    vkc_status st = launched(ctx, "batch_keys");
-    if (st) return st;
-    // Key digits: given, or all eight.
-    int shifts[8], np = 0;
+    const auto *ch = static_cast<const int64_t *>(keys->chunks.ptr);
+    int64_t nchunks = 0;
+    for (const BSeg &g : keys->host) nchunks += (g.n + BC_ROWS - 1) / BC_ROWS;
+    // Key digits: given, or all eight. Then the array's number, one or two digits.
     if (key_digits == 0) key_digits = 0xff;
-    for (int d = 0; d < 8; ++d)
-        if ((key_digits >> d) & 1u) shifts[np++] = 8 * d;
-    int which = 0;
-    if ((st = radix_pairs(ctx, keys->img, keys->pos, total, shifts, np, keys->counts, keys->offs, keys->sums, &which)))
-        return st;
-    // Then by array index (two 8-bit digits cover 65536 arrays).
-    const int grid = stream_grid(ctx, total, 256, 8, 2048);
-    batch_owner_kernel<<<grid, 256, 0, ctx->stream>>>(bases, n, keys->pos[which], keys->img[which], total);
+    BatchDigits d{};
+    for (int k = 0; k < 8; ++k)
+        if ((key_digits >> k) & 1u) d.shift[d.n++] = 8 * k;
+    const int numbers = n > 256 ? 2 : 1, digits = d.n + numbers;
+    int shifts[8];
+    for (int k = 0; k < 8; ++k) shifts[k] = 8 * k;
+    const RadixTables t{keys->counts, keys->offs, keys->sums};
+    BatchOut batch{bases, static_cast<const unsigned long long *>(keys->outs.ptr), 8 * d.n};
+    const int blocks = static_cast<int>(nchunks);
+    vkc_status st;
+    if (digits <= 4) {
+        batch_images_kernel<unsigned, true><<<blocks, 256, 0, ctx->stream>>>(tab, n, ch, d, static_cast<unsigned *>(keys->img[1]));
+        if ((st = launched(ctx, "batch_images"))) return st;
+        return radix_batch(ctx, false, keys->img[1], keys->img, keys->pos, batch, total, shifts, digits, t);
+    }
+    auto *wide = static_cast<unsigned long long *>(keys->img[1]);
+    if (digits <= 8) {
+        batch_images_kernel<unsigned long long, true><<<blocks, 256, 0, ctx->stream>>>(tab, n, ch, d, wide);
+        if ((st = launched(ctx, "batch_images"))) return st;
+        return radix_batch(ctx, true, wide, keys->img, keys->pos, batch, total, shifts, digits, t);
+    }
+    batch_images_kernel<unsigned long long, false><<<blocks, 256, 0, ctx->stream>>>(tab, n, ch, d, wide);
+    if ((st = launched(ctx, "batch_images"))) return st;
+    if ((st = radix_batch_keys(ctx, wide, keys->img, keys->pos, total, shifts, d.n, t))) return st;
+    const int at = (d.n - 1) & 1;
+    auto *number = static_cast<unsigned *>(keys->img[1 - at]);
+    batch_owner_kernel<<<stream_grid(ctx, total, 256, 8, 2048), 256, 0, ctx->stream>>>(bases, n, keys->pos[at], number, total);
     if ((st = launched(ctx, "batch_owner"))) return st;
-    if (n > 65536) return fail(ctx, VKC_USAGE, "batch argsort of more than 65536 arrays");
-    const int seg_shifts[2] = {0, 8};
-    unsigned long long *img2[2] = {keys->img[which], keys->img[1 - which]};
-    unsigned *pos2[2] = {keys->pos[which], keys->pos[1 - which]};
-    int w2 = 0;
-    if ((st = radix_pairs(ctx, img2, pos2, total, seg_shifts, n > 256 ? 2 : 1, keys->counts, keys->offs, keys->sums, &w2)))
-        return st;
-    batch_split_kernel<<<grid, 256, 0, ctx->stream>>>(bases, n, pos2[w2], static_cast<long long *const *>(keys->outs.ptr),
-                                                     total);
-    return launched(ctx, "batch_split");
+    batch.index_shift = 0;
+    return radix_batch_numbers(ctx, number, keys->pos[at], static_cast<unsigned *>(keys->img[at]), keys->pos[1 - at], batch,
+                               total, numbers, t);
 }
 
 extern "C" VKC_API vkc_status vkc_batch_concat(vkc_ctx *ctx, vkc_batch *b, vkc_array **rows, vkc_array **index) {

@@ -45,12 +45,11 @@
 #include <cmath>
 
 #include "lookback.cuh"
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
 
-int64_t scan_counts_sum_words(int64_t m);
-void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, unsigned *out);
 
 constexpr int CT_THREADS = 256;
 constexpr int CT_SEGS = 32;       // segments per tile

@@ -8,7 +8,7 @@
 //               (src/kernels/scalar/fused.rs:73-379)
 //   scans       scan_<fold>_T, scan_by_<fold>_T, reduce_into_<fold>_T, prev_T
 //               (src/kernels/scalar/scan.rs:16-439)
-//   whole       argsort_T, group_id_T, group_id2_A_B (index.rs:159-173, group.rs:259-363),
+//   whole       group_id_T, group_id2_A_B (group.rs:259-363),
 //               fill_T, same_len_T (construct.rs:49-120), slice_T (index.rs:240-258)
 //
 // Values travel as 64-bit words: i32 sign-extended, u8 and bool zero-extended, f32 as its 32
@@ -907,24 +907,21 @@ vkc_status filter_fam(vkc_ctx *ctx, const Arg *args, int nargs, int64_t base, Bu
 
 // ------------------------------------------------------------------ whole kernels
 
-// Widens keys to i64 for the i64 entries: for argsort an image whose i64 order is the key
-// order (u64: flip the top bit; i32 and u8: the value), for group ids any one-to-one image.
-template <vkc_type T, bool ORDER>
+// Widens keys to i64 for the i64 group ids (any one-to-one image serves).
+template <vkc_type T>
 __global__ void fam_widen_kernel(const void *x, int64_t n, long long *o) {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        u64 w = ld_word<T>(x, i);
-        if (ORDER && T == VKC_U64) w ^= 1ull << 63;
-        o[i] = static_cast<long long>(w);
+        o[i] = static_cast<long long>(ld_word<T>(x, i));
     }
 }
 
-template <vkc_type T, bool ORDER> vkc_status widen(vkc_ctx *ctx, const vkc_array *a, vkc_array **out) {
+template <vkc_type T> vkc_status widen(vkc_ctx *ctx, const vkc_array *a, vkc_array **out) {
     vkc_status st;
     if ((st = new_array(ctx, VKC_I64, a->len, false, out))) return st;
     if (a->len > 0) {
         const int g = stream_grid(ctx, a->len, 256, 8, 2048);
-        fam_widen_kernel<T, ORDER><<<g, 256, 0, ctx->stream>>>(a->data(), a->len, static_cast<long long *>((*out)->data()));
+        fam_widen_kernel<T><<<g, 256, 0, ctx->stream>>>(a->data(), a->len, static_cast<long long *>((*out)->data()));
         if ((st = launched(ctx, "family_widen"))) {
             vkc_array_release(*out);
             return st;
@@ -933,29 +930,13 @@ template <vkc_type T, bool ORDER> vkc_status widen(vkc_ctx *ctx, const vkc_array
     return VKC_OK;
 }
 
-// argsort_T (index.rs:159-173): the stable ascending positions, those of the widened keys.
-template <vkc_type T> vkc_status argsort_fam(vkc_ctx *ctx, const vkc_value *args, int nargs, vkc_value *out) {
-    vkc_status st;
-    if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));
-    if (!array_arg(ctx, args[0], T, &st)) return st;
-    vkc_array *w;
-    if ((st = widen<T, true>(ctx, args[0].array, &w))) return st;
-    static const KernelDef *d = kernel_def("argsort_i64");
-    vkc_value a{};
-    a.kind = VKC_VALUE_ARRAY;
-    a.array = w;
-    st = d->whole(ctx, &a, 1, out);
-    vkc_array_release(w);
-    return st;
-}
-
 // group_id_T (group.rs:259-274): ids by first occurrence depend only on which rows are equal.
 template <vkc_type T> vkc_status group_id_fam(vkc_ctx *ctx, const vkc_value *args, int nargs, vkc_value *out) {
     vkc_status st;
     if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));
     if (!array_arg(ctx, args[0], T, &st)) return st;
     vkc_array *w;
-    if ((st = widen<T, false>(ctx, args[0].array, &w))) return st;
+    if ((st = widen<T>(ctx, args[0].array, &w))) return st;
     static const KernelDef *d = kernel_def("group_id_i64");
     vkc_value a{};
     a.kind = VKC_VALUE_ARRAY;
@@ -974,8 +955,8 @@ template <vkc_type A, vkc_type B> vkc_status group_id2_fam(vkc_ctx *ctx, const v
         return fail(ctx, VKC_RUNTIME, "length mismatch: " + std::to_string(args[0].array->len) + " vs " +
                                           std::to_string(args[1].array->len));
     vkc_array *wa, *wb;
-    if ((st = widen<A, false>(ctx, args[0].array, &wa))) return st;
-    if ((st = widen<B, false>(ctx, args[1].array, &wb))) {
+    if ((st = widen<A>(ctx, args[0].array, &wa))) return st;
+    if ((st = widen<B>(ctx, args[1].array, &wb))) {
         vkc_array_release(wa);
         return st;
     }
@@ -1254,9 +1235,6 @@ void register_families(std::vector<KernelDef> &t) {
     reg_prev<VKC_U8>(t);
     reg_prev<VKC_BOOL>(t);
     // index.rs:290-325, group.rs:352-363, construct.rs:214-270
-    add_whole(t, "argsort_u64", {arr(VKC_U64)}, VKC_I64, 16, argsort_fam<VKC_U64>);
-    add_whole(t, "argsort_i32", {arr(VKC_I32)}, VKC_I64, 12, argsort_fam<VKC_I32>);
-    add_whole(t, "argsort_u8", {arr(VKC_U8)}, VKC_I64, 9, argsort_fam<VKC_U8>);
     add_whole(t, "group_id_u64", {arr(VKC_U64)}, VKC_I64, 16, group_id_fam<VKC_U64>);
     add_whole(t, "group_id_i32", {arr(VKC_I32)}, VKC_I64, 12, group_id_fam<VKC_I32>);
     add_whole(t, "group_id_u8", {arr(VKC_U8)}, VKC_I64, 9, group_id_fam<VKC_U8>);

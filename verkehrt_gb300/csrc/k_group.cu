@@ -18,6 +18,7 @@
 // overflow flag) once half its slots hold keys or a probe of 64 slots is reached, and only then
 // is the full table filled. Inputs with few distinct keys never touch the large table.
 #include "lookback.cuh"
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
@@ -624,8 +625,6 @@ static void launch_insert(vkc_ctx *ctx, bool small, const long long *a, const lo
     kern<<<grid, GI_THREADS, 0, ctx->stream>>>(a, b, n, t, slot_of, flags, ctx->status);
 }
 
-int64_t scan_counts_sum_words(int64_t m);
-void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, unsigned *out);
 
 // Single keys, many distinct, at least GR_MIN_ROWS rows: the region-partitioned path above.
 constexpr int64_t GR_MIN_ROWS = int64_t(1) << 22;

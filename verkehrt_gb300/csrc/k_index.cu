@@ -5,12 +5,11 @@
 // value in index order (first_out_of_range, index.rs:102-111). Here the check is fused into
 // the kernel: each offending row does an atomicMin of its row number into the status word,
 // and the host reports the value at that row and discards the output.
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
 
-int64_t scan_counts_sum_words(int64_t m);
-void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, unsigned *out);
 
 // ------------------------------------------------------------------ gather
 

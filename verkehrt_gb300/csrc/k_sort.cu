@@ -1,26 +1,31 @@
-// argsort_i64: the stable ascending positions of the rows (src/kernels/scalar/index.rs:159-173,
-// src/kernels/scalar/index/radix.rs:126-259).
+// argsort_T: the stable ascending positions of the rows (src/kernels/scalar/index.rs:159-173,
+// src/kernels/scalar/index/radix.rs:126-259), for i64, u64, i32 and u8 keys; and the radix passes
+// that the batched argsort and the float bucket sums use.
 //
-// LSD radix sort over the 8-bit digits of the sign-flipped image (radix.rs:58-61) of
-// (key, position) pairs, as the reference does, restated for the GPU:
-//  * one histogram kernel counts all 8 digits in one read (radix.rs:199-202);
-//  * a digit that is equal in every row leaves the order unchanged and its pass is skipped
-//    (radix.rs:203-211);
-//  * each remaining digit is one reduce-then-scan pass over tiles of 256 x radix_items rows (the
-//    autotuner's table: 2048, 3072 or 4096 rows by size): `up` counts each
-//    tile's digits into a digit-major table, one exclusive scan of that table gives every
-//    (digit, tile) its first output row, and `down` ranks the tile's rows stably by digit
-//    (a ballot per digit bit, in row order) and scatters them. The first pass reads the keys, the
-//    last writes the positions as i64. (A single-pass lookback per digit was slower here: the
-//    lookback of 256 digits per tile advances a few tiles per L2 round trip. A persistent
-//    `down` whose next tile arrives by TMA while it ranks the current one was no faster
-//    either: the pass is bound by instruction issue, about 3.8 warp instructions per row.)
+// LSD radix sort over 8-bit digits of (image, payload) pairs, as the reference does, restated for
+// the GPU:
+//  * the image of a key is its order-preserving unsigned value (radix.rs:58-61: the sign bit
+//    flipped); one reduction finds the images' least and greatest value and the bits that vary.
+//    The passes cover the bytes that vary (radix.rs:203-211: an equal digit leaves the order
+//    unchanged), or, when those are fewer, the bytes of the image's distance from the least one
+//    (signed keys of a small range vary in every byte, but not in their distance);
+//  * each pass is reduce-then-scan over tiles of 256 x radix_items rows (the autotuner's table:
+//    2048, 3072 or 4096 rows by size): `up` counts each tile's digits into a digit-major table, one
+//    exclusive scan of that table gives every (digit, tile) its first output row, and `down` ranks
+//    the tile's rows stably by digit and scatters them. The first pass reads the keys, the last
+//    writes the positions as i64. (A single-pass lookback per digit was slower here: the lookback
+//    of 256 digits per tile advances a few tiles per L2 round trip.)
+//  * `down` finds the lanes of a warp that share a digit by a ballot per digit bit. (An atomic OR of
+//    the lane's bit into the digit's shared word took a third of the instructions, 1.6 a row against
+//    3.8, but twice the shared-memory wavefronts, and these then bound the pass: 101 us against 79
+//    for 2^24 rows.)
 // Stability makes the output the reference's; inputs of at most 2048 rows are sorted in one
 // block by comparison (as the reference does below 1024 rows, radix.rs:140-151), inputs of at
 // most 8192 rows by the same radix passes inside one block.
 #include <algorithm>
 
 #include "lookback.cuh"
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
@@ -31,56 +36,86 @@ constexpr int RADIX = 256;
 
 // Rows per thread of a pass (the autotuner's radix_items: 8, 12 or 16; even, as ranks are
 // packed in pairs), the tile, and the resident blocks per SM that the down kernel's registers
-// allow (the best of a sweep over 3-6 per shape).
-template <int ITEMS> struct RsShape {
-    static_assert(ITEMS % 2 == 0, "ranks are packed two per word");
+// allow. PAIR: bytes of an image and its payload.
+template <int ITEMS, int PAIR> struct RsShape {
+    static_assert(ITEMS % 4 == 0, "ranks are packed two per word, images counted four at a time");
     static constexpr int TILE = RS_THREADS * ITEMS;
-    static constexpr int MIN_BLOCKS = ITEMS >= 16 ? 3 : (ITEMS >= 12 ? 4 : 5);
-    // Dynamic shared memory of the down kernel: the tile's images and positions sorted by digit.
-    static constexpr size_t DOWN_SMEM = (sizeof(unsigned long long) + sizeof(unsigned)) * TILE;
+    static constexpr int MIN_BLOCKS = ITEMS >= 16 ? (PAIR == 8 ? 4 : 3) : (ITEMS >= 12 ? 4 : 5);
+    // Dynamic shared memory of the down kernel: the tile's images and payloads sorted by digit.
+    static constexpr size_t DOWN_SMEM = static_cast<size_t>(PAIR) * TILE;
 };
 constexpr int RS_MIN_TILE = RS_THREADS * 8;
 
-__device__ __forceinline__ unsigned long long image_of(long long k) {
-    return static_cast<unsigned long long>(k) ^ 0x8000000000000000ull;
+// The keys of the first pass: the image of the key word k is (k ^ flip) - low, W bytes wide.
+template <int W> struct KeyWord;
+template <> struct KeyWord<8> { using T = unsigned long long; };
+template <> struct KeyWord<4> { using T = unsigned; };
+template <> struct KeyWord<1> { using T = unsigned char; };
+struct KeySource {
+    const void *keys;
+    unsigned long long flip, low;
+};
+template <int W> __device__ __forceinline__ unsigned long long key_image(const KeySource &k, int64_t r) {
+    using T = typename KeyWord<W>::T;
+    return (static_cast<unsigned long long>(__ldcs(static_cast<const T *>(k.keys) + r)) ^ k.flip) - k.low;
 }
 
-// Counts every digit of every row into hist[8][256]. (One atomic per warp for a digit all 32
-// rows share, found by warp votes, was slower: shared-memory atomics on one address are cheap
-// here, the votes are not.)
-__global__ void __launch_bounds__(256) rs_hist_kernel(const long long *__restrict__ keys, int64_t n,
-                                                      unsigned *__restrict__ hist) {
-    __shared__ unsigned h[8][RADIX];
-    for (int i = threadIdx.x; i < 8 * RADIX; i += blockDim.x) (&h[0][0])[i] = 0;
-    __syncthreads();
-    // Eight rows a thread per loop pass, all loaded before the first atomic (the atomics keep the
-    // program's order, so a load after one would wait for it).
-    constexpr int R = 8;
+// range[0..3]: the AND and the least (from all ones), the OR and the greatest (from zero) of the
+// images.
+template <int W>
+__global__ void __launch_bounds__(256) rs_range_kernel(KeySource k, int64_t n, unsigned long long *range) {
+    constexpr int R = 8;  // rows a thread loads together
+    unsigned long long all = ~0ull, lo = ~0ull, any = 0, hi = 0;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
     for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < n; i0 += R * stride) {
-        unsigned long long k[R];
+        unsigned long long v[R];
 #pragma unroll
-        for (int j = 0; j < R; ++j) k[j] = i0 + j * stride < n ? image_of(__ldcs(keys + i0 + j * stride)) : 0ull;
+        for (int j = 0; j < R; ++j) v[j] = key_image<W>(k, i0 + j * stride < n ? i0 + j * stride : i0);
 #pragma unroll
-        for (int j = 0; j < R; ++j)
-            if (i0 + j * stride < n)
+        for (int j = 0; j < R; ++j) {
+            all &= v[j];
+            any |= v[j];
+            lo = min(lo, v[j]);
+            hi = max(hi, v[j]);
+        }
+    }
 #pragma unroll
-                for (int p = 0; p < 8; ++p) atomicAdd(&h[p][(k[j] >> (8 * p)) & 0xff], 1u);
+    for (int o = 16; o > 0; o >>= 1) {
+        all &= __shfl_xor_sync(FULL, all, o);
+        any |= __shfl_xor_sync(FULL, any, o);
+        lo = min(lo, __shfl_xor_sync(FULL, lo, o));
+        hi = max(hi, __shfl_xor_sync(FULL, hi, o));
+    }
+    __shared__ unsigned long long s[4][8];
+    if ((threadIdx.x & 31) == 0) {
+        const int w = threadIdx.x >> 5;
+        s[0][w] = all;
+        s[1][w] = lo;
+        s[2][w] = any;
+        s[3][w] = hi;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 8 * RADIX; i += blockDim.x) {
-        unsigned v = (&h[0][0])[i];
-        if (v) atomicAdd(hist + i, v);
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) {
+            all &= s[0][w];
+            lo = min(lo, s[1][w]);
+            any |= s[2][w];
+            hi = max(hi, s[3][w]);
+        }
+        atomicAnd(range, all);
+        atomicMin(range + 1, lo);
+        atomicOr(range + 2, any);
+        atomicMax(range + 3, hi);
     }
 }
 
 // Up: the digit counts of every tile, digit-major: counts[d * tiles + tile]. Shared-memory
-// atomics into one histogram per warp (the order of the increments does not matter here).
-template <int RS_ITEMS, bool FIRST, class IMG>
-__global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(const long long *__restrict__ keys_in,
-                                                           const IMG *__restrict__ img_in, int64_t n,
+// atomics into one histogram per warp (the order of the increments does not matter here). W: the
+// first pass, from keys of W bytes; 0: from images.
+template <int RS_ITEMS, int W, class IMG>
+__global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IMG *__restrict__ img_in, int64_t n,
                                                            int shift, int tiles, unsigned *__restrict__ counts) {
-    constexpr int RS_TILE = RsShape<RS_ITEMS>::TILE;
+    constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     __shared__ unsigned s_cnt[RS_WARPS][RADIX];
     const int tile = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -89,10 +124,24 @@ __global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(const long long *__re
     const int64_t base = static_cast<int64_t>(tile) * RS_TILE + static_cast<int64_t>(w) * (32 * RS_ITEMS);
     if (base + 32 * RS_ITEMS <= n) {
         IMG img[RS_ITEMS];
+        if constexpr (W != 0) {
 #pragma unroll
-        for (int j = 0; j < RS_ITEMS; ++j) {
-            const int64_t r = base + j * 32 + lane;
-            img[j] = FIRST ? static_cast<IMG>(image_of(__ldcs(keys_in + r))) : __ldcs(img_in + r);
+            for (int j = 0; j < RS_ITEMS; ++j) img[j] = static_cast<IMG>(key_image<W>(k, base + j * 32 + lane));
+        } else {
+            constexpr int V = 16 / sizeof(IMG);  // images of a 16-byte load (image buffers start aligned)
+#pragma unroll
+            for (int j = 0; j < RS_ITEMS / V; ++j) {
+                const uint4 u = __ldcs(reinterpret_cast<const uint4 *>(img_in + base) + j * 32 + lane);
+                if constexpr (V == 4) {
+                    img[4 * j] = u.x;
+                    img[4 * j + 1] = u.y;
+                    img[4 * j + 2] = u.z;
+                    img[4 * j + 3] = u.w;
+                } else {
+                    img[2 * j] = (static_cast<unsigned long long>(u.y) << 32) | u.x;
+                    img[2 * j + 1] = (static_cast<unsigned long long>(u.w) << 32) | u.z;
+                }
+            }
         }
 #pragma unroll
         for (int j = 0; j < RS_ITEMS; ++j) atomicAdd(&s_cnt[w][static_cast<unsigned>(img[j] >> shift) & 0xffu], 1u);
@@ -100,7 +149,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(const long long *__re
         for (int j = 0; j < RS_ITEMS; ++j) {
             const int64_t r = base + j * 32 + lane;
             if (r < n) {
-                const IMG im = FIRST ? static_cast<IMG>(image_of(__ldcs(keys_in + r))) : __ldcs(img_in + r);
+                const IMG im = W != 0 ? static_cast<IMG>(key_image<W ? W : 8>(k, r)) : img_in[r];
                 atomicAdd(&s_cnt[w][static_cast<unsigned>(im >> shift) & 0xffu], 1u);
             }
         }
@@ -163,24 +212,48 @@ __global__ void __launch_bounds__(1024) rs_scan_top(unsigned *sums, int k) {
     }
 }
 
+// Thread t holds the chunk's rows t * SCAN_ITEMS .. + SCAN_ITEMS - 1 (contiguous), so a block
+// exclusive sum of the thread totals orders them. VEC: both arrays start on 16-byte boundaries, so a
+// thread's rows move as four 16-byte accesses (one word at a time, each warp access touched 32
+// sectors: 17 us for 2.5 M counts).
+template <bool VEC>
 __global__ void __launch_bounds__(SCAN_THREADS) rs_scan_apply(const unsigned *__restrict__ c, int64_t m,
                                                                const unsigned *__restrict__ sums,
                                                                unsigned *__restrict__ out) {
-    // Thread t holds the chunk's rows t*SCAN_ITEMS .. +SCAN_ITEMS-1 (contiguous), so a block
-    // exclusive sum of the thread totals orders them.
     const int64_t b0 = static_cast<int64_t>(blockIdx.x) * SCAN_CHUNK + static_cast<int64_t>(threadIdx.x) * SCAN_ITEMS;
+    const bool whole = VEC && b0 + SCAN_ITEMS <= m;
     unsigned v[SCAN_ITEMS], t = 0;
+    if (whole) {
 #pragma unroll
-    for (int j = 0; j < SCAN_ITEMS; ++j) {
-        v[j] = b0 + j < m ? c[b0 + j] : 0u;
-        t += v[j];
+        for (int q = 0; q < SCAN_ITEMS / 4; ++q) {
+            const uint4 u = *reinterpret_cast<const uint4 *>(c + b0 + 4 * q);
+            v[4 * q] = u.x;
+            v[4 * q + 1] = u.y;
+            v[4 * q + 2] = u.z;
+            v[4 * q + 3] = u.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j) v[j] = b0 + j < m ? c[b0 + j] : 0u;
     }
+#pragma unroll
+    for (int j = 0; j < SCAN_ITEMS; ++j) t += v[j];
     unsigned total;
     unsigned run = sums[blockIdx.x] + block_exclusive_sum<unsigned>(t, &total);
 #pragma unroll
     for (int j = 0; j < SCAN_ITEMS; ++j) {
-        if (b0 + j < m) out[b0 + j] = run;
-        run += v[j];
+        const unsigned x = v[j];
+        v[j] = run;
+        run += x;
+    }
+    if (whole) {
+#pragma unroll
+        for (int q = 0; q < SCAN_ITEMS / 4; ++q)
+            *reinterpret_cast<uint4 *>(out + b0 + 4 * q) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < SCAN_ITEMS; ++j)
+            if (b0 + j < m) out[b0 + j] = v[j];
     }
 }
 
@@ -191,39 +264,60 @@ void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, uns
     const int chunks = static_cast<int>(scan_counts_sum_words(m));
     rs_scan_sums<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums);
     rs_scan_top<<<1, 1024, 0, ctx->stream>>>(sums, chunks);
-    rs_scan_apply<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
+    if (((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(out)) & 15) == 0)
+        rs_scan_apply<true><<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
+    else
+        rs_scan_apply<false><<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
 }
 
+// Where a pass reads and writes. W (template): keys of W bytes with the row numbers as payloads
+// (the first pass of a sort), or 0: images and payloads. OUT (template): images and payloads, the
+// payloads alone as i64 rows (the last pass of an argsort), or each array's rows to its own output
+// (the last pass of a batched argsort, whose images hold the array's number above `index_shift`).
+enum RsOut { OUT_PAIRS = 0, OUT_ROWS = 1, OUT_BATCH = 2 };
+template <class IMG, class PAY> struct RsArgs {
+    KeySource k;
+    const IMG *img_in;
+    const PAY *pay_in;
+    IMG *img_out;
+    PAY *pay_out;
+    long long *out;
+    BatchOut batch;
+};
+
 // Down: one pass over digit `shift` with the tile's first output row per digit in
-// offsets[d * tiles + tile]. FIRST reads the i64 keys (positions are the row numbers); LAST
-// writes only the positions, as i64. IMG is the key image carried between passes: 64 bits, or
-// its low 32 bits when every active digit lies there.
+// offsets[d * tiles + tile]. Bound by issue and by its shared-memory wavefronts: 40 M rows of 32-bit
+// images take about 170 us (190 with two table lookups a row and three blocks an SM) against 95 us
+// for the 640 MB moved.
+struct __align__(16) RsShared {
+    // Per warp and digit: the warp's rows of the digit so far; after the ranking, the first row of
+    // the warp's rows of the digit in the sorted tile.
+    unsigned short w[RS_WARPS][RADIX];
+    unsigned excl[RADIX];  // the output row of sorted-tile row l is excl[d] + l
+};
+
 // The body of a down tile; WHOLE when every row of the tile is below n (all but the last
 // tile), which drops the per-row bounds checks.
-template <int RS_ITEMS, bool FIRST, bool LAST, class IMG, bool WHOLE>
-__device__ __forceinline__ void rs_down_tile(const long long *__restrict__ keys_in, const IMG *__restrict__ img_in,
-                                             const unsigned *__restrict__ pos_in, IMG *__restrict__ img_out,
-                                             unsigned *__restrict__ pos_out, long long *__restrict__ out, int64_t n,
-                                             int shift, int tile, unsigned short (*s_wcnt)[RADIX],
-                                             unsigned *s_tile_excl, unsigned *s_dstart, unsigned char *smem) {
-    constexpr int RS_TILE = RsShape<RS_ITEMS>::TILE;
+template <int RS_ITEMS, int W, int OUT, class IMG, class PAY, bool WHOLE>
+__device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, int64_t n, int shift, int tile, RsShared &sm,
+                                             unsigned char *smem) {
+    constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // Rows of this warp: warp-striped, row = base + j*32 + lane, so (j, lane) is row order.
     const int64_t base = static_cast<int64_t>(tile) * RS_TILE + static_cast<int64_t>(w) * (32 * RS_ITEMS);
     IMG img[RS_ITEMS];
-    unsigned pos[RS_ITEMS];
+    PAY pay[W ? 1 : RS_ITEMS];
     unsigned rank2[RS_ITEMS / 2];  // two 16-bit ranks per word
     const unsigned lt = (1u << lane) - 1;
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j) {
         const int64_t r = base + j * 32 + lane;
         const bool in = WHOLE || r < n;
-        if (FIRST) {
-            img[j] = in ? static_cast<IMG>(image_of(__ldcs(keys_in + r))) : static_cast<IMG>(~0ull);
-            pos[j] = 0u;  // the row number, recomputed when stored
+        if constexpr (W != 0) {
+            img[j] = in ? static_cast<IMG>(key_image<W>(a.k, r)) : IMG(0);
         } else {
-            img[j] = in ? __ldcs(img_in + r) : static_cast<IMG>(~0ull);
-            pos[j] = in ? __ldcs(pos_in + r) : 0u;
+            img[j] = in ? __ldcs(a.img_in + r) : IMG(0);
+            pay[j] = in ? __ldcs(a.pay_in + r) : PAY(0);
         }
     }
 #pragma unroll
@@ -232,56 +326,62 @@ __device__ __forceinline__ void rs_down_tile(const long long *__restrict__ keys_
         const unsigned d = static_cast<unsigned>(img[j] >> shift) & 0xffu;
         // Rank among this warp's earlier rows with the same digit.
         const unsigned peers = digit_peers(d, WHOLE ? FULL : __ballot_sync(FULL, in));
-        const unsigned short before = s_wcnt[w][d];
+        const unsigned before = sm.w[w][d];
         __syncwarp();
         if (in) {
             const unsigned rk = before + __popc(peers & lt);
             rank2[j / 2] = (j & 1) ? (rank2[j / 2] | (rk << 16)) : rk;
-            if ((peers & lt) == 0) s_wcnt[w][d] = static_cast<unsigned short>(before + __popc(peers));
+            if ((peers & lt) == 0) sm.w[w][d] = static_cast<unsigned short>(before + __popc(peers));
         }
         __syncwarp();
     }
     __syncthreads();
-    // Per digit: exclusive offsets of the warps within the digit, and the digit's first row in
-    // the tile sorted by digit.
+    // Per digit: the digit's first row in the tile sorted by digit, and each warp's within it.
     {
         const int d = threadIdx.x;
-        unsigned total = 0;
+        unsigned c[RS_WARPS], total = 0;
 #pragma unroll
         for (int ww = 0; ww < RS_WARPS; ++ww) {
-            const unsigned c = s_wcnt[ww][d];
-            s_wcnt[ww][d] = static_cast<unsigned short>(total);
-            total += c;
+            c[ww] = sm.w[ww][d];
+            total += c[ww];
         }
         unsigned tile_total;
-        const unsigned start = block_exclusive_sum<unsigned>(total, &tile_total);
-        s_dstart[d] = start;
-        s_tile_excl[d] -= start;  // from here: the output row of sorted-tile row l is s_tile_excl[d] + l
+        unsigned start = block_exclusive_sum<unsigned>(total, &tile_total);
+        sm.excl[d] -= start;
+#pragma unroll
+        for (int ww = 0; ww < RS_WARPS; ++ww) {
+            sm.w[ww][d] = static_cast<unsigned short>(start);
+            start += c[ww];
+        }
     }
     __syncthreads();
     // The tile sorted by digit (stable) in shared memory, then written out with consecutive
     // threads on consecutive rows of each digit's run, so the stores coalesce.
-    IMG *s_img = reinterpret_cast<IMG *>(smem);
-    unsigned *s_pos = reinterpret_cast<unsigned *>(smem + sizeof(IMG) * RS_TILE);
+    PAY *s_pay = reinterpret_cast<PAY *>(smem);
+    IMG *s_img = reinterpret_cast<IMG *>(smem + sizeof(PAY) * RS_TILE);
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j) {
         if (WHOLE || base + j * 32 + lane < n) {
-            const unsigned d = static_cast<unsigned>(img[j] >> shift) & 0xffu;
-            const unsigned l = s_dstart[d] + s_wcnt[w][d] + ((rank2[j / 2] >> (16 * (j & 1))) & 0xffffu);
+            const unsigned l = sm.w[w][static_cast<unsigned>(img[j] >> shift) & 0xffu] +
+                               ((rank2[j / 2] >> (16 * (j & 1))) & 0xffffu);
             s_img[l] = img[j];
-            s_pos[l] = FIRST ? static_cast<unsigned>(base + j * 32 + lane) : pos[j];
+            if constexpr (W != 0) s_pay[l] = static_cast<PAY>(base + j * 32 + lane);
+            else s_pay[l] = pay[j];
         }
     }
     __syncthreads();
     auto put = [&](int l) {
         const IMG im = s_img[l];
-        const unsigned d = static_cast<unsigned>(im >> shift) & 0xffu;
-        const unsigned dst = s_tile_excl[d] + static_cast<unsigned>(l);
-        if (LAST) {
-            out[dst] = static_cast<long long>(s_pos[l]);
+        const unsigned dst = sm.excl[static_cast<unsigned>(im >> shift) & 0xffu] + static_cast<unsigned>(l);
+        if constexpr (OUT == OUT_ROWS) {
+            a.out[dst] = static_cast<long long>(s_pay[l]);
+        } else if constexpr (OUT == OUT_BATCH) {
+            const unsigned i = static_cast<unsigned>(im >> a.batch.index_shift);
+            const int64_t first = __ldg(a.batch.bases + i);
+            reinterpret_cast<long long *>(__ldg(a.batch.outs + i))[dst - first] = static_cast<long long>(s_pay[l]) - first;
         } else {
-            img_out[dst] = im;
-            pos_out[dst] = s_pos[l];
+            a.img_out[dst] = im;
+            a.pay_out[dst] = s_pay[l];
         }
     };
     if (WHOLE) {
@@ -293,64 +393,134 @@ __device__ __forceinline__ void rs_down_tile(const long long *__restrict__ keys_
     }
 }
 
-template <int RS_ITEMS, bool FIRST, bool LAST, class IMG>
-__global__ void __launch_bounds__(RS_THREADS, RsShape<RS_ITEMS>::MIN_BLOCKS) rs_down_kernel(
-    const long long *__restrict__ keys_in, const IMG *__restrict__ img_in,
-    const unsigned *__restrict__ pos_in, IMG *__restrict__ img_out,
-    unsigned *__restrict__ pos_out, long long *__restrict__ out, int64_t n, int shift, int tiles,
-    const unsigned *__restrict__ offsets) {
-    constexpr int RS_TILE = RsShape<RS_ITEMS>::TILE;
-    __shared__ unsigned short s_wcnt[RS_WARPS][RADIX];  // per-warp digit counts, then offsets
-    __shared__ unsigned s_tile_excl[RADIX];             // the digit's first output row
-    __shared__ unsigned s_dstart[RADIX];                // the digit's first row in the sorted tile
+template <int RS_ITEMS, int W, int OUT, class IMG, class PAY>
+__global__ void __launch_bounds__(RS_THREADS, (RsShape<RS_ITEMS, sizeof(IMG) + sizeof(PAY)>::MIN_BLOCKS))
+    rs_down_kernel(RsArgs<IMG, PAY> a, int64_t n, int shift, int tiles, const unsigned *__restrict__ offsets) {
+    __shared__ RsShared sm;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     const int tile = blockIdx.x;
-    for (int i = threadIdx.x; i < RS_WARPS * RADIX; i += RS_THREADS) (&s_wcnt[0][0])[i] = 0;
-    s_tile_excl[threadIdx.x] = offsets[static_cast<int64_t>(threadIdx.x) * tiles + tile];  // RS_THREADS == RADIX
+    for (int i = threadIdx.x; i < RS_WARPS * RADIX / 2; i += RS_THREADS) reinterpret_cast<unsigned *>(&sm.w[0][0])[i] = 0u;
+    sm.excl[threadIdx.x] = offsets[static_cast<int64_t>(threadIdx.x) * tiles + tile];  // RS_THREADS == RADIX
     __syncthreads();
-    if (static_cast<int64_t>(tile + 1) * RS_TILE <= n)
-        rs_down_tile<RS_ITEMS, FIRST, LAST, IMG, true>(keys_in, img_in, pos_in, img_out, pos_out, out, n, shift, tile,
-                                                       s_wcnt, s_tile_excl, s_dstart, rs_smem);
+    if (static_cast<int64_t>(tile + 1) * (RS_THREADS * RS_ITEMS) <= n)
+        rs_down_tile<RS_ITEMS, W, OUT, IMG, PAY, true>(a, n, shift, tile, sm, rs_smem);
     else
-        rs_down_tile<RS_ITEMS, FIRST, LAST, IMG, false>(keys_in, img_in, pos_in, img_out, pos_out, out, n, shift, tile,
-                                                        s_wcnt, s_tile_excl, s_dstart, rs_smem);
+        rs_down_tile<RS_ITEMS, W, OUT, IMG, PAY, false>(a, n, shift, tile, sm, rs_smem);
 }
 
-// Launches of one pass's kernels for the tuned shape.
-template <bool FIRST, class IMG>
-static void launch_up(vkc_ctx *ctx, int items, int tiles, const long long *keys, const IMG *img, int64_t n, int shift,
-                      unsigned *counts) {
-    switch (items) {
-    case 8: rs_up_kernel<8, FIRST, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(keys, img, n, shift, tiles, counts); break;
-    case 16: rs_up_kernel<16, FIRST, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(keys, img, n, shift, tiles, counts); break;
-    default: rs_up_kernel<12, FIRST, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(keys, img, n, shift, tiles, counts); break;
-    }
-}
-
-template <int ITEMS, bool FIRST, bool LAST, class IMG> static void set_down_smem() {
-    cudaFuncSetAttribute(rs_down_kernel<ITEMS, FIRST, LAST, IMG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         static_cast<int>(RsShape<ITEMS>::DOWN_SMEM));
-}
-
-template <bool FIRST, bool LAST, class IMG>
-static void launch_down(vkc_ctx *ctx, int items, int tiles, const long long *keys, const IMG *img_in,
-                        const unsigned *pos_in, IMG *img_out, unsigned *pos_out, long long *out, int64_t n, int shift,
-                        const unsigned *offs) {
+// One pass in the tuned shape: up, the scan, down.
+template <int ITEMS, int W, int OUT, class IMG, class PAY>
+static void radix_pass_shape(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t) {
+    using S = RsShape<ITEMS, sizeof(IMG) + sizeof(PAY)>;
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {
-        set_down_smem<8, FIRST, LAST, IMG>();
-        set_down_smem<12, FIRST, LAST, IMG>();
-        set_down_smem<16, FIRST, LAST, IMG>();
+        cudaFuncSetAttribute(rs_down_kernel<ITEMS, W, OUT, IMG, PAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(S::DOWN_SMEM));
     });
-#define RS_DOWN(I)                                                                                             \
-    rs_down_kernel<I, FIRST, LAST, IMG><<<tiles, RS_THREADS, (sizeof(IMG) + sizeof(unsigned)) * RsShape<I>::TILE, \
-                                          ctx->stream>>>(keys, img_in, pos_in, img_out, pos_out, out, n, shift, tiles, offs)
-    switch (items) {
-    case 8: RS_DOWN(8); break;
-    case 16: RS_DOWN(16); break;
-    default: RS_DOWN(12); break;
+    const int tiles = static_cast<int>((n + S::TILE - 1) / S::TILE);
+    rs_up_kernel<ITEMS, W, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(a.k, a.img_in, n, shift, tiles, t.counts);
+    scan_counts(ctx, t.counts, static_cast<int64_t>(RADIX) * tiles, t.sums, t.offs);
+    rs_down_kernel<ITEMS, W, OUT, IMG, PAY><<<tiles, RS_THREADS, S::DOWN_SMEM, ctx->stream>>>(a, n, shift, tiles, t.offs);
+}
+template <int W, int OUT, class IMG, class PAY>
+static vkc_status radix_pass(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t) {
+    switch (tune(ctx, TK_RADIX_ITEMS, n)) {
+    case 8: radix_pass_shape<8, W, OUT, IMG, PAY>(ctx, a, n, shift, t); break;
+    case 16: radix_pass_shape<16, W, OUT, IMG, PAY>(ctx, a, n, shift, t); break;
+    default: radix_pass_shape<12, W, OUT, IMG, PAY>(ctx, a, n, shift, t); break;
     }
-#undef RS_DOWN
+    return launched(ctx, "radix_pass");
+}
+
+// Words of the passes' tables for n rows: counts and offs each, and sums (for the smallest tile, so
+// any tuned shape fits).
+void radix_table_words(int64_t n, int64_t *count_words, int64_t *sum_words) {
+    const int64_t tiles = (n + RS_MIN_TILE - 1) / RS_MIN_TILE;
+    *count_words = static_cast<int64_t>(RADIX) * tiles;
+    *sum_words = scan_counts_sum_words(*count_words);
+}
+
+template <class IMG, class PAY>
+vkc_status radix_pairs(vkc_ctx *ctx, const RadixPairs<IMG, PAY> &p, int64_t n, const int *shifts, int passes,
+                       const RadixTables &t, int *which) {
+    int cur = 0;
+    for (int i = 0; i < passes; ++i) {
+        RsArgs<IMG, PAY> a{};
+        a.img_in = i ? p.img[cur] : p.img_first;
+        a.pay_in = i ? p.pay[cur] : p.pay_first;
+        const int to = i ? 1 - cur : 0;
+        a.img_out = p.img[to];
+        a.pay_out = p.pay[to];
+        const vkc_status st = radix_pass<0, OUT_PAIRS>(ctx, a, n, shifts[i], t);
+        if (st) return st;
+        cur = to;
+    }
+    *which = cur;
+    return VKC_OK;
+}
+template vkc_status radix_pairs(vkc_ctx *, const RadixPairs<unsigned, unsigned long long> &, int64_t, const int *, int,
+                                const RadixTables &, int *);
+
+// The passes of an argsort: images from keys of W bytes, row numbers as payloads; the last pass
+// writes OUT. img and pos hold two buffers of n rows each (the second is read only by three passes
+// or more, the first only by two or more).
+template <int W, int OUT, class IMG>
+static vkc_status radix_argsort(vkc_ctx *ctx, const KeySource &k, IMG *const img[2], unsigned *const pos[2], long long *out,
+                                const BatchOut &batch, int64_t n, const int *shifts, int passes, const RadixTables &t) {
+    vkc_status st;
+    int cur = 0;
+    for (int i = 0; i < passes; ++i) {
+        RsArgs<IMG, unsigned> a{};
+        a.k = k;
+        a.out = out;
+        a.batch = batch;
+        a.img_in = img[cur];
+        a.pay_in = pos[cur];
+        const int to = i ? 1 - cur : 0;
+        a.img_out = img[to];
+        a.pay_out = pos[to];
+        const bool last = i == passes - 1;
+        if (i == 0) st = last ? radix_pass<W, OUT>(ctx, a, n, shifts[i], t) : radix_pass<W, OUT_PAIRS>(ctx, a, n, shifts[i], t);
+        else st = last ? radix_pass<0, OUT>(ctx, a, n, shifts[i], t) : radix_pass<0, OUT_PAIRS>(ctx, a, n, shifts[i], t);
+        if (st) return st;
+        cur = to;
+    }
+    return VKC_OK;
+}
+
+vkc_status radix_batch(vkc_ctx *ctx, bool wide, const void *images, void *const img[2], unsigned *const pos[2],
+                       const BatchOut &batch, int64_t n, const int *shifts, int passes, const RadixTables &t) {
+    const KeySource k{images, 0ull, 0ull};
+    if (wide) {
+        unsigned long long *b[2] = {static_cast<unsigned long long *>(img[0]), static_cast<unsigned long long *>(img[1])};
+        return radix_argsort<8, OUT_BATCH, unsigned long long>(ctx, k, b, pos, nullptr, batch, n, shifts, passes, t);
+    }
+    unsigned *b[2] = {static_cast<unsigned *>(img[0]), static_cast<unsigned *>(img[1])};
+    return radix_argsort<4, OUT_BATCH, unsigned>(ctx, k, b, pos, nullptr, batch, n, shifts, passes, t);
+}
+
+// The two halves of a batched argsort whose key digits and array number do not fit one image: the
+// stable order by the 64-bit key images, then by the array numbers (images_n, payloads pay_n).
+vkc_status radix_batch_keys(vkc_ctx *ctx, const void *images, void *const img[2], unsigned *const pos[2], int64_t n,
+                            const int *shifts, int passes, const RadixTables &t) {
+    unsigned long long *b[2] = {static_cast<unsigned long long *>(img[0]), static_cast<unsigned long long *>(img[1])};
+    return radix_argsort<8, OUT_PAIRS, unsigned long long>(ctx, KeySource{images, 0ull, 0ull}, b, pos, nullptr, BatchOut{}, n,
+                                                           shifts, passes, t);
+}
+vkc_status radix_batch_numbers(vkc_ctx *ctx, const unsigned *numbers, const unsigned *pay, unsigned *img_tmp,
+                               unsigned *pay_tmp, const BatchOut &batch, int64_t n, int passes, const RadixTables &t) {
+    RsArgs<unsigned, unsigned> a{};
+    a.batch = batch;
+    a.img_in = numbers;
+    a.pay_in = pay;
+    a.img_out = img_tmp;
+    a.pay_out = pay_tmp;
+    if (passes == 1) return radix_pass<0, OUT_BATCH>(ctx, a, n, 0, t);
+    vkc_status st = radix_pass<0, OUT_PAIRS>(ctx, a, n, 0, t);
+    if (st) return st;
+    a.img_in = img_tmp;
+    a.pay_in = pay_tmp;
+    return radix_pass<0, OUT_BATCH>(ctx, a, n, 8, t);
 }
 
 __global__ void rs_iota_kernel(long long *out, int64_t n) {
@@ -364,14 +534,14 @@ __global__ void rs_iota_kernel(long long *out, int64_t n) {
 // image, position >= n) sort after every row.
 constexpr int SMALL_SORT = 2048;
 
-__global__ void __launch_bounds__(1024) small_argsort_kernel(const long long *__restrict__ keys, int n,
-                                                              long long *__restrict__ out) {
+template <int W>
+__global__ void __launch_bounds__(1024) small_argsort_kernel(KeySource key, int n, long long *__restrict__ out) {
     __shared__ unsigned long long s_img[SMALL_SORT];
     __shared__ unsigned s_pos[SMALL_SORT];
     int p = 1;
     while (p < n) p <<= 1;
     for (int i = threadIdx.x; i < p; i += blockDim.x) {
-        s_img[i] = i < n ? image_of(keys[i]) : ~0ull;
+        s_img[i] = i < n ? key_image<W>(key, i) : ~0ull;
         s_pos[i] = static_cast<unsigned>(i);
     }
     __syncthreads();
@@ -412,14 +582,14 @@ struct MidSmem {
     unsigned long long all_and[MID_WARPS], all_or[MID_WARPS];
 };
 
-__global__ void __launch_bounds__(MID_THREADS) mid_argsort_kernel(const long long *__restrict__ keys, int n,
-                                                                   long long *__restrict__ out) {
+template <int W>
+__global__ void __launch_bounds__(MID_THREADS) mid_argsort_kernel(KeySource key, int n, long long *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char mid_smem[];
     MidSmem &sm = *reinterpret_cast<MidSmem *>(mid_smem);
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
     unsigned long long a = ~0ull, o = 0;
     for (int i = t; i < n; i += MID_THREADS) {
-        const unsigned long long im = image_of(keys[i]);
+        const unsigned long long im = key_image<W>(key, i);
         sm.img[0][i] = im;
         sm.pos[0][i] = static_cast<unsigned short>(i);
         a &= im;
@@ -523,44 +693,12 @@ __global__ void __launch_bounds__(MID_THREADS) mid_argsort_kernel(const long lon
     for (int i = t; i < n; i += MID_THREADS) out[i] = static_cast<long long>(sm.pos[cur][i]);
 }
 
-// The active-digit passes of argsort over (image, position) ping-pong buffers of image type IMG.
-template <class IMG>
-static vkc_status radix_argsort_passes(vkc_ctx *ctx, int items, int tiles, int64_t m, int chunks, const long long *keys,
-                                       void *const img_v[2], unsigned *const pos[2], unsigned *counts, unsigned *offs,
-                                       unsigned *sums, long long *oo, int64_t n, const int *active, int passes) {
-    IMG *img[2] = {static_cast<IMG *>(img_v[0]), static_cast<IMG *>(img_v[1])};
-    int cur = 0;
-    for (int a = 0; a < passes; ++a) {
-        const bool fst = a == 0, lst = a == passes - 1;
-        const int shift = 8 * active[a];
-        const int src = cur, dst = passes > 2 ? 1 - cur : 0;
-        if (fst) launch_up<true, IMG>(ctx, items, tiles, keys, nullptr, n, shift, counts);
-        else launch_up<false, IMG>(ctx, items, tiles, nullptr, img[src], n, shift, counts);
-        rs_scan_sums<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(counts, m, sums);
-        rs_scan_top<<<1, 1024, 0, ctx->stream>>>(sums, chunks);
-        rs_scan_apply<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(counts, m, sums, offs);
-        if (fst && lst)
-            launch_down<true, true, IMG>(ctx, items, tiles, keys, nullptr, nullptr, nullptr, nullptr, oo, n, shift, offs);
-        else if (fst)
-            launch_down<true, false, IMG>(ctx, items, tiles, keys, nullptr, nullptr, img[0], pos[0], nullptr, n, shift, offs);
-        else if (lst)
-            launch_down<false, true, IMG>(ctx, items, tiles, nullptr, img[src], pos[src], nullptr, nullptr, oo, n, shift, offs);
-        else
-            launch_down<false, false, IMG>(ctx, items, tiles, nullptr, img[src], pos[src], img[dst], pos[dst], nullptr, n,
-                                           shift, offs);
-        vkc_status st = launched(ctx, "rs_pass");
-        if (st) return st;
-        if (fst) cur = 0;
-        else if (!lst) cur = dst;
-    }
-    return VKC_OK;
-}
-
 // index.rs:159-173 (ArgSort::run).
-static vkc_status argsort_i64(vkc_ctx *ctx, const vkc_value *args, int nargs, vkc_value *out) {
+template <vkc_type T> static vkc_status argsort(vkc_ctx *ctx, const vkc_value *args, int nargs, vkc_value *out) {
+    constexpr int W = T == VKC_I64 || T == VKC_U64 ? 8 : (T == VKC_I32 ? 4 : 1);
     vkc_status st;
     if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));
-    if (!array_arg(ctx, args[0], VKC_I64, &st)) return st;
+    if (!array_arg(ctx, args[0], T, &st)) return st;
     const vkc_array *xs = args[0].array;
     int64_t n = xs->len;
     if (n >= (int64_t(1) << 32))
@@ -571,157 +709,103 @@ static vkc_status argsort_i64(vkc_ctx *ctx, const vkc_value *args, int nargs, vk
         vkc_array_release(o);
         return s;
     };
-    if (n == 0) {
+    auto finish = [&]() {
         out->kind = VKC_VALUE_ARRAY;
         out->array = o;
         return VKC_OK;
-    }
-    const auto *keys = static_cast<const long long *>(xs->data());
+    };
+    if (n == 0) return finish();
+    KeySource key{xs->data(), T == VKC_I64 ? 1ull << 63 : (T == VKC_I32 ? 1ull << 31 : 0ull), 0ull};
+    auto *oo = static_cast<long long *>(o->data());
     if (n <= SMALL_SORT) {
-        small_argsort_kernel<<<1, 1024, 0, ctx->stream>>>(keys, static_cast<int>(n), static_cast<long long *>(o->data()));
+        small_argsort_kernel<W><<<1, 1024, 0, ctx->stream>>>(key, static_cast<int>(n), oo);
         if ((st = launched(ctx, "small_argsort"))) return release(st);
-        out->kind = VKC_VALUE_ARRAY;
-        out->array = o;
-        return VKC_OK;
+        return finish();
     }
     if (n <= MID_SORT) {
         static std::atomic<unsigned long long> configured{0};
         once_per_device(configured, ctx->device, [] {
-            cudaFuncSetAttribute(mid_argsort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(mid_argsort_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(sizeof(MidSmem)));
         });
-        mid_argsort_kernel<<<1, MID_THREADS, sizeof(MidSmem), ctx->stream>>>(keys, static_cast<int>(n),
-                                                                              static_cast<long long *>(o->data()));
+        mid_argsort_kernel<W><<<1, MID_THREADS, sizeof(MidSmem), ctx->stream>>>(key, static_cast<int>(n), oo);
         if ((st = launched(ctx, "mid_argsort"))) return release(st);
-        out->kind = VKC_VALUE_ARRAY;
-        out->array = o;
-        return VKC_OK;
+        return finish();
     }
-    // Histogram of every digit.
-    void *p;
-    if ((st = scratch(ctx, 8 * RADIX * sizeof(unsigned), &p))) return release(st);
-    auto *hist = static_cast<unsigned *>(p);
-    VKC_CUDA(ctx, cudaMemsetAsync(hist, 0, 8 * RADIX * sizeof(unsigned), ctx->stream));
-    rs_hist_kernel<<<stream_grid(ctx, n, 256, 6, 16384), 256, 0, ctx->stream>>>(keys, n, hist);
-    if ((st = launched(ctx, "rs_hist"))) return release(st);
-    void *h;
-    if ((st = pinned(ctx, 2 * 8 * RADIX * sizeof(unsigned) + 16, &h))) return release(st);
-    auto *hh = static_cast<unsigned *>(h);
-    auto *first = reinterpret_cast<long long *>(hh + 2 * 8 * RADIX);
-    VKC_CUDA(ctx, cudaMemcpyAsync(hh, hist, 8 * RADIX * sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    VKC_CUDA(ctx, cudaMemcpyAsync(first, keys, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    // The images' range and varying bits.
+    void *p, *h;
+    if ((st = scratch(ctx, 4 * sizeof(unsigned long long), &p))) return release(st);
+    auto *range = static_cast<unsigned long long *>(p);
+    VKC_CUDA(ctx, cudaMemsetAsync(range, 0xff, 16, ctx->stream));
+    VKC_CUDA(ctx, cudaMemsetAsync(range + 2, 0, 16, ctx->stream));
+    rs_range_kernel<W><<<stream_grid(ctx, n, 256, 6, 16384), 256, 0, ctx->stream>>>(key, n, range);
+    if ((st = launched(ctx, "rs_range"))) return release(st);
+    if ((st = pinned(ctx, 32, &h))) return release(st);
+    VKC_CUDA(ctx, cudaMemcpyAsync(h, range, 32, cudaMemcpyDeviceToHost, ctx->stream));
     VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    // Active digits (radix.rs:203-211): a digit whose bucket of the first row holds every row.
-    unsigned long long first_img = static_cast<unsigned long long>(*first) ^ 0x8000000000000000ull;
-    int active[8], passes = 0;
-    for (int pss = 0; pss < 8; ++pss) {
-        unsigned fd = static_cast<unsigned>(first_img >> (8 * pss)) & 0xffu;
-        if (hh[pss * RADIX + fd] != static_cast<unsigned>(n)) active[passes++] = pss;
+    const auto *r = static_cast<const unsigned long long *>(h);
+    const unsigned long long varies = r[0] ^ r[2], spread = r[3] - r[1], least = r[1];
+    int shifts[8], passes = 0, wide = 0;
+    for (int b = 0; b < 8; ++b) {
+        if ((varies >> (8 * b)) & 0xffu) shifts[passes++] = 8 * b;
+        if (spread >> (8 * b)) ++wide;
     }
-    auto *oo = static_cast<long long *>(o->data());
+    if (wide < passes || (wide == passes && passes > 0 && spread >> 32 == 0 && shifts[passes - 1] >= 32)) {
+        // Fewer bytes (or as many, in narrower images) in the distance from the least image.
+        key.low = least;
+        passes = wide;
+        for (int b = 0; b < wide; ++b) shifts[b] = 8 * b;
+    }
     if (passes == 0) {
         rs_iota_kernel<<<stream_grid(ctx, n, 256, 8, 2048), 256, 0, ctx->stream>>>(oo, n);
         if ((st = launched(ctx, "rs_iota"))) return release(st);
-        out->kind = VKC_VALUE_ARRAY;
-        out->array = o;
-        return VKC_OK;
+        return finish();
     }
-    // Ping-pong buffers of (image, position), as radix.rs:224-232.
-    vkc_array *ia = nullptr, *ib = nullptr, *pa = nullptr, *pb = nullptr, *ca = nullptr, *oa = nullptr,
-              *sa = nullptr;
+    // Ping-pong buffers of (image, position), as radix.rs:224-232, and the passes' tables. When
+    // every digit lies in the low 32 bits, the passes carry the image's low 32 bits: 16 bytes a
+    // row per pass, not 24.
+    vkc_array *ia = nullptr, *ib = nullptr, *pa = nullptr, *pb = nullptr, *ca = nullptr, *oa = nullptr, *sa = nullptr;
     auto cleanup = [&]() {
         for (vkc_array *a : {ia, ib, pa, pb, ca, oa, sa})
             if (a) vkc_array_release(a);
     };
-    // When every active digit lies in the low 32 bits, rows with equal high halves differ only
-    // there, so the passes carry the image's low 32 bits: 16 bytes a row per pass, not 24.
-    const bool narrow = active[passes - 1] < 4;
+    const bool narrow = W < 8 || shifts[passes - 1] < 32;
     const vkc_type img_type = narrow ? VKC_I32 : VKC_U64;
-    if (passes > 1) {
-        if ((st = new_array(ctx, img_type, n, false, &ia)) || (st = new_array(ctx, VKC_I32, n, false, &pa))) {
-            cleanup();
-            return release(fail(ctx, VKC_ALLOC, "cannot allocate argsort scratch for " + std::to_string(n) + " rows"));
-        }
-        if (passes > 2 && ((st = new_array(ctx, img_type, n, false, &ib)) || (st = new_array(ctx, VKC_I32, n, false, &pb)))) {
-            cleanup();
-            return release(fail(ctx, VKC_ALLOC, "cannot allocate argsort scratch for " + std::to_string(n) + " rows"));
-        }
-    }
-    // Digit-major tile counts, their exclusive scan, and the scan's block sums.
-    const int items = tune(ctx, TK_RADIX_ITEMS, n);
-    const int64_t tile_rows = static_cast<int64_t>(RS_THREADS) * items;
-    const int tiles = static_cast<int>((n + tile_rows - 1) / tile_rows);
-    const int64_t m = static_cast<int64_t>(RADIX) * tiles;
-    const int chunks = static_cast<int>((m + SCAN_CHUNK - 1) / SCAN_CHUNK);
-    if ((st = new_array(ctx, VKC_I32, m, false, &ca)) || (st = new_array(ctx, VKC_I32, m, false, &oa)) ||
-        (st = new_array(ctx, VKC_I32, chunks, false, &sa))) {
+    int64_t cw, sw;
+    radix_table_words(n, &cw, &sw);
+    if ((passes > 1 && (new_array(ctx, img_type, n, false, &ia) || new_array(ctx, VKC_I32, n, false, &pa))) ||
+        (passes > 2 && (new_array(ctx, img_type, n, false, &ib) || new_array(ctx, VKC_I32, n, false, &pb))) ||
+        new_array(ctx, VKC_I32, cw, false, &ca) || new_array(ctx, VKC_I32, cw, false, &oa) ||
+        new_array(ctx, VKC_I32, sw, false, &sa)) {
         cleanup();
         return release(fail(ctx, VKC_ALLOC, "cannot allocate argsort scratch for " + std::to_string(n) + " rows"));
     }
-    auto *counts = static_cast<unsigned *>(ca->data());
-    auto *offs = static_cast<unsigned *>(oa->data());
-    auto *sums = static_cast<unsigned *>(sa->data());
-    void *img[2] = {ia ? ia->data() : nullptr, ib ? ib->data() : nullptr};
-    unsigned *pos[2] = {pa ? static_cast<unsigned *>(pa->data()) : nullptr,
-                        pb ? static_cast<unsigned *>(pb->data()) : nullptr};
-    const vkc_status pst = narrow ? radix_argsort_passes<unsigned>(ctx, items, tiles, m, chunks, keys, img, pos, counts,
-                                                                    offs, sums, oo, n, active, passes)
-                                  : radix_argsort_passes<unsigned long long>(ctx, items, tiles, m, chunks, keys, img, pos,
-                                                                             counts, offs, sums, oo, n, active, passes);
-    if (pst) {
-        cleanup();
-        return release(pst);
+    auto words = [](vkc_array *a) { return a ? static_cast<unsigned *>(a->data()) : nullptr; };
+    const RadixTables t{words(ca), words(oa), words(sa)};
+    unsigned *pos[2] = {words(pa), words(pb)};
+    if (narrow) {
+        unsigned *img[2] = {words(ia), words(ib)};
+        st = radix_argsort<W, OUT_ROWS, unsigned>(ctx, key, img, pos, oo, BatchOut{}, n, shifts, passes, t);
+    } else if constexpr (W == 8) {
+        unsigned long long *img[2] = {ia ? static_cast<unsigned long long *>(ia->data()) : nullptr,
+                                      ib ? static_cast<unsigned long long *>(ib->data()) : nullptr};
+        st = radix_argsort<8, OUT_ROWS, unsigned long long>(ctx, key, img, pos, oo, BatchOut{}, n, shifts, passes, t);
     }
-    DevStatus ds;
-    st = read_status(ctx, &ds);
     cleanup();
-    if (st) return release(st);
-    out->kind = VKC_VALUE_ARRAY;
-    out->array = o;
-    return VKC_OK;
-}
-
-// Stable LSD passes over (image, position) pairs that are already in img[0] / pos[0], one per
-// entry of `shifts`, ping-ponging between the two buffers; *which gets the buffer that holds
-// the result. counts and offs hold radix_pairs_scratch's words and sums
-// ceil(that / SCAN_CHUNK). Enqueue only: no host synchronisation and no allocation.
-vkc_status radix_pairs(vkc_ctx *ctx, unsigned long long *img[2], unsigned *pos[2], int64_t n, const int *shifts,
-                       int npasses, unsigned *counts, unsigned *offs, unsigned *sums, int *which) {
-    vkc_status st;
-    const int items = tune(ctx, TK_RADIX_ITEMS, n);
-    const int64_t tile_rows = static_cast<int64_t>(RS_THREADS) * items;
-    const int tiles = static_cast<int>((n + tile_rows - 1) / tile_rows);
-    const int64_t m = static_cast<int64_t>(RADIX) * tiles;
-    const int chunks = static_cast<int>((m + SCAN_CHUNK - 1) / SCAN_CHUNK);
-    int cur = 0;
-    for (int a = 0; a < npasses; ++a) {
-        const int shift = shifts[a];
-        launch_up<false, unsigned long long>(ctx, items, tiles, nullptr, img[cur], n, shift, counts);
-        rs_scan_sums<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(counts, m, sums);
-        rs_scan_top<<<1, 1024, 0, ctx->stream>>>(sums, chunks);
-        rs_scan_apply<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(counts, m, sums, offs);
-        launch_down<false, false, unsigned long long>(ctx, items, tiles, nullptr, img[cur], pos[cur], img[1 - cur], pos[1 - cur], nullptr, n,
-                                  shift, offs);
-        if ((st = launched(ctx, "radix_pairs"))) return st;
-        cur = 1 - cur;
-    }
-    *which = cur;
-    return VKC_OK;
-}
-
-// Words of the radix_pairs scratch for n rows: counts/offs each, and sums (for the smallest
-// tile, so any tuned shape fits).
-void radix_pairs_scratch(int64_t n, int64_t *count_words, int64_t *sum_words) {
-    const int64_t tiles = (n + RS_MIN_TILE - 1) / RS_MIN_TILE;
-    *count_words = static_cast<int64_t>(RADIX) * tiles;
-    *sum_words = (*count_words + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    return st ? release(st) : finish();
 }
 
 void register_sort(std::vector<KernelDef> &t) {
-    // index.rs:241-255: cost = key width + 8.
-    KernelDef d{"argsort_i64", VKC_WHOLE, {InSpec{IN_ARRAY, VKC_I64}}, true, VKC_I64, 16};
-    d.whole = argsort_i64;
-    t.push_back(d);
+    // index.rs:241-255, :290-325: cost = key width + 8.
+    struct S { vkc_type t; WholeFn f; };
+    const S sorts[] = {{VKC_I64, argsort<VKC_I64>}, {VKC_U64, argsort<VKC_U64>}, {VKC_I32, argsort<VKC_I32>},
+                       {VKC_U8, argsort<VKC_U8>}};
+    for (const S &s : sorts) {
+        KernelDef d{std::string("argsort_") + type_name(s.t), VKC_WHOLE, {InSpec{IN_ARRAY, s.t}}, true, VKC_I64,
+                    static_cast<uint64_t>(type_width(s.t) + 8)};
+        d.whole = s.f;
+        t.push_back(d);
+    }
 }
 
 }  // namespace vkc
