@@ -310,13 +310,14 @@ __global__ void __launch_bounds__(GP_THREADS, 6) gp_restore_kernel(const unsigne
     }
 }
 
-// The partitioned path pays when the source is well beyond L2 (2^26 rows, 512 MiB; at 2^25
-// rows the one-pass gather still hits L2 often enough) and the index rows are at least half
-// the source rows, so that each region line fetched into L2 is read about twice (with fewer,
-// the one-pass gather moves fewer DRAM bytes). Measured on GB300 at n = 2^28 index rows into
-// 2^28 source rows: 68 G rows/s against 45 G. Positions are u32: fewer than 2^32 index rows.
+// The partitioned path pays when the source is beyond L2 (7 * 2^22 rows, 224 MiB; smaller ones hit
+// L2 often enough) and the index rows are at least half the source rows, so that each region line
+// fetched into L2 is read about twice (with fewer, the one-pass gather moves fewer DRAM bytes).
+// Measured on GB300 with as many index rows as source rows, one pass against four: 20 M rows 260
+// against 312 us, 28 M 421 / 410, 40 M 667 / 545, 2^28 45 against 68 G rows/s. Positions are u32:
+// fewer than 2^32 index rows.
 static bool gather_partitions(uint64_t nsrc, int64_t n) {
-    return nsrc >= (uint64_t(1) << 26) && nsrc <= (uint64_t(1) << 38) && n >= (int64_t(1) << 22) &&
+    return nsrc >= (uint64_t(7) << 22) && nsrc <= (uint64_t(1) << 38) && n >= (int64_t(1) << 22) &&
            2 * static_cast<uint64_t>(n) >= nsrc && n < (int64_t(1) << 32);
 }
 
