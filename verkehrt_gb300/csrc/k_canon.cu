@@ -44,6 +44,7 @@
 #include <climits>
 #include <cmath>
 
+#include "add_bits.cuh"
 #include "lookback.cuh"
 #include "radix.h"
 #include "reduce_common.h"
@@ -55,8 +56,6 @@ constexpr int CT_THREADS = 256;
 constexpr int CT_SEGS = 32;       // segments per tile
 constexpr int CT_SEG_BLOCKS = 8;  // 16-row blocks per segment
 constexpr int CT_BLOCKS = CT_SEGS * CT_SEG_BLOCKS;  // 256 blocks = 4096 rows per tile
-constexpr unsigned long long MANT = 0xfffffffffffffull;
-constexpr unsigned long long ONE52 = 1ull << 52;
 constexpr unsigned long long SAT = 1ull << 60;
 constexpr int NO_E = INT_MIN;
 
@@ -68,9 +67,6 @@ struct RowArgs {
     CmpRange r;
     unsigned long long e;
 };
-
-__device__ __forceinline__ double as_f64(unsigned long long b) { return __longlong_as_double(static_cast<long long>(b)); }
-__device__ __forceinline__ unsigned long long as_bits(double d) { return static_cast<unsigned long long>(__double_as_longlong(d)); }
 
 // The row value fed to the lane (fused.rs:77-98, :112-127, :190-203). Products are single
 // IEEE multiplies (no FMA contraction: the file is built with -fmad=false).
@@ -1517,27 +1513,6 @@ struct ScanSmem {
     double c[CT_BLOCKS + 1];  // the combines of st[j]
     int serial[16];           // lanes whose segments do not all carry a transfer function
 };
-
-// fl(s + x) on bits. When s is a positive normal in binade E >= -959, x is non-negative and below
-// that binade and the sum stays in it, s = S u with u = 2^(E-52) and fl(s + x) = (S + RNE(x/u)) u
-// with ties to the even S (the integer steps of seg_tf for one row); otherwise the FP64 add.
-__device__ __forceinline__ unsigned long long add_bits(unsigned long long s, unsigned long long x) {
-    const unsigned KE = static_cast<unsigned>(s >> 52);  // with the sign bit: a negative s is above 2047
-    const unsigned ex = static_cast<unsigned>(x >> 52);  // likewise a negative x
-    if (KE >= 64u && KE <= 2046u && ex < KE) {
-        const unsigned k = min(KE - ex, 63u);  // zero and subnormal rows: k = 63, no increment
-        const unsigned long long w = ((x & MANT) | ONE52) + (1ull << (k - 1));
-        unsigned long long inc = w >> k;
-        const unsigned long long S = (s & MANT) | ONE52;
-        if ((w << (64 - k)) == 0) {  // exactly halfway: to the even neighbour
-            inc -= 1;
-            inc += (S + inc) & 1;
-        }
-        const unsigned long long S2 = S + inc;
-        if (S2 < (ONE52 << 1)) return (static_cast<unsigned long long>(KE) << 52) | (S2 & MANT);
-    }
-    return as_bits(__dadd_rn(as_f64(s), as_f64(x)));
-}
 
 // One block per tile. (1) Each (segment, lane pair) thread computes its segments' transfer
 // functions at the binade of the lane's state before the tile (K3's layout: 8 lane pairs x 32

@@ -9,26 +9,40 @@
 //
 // Equivalently, out[k] is the canonical sum of the rows with every row of another bucket read as
 // +0.0: a stripe starts at +0.0 and never holds -0.0 (a sum is -0.0 only when both terms are), so
-// adding +0.0 leaves it unchanged. Two paths:
-//  * few buckets (at most 16): that identity, per bucket: the masked rows, then reduce_add_f64
-//    (one canonical pass each, about 1 ms per bucket at 2^27 rows);
-//  * otherwise: a stable argsort of the rows below b by (key, stripe), after which each stripe of
-//    each bucket is a contiguous chain that one warp adds in index order (32 rows per load, the
-//    adds in order through shuffles); the chains of a bucket combine pairwise, and one thread
-//    folds the tail rows in order.
+// adding +0.0 leaves it unchanged. Three paths:
+//  * very few buckets of many rows (rif_masks): that identity, per bucket: the masked rows, then
+//    reduce_add_f64;
+//  * otherwise the rows below b are sorted, stably, by (key, stripe), a 32-bit image whose radix
+//    passes carry the values; each stripe of each bucket is then a contiguous chain that one thread
+//    adds in index order, the sixteen of a bucket side by side, so that they combine by shuffles;
+//    one thread folds the tail rows in order. (Until now an argsort, two gathers by its order and a
+//    warp a chain whose 32 lanes all ran the chain: 4.36 ms against 0.72 for 33 M rows in 1024
+//    buckets, 2.26 ms of it FP64 adds that 31 lanes repeated.)
+//  * buckets so many that a table of their chains would dwarf the rows (rif_tables): the chains are
+//    found by a scan over the sorted rows instead.
 // Arguments and errors follow reduce_into_add_i64 (index.rs:194-222): the values' kind first,
 // then the keys (checked_keys, index.rs:116-130), a length mismatch, the result's allocation.
+#include <algorithm>
+
+#include "add_bits.cuh"
+#include "radix.h"
 #include "reduce_common.h"
 
 namespace vkc {
 
-int64_t scan_counts_sum_words(int64_t m);
-void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, unsigned *out);
 vkc_status bucket_key_error(vkc_ctx *ctx, const long long *k, int64_t n, int64_t nb, bool *found);
 
-constexpr int64_t RIF_MASKED_BUCKETS = 16;
-
-__device__ __forceinline__ double rif_f64(unsigned long long b) { return __longlong_as_double(static_cast<long long>(b)); }
+// Measured: the masked path costs about 130 us a bucket and 7.2 us a bucket per million rows; the
+// sorted one 100 us, 16 us per million rows and its chains at 40 ns a row (n / (16 nb) rows each when
+// the buckets are even). Masked where that is less: up to 1 bucket of 2^17 rows, 4 of 2^20, 15 of 2^25.
+static bool rif_masks(int64_t n, int64_t nb) {
+    const double m = static_cast<double>(n) * 1e-6, k = static_cast<double>(nb);
+    return k * (130.0 + 7.2 * m) < 100.0 + 16.0 * m + 2500.0 * m / k;
+}
+// Images (key * 16 + stripe) of 32 bits, and a table of every chain no larger than a few rows' worth.
+static bool rif_tables(int64_t n, int64_t nb) {
+    return n < (int64_t(1) << 32) && nb <= (int64_t(1) << 28) && nb <= n + (int64_t(1) << 16);
+}
 
 // v[i] = x[i] for rows of bucket k, else +0.0.
 __global__ void rif_mask_kernel(const long long *__restrict__ keys, const unsigned long long *__restrict__ x,
@@ -87,7 +101,7 @@ __global__ void __launch_bounds__(256) rif_chain_kernel(const long long *__restr
             for (int u = 0; u < RIF_U; ++u) {
                 const int64_t q = q0 + u * 32 + lane;
                 in[u] = q < b && cs[q] == key;
-                x[u] = q < b ? rif_f64(v[q]) : 0.0;
+                x[u] = q < b ? as_f64(v[q]) : 0.0;
             }
             bool more = true;
 #pragma unroll
@@ -122,7 +136,7 @@ __global__ void rif_combine_kernel(const long long *__restrict__ chain_key,
         double s[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) s[j] = 0.0;
-        for (int64_t o2 = o; o2 < m && (chain_key[o2] >> 4) == k; ++o2) s[chain_key[o2] & 15] = rif_f64(chain_sum[o2]);
+        for (int64_t o2 = o; o2 < m && (chain_key[o2] >> 4) == k; ++o2) s[chain_key[o2] & 15] = as_f64(chain_sum[o2]);
 #pragma unroll
         for (int step = 8; step > 0; step >>= 1)
 #pragma unroll
@@ -133,9 +147,9 @@ __global__ void rif_combine_kernel(const long long *__restrict__ chain_key,
 
 // The rows from b on, fewer than 16, fold into their buckets in index order.
 __global__ void rif_tail_kernel(const long long *__restrict__ keys, const unsigned long long *__restrict__ x,
-                                int64_t b, int64_t n, unsigned long long *__restrict__ out) {
+                                int64_t b, int64_t n, uint64_t nb, unsigned long long *__restrict__ out) {
     for (int64_t i = b; i < n; ++i)
-        out[keys[i]] = static_cast<unsigned long long>(__double_as_longlong(__dadd_rn(rif_f64(out[keys[i]]), rif_f64(x[i]))));
+        if (static_cast<uint64_t>(keys[i]) < nb) out[keys[i]] = static_cast<unsigned long long>(__double_as_longlong(__dadd_rn(as_f64(out[keys[i]]), as_f64(x[i]))));
 }
 
 // A whole entry of the table by name, on array arguments; the result array in *res.
@@ -155,6 +169,185 @@ static vkc_status call_whole(vkc_ctx *ctx, const char *name, std::initializer_li
     *res = st ? nullptr : out.array;
     return st;
 }
+
+// ------------------------------------------------------------------ the sorted path
+
+// Images of the rows below b (a row out of range gets image 0, so that no later kernel leaves its
+// tables: the call fails), and the first key out of range among all n rows.
+__global__ void __launch_bounds__(256) rif_images_kernel(const long long *__restrict__ keys, int64_t n, int64_t b, uint64_t nb,
+                                                         unsigned *__restrict__ img, DevStatus *status) {
+    constexpr int R = 4;
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    unsigned long long bad = ~0ull;
+    for (int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i0 < n; i0 += R * stride) {
+        unsigned long long k[R];
+#pragma unroll
+        for (int j = 0; j < R; ++j) k[j] = i0 + j * stride < n ? static_cast<unsigned long long>(__ldcs(keys + i0 + j * stride)) : 0ull;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int64_t i = i0 + j * stride;
+            if (i >= n) break;
+            const bool ok = k[j] < nb;
+            if (!ok && static_cast<unsigned long long>(i) < bad) bad = static_cast<unsigned long long>(i);
+            if (i < b) img[i] = ok ? static_cast<unsigned>(k[j]) * 16u + static_cast<unsigned>(i & 15) : 0u;
+        }
+    }
+    if (bad != ~0ull) atomicMin(&status->first_bad, bad);
+}
+
+// span[c] = the rows [x, y) of chain c among the sorted images (zeroed: empty chains).
+__global__ void __launch_bounds__(256) rif_spans_kernel(const unsigned *__restrict__ img, int64_t b, uint2 *__restrict__ span) {
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * 4;
+    for (int64_t p = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4; p < b; p += stride) {
+        // b is a multiple of 16, so four images from p on are there.
+        const uint4 q = *reinterpret_cast<const uint4 *>(img + p);
+        const unsigned v[6] = {p ? img[p - 1] : ~q.x, q.x, q.y, q.z, q.w, p + 4 < b ? img[p + 4] : ~q.w};
+#pragma unroll
+        for (int j = 1; j < 5; ++j) {
+            if (v[j] != v[j - 1]) span[v[j]].x = static_cast<unsigned>(p + j - 1);
+            if (v[j] != v[j + 1]) span[v[j]].y = static_cast<unsigned>(p + j);
+        }
+    }
+}
+
+// One block per two buckets: a warp adds, one thread per chain, and a second warp copies the next
+// RC_ROWS rows of each of the 32 chains into shared memory (each a coalesced run, RC_STAGES - 1
+// stages ahead; by the adding warp itself the copies' issue took half as long again as the adds). A
+// row of a chain costs 31 ns, the latency of an FP64 add. (add_bits, the adds as integer steps, took
+// 110 ns: it pays where a chain's neighbours fill the pipe, not here.)
+constexpr int RC_ROWS = 32, RC_STAGES = 3, RC_PITCH = RC_ROWS + 1;
+
+__global__ void __launch_bounds__(64) rif_sum_kernel(const uint2 *__restrict__ span, const unsigned long long *__restrict__ v,
+                                                     int64_t nb, unsigned long long *__restrict__ out) {
+    __shared__ unsigned long long buf[RC_STAGES][32][RC_PITCH];
+    const int lane = threadIdx.x & 31;
+    const bool copies = threadIdx.x >= 32;
+    for (int64_t pair = blockIdx.x; pair * 2 < nb; pair += gridDim.x) {
+        const int64_t c = pair * 32 + lane;
+        const uint2 s = c < nb * 16 ? span[c] : make_uint2(0u, 0u);
+        const unsigned len = s.y - s.x, most = __reduce_max_sync(FULL, len);
+        const int steps = static_cast<int>((static_cast<int64_t>(most) + RC_ROWS - 1) / RC_ROWS);
+        auto issue = [&](int k) {
+            if (k < steps) {
+#pragma unroll 8
+                for (int t = 0; t < 32; ++t) {
+                    const unsigned first = __shfl_sync(FULL, s.x, t), n = __shfl_sync(FULL, len, t);
+                    const unsigned r = static_cast<unsigned>(k) * RC_ROWS + lane;
+                    if (r < n)
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<unsigned>(
+                                         __cvta_generic_to_shared(&buf[k % RC_STAGES][t][lane]))),
+                                     "l"(v + first + r)
+                                     : "memory");
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        if (copies)
+            for (int k = 0; k < RC_STAGES - 1; ++k) issue(k);
+        double acc = 0.0;
+        for (int k = 0; k < steps; ++k) {
+            if (copies) asm volatile("cp.async.wait_group %0;" ::"n"(RC_STAGES - 2) : "memory");
+            __syncthreads();  // step k's rows have landed, and the buffer of step k - 1 is free
+            if (copies) {
+                issue(k + RC_STAGES - 1);
+            } else {
+                const unsigned done = static_cast<unsigned>(k) * RC_ROWS;
+                const int rows = len > done ? static_cast<int>(min(len - done, static_cast<unsigned>(RC_ROWS))) : 0;
+                const unsigned long long *x = buf[k % RC_STAGES][lane];
+                int i = 0;
+                for (; i + 8 <= rows; i += 8) {
+                    double t[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) t[j] = as_f64(x[i + j]);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) acc = __dadd_rn(acc, t[j]);
+                }
+                for (; i < rows; ++i) acc = __dadd_rn(acc, as_f64(x[i]));
+            }
+        }
+        if (copies) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        // +8, +4, +2, +1 over the bucket's sixteen stripes.
+        if (!copies) {
+#pragma unroll
+            for (int step = 8; step > 0; step >>= 1) {
+                const double other = __shfl_down_sync(FULL, acc, step, 16);
+                if ((lane & 15) < step) acc = __dadd_rn(acc, other);
+            }
+            if ((lane & 15) == 0 && c < nb * 16) out[c >> 4] = as_bits(acc);
+        }
+        __syncthreads();  // the buffers are free for the next pair
+    }
+}
+
+// Many buckets of few rows: one thread per chain reads its rows itself, the chains of a warp lying
+// side by side. (The staged form spends about 2 us a block on a pair of buckets however short: 2^20
+// buckets of 2^20 rows took 883 us.)
+constexpr int64_t RIF_SHORT_ROWS = 4;  // average rows of a chain below which this form runs
+__global__ void __launch_bounds__(256) rif_short_kernel(const uint2 *__restrict__ span, const unsigned long long *__restrict__ v,
+                                                        int64_t nb, unsigned long long *__restrict__ out) {
+    const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const uint2 s = c < nb * 16 ? span[c] : make_uint2(0u, 0u);
+    double acc = 0.0;
+    for (unsigned p = s.x; p < s.y; p += 4) {
+        double t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) t[j] = p + j < s.y ? as_f64(v[p + j]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc = __dadd_rn(acc, t[j]);  // +0.0 changes no sum
+    }
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1) {
+        const double other = __shfl_down_sync(FULL, acc, step, 16);
+        if ((threadIdx.x & 15) < step) acc = __dadd_rn(acc, other);
+    }
+    if ((threadIdx.x & 15) == 0 && c < nb * 16) out[c >> 4] = as_bits(acc);
+}
+
+static vkc_status rif_sorted(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t n, int64_t b,
+                             int64_t nb, unsigned long long *out) {
+    int passes = 1;  // of the image's bits: the largest is 16 nb - 1
+    while (passes < 4 && ((16 * static_cast<uint64_t>(nb) - 1) >> (8 * passes))) ++passes;
+    static const int shifts[4] = {0, 8, 16, 24};
+    vkc_array *ia = nullptr, *ib = nullptr, *va = nullptr, *vb = nullptr, *ca = nullptr, *oa = nullptr, *sa = nullptr,
+              *sp = nullptr;
+    auto done = [&](vkc_status st) {
+        for (vkc_array *a : {ia, ib, va, vb, ca, oa, sa, sp})
+            if (a) vkc_array_release(a);
+        return st;
+    };
+    int64_t cw, sw;
+    radix_table_words(b, &cw, &sw);
+    vkc_status st;
+    if ((st = new_array(ctx, VKC_I32, b, false, &ia)) || (st = new_array(ctx, VKC_I32, b, false, &ib)) ||
+        (st = new_array(ctx, VKC_F64, b, false, &va)) || (passes > 1 && (st = new_array(ctx, VKC_F64, b, false, &vb))) ||
+        (st = new_array(ctx, VKC_I32, cw, false, &ca)) || (st = new_array(ctx, VKC_I32, cw, false, &oa)) ||
+        (st = new_array(ctx, VKC_I32, sw, false, &sa)) || (st = new_array(ctx, VKC_U64, 16 * nb, true, &sp)))
+        return done(st);
+    auto *first = static_cast<unsigned *>(ib->data());
+    rif_images_kernel<<<stream_grid(ctx, n, 256, 8, 4096), 256, 0, ctx->stream>>>(keys, n, b, static_cast<uint64_t>(nb), first,
+                                                                                  ctx->status);
+    if ((st = launched(ctx, "rif_images"))) return done(st);
+    const RadixTables t{static_cast<unsigned *>(ca->data()), static_cast<unsigned *>(oa->data()),
+                        static_cast<unsigned *>(sa->data())};
+    const RadixPairs<unsigned, unsigned long long> p{
+        first, x, {static_cast<unsigned *>(ia->data()), first},
+        {static_cast<unsigned long long *>(va->data()), vb ? static_cast<unsigned long long *>(vb->data()) : nullptr}};
+    int at = 0;
+    if ((st = radix_pairs(ctx, p, b, shifts, passes, t, &at))) return done(st);
+    auto *span = static_cast<uint2 *>(sp->data());
+    rif_spans_kernel<<<stream_grid(ctx, b / 4, 256, 8, 1024), 256, 0, ctx->stream>>>(p.img[at], b, span);
+    if (b < RIF_SHORT_ROWS * 16 * nb) {
+        rif_short_kernel<<<static_cast<int>((16 * nb + 255) / 256), 256, 0, ctx->stream>>>(span, p.pay[at], nb, out);
+    } else {
+        // Every pair of buckets that fits a wave of resident blocks, then further ones by stride.
+        const int64_t pairs = (nb + 1) / 2;
+        const int grid = static_cast<int>(std::min<int64_t>(pairs, static_cast<int64_t>(ctx->sms) * 8));
+        rif_sum_kernel<<<grid, 64, 0, ctx->stream>>>(span, p.pay[at], nb, out);
+    }
+    return done(launched(ctx, "rif_sums"));
+}
+
+// ------------------------------------------------------------------ the other paths
 
 // The masked path: for each bucket, reduce_add_f64 of the rows with the others read as +0.0.
 static vkc_status rif_masked(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t n,
@@ -185,8 +378,8 @@ static vkc_status rif_masked(vkc_ctx *ctx, const long long *keys, const unsigned
     return st;
 }
 
-// The sorted path over the rows below b (b > 0).
-static vkc_status rif_sorted(vkc_ctx *ctx, const vkc_array *keys, const vkc_array *vals, int64_t b,
+// Without a table of the chains, over the rows below b (b > 0).
+static vkc_status rif_scanned(vkc_ctx *ctx, const vkc_array *keys, const vkc_array *vals, int64_t b,
                              unsigned long long *out) {
     vkc_array *c = nullptr, *perm = nullptr, *cs = nullptr, *v = nullptr, *heads = nullptr, *ord = nullptr,
               *sums = nullptr, *ckey = nullptr, *csum = nullptr;
@@ -248,20 +441,28 @@ static vkc_status reduce_into_add_f64(vkc_ctx *ctx, const vkc_value *args, int n
         if (kst) return kst;
         return fail(ctx, st, msg);
     }
-    if ((st = bucket_key_error(ctx, k, n, nb, &found))) {
-        vkc_array_release(o);
-        return st;
-    }
     auto *ov = static_cast<unsigned long long *>(o->data());
     const auto *x = static_cast<const unsigned long long *>(vals->data());
     const int64_t b = n - n % 16;
-    if (n > 0 && nb <= RIF_MASKED_BUCKETS) {
-        st = rif_masked(ctx, k, x, n, nb, ov);
-    } else if (n > 0) {
-        if (b > 0) st = rif_sorted(ctx, keys, vals, b, ov);
+    if (b > 0 && nb > 0 && !rif_masks(n, nb) && rif_tables(n, nb)) {
+        // The keys are checked with their images; an error is found once the sums are done.
+        st = rif_sorted(ctx, k, x, n, b, nb, ov);
         if (!st && b < n) {
-            rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(k, x, b, n, ov);
+            rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(k, x, b, n, static_cast<uint64_t>(nb), ov);
             st = launched(ctx, "rif_tail");
+        }
+        DevStatus ds;
+        if (!st) st = read_status(ctx, &ds);
+        if (!st && ds.first_bad != ~0ull) st = bucket_key_error(ctx, k, n, nb, &found);
+    } else if (!(st = bucket_key_error(ctx, k, n, nb, &found)) && n > 0) {
+        if (rif_masks(n, nb)) {
+            st = rif_masked(ctx, k, x, n, nb, ov);
+        } else {
+            if (b > 0) st = rif_scanned(ctx, keys, vals, b, ov);
+            if (!st && b < n) {
+                rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(k, x, b, n, static_cast<uint64_t>(nb), ov);
+                st = launched(ctx, "rif_tail");
+            }
         }
     }
     if (st) {
