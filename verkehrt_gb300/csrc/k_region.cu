@@ -21,6 +21,7 @@
 
 #include "kcommon.cuh"
 #include "region.h"
+#include "reduce_common.h"
 #include "registry.h"
 
 namespace vkc {
@@ -114,6 +115,16 @@ bool plan_region(const vkc_region_kernel *ks, int nk, const vkc_value *in, int n
         if (d->ew_fn == EF_DIVC && !make_ew_divider(d->ew_ty, in[src_of(ks[k].args[1]).i].scalar.bits, &o.dv))
             return false;  // division by zero
         ty[static_cast<size_t>(k)] = d->out_type;
+        // An f64 comparison with a constant holds on a range of the other operand's order keys.
+        if (o.ty == ET_F64 && o.fn >= EF_LT && o.fn <= EF_NE && (o.kind[0] == RK_CONST) != (o.kind[1] == RK_CONST)) {
+            static const int of[6] = {2, 3, 4, 5, 0, 1};       // lt le gt ge eq ne
+            static const int mirrored[6] = {4, 5, 2, 3, 0, 1};  // c < x is x > c
+            const int at = o.kind[0] == RK_CONST ? 0 : 1;
+            double c;
+            memcpy(&c, &o.c[at], 8);
+            o.ranged = static_cast<unsigned char>(at == 1 ? 1 : 2);
+            o.range = cmp_range((at == 1 ? of : mirrored)[o.fn - EF_LT], c);
+        }
     }
     // Slots of the kept values, in kernel order.
     std::vector<int> slot(static_cast<size_t>(nk), -1);

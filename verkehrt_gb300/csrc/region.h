@@ -4,6 +4,7 @@
 // entries that check a region and fall back to whole evaluation).
 #pragma once
 
+#include "kcommon.cuh"
 #include "vkc_internal.h"
 
 namespace vkc {
@@ -45,12 +46,14 @@ struct RgOp {
     unsigned char fn, ty, dst;
     unsigned char kind[3], idx[3];
     unsigned char keep, slot;
+    unsigned char ranged;  // an f64 comparison with a constant: 1 or 2, the other operand's place + 1
     unsigned long long c[3];
     Divider dv;
+    CmpRange range;  // the values of that operand for which it holds
 };
 struct RegionProg {
     int nk, nslots, out_width, narr;
-    int f64only;  // every kernel f64 arithmetic or an f64 comparison, every input f64 (region_f64_kernel)
+    int f64only;  // every kernel f64 arithmetic or an f64 comparison, every input f64 (the f64 evaluator)
     RgIn in[RG_MAX_ARR];  // the array inputs, numbered in input order
     RgOp op[RG_MAX_K];
 };
