@@ -1071,22 +1071,59 @@ __global__ void __launch_bounds__(256) canon_fill_kernel(RowArgs args, int64_t n
 }
 
 // Short inputs: the reference's own order, each lane a chain of IEEE adds over its rows
-// (reduce.rs:45-62), from the lane states. The block first stages every row value in shared
-// memory (coalesced, all loads in flight at once); then 16 threads run the lane chains.
+// (reduce.rs:45-62), from the lane states (+0.0 when `fresh`). The block first stages every row value
+// in shared memory (coalesced, all loads in flight at once); then 16 threads run the lane chains, 31
+// ns a row, the latency of an FP64 add. With `result` the same launch combines the lanes and folds
+// the tail in (finish_lanes), else the lanes and the tail rows go to the state.
 constexpr int64_t CANON_SEQ_BLOCKS = 256;  // 16-row blocks (4096 rows) up to which this path runs
 
 template <int OP>
-__global__ void __launch_bounds__(256) canon_seq_kernel(RowArgs args, int nb, CanonState *state) {
-    __shared__ unsigned long long s_v[CANON_SEQ_BLOCKS * 16];
-    const int rows = nb * 16;
-    for (int i = threadIdx.x; i < rows; i += blockDim.x)
-        s_v[i] = row_value<OP>(args, args.x[i], OP == ROW_DOT ? args.y[i] : 0ull);
+__global__ void __launch_bounds__(256) canon_seq_kernel(RowArgs args, int nb, int rest, bool fresh, CanonState *state,
+                                                        unsigned long long *result) {
+    __shared__ unsigned long long s_v[CANON_SEQ_BLOCKS * 16 + 16];
+    const int rows = nb * 16 + rest;
+    constexpr int Q = CANON_SEQ_BLOCKS * 16 / 256 + 1;
+    unsigned long long x[Q], y[Q];
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int i = threadIdx.x + q * 256;
+        x[q] = i < rows ? args.x[i] : 0ull;
+        if (OP == ROW_DOT) y[q] = i < rows ? args.y[i] : 0ull;
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        const int i = threadIdx.x + q * 256;
+        if (i < rows) s_v[i] = row_value<OP>(args, x[q], OP == ROW_DOT ? y[q] : 0ull);
+    }
     __syncthreads();
     const int j = threadIdx.x;
-    if (j >= 16) return;
-    double s = as_f64(state->lanes[j]);
-    for (int b = 0; b < nb; ++b) s = __dadd_rn(s, as_f64(s_v[b * 16 + j]));
-    state->lanes[j] = as_bits(s);
+    if (j >= 32) return;
+    double s = fresh || j >= 16 ? 0.0 : as_f64(state->lanes[j]);
+    if (j < 16) {
+        int b = 0;
+        for (; b + 8 <= nb; b += 8) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = as_f64(s_v[(b + u) * 16 + j]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s = __dadd_rn(s, v[u]);
+        }
+        for (; b < nb; ++b) s = __dadd_rn(s, as_f64(s_v[b * 16 + j]));
+    }
+    if (!result) {
+        if (j < 16) state->lanes[j] = as_bits(s);
+        if (j < rest) state->tail[j] = s_v[nb * 16 + j];
+        return;
+    }
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1) {
+        const double other = __shfl_down_sync(FULL, s, step);
+        if (j < step) s = __dadd_rn(s, other);
+    }
+    if (j == 0) {
+        for (int i = 0; i < rest; ++i) s = __dadd_rn(s, as_f64(s_v[nb * 16 + i]));
+        *result = as_bits(s);
+    }
 }
 
 // Stores the row values of the rest rows (fewer than 16) as the pending tail.
@@ -1100,7 +1137,7 @@ __global__ void canon_tail(RowArgs args, int64_t first, int rest, CanonState *st
 }
 
 // reduce.rs:77-91 (finish_lanes): +8, +4, +2, +1, then the tail into lane 0 in order.
-__global__ void canon_finish(CanonState *state, int tail_len) {
+__global__ void canon_finish(CanonState *state, int tail_len, unsigned long long *host) {
     double acc[16];
     for (int j = 0; j < 16; ++j) acc[j] = as_f64(state->lanes[j]);
     for (int step = 8; step > 0; step >>= 1)
@@ -1108,6 +1145,7 @@ __global__ void canon_finish(CanonState *state, int tail_len) {
     double r = acc[0];
     for (int j = 0; j < tail_len; ++j) r = __dadd_rn(r, as_f64(state->tail[j]));
     state->result = as_bits(r);
+    if (host) *host = as_bits(r);
 }
 
 // ---------------------------------------------------------------------------- the lane chain
@@ -1396,10 +1434,12 @@ struct CanonReducer : DevReducer {
     int cmp = -1;
     int tail_len = 0;
 
-    vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
+    // The update's arguments, checked in the order of each reducer's update (fused.rs:77-203,
+    // reduce.rs:612-617).
+    vkc_status take(vkc_ctx *ctx, const Arg *args, int nargs, RowArgs *out) {
         vkc_status st;
-        RowArgs a{};
-        // Argument checks in the order of each reducer's update (fused.rs:77-203, reduce.rs:612-617).
+        RowArgs &a = *out;
+        a = RowArgs{};
         switch (op) {
         case ROW_SUM:
         case ROW_SUMSQ:
@@ -1424,22 +1464,37 @@ struct CanonReducer : DevReducer {
             break;
         }
         a.x = args[0].ptr<unsigned long long>();
-        const int64_t n = args[0].len();
         // reduce.rs:297-303: rows may only follow whole blocks.
         if (tail_len != 0) return fail(ctx, VKC_RUNTIME, "canonical update after a partial block");
-        const int64_t nb = n / 16;
+        return VKC_OK;
+    }
+    vkc_status seq(vkc_ctx *ctx, const RowArgs &a, int64_t n, unsigned long long *result) {
+        const int nb = static_cast<int>(n / 16), rest = static_cast<int>(n % 16);
+        auto *cs = static_cast<CanonState *>(state);
+        switch (op) {
+        case ROW_SUM: canon_seq_kernel<ROW_SUM><<<1, 256, 0, ctx->stream>>>(a, nb, rest, fresh, cs, result); break;
+        case ROW_DOT: canon_seq_kernel<ROW_DOT><<<1, 256, 0, ctx->stream>>>(a, nb, rest, fresh, cs, result); break;
+        case ROW_SUMSQ: canon_seq_kernel<ROW_SUMSQ><<<1, 256, 0, ctx->stream>>>(a, nb, rest, fresh, cs, result); break;
+        default: canon_seq_kernel<ROW_CONDSUM><<<1, 256, 0, ctx->stream>>>(a, nb, rest, fresh, cs, result); break;
+        }
+        updated(ctx);
+        return launched(ctx, "canon_seq");
+    }
+
+    vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
+        RowArgs a;
+        vkc_status st = take(ctx, args, nargs, &a);
+        if (st) return st;
+        const int64_t n = args[0].len(), nb = n / 16;
         const int rest = static_cast<int>(n % 16);
         auto *cs = static_cast<CanonState *>(state);
-        if (nb > 0 && nb <= CANON_SEQ_BLOCKS) {
-            const int nbi = static_cast<int>(nb);
-            switch (op) {
-            case ROW_SUM: canon_seq_kernel<ROW_SUM><<<1, 256, 0, ctx->stream>>>(a, nbi, cs); break;
-            case ROW_DOT: canon_seq_kernel<ROW_DOT><<<1, 256, 0, ctx->stream>>>(a, nbi, cs); break;
-            case ROW_SUMSQ: canon_seq_kernel<ROW_SUMSQ><<<1, 256, 0, ctx->stream>>>(a, nbi, cs); break;
-            default: canon_seq_kernel<ROW_CONDSUM><<<1, 256, 0, ctx->stream>>>(a, nbi, cs); break;
-            }
-            if ((st = launched(ctx, "canon_seq"))) return st;
-        } else if (nb > 0) {
+        if (n == 0) return VKC_OK;
+        if (nb <= CANON_SEQ_BLOCKS) {
+            tail_len = rest;
+            return seq(ctx, a, n, nullptr);
+        }
+        if (fresh && (st = zero(ctx))) return st;
+        {
             const int64_t T64 = (nb + CT_BLOCKS - 1) / CT_BLOCKS;
             if (T64 > (int64_t(1) << 26)) return fail(ctx, VKC_USAGE, "array too long for one update");
             const int T = static_cast<int>(T64), C = (T + 31) / 32;
@@ -1468,20 +1523,37 @@ struct CanonReducer : DevReducer {
             if ((st = launched(ctx, "canon_tail"))) return st;
             tail_len = rest;
         }
+        updated(ctx);
         return VKC_OK;
     }
+    vkc_status once(vkc_ctx *ctx, const Arg *args, int nargs, vkc_scalar *out, void *dst, bool *done) override {
+        *done = args[0].rows && args[0].len() / 16 <= CANON_SEQ_BLOCKS;
+        if (!*done) return VKC_OK;
+        RowArgs a;
+        vkc_status st = take(ctx, args, nargs, &a);
+        if (st) return st;
+        auto *to = static_cast<unsigned long long *>(dst ? dst : (host ? host : &static_cast<CanonState *>(state)->result));
+        if ((st = seq(ctx, a, args[0].len(), to)) || dst) return st;
+        out->type = VKC_F64;
+        return host ? result(ctx, &out->bits, 8) : download(ctx, &out->bits, 8, offsetof(CanonState, result));
+    }
 
+    // finish_lanes on the device; the result in the state and the slot.
+    vkc_status combine(vkc_ctx *ctx) {
+        vkc_status st;
+        if (fresh && (st = zero(ctx))) return st;
+        canon_finish<<<1, 1, 0, ctx->stream>>>(static_cast<CanonState *>(state), tail_len, static_cast<unsigned long long *>(host));
+        updated(ctx);
+        return launched(ctx, "canon_finish");
+    }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
-        auto *cs = static_cast<CanonState *>(state);
-        canon_finish<<<1, 1, 0, ctx->stream>>>(cs, tail_len);
-        vkc_status st = launched(ctx, "canon_finish");
+        const vkc_status st = combine(ctx);
         if (st) return st;
         out->type = VKC_F64;
-        return download(ctx, &out->bits, 8, offsetof(CanonState, result));
+        return host ? result(ctx, &out->bits, 8) : download(ctx, &out->bits, 8, offsetof(CanonState, result));
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        canon_finish<<<1, 1, 0, ctx->stream>>>(static_cast<CanonState *>(state), tail_len);
-        vkc_status st = launched(ctx, "canon_finish");
+        const vkc_status st = combine(ctx);
         return st ? st : copy_out(ctx, dst, 8, offsetof(CanonState, result));
     }
 };

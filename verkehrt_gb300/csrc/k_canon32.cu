@@ -516,12 +516,17 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
 }
 
 // Short inputs: the sixteen chains themselves, one block. The other warps stage the row values in
-// shared memory, chunk after chunk, while sixteen threads add (4.4 cycles a row of a lane).
+// shared memory, chunk after chunk, while sixteen threads add (4.4 cycles a row of a lane). With
+// `result` the same launch combines the lanes and folds the tail in (finish_lanes).
 constexpr int S32_BLOCKS = 512;           // 16-row blocks per staged chunk (32 KB)
-constexpr int64_t C32_SEQ_BLOCKS = 4096;  // up to 2^16 rows
+// Up to 2^16 rows the chains themselves, else the tile passes: the chains take about 0.3 ns a row,
+// the passes' five launches about 75 us up to a few million rows.
+constexpr int64_t C32_SEQ_BLOCKS = 4096;
 
-template <int OP> __global__ void __launch_bounds__(512) c32_chain(Args32 a, int nb, State32 *state) {
+template <int OP>
+__global__ void __launch_bounds__(512) c32_chain(Args32 a, int nb, int rest, bool fresh, State32 *state, float *result) {
     extern __shared__ __align__(16) float chain32[];
+    __shared__ float s_tail[16];
     const int t = threadIdx.x, chunks = (nb + S32_BLOCKS - 1) / S32_BLOCKS;
     auto stage = [&](int k, int first, int step) {
         const int r0 = k * S32_BLOCKS * 16, rows = min(S32_BLOCKS * 16, nb * 16 - r0);
@@ -530,8 +535,10 @@ template <int OP> __global__ void __launch_bounds__(512) c32_chain(Args32 a, int
         for (int i = first; i < rows; i += step)
             to[i] = value32<OP>(a, __ldg(a.x + r0 + i), OP == R32_DOT ? __ldg(a.y + r0 + i) : 0.f);
     };
-    float s = t < 16 ? state->lanes[t] : 0.f;
-    stage(0, t, 512);
+    float s = t < 16 && !fresh ? state->lanes[t] : 0.f;
+    if (t < rest)
+        s_tail[t] = value32<OP>(a, a.x[static_cast<int64_t>(nb) * 16 + t], OP == R32_DOT ? a.y[static_cast<int64_t>(nb) * 16 + t] : 0.f);
+    if (chunks > 0) stage(0, t, 512);
     __syncthreads();
     for (int k = 0; k < chunks; ++k) {
         if (t >= 32) {
@@ -551,7 +558,21 @@ template <int OP> __global__ void __launch_bounds__(512) c32_chain(Args32 a, int
         }
         __syncthreads();
     }
-    if (t < 16) state->lanes[t] = s;
+    if (!result) {
+        if (t < 16) state->lanes[t] = s;
+        if (t < rest) state->tail[t] = s_tail[t];
+        return;
+    }
+    if (t >= 32) return;
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1) {
+        const float other = __shfl_down_sync(FULL, s, step);
+        if (t < step) s = __fadd_rn(s, other);
+    }
+    if (t == 0) {
+        for (int i = 0; i < rest; ++i) s = __fadd_rn(s, s_tail[i]);
+        *result = s;
+    }
 }
 
 // The rest rows (fewer than 16), kept as row values until finish.
@@ -561,7 +582,7 @@ template <int OP> __global__ void c32_tail(Args32 a, int64_t first, int rest, St
 }
 
 // reduce.rs:77-91 (finish_lanes).
-__global__ void c32_finish(State32 *state, int tail_len) {
+__global__ void c32_finish(State32 *state, int tail_len, float *host) {
     float acc[16];
     for (int j = 0; j < 16; ++j) acc[j] = state->lanes[j];
     for (int step = 8; step > 0; step >>= 1)
@@ -569,6 +590,7 @@ __global__ void c32_finish(State32 *state, int tail_len) {
     float r = acc[0];
     for (int j = 0; j < tail_len; ++j) r = __fadd_rn(r, state->tail[j]);
     state->result = r;
+    if (host) *host = r;
 }
 
 size_t layout32(int T, int C, char *b, Work32 *wk) {
@@ -583,20 +605,19 @@ size_t layout32(int T, int C, char *b, Work32 *wk) {
     return o_ccode + up(c16 * 4);
 }
 
-// Which way: up to 2^16 rows the chains themselves, else the tile passes. The chains take about
-// 0.3 ns a row (45 us a call at 2^16 rows, 93 with the former staging), the passes' five launches
-// about 75 us up to a few million rows.
+template <int OP>
+vkc_status launch_chain32(vkc_ctx *ctx, const Args32 &a, int nb, int rest, bool fresh, State32 *state, float *result) {
+    constexpr size_t smem = 2 * S32_BLOCKS * 16 * sizeof(float);
+    static std::atomic<unsigned long long> configured{0};
+    once_per_device(configured, ctx->device, [] {
+        cudaFuncSetAttribute(c32_chain<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    });
+    c32_chain<OP><<<1, 512, smem, ctx->stream>>>(a, nb, rest, fresh, state, result);
+    return launched(ctx, "canon32_chain");
+}
+
 template <int OP> vkc_status launch_canon32(vkc_ctx *ctx, const Args32 &a, int64_t nb, State32 *state) {
     vkc_status st;
-    if (nb <= C32_SEQ_BLOCKS) {
-        constexpr size_t smem = 2 * S32_BLOCKS * 16 * sizeof(float);
-        static std::atomic<unsigned long long> configured{0};
-        once_per_device(configured, ctx->device, [] {
-            cudaFuncSetAttribute(c32_chain<OP>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        });
-        c32_chain<OP><<<1, 512, smem, ctx->stream>>>(a, static_cast<int>(nb), state);
-        return launched(ctx, "canon32_chain");
-    }
     const int64_t T64 = (nb + C32_BLOCKS - 1) / C32_BLOCKS;
     if (T64 > (int64_t(1) << 26)) return fail(ctx, VKC_USAGE, "array too long for one update");
     const int T = static_cast<int>(T64), C = (T + C32_CHUNK - 1) / C32_CHUNK;
@@ -636,12 +657,13 @@ template <int OP> struct Canon32Reducer : DevReducer {
     int cmp = 0;
     int tail_len = 0;
 
-    vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
+    vkc_status take(vkc_ctx *ctx, const Arg *args, int nargs, Args32 *out) {
         vkc_status st;
         constexpr int want = OP == R32_DOT ? 2 : (OP == R32_COND ? 3 : 1);
         if (nargs != want) return fail(ctx, VKC_RUNTIME, arity_error(want, nargs));
         if (!rows_arg(ctx, args[0], VKC_F32, &st)) return st;
-        Args32 a{args[0].ptr<float>(), nullptr, cmp, 0.f, 0.f};
+        Args32 &a = *out;
+        a = Args32{args[0].ptr<float>(), nullptr, cmp, 0.f, 0.f};
         if (OP == R32_DOT) {
             if (!rows_arg(ctx, args[1], VKC_F32, &st)) return st;
             if (args[0].len() != args[1].len())
@@ -655,39 +677,70 @@ template <int OP> struct Canon32Reducer : DevReducer {
         }
         // reduce.rs:297-303: rows may only follow whole blocks.
         if (tail_len != 0) return fail(ctx, VKC_RUNTIME, "canonical update after a partial block");
-        const int64_t n = args[0].len(), nb = n / 16;
-        auto *s = static_cast<State32 *>(state);
-        if (nb > 0 && (st = launch_canon32<OP>(ctx, a, nb, s))) return st;
-        const int rest = static_cast<int>(n % 16);
-        if (rest > 0) {
-            c32_tail<OP><<<1, 16, 0, ctx->stream>>>(a, nb * 16, rest, s);
-            if ((st = launched(ctx, "canon32_tail"))) return st;
-            tail_len = rest;
-        }
         return VKC_OK;
     }
-    vkc_status result(vkc_ctx *ctx) {
-        c32_finish<<<1, 1, 0, ctx->stream>>>(static_cast<State32 *>(state), tail_len);
+    vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
+        Args32 a;
+        vkc_status st = take(ctx, args, nargs, &a);
+        if (st) return st;
+        const int64_t n = args[0].len(), nb = n / 16;
+        const int rest = static_cast<int>(n % 16);
+        auto *s = static_cast<State32 *>(state);
+        if (n == 0) return VKC_OK;
+        if (nb <= C32_SEQ_BLOCKS) {
+            st = launch_chain32<OP>(ctx, a, static_cast<int>(nb), rest, fresh, s, nullptr);
+        } else {
+            if (fresh && (st = zero(ctx))) return st;
+            st = launch_canon32<OP>(ctx, a, nb, s);
+            if (!st && rest > 0) {
+                c32_tail<OP><<<1, 16, 0, ctx->stream>>>(a, nb * 16, rest, s);
+                st = launched(ctx, "canon32_tail");
+            }
+        }
+        updated(ctx);
+        tail_len = rest;
+        return st;
+    }
+    vkc_status read(vkc_ctx *ctx, vkc_scalar *out) {
+        unsigned b = 0;
+        const vkc_status st = host ? result(ctx, &b, 4) : download(ctx, &b, 4, offsetof(State32, result));
+        out->type = VKC_F32;
+        out->bits = b;
+        return st;
+    }
+    vkc_status once(vkc_ctx *ctx, const Arg *args, int nargs, vkc_scalar *out, void *dst, bool *done) override {
+        *done = args[0].rows && args[0].len() / 16 <= C32_SEQ_BLOCKS;
+        if (!*done) return VKC_OK;
+        Args32 a;
+        vkc_status st = take(ctx, args, nargs, &a);
+        if (st) return st;
+        const int64_t n = args[0].len();
+        auto *s = static_cast<State32 *>(state);
+        auto *to = static_cast<float *>(dst ? dst : (host ? host : &s->result));
+        st = launch_chain32<OP>(ctx, a, static_cast<int>(n / 16), static_cast<int>(n % 16), fresh, s, to);
+        updated(ctx);
+        return st || dst ? st : read(ctx, out);
+    }
+    vkc_status combine(vkc_ctx *ctx) {
+        vkc_status st;
+        if (fresh && (st = zero(ctx))) return st;
+        c32_finish<<<1, 1, 0, ctx->stream>>>(static_cast<State32 *>(state), tail_len, static_cast<float *>(host));
+        updated(ctx);
         return launched(ctx, "canon32_finish");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
-        vkc_status st = result(ctx);
-        if (st) return st;
-        unsigned b = 0;
-        if ((st = download(ctx, &b, 4, offsetof(State32, result)))) return st;
-        out->type = VKC_F32;
-        out->bits = b;
-        return VKC_OK;
+        const vkc_status st = combine(ctx);
+        return st ? st : read(ctx, out);
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        const vkc_status st = result(ctx);
+        const vkc_status st = combine(ctx);
         return st ? st : copy_out(ctx, dst, 4, offsetof(State32, result));
     }
 };
 
 template <int OP> ReducerImpl *make32(vkc_ctx *ctx, int cmp) {
     auto *r = new Canon32Reducer<OP>;
-    if (r->alloc(ctx, sizeof(State32))) {  // lanes at +0.0
+    if (r->alloc(ctx, sizeof(State32))) {
         delete r;
         return nullptr;
     }

@@ -793,7 +793,8 @@ __global__ void __launch_bounds__(RG_THREADS, 4) region_f64_kernel(const RegionP
 }
 
 template <int NARR, int MODE>
-static vkc_status launch_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *work, unsigned *done) {
+static vkc_status launch_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *partials, unsigned *done,
+                             RgFold *result) {
     constexpr int RF_BLOCK_ROWS = RG_THREADS * rf_rows<NARR>();
     const size_t smem = static_cast<size_t>(p.nslots) * RF_BLOCK_ROWS * sizeof(double);
     static std::atomic<unsigned long long> configured{0};
@@ -808,25 +809,25 @@ static vkc_status launch_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void 
     const int64_t blocks = (n + RF_BLOCK_ROWS - 1) / RF_BLOCK_ROWS;
     const int64_t most = std::min<int64_t>(static_cast<int64_t>(ctx->sms) * std::max(1, per_sm), RG_FOLD_MAX_GRID);
     const int grid = static_cast<int>(std::min<int64_t>(blocks, most));
-    region_f64_kernel<NARR, MODE><<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, aligned, out, kind, work ? work + 1 : nullptr,
-                                                                         done, work);
+    region_f64_kernel<NARR, MODE><<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, aligned, out, kind, partials, done, result);
     return launched(ctx, "region_f64");
 }
 
 template <int MODE>
-static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *work, unsigned *done) {
+static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *partials, unsigned *done,
+                          RgFold *result) {
     switch (p.narr) {
-    case 1: return launch_f64<1, MODE>(ctx, p, n, out, kind, work, done);
-    case 2: return launch_f64<2, MODE>(ctx, p, n, out, kind, work, done);
-    case 3: return launch_f64<3, MODE>(ctx, p, n, out, kind, work, done);
-    default: return launch_f64<4, MODE>(ctx, p, n, out, kind, work, done);
+    case 1: return launch_f64<1, MODE>(ctx, p, n, out, kind, partials, done, result);
+    case 2: return launch_f64<2, MODE>(ctx, p, n, out, kind, partials, done, result);
+    case 3: return launch_f64<3, MODE>(ctx, p, n, out, kind, partials, done, result);
+    default: return launch_f64<4, MODE>(ctx, p, n, out, kind, partials, done, result);
     }
 }
 
-vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *work,
-                              unsigned *done) {
+vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *partials,
+                              unsigned *done, RgFold *result) {
     if (n <= 0) return VKC_OK;
-    if (p.f64only && f64) return run_f64<RF_FOLD>(ctx, p, n, nullptr, kind, work, done);
+    if (p.f64only && f64) return run_f64<RF_FOLD>(ctx, p, n, nullptr, kind, partials, done, result);
     const size_t smem = static_cast<size_t>(p.nslots) * RG_BLOCK_ROWS * sizeof(unsigned long long);
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {
@@ -838,15 +839,15 @@ vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int 
     const int64_t blocks = (n + RG_BLOCK_ROWS - 1) / RG_BLOCK_ROWS;
     int64_t g = std::min<int64_t>(blocks, static_cast<int64_t>(ctx->sms) * std::max(1, per_sm));
     const int grid = static_cast<int>(std::min<int64_t>(g, RG_FOLD_MAX_GRID));
-    region_fold_kernel<<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, kind, f64, work + 1, done, work);
+    region_fold_kernel<<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, kind, f64, partials, done, result);
     return launched(ctx, "region_fold");
 }
 
 vkc_status launch_region(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, bool count) {
     if (n <= 0) return VKC_OK;
     if (p.f64only)
-        return count ? run_f64<RF_COUNT>(ctx, p, n, out, 0, nullptr, nullptr)
-                     : run_f64<RF_STORE>(ctx, p, n, out, 0, nullptr, nullptr);
+        return count ? run_f64<RF_COUNT>(ctx, p, n, out, 0, nullptr, nullptr, nullptr)
+                     : run_f64<RF_STORE>(ctx, p, n, out, 0, nullptr, nullptr, nullptr);
     const size_t smem = static_cast<size_t>(p.nslots) * RG_BLOCK_ROWS * sizeof(unsigned long long);
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {

@@ -190,7 +190,8 @@ template <vkc_type T, int ROW> __device__ __forceinline__ u64 row_value(const Ro
 // block combine (the fold is commutative), and the last block to finish folds the block
 // partials into the reducer's state word.
 template <vkc_type T, int F, int ROW>
-__global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64 *partials, unsigned *done, u64 *state) {
+__global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64 *partials, unsigned *done, bool fresh, u64 *state,
+                                                       u64 *host) {
     constexpr vkc_type AT = ROW == R_PRED ? VKC_U64 : T;  // predicate counts add as u64
     u64 acc = identity<AT, F>();
     const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -218,8 +219,9 @@ __global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s = step<AT, F>(s, __shfl_xor_sync(FULL, s, o));
         if (threadIdx.x == 0) {
-            state[0] = step<AT, F>(state[0], s);
-            state[1] = 1;  // rows seen
+            if (!fresh) s = step<AT, F>(state[0], s);
+            state[0] = s;
+            if (host) host[0] = s;
         }
     }
 }
@@ -246,7 +248,7 @@ __device__ __forceinline__ void arg_better(u64 &h, u64 &r, u64 h2, u64 r2) {
 
 template <vkc_type T, bool MAX>
 __global__ void __launch_bounds__(256) fam_arg_kernel(const void *x, int64_t n, u64 base, ulonglong2 *partials,
-                                                      unsigned *done, u64 *state) {
+                                                      unsigned *done, bool fresh, u64 *state, u64 *host) {
     u64 h = ~0ull, r = ~0ull;
     const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -269,11 +271,13 @@ __global__ void __launch_bounds__(256) fam_arg_kernel(const void *x, int64_t n, 
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) arg_better(bh, br, __shfl_xor_sync(FULL, bh, o), __shfl_xor_sync(FULL, br, o));
         if (threadIdx.x == 0) {
-            u64 sh = state[0], sr = state[1];
-            arg_better(sh, sr, bh, br);
-            state[0] = sh;
-            state[1] = sr;
-            state[2] = 1;
+            if (!fresh) arg_better(bh, br, state[0], state[1]);
+            state[0] = bh;
+            state[1] = br;
+            if (host) {
+                host[0] = bh;
+                host[1] = br;
+            }
         }
     }
 }
@@ -294,8 +298,8 @@ u64 scalar_word(vkc_type t, const vkc_scalar &s) {
     return s.bits;
 }
 
-// Reducers of the order-free folds. State: [0] the folded word, [1] rows seen (argmin/argmax:
-// [0] key, [1] row, [2] rows seen). `base` counts the rows of earlier updates.
+// Reducers of the order-free folds. State: [0] the folded word (argmin/argmax: [0] key, [1] row).
+// `base` counts the rows of earlier updates.
 struct FamReducer : DevReducer {
     vkc_type in, out;
     int fold;      // F_*, or -1 argmin, -2 argmax
@@ -305,10 +309,10 @@ struct FamReducer : DevReducer {
     bool empty_error = false;  // min/max/argmin/argmax of no rows fail
     const char *what = "";
     u64 base = 0;
-    using Launch = void (*)(vkc_ctx *, const RowArgs &, int64_t, int, void *, u64, u64 *);
+    u64 empty = 0;  // the result word of no rows
+    using Launch = void (*)(vkc_ctx *, const RowArgs &, int64_t, int, void *, u64, bool, u64 *, u64 *);
     Launch launch = nullptr;
 
-    vkc_status init(vkc_ctx *ctx, u64 id0, u64 id1) { return fill(ctx, 3, id0, id1, 0); }
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != nargs_want) return fail(ctx, VKC_RUNTIME, arity_error(nargs_want, nargs));
@@ -331,40 +335,42 @@ struct FamReducer : DevReducer {
         const int grid = stream_grid(ctx, n, 256, tune(ctx, TK_STREAM_BLOCKS, n), 4096);
         void *part;
         if ((st = scratch(ctx, 16 * static_cast<size_t>(grid), &part))) return st;
-        launch(ctx, a, n, grid, part, base, static_cast<u64 *>(state));
+        launch(ctx, a, n, grid, part, base, fresh, static_cast<u64 *>(state), static_cast<u64 *>(host));
+        updated(ctx);
         base += static_cast<u64>(n);
         return launched(ctx, "family_fold");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out_s) override {
-        u64 h[3];
-        vkc_status st = download(ctx, h, sizeof h);
+        if (empty_error && fresh) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
+        u64 h[2] = {empty, 0};
+        vkc_status st = fresh ? VKC_OK : result(ctx, h, sizeof h);
         if (st) return st;
-        const bool arg = fold < 0;
-        if (empty_error && !(arg ? h[2] : h[1])) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
-        *out_s = arg ? scalar_i64(static_cast<int64_t>(h[1])) : word_scalar(out, h[0]);
+        *out_s = fold < 0 ? scalar_i64(static_cast<int64_t>(h[1])) : word_scalar(out, h[0]);
         return VKC_OK;
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        if (empty_error && base == 0) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
+        if (empty_error && fresh) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
+        const vkc_status st = fresh ? fill(ctx, 1, empty) : VKC_OK;
+        if (st) return st;
         // Words are little-endian: the result type's bytes are the word's low bytes.
         return fold < 0 ? copy_out(ctx, dst, 8, 8) : copy_out(ctx, dst, static_cast<size_t>(width_of(out)));
     }
 };
 
 template <vkc_type T, int F, int ROW>
-void launch_fold(vkc_ctx *ctx, const RowArgs &a, int64_t n, int grid, void *part, u64, u64 *state) {
-    fam_fold_kernel<T, F, ROW><<<grid, 256, 0, ctx->stream>>>(a, n, static_cast<u64 *>(part), ctx->counters + 1, state);
+void launch_fold(vkc_ctx *ctx, const RowArgs &a, int64_t n, int grid, void *part, u64, bool fresh, u64 *state, u64 *host) {
+    fam_fold_kernel<T, F, ROW><<<grid, 256, 0, ctx->stream>>>(a, n, static_cast<u64 *>(part), ctx->counters + 1, fresh, state, host);
 }
 template <vkc_type T, bool MAX>
-void launch_arg(vkc_ctx *ctx, const RowArgs &a, int64_t n, int grid, void *part, u64 base, u64 *state) {
+void launch_arg(vkc_ctx *ctx, const RowArgs &a, int64_t n, int grid, void *part, u64 base, bool fresh, u64 *state, u64 *host) {
     fam_arg_kernel<T, MAX><<<grid, 256, 0, ctx->stream>>>(a.x, n, base, static_cast<ulonglong2 *>(part),
-                                                          ctx->counters + 1, state);
+                                                          ctx->counters + 1, fresh, state, host);
 }
 
 template <vkc_type T, int F, int ROW, int NARGS>
 ReducerImpl *make_fold(vkc_ctx *ctx, vkc_type out, int cmp, bool empty_error, const char *what) {
     auto *r = new FamReducer;
-    if (r->alloc(ctx, 24)) {
+    if (r->alloc(ctx, 16)) {
         delete r;
         return nullptr;
     }
@@ -377,17 +383,13 @@ ReducerImpl *make_fold(vkc_ctx *ctx, vkc_type out, int cmp, bool empty_error, co
     r->empty_error = empty_error;
     r->what = what;
     r->launch = launch_fold<T, F, ROW>;
-    constexpr vkc_type AT = ROW == R_PRED ? VKC_U64 : T;
-    if (r->init(ctx, identity<AT, F>(), 0)) {
-        delete r;
-        return nullptr;
-    }
+    r->empty = identity<ROW == R_PRED ? VKC_U64 : T, F>();
     return r;
 }
 
 template <vkc_type T, bool MAX> ReducerImpl *make_arg(vkc_ctx *ctx) {
     auto *r = new FamReducer;
-    if (r->alloc(ctx, 24)) {
+    if (r->alloc(ctx, 16)) {
         delete r;
         return nullptr;
     }
@@ -399,10 +401,6 @@ template <vkc_type T, bool MAX> ReducerImpl *make_arg(vkc_ctx *ctx) {
     r->empty_error = true;
     r->what = MAX ? "argmax" : "argmin";
     r->launch = launch_arg<T, MAX>;
-    if (r->init(ctx, ~0ull, ~0ull)) {
-        delete r;
-        return nullptr;
-    }
     return r;
 }
 
@@ -444,7 +442,7 @@ template <vkc_type T> __global__ void fam_chain_tail(const void *x, int64_t firs
 }
 
 // reduce.rs:77-91 (finish_lanes).
-template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len) {
+template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len, u64 *host) {
     u64 acc[16];
     for (int j = 0; j < 16; ++j) acc[j] = st[j];
     for (int s = 8; s > 0; s >>= 1)
@@ -452,6 +450,7 @@ template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len) {
     u64 r = acc[0];
     for (int j = 0; j < tail_len; ++j) r = mul_t<T>(r, st[16 + j]);
     st[32] = r;
+    if (host) *host = r;
 }
 
 // CanonicalAcc (reduce.rs:253-323) on the device. State: [0..15] lanes, [16..31] tail, [32] result.
@@ -473,20 +472,21 @@ template <vkc_type T> struct ChainReducer : DevReducer {
         tail_len = rest;
         return launched(ctx, "family_chain");
     }
-    vkc_status result(vkc_ctx *ctx) {
-        fam_chain_finish<T><<<1, 1, 0, ctx->stream>>>(static_cast<u64 *>(state), tail_len);
+    vkc_status combine(vkc_ctx *ctx) {
+        fam_chain_finish<T><<<1, 1, 0, ctx->stream>>>(static_cast<u64 *>(state), tail_len, static_cast<u64 *>(host));
+        updated(ctx);
         return launched(ctx, "family_chain_finish");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
-        vkc_status st = result(ctx);
+        vkc_status st = combine(ctx);
         if (st) return st;
         u64 r = 0;
-        if ((st = download(ctx, &r, 8, 32 * 8))) return st;
+        if ((st = host ? result(ctx, &r, 8) : download(ctx, &r, 8, 32 * 8))) return st;
         *out = word_scalar(T, r);
         return VKC_OK;
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        const vkc_status st = result(ctx);
+        const vkc_status st = combine(ctx);
         return st ? st : copy_out(ctx, dst, static_cast<size_t>(width_of(T)), 32 * 8);
     }
 };

@@ -4,7 +4,7 @@
 //
 // Each reducer keeps its running state in a small device buffer. An update is one kernel: every
 // block folds its rows, and the last block to finish (last-block-done) folds the block
-// partials into the state, so the only host sync is the download at finish.
+// partials into the state and into the reducer's host slot, so finish only waits for the stream.
 #include <cmath>
 #include <cstring>
 
@@ -58,7 +58,8 @@ CmpRange cmp_range(int cmp, double c) {
 template <bool BOOL, bool POS>
 __global__ void __launch_bounds__(256) count_kernel(const void *__restrict__ xv, int64_t n,
                                                     CmpRange r, unsigned long long *partials,
-                                                    unsigned *done, unsigned long long *state) {
+                                                    unsigned *done, bool fresh, unsigned long long *state,
+                                                    unsigned long long *host) {
     unsigned long long c = 0;
     int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -114,7 +115,11 @@ __global__ void __launch_bounds__(256) count_kernel(const void *__restrict__ xv,
         unsigned long long s = 0;
         for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) s += partials[b];
         s = warp_sum(s);
-        if (threadIdx.x == 0) *state += s;
+        if (threadIdx.x == 0) {
+            if (!fresh) s += *state;
+            *state = s;
+            if (host) *host = s;
+        }
     }
 }
 
@@ -137,23 +142,28 @@ struct CountReducer : DevReducer {
         if ((st = scratch(ctx, sizeof(unsigned long long) * grid, &part))) return st;
         auto *s = static_cast<unsigned long long *>(state);
         auto *pp = static_cast<unsigned long long *>(part);
+        auto *hs = static_cast<unsigned long long *>(host);
         if (cmp < 0) {
-            count_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, CmpRange{}, pp, ctx->counters + 1, s);
+            count_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, CmpRange{}, pp, ctx->counters + 1, fresh, s, hs);
         } else {
             const CmpRange r = cmp_range(cmp, args[1].f64());
-            if (pos_range(r)) count_kernel<false, true><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, r, pp, ctx->counters + 1, s);
-            else count_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, r, pp, ctx->counters + 1, s);
+            if (pos_range(r)) count_kernel<false, true><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, r, pp, ctx->counters + 1, fresh, s, hs);
+            else count_kernel<false, false><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, r, pp, ctx->counters + 1, fresh, s, hs);
         }
+        updated(ctx);
         return launched(ctx, "count");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
         unsigned long long v = 0;
-        vkc_status st = download(ctx, &v, sizeof v);
+        vkc_status st = fresh ? VKC_OK : result(ctx, &v, sizeof v);
         if (st) return st;
         *out = scalar_i64(static_cast<int64_t>(v));
         return VKC_OK;
     }
-    vkc_status finish_into(vkc_ctx *ctx, void *dst) override { return copy_out(ctx, dst, 8); }
+    vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
+        const vkc_status st = fresh ? zero(ctx) : VKC_OK;
+        return st ? st : copy_out(ctx, dst, 8);
+    }
 };
 
 // ------------------------------------------------------------------ extremes
@@ -186,7 +196,7 @@ __device__ __forceinline__ void better(long long &k, unsigned long long &i, long
 template <bool MAX, bool F64, bool ARG>
 __global__ void __launch_bounds__(256) extreme_kernel(const long long *__restrict__ x, int64_t n,
                                                       unsigned long long base, ExtState *partials,
-                                                      unsigned *done, ExtState *state) {
+                                                      unsigned *done, bool fresh, ExtState *state, ExtState *host) {
     long long bk = MAX ? LLONG_MIN : LLONG_MAX;
     unsigned bpos = ~0u, npos = ~0u;  // best and first-NaN positions (step * 8 + slot)
     unsigned long long maxabs = 0;     // min/max only: NaN when above +inf's bits
@@ -326,9 +336,12 @@ __global__ void __launch_bounds__(256) extreme_kernel(const long long *__restric
         __syncthreads();
         if (threadIdx.x == 0) {
             for (int w = 1; w < 8; ++w) take(ws[w].key, ws[w].idx, ws[w].nan_idx);
-            const ExtState s = *state;
-            if (s.seen) take(s.key, s.idx, s.nan_idx);
+            if (!fresh) {
+                const ExtState s = *state;
+                take(s.key, s.idx, s.nan_idx);
+            }
             *state = ExtState{k, i, nn, 1};
+            if (host) *host = ExtState{k, i, nn, 1};
         }
     }
 }
@@ -344,7 +357,6 @@ struct ExtremeReducer : DevReducer {
     bool max, arg;
     vkc_type type;
     unsigned long long consumed = 0;
-    vkc_status init(vkc_ctx *ctx) { return fill(ctx, 4, 0, ~0ull, ~0ull, 0); }  // ExtState{0, ~0, ~0, 0}
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));
@@ -358,7 +370,7 @@ struct ExtremeReducer : DevReducer {
         auto *s = static_cast<ExtState *>(state);
         const long long *x = static_cast<const long long *>(args[0].a->data());
         bool f = type == VKC_F64;
-#define EXT_LAUNCH(MX, F, A) extreme_kernel<MX, F, A><<<grid, 256, 0, ctx->stream>>>(x, n, consumed, p, ctx->counters + 1, s)
+#define EXT_LAUNCH(MX, F, A) extreme_kernel<MX, F, A><<<grid, 256, 0, ctx->stream>>>(x, n, consumed, p, ctx->counters + 1, fresh, s, static_cast<ExtState *>(host))
         if (arg) {
             if (max && f) EXT_LAUNCH(true, true, true);
             else if (max) EXT_LAUNCH(true, false, true);
@@ -372,12 +384,13 @@ struct ExtremeReducer : DevReducer {
         }
 #undef EXT_LAUNCH
         consumed += static_cast<unsigned long long>(n);
+        updated(ctx);
         return launched(ctx, "extreme");
     }
     // reduce.rs:401-411 and :454-467: empty input is an error; a NaN decides the result.
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
-        ExtState s;
-        vkc_status st = download(ctx, &s, sizeof s);
+        ExtState s{0, 0, 0, 0};
+        vkc_status st = fresh ? VKC_OK : result(ctx, &s, sizeof s);
         if (st) return st;
         if (!s.seen) {
             std::string what = arg ? (max ? "argmax" : "argmin") : (max ? "reduce_max" : "reduce_min");
@@ -411,8 +424,8 @@ struct ExtremeReducer : DevReducer {
 // ------------------------------------------------------------------ integer sum
 
 __global__ void __launch_bounds__(256) isum_kernel(const unsigned long long *__restrict__ x, int64_t n,
-                                                   unsigned long long *partials, unsigned *done,
-                                                   unsigned long long *state) {
+                                                   unsigned long long *partials, unsigned *done, bool fresh,
+                                                   unsigned long long *state, unsigned long long *host) {
     unsigned long long c = 0;
     int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -442,7 +455,11 @@ __global__ void __launch_bounds__(256) isum_kernel(const unsigned long long *__r
         unsigned long long s = 0;
         for (unsigned b = threadIdx.x; b < gridDim.x; b += 32) s += partials[b];
         s = warp_sum(s);
-        if (threadIdx.x == 0) *state += s;
+        if (threadIdx.x == 0) {
+            if (!fresh) s += *state;
+            *state = s;
+            if (host) *host = s;
+        }
     }
 }
 
@@ -459,18 +476,22 @@ struct IntSumReducer : DevReducer {
         if ((st = scratch(ctx, sizeof(unsigned long long) * grid, &part))) return st;
         isum_kernel<<<grid, 256, 0, ctx->stream>>>(
             static_cast<const unsigned long long *>(args[0].a->data()), n,
-            static_cast<unsigned long long *>(part), ctx->counters + 1,
-            static_cast<unsigned long long *>(state));
+            static_cast<unsigned long long *>(part), ctx->counters + 1, fresh,
+            static_cast<unsigned long long *>(state), static_cast<unsigned long long *>(host));
+        updated(ctx);
         return launched(ctx, "isum");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out) override {
         unsigned long long v = 0;
-        vkc_status st = download(ctx, &v, sizeof v);
+        vkc_status st = fresh ? VKC_OK : result(ctx, &v, sizeof v);
         if (st) return st;
         *out = scalar_i64(static_cast<int64_t>(v));
         return VKC_OK;
     }
-    vkc_status finish_into(vkc_ctx *ctx, void *dst) override { return copy_out(ctx, dst, 8); }
+    vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
+        const vkc_status st = fresh ? zero(ctx) : VKC_OK;
+        return st ? st : copy_out(ctx, dst, 8);
+    }
 };
 
 // ------------------------------------------------------------------ registration
@@ -498,10 +519,6 @@ template <bool MAX, bool ARG, vkc_type T> static ReducerImpl *make_ext(vkc_ctx *
     r->max = MAX;
     r->arg = ARG;
     r->type = T;
-    if (r->init(ctx)) {
-        delete r;
-        return nullptr;
-    }
     return r;
 }
 

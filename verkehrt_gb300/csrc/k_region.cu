@@ -357,16 +357,15 @@ vkc_status vkc_region_reduce(vkc_ctx *ctx, int root, const int32_t *root_args, i
             t != (f.f64 ? VKC_F64 : VKC_I64) || n == 0)
             break;  // the root over the materialised value gives the value and the errors
         await_values(ctx, inputs, ninputs);
-        vkc_array *w;
-        const int64_t words = 4 * (RG_FOLD_MAX_GRID + 1) + 1;
-        if ((st = new_array(ctx, VKC_U64, words, true, &w))) return st;
-        auto *work = static_cast<RgFold *>(w->data());
-        RgFold r{};
-        st = launch_region_fold(ctx, p, n, f.kind, f.f64, work,
-                                reinterpret_cast<unsigned *>(static_cast<unsigned long long *>(w->data()) + words - 1));
-        if (!st) st = vkc_array_download(ctx, w, &r, 4);
-        vkc_array_release(w);
+        // The last block writes the fold into pinned memory, so the call is one launch and one wait.
+        void *partials, *host;
+        if ((st = scratch(ctx, sizeof(RgFold) * RG_FOLD_MAX_GRID, &partials))) return st;
+        if ((st = pinned(ctx, sizeof(RgFold), &host))) return st;
+        st = launch_region_fold(ctx, p, n, f.kind, f.f64, static_cast<RgFold *>(partials), ctx->counters + 1,
+                                static_cast<RgFold *>(host));
         if (st) return st;
+        VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        const RgFold r = *static_cast<const RgFold *>(host);
         out->kind = VKC_VALUE_SCALAR;
         const bool arg = f.kind == RF_ARGMIN || f.kind == RF_ARGMAX;
         if (f.kind == RF_SUM) {

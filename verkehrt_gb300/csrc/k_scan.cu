@@ -300,12 +300,12 @@ __global__ void __launch_bounds__(SC_THREADS + 64, SC_BLOCKS) scan_kernel(const 
                                                                   const unsigned char *__restrict__ starts,
                                                                   unsigned long long *__restrict__ out, int64_t n,
                                                                   bool aligned, int tiles, ulonglong2 *recs,
-                                                                  unsigned epoch, ScanState *state,
+                                                                  unsigned epoch, bool fresh, ScanState *state,
                                                                   unsigned *counters, DevStatus *status) {
-    // The carried state is read once, before this block publishes anything; the block that
-    // finishes last rewrites it, after every block has read it.
-    const bool seen = state->seen != 0;
-    const unsigned long long carried = state->last;
+    // The carried state (none in a first update) is read once, before this block publishes
+    // anything; the block that finishes last rewrites it, after every block has read it.
+    const bool seen = !fresh && state->seen != 0;
+    const unsigned long long carried = fresh ? 0ull : state->last;
     ScanPass<BY> p{x, starts, out, n, seen, aligned};
     // The last row's output, the last tile's inclusive value, is the carried state.
     if (tile_pass<SC_WINDOW>(p, recs, tiles, epoch, counters, status, Seg{carried, 0}) && threadIdx.x == 0) {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(SC_THREADS + 64, SC_BLOCKS) scan_kernel(const 
 // Launches a scan on `stream` with the tile records at `recs` (REC_STRIDE bytes per tile).
 template <bool BY>
 static void launch_scan(int device, int sms, cudaStream_t stream, const unsigned long long *x, const unsigned char *s,
-                        unsigned long long *o, int64_t n, int tiles, ulonglong2 *recs, unsigned epoch,
+                        unsigned long long *o, int64_t n, int tiles, ulonglong2 *recs, unsigned epoch, bool fresh,
                         ScanState *state, unsigned *counters, DevStatus *status) {
     const bool aligned = (reinterpret_cast<uintptr_t>(x) & 31) == 0 && (reinterpret_cast<uintptr_t>(o) & 31) == 0 &&
                          (reinterpret_cast<uintptr_t>(s) & 15) == 0;
@@ -334,13 +334,14 @@ static void launch_scan(int device, int sms, cudaStream_t stream, const unsigned
     }
     const long long g = static_cast<long long>(per_sm) * sms;
     const int grid = static_cast<int>(g < tiles ? g : tiles);
-    scan_kernel<BY><<<grid, SC_THREADS + 64, smem, stream>>>(x, s, o, n, aligned, tiles, recs, epoch, state, counters,
+    scan_kernel<BY><<<grid, SC_THREADS + 64, smem, stream>>>(x, s, o, n, aligned, tiles, recs, epoch, fresh, state, counters,
                                                              status);
 }
 
 struct ScanImpl : ScannerImpl {
     bool by;
-    ScanState *state = nullptr;
+    ScanState *state = nullptr;  // uninitialised until the first update (fresh)
+    bool fresh = true;
     DeviceMem mem;  // owns `state`
     // scan.rs:228-282 (tile_rows): arity, kinds, then destination rows.
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs, vkc_array *out) override {
@@ -363,25 +364,18 @@ struct ScanImpl : ScannerImpl {
         const auto *x = args[0].ptr<unsigned long long>();
         const unsigned char *s = by ? args[1].ptr<unsigned char>() : nullptr;
         auto *o = static_cast<unsigned long long *>(out->data());
-        if (by) launch_scan<true>(ctx->device, ctx->sms, ctx->stream, x, s, o, n, tiles, recs, epoch, state, ctx->counters, ctx->status);
-        else launch_scan<false>(ctx->device, ctx->sms, ctx->stream, x, s, o, n, tiles, recs, epoch, state, ctx->counters, ctx->status);
+        if (by) launch_scan<true>(ctx->device, ctx->sms, ctx->stream, x, s, o, n, tiles, recs, epoch, fresh, state, ctx->counters, ctx->status);
+        else launch_scan<false>(ctx->device, ctx->sms, ctx->stream, x, s, o, n, tiles, recs, epoch, fresh, state, ctx->counters, ctx->status);
+        fresh = false;
         return launched(ctx, "scan");
     }
 };
 
-// A zeroed ScanState on the context's stream, owned by `mem`.
+// A ScanState owned by `mem`, uninitialised.
 static bool alloc_scan_state(vkc_ctx *ctx, ScanState **state, DeviceMem *mem) {
-    if (cudaMallocAsync(reinterpret_cast<void **>(state), sizeof(ScanState), ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        *state = nullptr;
-        return false;
-    }
-    mem->ptr = *state;
-    mem->box = ctx->box;
-    if (cudaMemsetAsync(*state, 0, sizeof(ScanState), ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
+    bool captured;
+    if (state_block(ctx, sizeof(ScanState), mem, &captured)) return false;
+    *state = static_cast<ScanState *>(mem->ptr);
     return true;
 }
 
@@ -436,7 +430,9 @@ struct PrevImpl : ScannerImpl {
 
 static ScannerImpl *make_prev(vkc_ctx *ctx) {
     auto *s = new PrevImpl;
-    if (!alloc_scan_state(ctx, &s->state, &s->mem)) {
+    if (!alloc_scan_state(ctx, &s->state, &s->mem) ||
+        cudaMemsetAsync(s->state, 0, sizeof(ScanState), ctx->stream) != cudaSuccess) {
+        cudaGetLastError();
         delete s;
         return nullptr;
     }
@@ -584,7 +580,7 @@ extern "C" vkc_status vkc_scan_add_i64_noalloc(int device, const int64_t *in, in
         return done(VKC_DEVICE, std::string("vkc_scan_add_i64_noalloc: ") + cudaGetErrorString(e));
     }
     launch_scan<false>(device, sms, s, reinterpret_cast<const unsigned long long *>(in), nullptr,
-                       reinterpret_cast<unsigned long long *>(out), n, tiles, recs, 1u, state, counters, status);
+                       reinterpret_cast<unsigned long long *>(out), n, tiles, recs, 1u, true, state, counters, status);
     e = cudaGetLastError();
     if (e != cudaSuccess) return done(VKC_DEVICE, std::string("vkc_scan_add_i64_noalloc: ") + cudaGetErrorString(e));
     // Synchronous, like the other entries: read the status word into host memory.

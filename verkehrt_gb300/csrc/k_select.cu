@@ -34,6 +34,7 @@ struct SelArgs {
     int64_t base;           // where: global row of row 0
     void *out;
     unsigned long long *total;  // survivor count of the launch
+    unsigned long long *host;   // pinned: the count and the status word's timeout, written by the last block
     bool aligned;           // values and mask start on 16-byte boundaries: whole tiles go by TMA
 };
 
@@ -271,52 +272,119 @@ __global__ void __launch_bounds__(SEL_THREADS + 64, SEL_BLOCKS) select_kernel(Se
                                                                      unsigned epoch, unsigned *counters,
                                                                      DevStatus *status) {
     SelectPass<KIND, W, POS> p{a};
-    tile_pass<SEL_WINDOW>(p, recs, tiles, epoch, counters, status, 0ull);
+    if (tile_pass<SEL_WINDOW>(p, recs, tiles, epoch, counters, status, 0ull) && threadIdx.x == 0) {
+        a.host[0] = *a.total;
+        a.host[1] = *reinterpret_cast<volatile unsigned *>(&status->timeout);
+    }
+}
+
+// Few rows: one block, every row in a register (row 32 j + lane of warp w's slice in v[j]), ranked by
+// ballots and one scan of the warps' counts. The tile pass takes 17 us for a thousand rows (its only
+// tile is read row by row, and twice), this one about 3 (calls of 4096 rows 38 -> 19 us).
+constexpr int SEL_SMALL_ITEMS = 16, SEL_SMALL = 1024 * SEL_SMALL_ITEMS;
+
+template <int KIND, int W>
+__global__ void __launch_bounds__(1024) select_small_kernel(SelArgs a, DevStatus *status) {
+    using T = typename Word<W>::T;
+    using O = typename Word<KIND == SEL_WHERE ? 8 : W>::T;
+    constexpr int I = SEL_SMALL_ITEMS;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = static_cast<int>(a.n);
+    const int per = (n + 1023) / 1024 * 32;  // rows of a warp
+    T v[KIND == SEL_WHERE ? 1 : I];
+    unsigned m[I];
+    unsigned char mb[KIND == SEL_FILTER ? 1 : I];
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+        const int r = w * per + j * 32 + lane;
+        const bool in = j * 32 < per && r < n;
+        if (KIND != SEL_WHERE) v[j] = in ? static_cast<const T *>(a.x)[r] : T(0);
+        if (KIND != SEL_FILTER) mb[j] = in ? a.m[r] : 0;
+    }
+    unsigned count = 0;
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+        const bool in = j * 32 < per && w * per + j * 32 + lane < n;
+        bool keep = false;
+        if constexpr (KIND == SEL_FILTER) keep = in && in_range(a.r, static_cast<unsigned long long>(v[j]));
+        else keep = in && mb[j] != 0;
+        m[j] = __ballot_sync(FULL, keep);
+        count += __popc(m[j]);
+    }
+    __shared__ unsigned warp_count[32];
+    if (lane == 0) warp_count[w] = count;
+    __syncthreads();
+    const unsigned mine = warp_count[lane];
+    unsigned inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(FULL, inc, o);
+        if (lane >= o) inc += y;
+    }
+    unsigned at = __shfl_sync(FULL, inc - mine, w);
+    O *out = static_cast<O *>(a.out);
+#pragma unroll
+    for (int j = 0; j < I; ++j) {
+        if ((m[j] >> lane) & 1u) {
+            const unsigned q = at + __popc(m[j] & ((1u << lane) - 1u));
+            if constexpr (KIND == SEL_WHERE) out[q] = static_cast<O>(a.base + w * per + j * 32 + lane);
+            else out[q] = static_cast<O>(v[j]);
+        }
+        at += __popc(m[j]);
+    }
+    if (threadIdx.x == 31) {
+        a.host[0] = inc;
+        a.host[1] = *reinterpret_cast<volatile unsigned *>(&status->timeout);
+    }
 }
 
 template <int KIND, int W>
 static vkc_status run_select(vkc_ctx *ctx, SelArgs a, int64_t n, Builder *b) {
     if (n >= (int64_t(1) << 38)) return fail(ctx, VKC_USAGE, "selection of 2^38 rows or more");
-    const int64_t tiles64 = (n + SEL_TILE - 1) / SEL_TILE;
-    const int tiles = static_cast<int>(tiles64);
-    void *p;
-    unsigned long long *recs;
     vkc_status st;
-    if ((st = scratch(ctx, 256, &p))) return st;
-    if ((st = rec_arena(ctx, tiles, &recs))) return st;
-    a.total = static_cast<unsigned long long *>(p);
-    void *at;
+    void *at, *h;
     if ((st = b->reserve(n, &at))) return st;
+    if ((st = pinned(ctx, 16, &h))) return st;
     a.out = at;
-    const unsigned epoch = next_epoch(ctx);
-    a.aligned = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.m) & 15) == 0;
-    constexpr size_t smem = SEL_SLOTS * SelectPass<KIND, W>::SLOT_BYTES;
-    static std::atomic<unsigned long long> configured{0};
-    once_per_device(configured, ctx->device, [] {
-        cudaFuncSetAttribute(select_kernel<KIND, W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if constexpr (KIND == SEL_FILTER)
-            cudaFuncSetAttribute(select_kernel<KIND, W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-    });
-    bool launched_pos = false;
-    if constexpr (KIND == SEL_FILTER) {
-        if (pos_range(a.r)) {
-            const int grid = tile_pass_grid(ctx, select_kernel<KIND, W, true>, SEL_THREADS + 64, smem, tiles);
-            select_kernel<KIND, W, true><<<grid, SEL_THREADS + 64, smem, ctx->stream>>>(a, tiles, recs, epoch, ctx->counters, ctx->status);
-            launched_pos = true;
+    a.host = static_cast<unsigned long long *>(h);
+    if (n <= SEL_SMALL) {
+        select_small_kernel<KIND, W><<<1, 1024, 0, ctx->stream>>>(a, ctx->status);
+        if ((st = launched(ctx, "select_small"))) return st;
+    } else {
+        const int tiles = static_cast<int>((n + SEL_TILE - 1) / SEL_TILE);
+        void *p;
+        unsigned long long *recs;
+        if ((st = scratch(ctx, 256, &p))) return st;
+        if ((st = rec_arena(ctx, tiles, &recs))) return st;
+        a.total = static_cast<unsigned long long *>(p);
+        const unsigned epoch = next_epoch(ctx);
+        a.aligned = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.m) & 15) == 0;
+        constexpr size_t smem = SEL_SLOTS * SelectPass<KIND, W>::SLOT_BYTES;
+        static std::atomic<unsigned long long> configured{0};
+        once_per_device(configured, ctx->device, [] {
+            cudaFuncSetAttribute(select_kernel<KIND, W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if constexpr (KIND == SEL_FILTER)
+                cudaFuncSetAttribute(select_kernel<KIND, W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        });
+        bool launched_pos = false;
+        if constexpr (KIND == SEL_FILTER) {
+            if (pos_range(a.r)) {
+                const int grid = tile_pass_grid(ctx, select_kernel<KIND, W, true>, SEL_THREADS + 64, smem, tiles);
+                select_kernel<KIND, W, true><<<grid, SEL_THREADS + 64, smem, ctx->stream>>>(a, tiles, recs, epoch, ctx->counters, ctx->status);
+                launched_pos = true;
+            }
         }
+        if (!launched_pos) {
+            const int grid = tile_pass_grid(ctx, select_kernel<KIND, W, false>, SEL_THREADS + 64, smem, tiles);
+            select_kernel<KIND, W, false><<<grid, SEL_THREADS + 64, smem, ctx->stream>>>(a, tiles, recs, epoch, ctx->counters, ctx->status);
+        }
+        if ((st = launched(ctx, "select"))) return st;
     }
-    if (!launched_pos) {
-        const int grid = tile_pass_grid(ctx, select_kernel<KIND, W, false>, SEL_THREADS + 64, smem, tiles);
-        select_kernel<KIND, W, false><<<grid, SEL_THREADS + 64, smem, ctx->stream>>>(a, tiles, recs, epoch, ctx->counters, ctx->status);
-    }
-    if ((st = launched(ctx, "select"))) return st;
-    DevStatus ds;
-    if ((st = read_status(ctx, &ds))) return st;
-    void *h;
-    if ((st = pinned(ctx, 8, &h))) return st;
-    VKC_CUDA(ctx, cudaMemcpyAsync(h, a.total, 8, cudaMemcpyDeviceToHost, ctx->stream));
     VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const unsigned long long k = *static_cast<unsigned long long *>(h);
+    const unsigned long long k = a.host[0];
+    if (a.host[1]) {  // a wait ran out, here or in work enqueued earlier: clear the status word
+        DevStatus ds;
+        if ((st = read_status(ctx, &ds))) return st;
+    }
     // The count can only be at most the rows reserved; anything else is a broken launch.
     if (k > static_cast<unsigned long long>(n))
         return fail(ctx, VKC_DEVICE, "selection returned " + std::to_string(k) + " rows for " +

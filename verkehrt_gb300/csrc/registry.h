@@ -47,6 +47,12 @@ struct ReducerImpl {
     // report, an empty input where that is an error, is decided by the rows the reducer was
     // given, which the host knows.
     virtual vkc_status finish_into(vkc_ctx *ctx, void *dst);
+    // One update with every row and finish, where a reducer can run both in one launch (*done): the
+    // result goes to *out, or with `dst` its bits to that device address, enqueued only.
+    virtual vkc_status once(vkc_ctx *, const Arg *, int, vkc_scalar *, void *, bool *done) {
+        *done = false;
+        return VKC_OK;
+    }
 };
 
 // Scanner (src/kernels.rs:65-88): carried state on the device.

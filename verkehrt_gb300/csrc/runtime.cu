@@ -19,6 +19,7 @@ StreamBox::~StreamBox() {
         for (auto &kv : free_blocks) cudaFreeAsync(kv.second, stream);
         free_blocks.clear();
         cudaStreamSynchronize(stream);
+        if (slots) cudaFreeHost(slots);
         cudaStreamDestroy(stream);
         cudaSetDevice(prev);
     }
@@ -56,8 +57,30 @@ void StreamBox::give(void *p, size_t cls) {
     cudaFreeAsync(p, stream);
 }
 
+void *StreamBox::take_slot() {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!slots && cudaMallocHost(reinterpret_cast<void **>(&slots), RESULT_SLOT * RESULT_SLOTS) != cudaSuccess) {
+        cudaGetLastError();
+        slots = nullptr;
+        return nullptr;
+    }
+    for (int i = 0; i < RESULT_SLOTS; ++i)
+        if (!((slots_used >> i) & 1)) {
+            slots_used |= uint64_t(1) << i;
+            return slots + i * RESULT_SLOT;
+        }
+    return nullptr;
+}
+
+void StreamBox::give_slot(void *slot) {
+    std::lock_guard<std::mutex> lock(mu);
+    slots_used &= ~(uint64_t(1) << ((static_cast<char *>(slot) - slots) / RESULT_SLOT));
+}
+
 DeviceMem::~DeviceMem() {
-    if (ptr && box) cudaFreeAsync(ptr, box->stream);
+    if (!ptr || !box) return;
+    if (cls) box->give(ptr, cls);
+    else cudaFreeAsync(ptr, box->stream);
 }
 
 Buffer::~Buffer() {
@@ -114,6 +137,18 @@ static bool stream_capturing(cudaStream_t stream) {
 static vkc_status copy_streams(vkc_ctx *ctx) {
     if (!ctx->h2d) VKC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
     if (!ctx->d2h) VKC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
+    return VKC_OK;
+}
+
+vkc_status state_block(vkc_ctx *ctx, size_t bytes, DeviceMem *m, bool *captured) {
+    *captured = stream_capturing(ctx->stream);
+    m->box = ctx->box;
+    if (*captured) {
+        VKC_CUDA(ctx, cudaMallocAsync(&m->ptr, bytes, ctx->stream));
+        return VKC_OK;
+    }
+    m->ptr = ctx->box->take(bytes, &m->cls);
+    if (!m->ptr) VKC_CUDA(ctx, cudaMallocAsync(&m->ptr, m->cls, ctx->stream));
     return VKC_OK;
 }
 
@@ -624,11 +659,12 @@ vkc_status vkc_tune_get(const vkc_ctx *ctx, const char *knob, int size_class, in
 }
 
 vkc_status vkc_synchronize(vkc_ctx *ctx) {
-    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const bool capturing = stream_capturing(ctx->stream);
+    if (capturing) VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if (ctx->h2d) VKC_CUDA(ctx, cudaStreamSynchronize(ctx->h2d));
     if (ctx->d2h) VKC_CUDA(ctx, cudaStreamSynchronize(ctx->d2h));
-    if (stream_capturing(ctx->stream)) return VKC_OK;
-    DevStatus ds;
+    if (capturing) return VKC_OK;
+    DevStatus ds;  // waits for the context stream
     return read_status(ctx, &ds);
 }
 
@@ -683,8 +719,8 @@ vkc_status vkc_array_download(vkc_ctx *ctx, const vkc_array *a, void *host, int6
     if (n > 0)
         VKC_CUDA(ctx, cudaMemcpyAsync(host, a->data(), static_cast<size_t>(n) * type_width(a->type),
                                       cudaMemcpyDeviceToHost, ctx->stream));
-    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    // A wait of earlier enqueued work that ran out (its call did not wait for the device).
+    // Waits for the copy; and a wait of earlier enqueued work that ran out (its call did not wait
+    // for the device).
     DevStatus ds;
     return read_status(ctx, &ds);
 }
@@ -834,9 +870,13 @@ vkc_status vkc_call(vkc_ctx *ctx, int id, const vkc_value *args, int nargs, vkc_
         if (rows < 0) return fail(ctx, VKC_USAGE, "a reduction needs an array operand");
         ReducerImpl *r = d->red(ctx);
         if (!r) return ctx->err.empty() ? fail(ctx, VKC_ALLOC, "cannot allocate a reducer") : VKC_ALLOC;
-        if (rows > 0) st = r->update(ctx, call.data(), nargs);
         vkc_scalar s{};
-        if (!st) st = r->finish(ctx, &s);
+        bool done = false;
+        if (rows > 0) st = r->once(ctx, call.data(), nargs, &s, nullptr, &done);
+        if (!done) {
+            if (!st && rows > 0) st = r->update(ctx, call.data(), nargs);
+            if (!st) st = r->finish(ctx, &s);
+        }
         delete r;
         if (st) return st;
         out->kind = VKC_VALUE_SCALAR;
@@ -939,8 +979,13 @@ vkc_status vkc_call_into(vkc_ctx *ctx, int id, const vkc_value *args, int nargs,
     ReducerImpl *r = d->red(ctx);
     if (!r) return ctx->err.empty() ? fail(ctx, VKC_ALLOC, "cannot allocate a reducer") : VKC_ALLOC;
     // As vkc_call: one update with all rows, none on empty input.
-    if (rows > 0) st = r->update(ctx, call.data(), nargs);
-    if (!st) st = r->finish_into(ctx, static_cast<char *>(out->data()) + row * type_width(out->type));
+    void *dst = static_cast<char *>(out->data()) + row * type_width(out->type);
+    bool done = false;
+    if (rows > 0) st = r->once(ctx, call.data(), nargs, nullptr, dst, &done);
+    if (!done) {
+        if (!st && rows > 0) st = r->update(ctx, call.data(), nargs);
+        if (!st) st = r->finish_into(ctx, dst);
+    }
     delete r;
     return st;
 }

@@ -50,6 +50,10 @@ struct StreamBox {
     size_t cached = 0;
     size_t limit = size_t(48) << 30;  // cached bytes at most (vkc_set_cache_limit)
     std::mutex mu;
+    // Pinned host slots of RESULT_SLOT bytes for results that kernels write themselves (made on
+    // first use, freed with the box): bit i of slots_used is set while slot i is taken.
+    char *slots = nullptr;
+    uint64_t slots_used = 0;
     ~StreamBox();
     // A block of at least `bytes` (its class size in *cls), or nullptr.
     void *take(size_t bytes, size_t *cls);
@@ -57,7 +61,11 @@ struct StreamBox {
     void give(void *p, size_t cls);
     // Frees every cached block.
     void release_all();
+    // A free result slot, or nullptr when all are taken.
+    void *take_slot();
+    void give_slot(void *slot);
 };
+constexpr int RESULT_SLOT = 64, RESULT_SLOTS = 64;
 
 // The size class of an allocation: 256-byte multiples below 1 MiB, then 2 MiB multiples.
 inline size_t size_class(size_t bytes) {
@@ -65,9 +73,11 @@ inline size_t size_class(size_t bytes) {
     return (bytes + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
 }
 
-// A device allocation freed stream-ordered on its context's stream, whenever it goes.
+// A device allocation freed stream-ordered on its context's stream, whenever it goes (into the
+// box's cache when it has a size class).
 struct DeviceMem {
     void *ptr = nullptr;
+    size_t cls = 0;
     std::shared_ptr<StreamBox> box;
     ~DeviceMem();
 };
@@ -209,6 +219,11 @@ vkc_status launched(vkc_ctx *ctx, const char *what);
 // New array of `len` rows (uninitialised unless `zero`). Message texts follow
 // src/value.rs:285-307.
 vkc_status new_array(vkc_ctx *ctx, vkc_type t, int64_t len, bool zero, vkc_array **out);
+// A device block for a small state (uninitialised), from the box's cache where that is possible: a
+// block taken while a graph is captured belongs to the graph's replays, so it is the graph's own
+// allocation then. *captured tells which.
+vkc_status state_block(vkc_ctx *ctx, size_t bytes, DeviceMem *m, bool *captured);
+
 // Shrinks an array's logical length (the allocation stays).
 inline void set_len(vkc_array *a, int64_t len) { a->len = len; }
 
