@@ -124,35 +124,17 @@ __device__ __forceinline__ TF compose(TF a, TF b) {
     return TF{sat_add(au, bu), sat_add(ad, bd) | SIGNED_TF};
 }
 
-// Applies f (valid in binade E) to the lane state with bits s. Fails when |s| is not a normal
-// in binade E or when a state on the way could leave the binade. A negative state is the
-// mirror image: round-to-nearest-even is symmetric, so its magnitude moves by the negated
-// increments (only for functions without a parity dependence). A signed function keeps every
-// state on the way at least one ulp above 2^E, so each exact sum lies in the binade.
-// SIGNED = false: positive states and unsigned functions only (fails otherwise).
-template <bool SIGNED = true>
-__device__ __forceinline__ bool apply(unsigned long long s, int E, TF f, unsigned long long *out) {
+// Applies the unsigned function f (valid in binade E) to the lane state with bits s. Fails when s is
+// not a positive normal in binade E or would leave it. (Signed functions and negative states:
+// apply_prefix, whose moves are the mirror image for a negative state, as round-to-nearest-even is
+// symmetric, and keep every state on the way at least one ulp above 2^E, so that each exact sum lies in
+// the binade.)
+__device__ __forceinline__ bool apply_positive(unsigned long long s, int E, TF f, unsigned long long *out) {
     const unsigned long long ef = static_cast<unsigned long long>(E + 1023);
-    const unsigned long long neg = SIGNED ? s >> 63 : 0;
-    if (!SIGNED && (s >> 63)) return false;
-    if (((s >> 52) & 0x7ff) != ef) return false;
-    const unsigned long long S = (s & MANT) | ONE52;
-    unsigned long long S2;
-    if (!SIGNED || (!neg && !(f.d1 & SIGNED_TF))) {
-        S2 = S + ((S & 1) ? f.d1 : f.d0);
-        if (S2 >= (ONE52 << 1)) return false;
-    } else {
-        unsigned long long up, dn;
-        if (!as_signed(f, &up, &dn)) return false;
-        if (neg) {
-            const unsigned long long x = up;
-            up = dn;
-            dn = x;
-        }
-        if (up >= ONE52 || dn >= ONE52 || S + up >= (ONE52 << 1) || (dn && S - dn <= ONE52)) return false;
-        S2 = S + up - dn;
-    }
-    *out = (neg << 63) | (ef << 52) | (S2 & MANT);
+    if ((s >> 52) != ef) return false;
+    const unsigned long long S = (s & MANT) | ONE52, S2 = S + ((S & 1) ? f.d1 : f.d0);
+    if (S2 >= (ONE52 << 1)) return false;
+    *out = (ef << 52) | (S2 & MANT);
     return true;
 }
 
@@ -311,7 +293,8 @@ struct CanonWork {
     int *chunkE;               // [16][C] binade of each 32-tile chunk's transfer function
     TF *chunkD;                // [16][C]
     double *gsum;              // [16][G] approximate sum of each group of CAND_GROUP tiles
-    int *flags;                // [T] tiles whose transfer functions are recomputed (K3 again);
+    bool listed = false;       // K3 lists the tiles with negative rows itself (no check follows)
+    int *flags = nullptr;      // [T] tiles whose transfer functions are recomputed (K3 again);
                                // [T]: some tile has a negative row; [T + 1]: the number of
                                // flagged tiles, listed from [T + 2]
     unsigned long long *tstate = nullptr;  // scans: [16][T + 1] exact lane state before each tile
@@ -435,6 +418,62 @@ __global__ void __launch_bounds__(CT_THREADS) canon_apx_kernel(RowArgs args, int
     }
 }
 
+// K1 of shorter inputs (T <= FULL_TILES): the approximate lane sums from every row. The sums then lie
+// within a few float roundings of the exact ones, far inside the candidates' margin, so the check
+// (K2c, K3 on the flagged tiles) is left out: it took five launches, about 35 us, where the whole
+// first read takes at most 20 (and the second comes from L2 up to about 2^23 rows).
+constexpr int FULL_TILES = 4096;
+
+template <int OP, bool ALIGNED>
+__global__ void __launch_bounds__(CT_THREADS) canon_sums_kernel(RowArgs args, int64_t nb, int T, CanonWork wk) {
+    __shared__ float part[CT_THREADS / 32][16];
+    const int t = threadIdx.x, lp = t & 7, seg = t >> 3, tile = blockIdx.x;
+    if (tile == 0 && t < 2) wk.flags[T + t] = 0;  // no negative row yet, no tile listed
+    unsigned long long x[CT_SEG_BLOCKS][2], y[CT_SEG_BLOCKS][2];
+#pragma unroll
+    for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
+        const int64_t b = static_cast<int64_t>(tile) * CT_BLOCKS + seg * CT_SEG_BLOCKS + i, r = b * 16 + 2 * lp;
+        x[i][0] = x[i][1] = y[i][0] = y[i][1] = 0;
+        if (b < nb) {
+            if (ALIGNED) {
+                const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2 *>(args.x + r));
+                x[i][0] = v.x;
+                x[i][1] = v.y;
+                if (OP == ROW_DOT) {
+                    const ulonglong2 u = __ldg(reinterpret_cast<const ulonglong2 *>(args.y + r));
+                    y[i][0] = u.x;
+                    y[i][1] = u.y;
+                }
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    x[i][h] = __ldg(args.x + r + h);
+                    if (OP == ROW_DOT) y[i][h] = __ldg(args.y + r + h);
+                }
+            }
+        }
+    }
+    float s[2] = {0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
+        const bool in = static_cast<int64_t>(tile) * CT_BLOCKS + seg * CT_SEG_BLOCKS + i < nb;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) s[h] += in ? approx_row<OP>(args, x[i][h], y[i][h]) : 0.f;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        s[h] += __shfl_xor_sync(FULL, s[h], 8);
+        s[h] += __shfl_xor_sync(FULL, s[h], 16);
+        if ((t & 31) < 8) part[t >> 5][2 * lp + h] = s[h];
+    }
+    __syncthreads();
+    if (t < 16) {
+        float a = 0.f;
+        for (int w = 0; w < CT_THREADS / 32; ++w) a += part[w][t];
+        wk.apx[static_cast<int64_t>(t) * T + tile] = a;
+    }
+}
+
 // K2a: per lane and group of CAND_GROUP tiles (one block each), the approximate sum of the
 // group's tiles.
 __global__ void __launch_bounds__(256) canon_gsum_kernel(int T, int G, CanonWork wk) {
@@ -463,10 +502,12 @@ constexpr int CAND_THREADS = 256;
 constexpr int CAND_PER = CAND_GROUP / CAND_THREADS;
 
 // CHECK (K2c, after K3 and the refined sums of canon_refine_kernel): a tile whose new
-// candidates include a binade that its K3 candidates did not gets the new ones and a flag.
-template <bool CHECK>
-__global__ void __launch_bounds__(CAND_THREADS) canon_cand_kernel(int T, int G, CanonWork wk, const CanonState *state) {
+// candidates include a binade that its K3 candidates did not gets the new ones and a flag. FULL (few
+// groups): the groups before this one are summed here, not by K2a.
+template <bool CHECK, bool FULL_SUMS>
+__global__ void __launch_bounds__(CAND_THREADS) canon_cand_kernel(int T, int G, CanonWork wk, bool fresh, const CanonState *state) {
     __shared__ double s_base;
+    __shared__ double s_before[CAND_THREADS / 32];
     const int L = blockIdx.x / G, g = blockIdx.x % G, t = threadIdx.x;
     const int k0 = g * CAND_GROUP + t * CAND_PER;
     const float *apx = wk.apx + static_cast<int64_t>(L) * T;
@@ -476,11 +517,22 @@ __global__ void __launch_bounds__(CAND_THREADS) canon_cand_kernel(int T, int G, 
         a[j] = k0 + j < T ? apx[k0 + j] : 0.f;
         tot += a[j];
     }
-    if (t < 32) {
+    const double from = fresh ? 0.0 : as_f64(state->lanes[L]);
+    if (FULL_SUMS) {
+        double b = 0.0;
+        for (int k = t; k < g * CAND_GROUP; k += CAND_THREADS) b += static_cast<double>(apx[k]);
+        b = warp_sum(b);
+        if ((t & 31) == 0) s_before[t >> 5] = b;
+        __syncthreads();
+        if (t == 0) {
+            for (int w = 1; w < CAND_THREADS / 32; ++w) b += s_before[w];
+            s_base = from + b;
+        }
+    } else if (t < 32) {
         double b = 0.0;
         for (int i = t; i < g; i += 32) b += wk.gsum[L * G + i];
         b = warp_sum(b);
-        if (t == 0) s_base = as_f64(state->lanes[L]) + b;
+        if (t == 0) s_base = from + b;
     }
     float total;
     float run = block_exclusive_sum<float>(tot, &total);  // synchronises the block
@@ -613,7 +665,8 @@ __device__ __forceinline__ void tf_tile(const RowArgs &args, int64_t nb, int T, 
     if (__syncthreads_or(sgn)) {  // also the barrier after s_E
         if (!FLAGGED) {
             if (t == 0) {
-                wk.flags[tile] = 2;
+                if (wk.listed) wk.flags[T + 2 + atomicAdd(&wk.flags[T + 1], 1)] = tile;
+                else wk.flags[tile] = 2;
                 wk.flags[T] = 1;  // some tile has a negative row
             }
             if (t < 32) wk.recE[(static_cast<int64_t>(t & 15) * T + tile) * 2 + (t >> 4)] = NO_E;
@@ -779,17 +832,60 @@ __device__ __forceinline__ int state_binade(unsigned long long s) {
 // Inclusive ordered prefix composition over the warp (lane 0 first), then the number of
 // leading lanes whose prefix applies to state s (usable and inside the binade). Returns that
 // count and, in *out, the state after them.
+//
+// SIGNED: every function as the move of the state's magnitude from an even and an odd start and the
+// bounds of the moves on the way, so that one composition without branches serves signed functions,
+// unsigned ones and ties (composing TFs as such, with both kinds in a warp, took about 4000 cycles a
+// call, and the walk of 2^27 rows of u - 1/4 1.0 ms, slow enough to hand some lanes to the chain).
+struct Move {
+    long long d0, d1, mn, mx;
+};
+
 template <bool SIGNED = true>
 __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long long s, int E,
                                             unsigned long long *out, unsigned long long *mine = nullptr) {
     const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        TF y = shfl_up_tf(f, o);
-        if (lane >= o) f = compose<SIGNED>(y, f);
-    }
     unsigned long long r = 0;
-    const bool ok = usable && apply<SIGNED>(s, E, f, &r);
+    bool ok = usable;
+    if constexpr (SIGNED) {
+        const bool neg = (s >> 63) != 0;
+        const unsigned long long up = f.d0, dn = (f.d1 & SIGNED_TF) ? f.d1 & ~SIGNED_TF : 0ull;
+        const bool parity = !(f.d1 & SIGNED_TF) && f.d0 != f.d1;  // only for states as the rows: not negative
+        ok = ok && max(up, parity ? f.d1 : dn) < (ONE52 << 1) && !(parity && neg);
+        Move m{0, 0, 0, 0};
+        if (ok) {
+            const long long u = static_cast<long long>(up), d = static_cast<long long>(dn);
+            m.d0 = neg ? d - u : u - d;
+            m.d1 = parity ? static_cast<long long>(f.d1) : m.d0;
+            m.mn = neg ? -u : -d;
+            m.mx = neg ? d : max(u, parity ? m.d1 : 0ll);
+        }
+        const bool ties = __any_sync(FULL, m.d0 != m.d1);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            Move a{__shfl_up_sync(FULL, m.d0, o), 0, __shfl_up_sync(FULL, m.mn, o), __shfl_up_sync(FULL, m.mx, o)};
+            a.d1 = ties ? __shfl_up_sync(FULL, m.d1, o) : a.d0;
+            if (lane >= o) {
+                m.mn = min(a.mn, min(a.d0, a.d1) + m.mn);
+                m.mx = max(a.mx, max(a.d0, a.d1) + m.mx);
+                const long long n0 = a.d0 + ((a.d0 & 1) ? m.d1 : m.d0);
+                m.d1 = a.d1 + ((a.d1 & 1) ? m.d0 : m.d1);
+                m.d0 = n0;
+            }
+        }
+        const unsigned long long ef = static_cast<unsigned long long>(E + 1023);
+        const long long S = static_cast<long long>((s & MANT) | ONE52);
+        ok = ok && ((s >> 52) & 0x7ff) == ef && S + m.mx < static_cast<long long>(ONE52 << 1) &&
+             (m.mn >= 0 || S + m.mn > static_cast<long long>(ONE52));
+        r = (s & (1ull << 63)) | (ef << 52) | (static_cast<unsigned long long>(S + ((S & 1) ? m.d1 : m.d0)) & MANT);
+    } else {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            TF y = shfl_up_tf(f, o);
+            if (lane >= o) f = compose<false>(y, f);
+        }
+        ok = ok && apply_positive(s, E, f, &r);
+    }
     if (mine) *mine = r;  // this lane's state (valid below the returned count)
     const unsigned bad = __ballot_sync(FULL, !ok);
     const int m = bad ? __ffs(bad) - 1 : 32;
@@ -799,14 +895,21 @@ __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long lon
 
 // Resolves tile `tp` for lane L from the state s: the warp recomputes the tile's 32 segment
 // transfer functions from the rows (lane j = segment j) for the state's binade and the next,
-// applies them in order, and adds the rows of any segment they do not carry one by one.
+// applies them in order, and adds the rows of any segment they do not carry one by one. `held`: the
+// row values in shared memory (WalkSmem), or nullptr.
 template <int OP, bool SIGNED>
-__device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int tp, int L, unsigned long long s) {
+__device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int tp, int L, unsigned long long s,
+                                           const unsigned long long *held) {
     const int lane = threadIdx.x & 31;
     unsigned long long v[CT_SEG_BLOCKS][2];
     const int64_t blk0 = static_cast<int64_t>(tp) * CT_BLOCKS + lane * CT_SEG_BLOCKS;
 #pragma unroll
     for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
+        if (held) {
+            v[i][0] = held[i * 32 + lane];
+            v[i][1] = 0;
+            continue;
+        }
         int64_t b = blk0 + i;
         unsigned long long xv = 0, yv = 0;
         if (b < nb) {
@@ -856,8 +959,9 @@ __device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int 
 // tiles inside mixed chunks, and resolves from the rows the tiles that none carries (binade
 // crossings, negative or special rows, the first rows of the lane).
 constexpr int WK_THREADS = 256;
-constexpr int WK_MAX_CHUNKS = 4096;  // chunk records held in shared memory
+constexpr int WK_MAX_CHUNKS = 2048;  // chunk records held in shared memory (2^28 rows)
 constexpr int WK_MAX_MIXED = 48;     // mixed chunks whose tile records are held there
+constexpr int WK_MAX_ROWS = 40;      // tiles whose rows are held there: those likely to be resolved
 
 // The walk's progress over windows of the SM clock: a window in which it advanced fewer tiles
 // than the lane chain would (WALK_MIN_TILES in WALK_WINDOW cycles, about 2 tiles a microsecond)
@@ -886,7 +990,10 @@ struct WalkSmem {
     int chunk_of[WK_MAX_MIXED];
     int mE[WK_MAX_MIXED][32][2];
     TF mD[WK_MAX_MIXED][32][2];
-    int nmixed;
+    unsigned long long rows[WK_MAX_ROWS][CT_BLOCKS];  // row values, row r at (r % 8) * 32 + r / 8
+    int tile_of[WK_MAX_ROWS];
+    short rows_of[WK_MAX_MIXED][32];
+    int nmixed, nrows;
 };
 
 // Chunk k of lane L tile by tile from state s (one warp): runs of tiles whose transfer
@@ -937,7 +1044,8 @@ __device__ __forceinline__ unsigned long long walk_chunk_tiles(const RowArgs &ar
             s = r;
             tp += mt;
         } else {
-            s = resolve_tile<OP, SIGNED>(args, nb, tp, L, s);
+            const int q = slot >= 0 ? sm->rows_of[slot][tp - k * 32] : -1;
+            s = resolve_tile<OP, SIGNED>(args, nb, tp, L, s, q >= 0 ? sm->rows[q] : nullptr);
             ++tp;
         }
     }
@@ -996,14 +1104,14 @@ __device__ __forceinline__ unsigned long long walk_lane(const RowArgs &args, int
 
 template <int OP, bool RECORD>
 __global__ void __launch_bounds__(WK_THREADS) canon_walk_kernel(RowArgs args, int64_t nb, int T, int C, CanonWork wk,
-                                                                CanonState *state) {
+                                                                bool fresh, CanonState *state) {
     extern __shared__ __align__(16) unsigned char walk_smem[];
     WalkSmem &sm = *reinterpret_cast<WalkSmem *>(walk_smem);
     const int L = blockIdx.x, t = threadIdx.x;
     const bool held = C <= WK_MAX_CHUNKS;
     const int *gE = wk.chunkE + static_cast<int64_t>(L) * C;
     const TF *gD = wk.chunkD + static_cast<int64_t>(L) * C;
-    if (t == 0) sm.nmixed = 0;
+    if (t == 0) sm.nmixed = sm.nrows = 0;
     __syncthreads();
     if (held) {
         for (int c = t; c < C; c += WK_THREADS) {
@@ -1037,12 +1145,36 @@ __global__ void __launch_bounds__(WK_THREADS) canon_walk_kernel(RowArgs args, in
             }
             sm.mE[slot][j][cand] = e;
             sm.mD[slot][j][cand] = d;
+            if (cand == 0) {
+                // No function, or a second candidate binade: the sum crosses in or near this tile.
+                short q = -1;
+                if (tp < T && (e == NO_E || wk.cand[(static_cast<int64_t>(tp) * 16 + L) * 2 + 1] != NO_E)) {
+                    const int k = atomicAdd(&sm.nrows, 1);
+                    if (k < WK_MAX_ROWS) {
+                        q = static_cast<short>(k);
+                        sm.tile_of[k] = tp;
+                    }
+                }
+                sm.rows_of[slot][j] = q;
+            }
+        }
+        __syncthreads();
+        // The rows of those tiles, all in flight at once (a walk that loaded each tile's when it came
+        // to it waited a DRAM round trip per crossing).
+        static_assert(WK_THREADS == CT_BLOCKS, "a thread per row of a lane's tile");
+        const int nr = min(sm.nrows, WK_MAX_ROWS);
+#pragma unroll 8
+        for (int k = 0; k < nr; ++k) {
+            const int64_t b = static_cast<int64_t>(sm.tile_of[k]) * CT_BLOCKS + t;
+            unsigned long long v = 0;
+            if (b < nb) v = row_value<OP>(args, args.x[b * 16 + L], OP == ROW_DOT ? args.y[b * 16 + L] : 0ull);
+            sm.rows[k][(t % CT_SEG_BLOCKS) * 32 + t / CT_SEG_BLOCKS] = v;
         }
     }
     __syncthreads();
     if (t >= 32) return;
     const int lane = t;
-    unsigned long long s = state->lanes[L];
+    unsigned long long s = fresh ? 0ull : state->lanes[L];
     int stop = -1;
     s = (wk.flags[T] != 0 || (s >> 63)) ? walk_lane<OP, true, RECORD>(args, nb, T, C, wk, sm, held, gE, gD, L, s, &stop)
                                         : walk_lane<OP, false, RECORD>(args, nb, T, C, wk, sm, held, gE, gD, L, s, &stop);
@@ -1187,9 +1319,8 @@ template <int OP, int ROWS> constexpr size_t chain_smem() {
 }
 
 template <int OP, int ROWS>
-__global__ void __launch_bounds__(32) canon_chain_kernel(RowArgs args, int64_t nb, int T, CanonWork wk,
-                                                         CanonState *state) {
-    extern __shared__ __align__(16) unsigned long long chain_smem_buf[];
+__device__ __forceinline__ void chain_lane(const RowArgs &args, int64_t nb, int T, const CanonWork &wk, CanonState *state,
+                                           unsigned long long *chain_smem_buf) {
     constexpr int NA = OP == ROW_DOT ? 2 : 1;
     constexpr int STEP = 32 * ROWS, PITCH = ROWS + 1;
     const int L = blockIdx.x, j = threadIdx.x;
@@ -1336,29 +1467,61 @@ __global__ void __launch_bounds__(32) canon_chain_kernel(RowArgs args, int64_t n
     if (j == 0) state->lanes[L] = s;
 }
 
+// One warp per lane. With `result` (the input is the whole sum's) the last block also combines the
+// lanes and folds the `rest` tail rows in (finish_lanes), which saves two launches.
+template <int OP, int ROWS>
+__global__ void __launch_bounds__(32) canon_chain_kernel(RowArgs args, int64_t nb, int T, CanonWork wk, CanonState *state,
+                                                         int rest, unsigned *done, unsigned long long *result) {
+    extern __shared__ __align__(16) unsigned long long chain_smem_buf[];
+    chain_lane<OP, ROWS>(args, nb, T, wk, state, chain_smem_buf);
+    if (!result || !last_block(done)) return;
+    const int j = threadIdx.x;
+    double s = j < 16 ? as_f64(*reinterpret_cast<volatile unsigned long long *>(&state->lanes[j])) : 0.0;
+    const int64_t r = nb * 16 + j;
+    const double v = j < rest ? as_f64(row_value<OP>(args, args.x[r], OP == ROW_DOT ? args.y[r] : 0ull)) : 0.0;
+#pragma unroll
+    for (int step = 8; step > 0; step >>= 1) {
+        const double other = __shfl_down_sync(FULL, s, step);
+        if (j < step) s = __dadd_rn(s, other);
+    }
+    for (int i = 0; i < rest; ++i) s = __dadd_rn(s, __shfl_sync(FULL, v, i));
+    if (j == 0) *result = as_bits(s);
+}
+
 // RECORD (scans): the walk also stores the exact lane state before every tile in wk.tstate.
+// `result`: the whole sum's bits go there, the rest rows included.
 template <int OP, bool ALIGNED, bool RECORD = false>
-static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T, int C, const CanonWork &wk,
-                               CanonState *state) {
+static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T, int C, const CanonWork &wk, bool fresh,
+                               CanonState *state, int rest = 0, unsigned long long *result = nullptr) {
     vkc_status st;
-    canon_apx_kernel<OP, ALIGNED><<<(T + APX_TILES - 1) / APX_TILES, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
-    if ((st = launched(ctx, "canon_apx"))) return st;
     const int G = (T + CAND_GROUP - 1) / CAND_GROUP;
-    canon_gsum_kernel<<<16 * G, 256, 0, ctx->stream>>>(T, G, wk);
-    if ((st = launched(ctx, "canon_gsum"))) return st;
-    canon_cand_kernel<false><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, state);
-    if ((st = launched(ctx, "canon_cand"))) return st;
-    VKC_CUDA(ctx, cudaMemsetAsync(wk.flags, 0, static_cast<size_t>(T + 2) * sizeof(int), ctx->stream));
-    canon_tf_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
-    if ((st = launched(ctx, "canon_tf"))) return st;
-    // The check of the sampled candidates: K3's sums, the prefixes again, K3 again on the tiles
-    // whose binades the first candidates missed and on the tiles with negative rows.
-    canon_refine_kernel<<<static_cast<int>((16 * static_cast<int64_t>(T) + 255) / 256), 256, 0, ctx->stream>>>(T, wk);
-    canon_gsum_kernel<<<16 * G, 256, 0, ctx->stream>>>(T, G, wk);
-    canon_cand_kernel<true><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, state);
-    canon_flag_list_kernel<<<std::min(T / 256 + 1, 1024), 256, 0, ctx->stream>>>(T, wk);
+    if (wk.listed) {
+        canon_sums_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+        if ((st = launched(ctx, "canon_sums"))) return st;
+        canon_cand_kernel<false, true><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, fresh, state);
+        if ((st = launched(ctx, "canon_cand"))) return st;
+        canon_tf_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+        if ((st = launched(ctx, "canon_tf"))) return st;
+    } else {
+        canon_apx_kernel<OP, ALIGNED><<<(T + APX_TILES - 1) / APX_TILES, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+        if ((st = launched(ctx, "canon_apx"))) return st;
+        canon_gsum_kernel<<<16 * G, 256, 0, ctx->stream>>>(T, G, wk);
+        if ((st = launched(ctx, "canon_gsum"))) return st;
+        canon_cand_kernel<false, false><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, fresh, state);
+        if ((st = launched(ctx, "canon_cand"))) return st;
+        VKC_CUDA(ctx, cudaMemsetAsync(wk.flags, 0, static_cast<size_t>(T + 2) * sizeof(int), ctx->stream));
+        canon_tf_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+        if ((st = launched(ctx, "canon_tf"))) return st;
+        // The check of the sampled candidates: K3's sums, the prefixes again, K3 again on the tiles
+        // whose binades the first candidates missed and on the tiles with negative rows.
+        canon_refine_kernel<<<static_cast<int>((16 * static_cast<int64_t>(T) + 255) / 256), 256, 0, ctx->stream>>>(T, wk);
+        canon_gsum_kernel<<<16 * G, 256, 0, ctx->stream>>>(T, G, wk);
+        canon_cand_kernel<true, false><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, fresh, state);
+        canon_flag_list_kernel<<<std::min(T / 256 + 1, 1024), 256, 0, ctx->stream>>>(T, wk);
+        if ((st = launched(ctx, "canon_check"))) return st;
+    }
     canon_tf_flagged_kernel<OP, ALIGNED><<<std::min(T, 4 * ctx->sms), CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
-    if ((st = launched(ctx, "canon_check"))) return st;
+    if ((st = launched(ctx, "canon_tf_flagged"))) return st;
     int warps = 16 * C;
     canon_chunk_kernel<<<(warps + 7) / 8, 256, 0, ctx->stream>>>(T, C, wk);
     if ((st = launched(ctx, "canon_chunk"))) return st;
@@ -1368,7 +1531,7 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
                              static_cast<int>(sizeof(WalkSmem)));
     });
     if constexpr (RECORD) VKC_CUDA(ctx, cudaMemsetAsync(wk.whole, 0, static_cast<size_t>(C) * 16 * sizeof(int), ctx->stream));
-    canon_walk_kernel<OP, RECORD><<<16, WK_THREADS, sizeof(WalkSmem), ctx->stream>>>(a, nb, T, C, wk, state);
+    canon_walk_kernel<OP, RECORD><<<16, WK_THREADS, sizeof(WalkSmem), ctx->stream>>>(a, nb, T, C, wk, fresh, state);
     if ((st = launched(ctx, "canon_walk"))) return st;
     if constexpr (!RECORD) {
         static std::atomic<unsigned long long> chain_configured{0};
@@ -1380,10 +1543,11 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
             cudaFuncSetAttribute(canon_chain_kernel<OP, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(chain_smem<OP, 16>()));
         });
+        unsigned *done = ctx->counters + 1;
         switch (tune(ctx, TK_CHAIN_ROWS, nb * 16)) {
-        case 4: canon_chain_kernel<OP, 4><<<16, 32, chain_smem<OP, 4>(), ctx->stream>>>(a, nb, T, wk, state); break;
-        case 16: canon_chain_kernel<OP, 16><<<16, 32, chain_smem<OP, 16>(), ctx->stream>>>(a, nb, T, wk, state); break;
-        default: canon_chain_kernel<OP, 8><<<16, 32, chain_smem<OP, 8>(), ctx->stream>>>(a, nb, T, wk, state); break;
+        case 4: canon_chain_kernel<OP, 4><<<16, 32, chain_smem<OP, 4>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
+        case 16: canon_chain_kernel<OP, 16><<<16, 32, chain_smem<OP, 16>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
+        default: canon_chain_kernel<OP, 8><<<16, 32, chain_smem<OP, 8>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
         }
         if ((st = launched(ctx, "canon_chain"))) return st;
     }
@@ -1417,7 +1581,7 @@ static size_t canon_layout(int T, int C, bool scan, char *b, CanonWork *wk, Cano
         *wk = CanonWork{reinterpret_cast<float *>(b), reinterpret_cast<int *>(b + o_cand),
                         reinterpret_cast<int *>(b + o_recE), reinterpret_cast<TF *>(b + o_recD),
                         reinterpret_cast<int *>(b + o_chE), reinterpret_cast<TF *>(b + o_chD),
-                        reinterpret_cast<double *>(b + o_gs), reinterpret_cast<int *>(b + o_fl)};
+                        reinterpret_cast<double *>(b + o_gs), T <= FULL_TILES, reinterpret_cast<int *>(b + o_fl)};
         if (!scan) wk->resume = reinterpret_cast<int *>(b + o_rs);
         if (scan) {
             wk->tstate = reinterpret_cast<unsigned long long *>(b + o_ts);
@@ -1489,30 +1653,10 @@ struct CanonReducer : DevReducer {
         const int rest = static_cast<int>(n % 16);
         auto *cs = static_cast<CanonState *>(state);
         if (n == 0) return VKC_OK;
-        if (nb <= CANON_SEQ_BLOCKS) {
-            tail_len = rest;
-            return seq(ctx, a, n, nullptr);
-        }
-        if (fresh && (st = zero(ctx))) return st;
-        {
-            const int64_t T64 = (nb + CT_BLOCKS - 1) / CT_BLOCKS;
-            if (T64 > (int64_t(1) << 26)) return fail(ctx, VKC_USAGE, "array too long for one update");
-            const int T = static_cast<int>(T64), C = (T + 31) / 32;
-            void *p;
-            if ((st = scratch(ctx, canon_layout(T, C, false, nullptr, nullptr, nullptr), &p))) return st;
-            CanonWork wk;
-            canon_layout(T, C, false, static_cast<char *>(p), &wk, nullptr);
-            const bool aligned = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 &&
-                                 (op != ROW_DOT || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0);
-            switch (op) {
-            case ROW_SUM: st = aligned ? launch_canon<ROW_SUM, true>(ctx, a, nb, T, C, wk, cs) : launch_canon<ROW_SUM, false>(ctx, a, nb, T, C, wk, cs); break;
-            case ROW_DOT: st = aligned ? launch_canon<ROW_DOT, true>(ctx, a, nb, T, C, wk, cs) : launch_canon<ROW_DOT, false>(ctx, a, nb, T, C, wk, cs); break;
-            case ROW_SUMSQ: st = aligned ? launch_canon<ROW_SUMSQ, true>(ctx, a, nb, T, C, wk, cs) : launch_canon<ROW_SUMSQ, false>(ctx, a, nb, T, C, wk, cs); break;
-            default: st = aligned ? launch_canon<ROW_CONDSUM, true>(ctx, a, nb, T, C, wk, cs) : launch_canon<ROW_CONDSUM, false>(ctx, a, nb, T, C, wk, cs); break;
-            }
-            if (st) return st;
-        }
-        if (rest > 0) {
+        tail_len = rest;
+        if (nb <= CANON_SEQ_BLOCKS) return seq(ctx, a, n, nullptr);
+        st = tiles(ctx, a, nb, 0, nullptr);
+        if (!st && rest > 0) {
             const int64_t first = nb * 16;
             switch (op) {
             case ROW_SUM: canon_tail<ROW_SUM><<<1, 16, 0, ctx->stream>>>(a, first, rest, cs); break;
@@ -1520,20 +1664,42 @@ struct CanonReducer : DevReducer {
             case ROW_SUMSQ: canon_tail<ROW_SUMSQ><<<1, 16, 0, ctx->stream>>>(a, first, rest, cs); break;
             default: canon_tail<ROW_CONDSUM><<<1, 16, 0, ctx->stream>>>(a, first, rest, cs); break;
             }
-            if ((st = launched(ctx, "canon_tail"))) return st;
-            tail_len = rest;
+            st = launched(ctx, "canon_tail");
+        }
+        return st;
+    }
+    // The tile passes over nb blocks; with `result` the rest rows and the finish too.
+    vkc_status tiles(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int rest, unsigned long long *result) {
+        vkc_status st;
+        auto *cs = static_cast<CanonState *>(state);
+        const int64_t T64 = (nb + CT_BLOCKS - 1) / CT_BLOCKS;
+        if (T64 > (int64_t(1) << 26)) return fail(ctx, VKC_USAGE, "array too long for one update");
+        const int T = static_cast<int>(T64), C = (T + 31) / 32;
+        void *p;
+        if ((st = scratch(ctx, canon_layout(T, C, false, nullptr, nullptr, nullptr), &p))) return st;
+        CanonWork wk;
+        canon_layout(T, C, false, static_cast<char *>(p), &wk, nullptr);
+        const bool aligned = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 &&
+                             (op != ROW_DOT || (reinterpret_cast<uintptr_t>(a.y) & 15) == 0);
+        switch (op) {
+        case ROW_SUM: st = aligned ? launch_canon<ROW_SUM, true>(ctx, a, nb, T, C, wk, fresh, cs, rest, result) : launch_canon<ROW_SUM, false>(ctx, a, nb, T, C, wk, fresh, cs, rest, result); break;
+        case ROW_DOT: st = aligned ? launch_canon<ROW_DOT, true>(ctx, a, nb, T, C, wk, fresh, cs, rest, result) : launch_canon<ROW_DOT, false>(ctx, a, nb, T, C, wk, fresh, cs, rest, result); break;
+        case ROW_SUMSQ: st = aligned ? launch_canon<ROW_SUMSQ, true>(ctx, a, nb, T, C, wk, fresh, cs, rest, result) : launch_canon<ROW_SUMSQ, false>(ctx, a, nb, T, C, wk, fresh, cs, rest, result); break;
+        default: st = aligned ? launch_canon<ROW_CONDSUM, true>(ctx, a, nb, T, C, wk, fresh, cs, rest, result) : launch_canon<ROW_CONDSUM, false>(ctx, a, nb, T, C, wk, fresh, cs, rest, result); break;
         }
         updated(ctx);
-        return VKC_OK;
+        return st;
     }
     vkc_status once(vkc_ctx *ctx, const Arg *args, int nargs, vkc_scalar *out, void *dst, bool *done) override {
-        *done = args[0].rows && args[0].len() / 16 <= CANON_SEQ_BLOCKS;
+        *done = args[0].rows;
         if (!*done) return VKC_OK;
         RowArgs a;
         vkc_status st = take(ctx, args, nargs, &a);
         if (st) return st;
+        const int64_t n = args[0].len();
         auto *to = static_cast<unsigned long long *>(dst ? dst : (host ? host : &static_cast<CanonState *>(state)->result));
-        if ((st = seq(ctx, a, args[0].len(), to)) || dst) return st;
+        st = n / 16 <= CANON_SEQ_BLOCKS ? seq(ctx, a, n, to) : tiles(ctx, a, n / 16, static_cast<int>(n % 16), to);
+        if (st || dst) return st;
         out->type = VKC_F64;
         return host ? result(ctx, &out->bits, 8) : download(ctx, &out->bits, 8, offsetof(CanonState, result));
     }
@@ -1738,11 +1904,10 @@ static vkc_status canon_scan_rows(vkc_ctx *ctx, const unsigned long long *x, int
         CanonWork wk;
         CanonState *cs = nullptr;
         canon_layout(T, C, true, static_cast<char *>(p), &wk, &cs);
-        VKC_CUDA(ctx, cudaMemsetAsync(cs, 0, sizeof(CanonState), ctx->stream));
         RowArgs a{};
         a.x = x;
-        st = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? launch_canon<ROW_SUM, true, true>(ctx, a, nb, T, C, wk, cs)
-                                                        : launch_canon<ROW_SUM, false, true>(ctx, a, nb, T, C, wk, cs);
+        st = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? launch_canon<ROW_SUM, true, true>(ctx, a, nb, T, C, wk, true, cs)
+                                                        : launch_canon<ROW_SUM, false, true>(ctx, a, nb, T, C, wk, true, cs);
         if (st) return st;
         tstate = wk.tstate;
     }
