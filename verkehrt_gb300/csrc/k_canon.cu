@@ -879,10 +879,21 @@ __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long lon
              (m.mn >= 0 || S + m.mn > static_cast<long long>(ONE52));
         r = (s & (1ull << 63)) | (ef << 52) | (static_cast<unsigned long long>(S + ((S & 1) ? m.d1 : m.d0)) & MANT);
     } else {
+        if (!__any_sync(FULL, usable && f.d0 != f.d1)) {
+            // No tie: the increments add up (above 2^54 they never apply, so 32 of them cannot wrap).
+            unsigned long long d = min(f.d0, ONE52 << 2);
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            TF y = shfl_up_tf(f, o);
-            if (lane >= o) f = compose<false>(y, f);
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long y = __shfl_up_sync(FULL, d, o);
+                if (lane >= o) d += y;
+            }
+            f = TF{d, d};
+        } else {
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                TF y = shfl_up_tf(f, o);
+                if (lane >= o) f = compose<false>(y, f);
+            }
         }
         ok = ok && apply_positive(s, E, f, &r);
     }
