@@ -9,9 +9,10 @@
 //     it belongs to the key EMPTY (or the pair (EMPTY, EMPTY)), whose rows go there directly.
 //     Each slot keeps the smallest row that holds its key (atomicMin, skipped when the stored
 //     row is already smaller), and each row records its slot. A thread probes four rows at once.
-//  2. number: a row is a first occurrence when its slot's smallest row is itself; a
-//     decoupled-lookback compaction over rows gives each first occurrence its rank, which is
-//     the group's id, stored in the slot; the same kernel writes every row's id.
+//  2. number: the smallest rows of the slots are the first occurrences, and a group's id is the rank
+//     of its first row among them. They are marked in a bitmap of the rows, whose words' counts are
+//     scanned; each occupied slot takes its id from there, and every row reads its slot's. Short
+//     inputs (GN_MIN_ROWS) do it in one kernel instead, a decoupled-lookback compaction over rows.
 // Table size: the reference's maximum is nextpow2(2n) slots (group.rs:226-229). When that is
 // above the first table's size (2^group_first_table_log2 slots from the autotuner's table,
 // 2^21 by default, which stays in L2), the insert first runs on that table; it gives up (an
@@ -84,29 +85,43 @@ __device__ __forceinline__ unsigned ld_relaxed32(const unsigned *p) {
     return v;
 }
 
-// SMALL: the attempt on the small table, which gives up through flags[1] (flags[0] counts the
-// distinct keys inserted). Otherwise the table has room for every key and a probe longer than
-// the table only records a timeout. Probes read the slot first and claim a free one by CAS,
+// SMALL: slots are read before they are claimed, the way of few distinct keys; with gives_up the
+// attempt on the first table, which gives up through flags[1] (flags[0] counts the distinct keys
+// inserted). Otherwise the table has room for every key and a probe longer than the table only records
+// a timeout. Probes read the slot first and claim a free one by CAS,
 // except for single keys on the full table (many distinct keys): there one 128-bit CAS both
 // reads the slot and claims it with the row as its smallest row.
+// Rows in flight together that share a key all try to claim it and to lower its smallest row, and
+// these atomics on few addresses take turns (10 keys in 2^20 rows: 176 us a call). So all blocks but
+// the first GI_AHEAD start GI_STAGGER_NS late: by then the frequent keys are there with the smallest
+// rows they ever will hold, and the others' rows find them by reading. (The sleep orders nothing: a row
+// that comes too early takes the atomics.)
+constexpr unsigned GI_AHEAD = 4, GI_STAGGER_NS = 4000;
+// (Slots read by way of L1 first, while few keys were seen: 10 keys in 30 M rows 372 us a call against
+// 428, but 2^16 keys 522 against 463, for the code around it; a launch of their own for the first rows
+// cost more than the sleep.) Measured, a call on 30 M rows of 10 / 1000 / 2^16 / 3.75 M / all distinct
+// keys: 1155 / 873 / 930 us / 10.1 / 11.5 ms when a key's slot and its row were two reads, the numbering
+// one lookback kernel and the regions 256 launches; now 445 / 385 / 485 us / 1.79 / 2.06 ms.
+
 template <bool PAIR, bool SMALL>
 __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *__restrict__ a,
                                                                const long long *__restrict__ b, int64_t n,
-                                                               GroupTable t, unsigned *__restrict__ slot_of,
+                                                               bool gives_up, GroupTable t, unsigned *__restrict__ slot_of,
                                                                unsigned *flags, DevStatus *st) {
     constexpr bool CAS_FIRST = !SMALL && !PAIR;
     const int lane = threadIdx.x & 31;
     const int64_t step = static_cast<int64_t>(gridDim.x) * GI_THREADS * GI_ROWS;
     // The full table always has a free slot, so a probe ends within `mask` steps.
-    const unsigned long long limit = SMALL ? GI_SMALL_PROBES : t.mask;
+    const unsigned long long limit = SMALL && gives_up ? GI_SMALL_PROBES : t.mask;
     const unsigned max_keys = static_cast<unsigned>((t.mask + 1) / 2);
+    if (SMALL && blockIdx.x >= GI_AHEAD && gridDim.x >= 8 * GI_AHEAD) __nanosleep(GI_STAGGER_NS);
     for (int64_t base = static_cast<int64_t>(blockIdx.x) * GI_THREADS * GI_ROWS; base < n; base += step) {
-        if (SMALL) {
-            unsigned ov = lane == 0 ? ld_relaxed32(flags + 1) : 0u;
+        if (SMALL && gives_up) {
+            const unsigned ov = lane == 0 ? ld_relaxed32(flags + 1) : 0u;
             if (__shfl_sync(FULL, ov, 0)) return;  // the whole warp leaves together
         }
         unsigned long long ka[GI_ROWS], kb[GI_ROWS], s[GI_ROWS];
-        unsigned cur[GI_ROWS];  // the slot's smallest row as last seen (CAS_FIRST)
+        unsigned cur[GI_ROWS];  // the slot's smallest row as last seen (single keys)
         unsigned pend = 0, in = 0, fresh = 0;
         bool gave_up = false;
 #pragma unroll
@@ -138,7 +153,9 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
                     } else if (PAIR) {
                         ld_relaxed_pair(t.words + 4 * s[j], va[j], vb[j]);
                     } else {
-                        va[j] = ld_relaxed64(t.words + 2 * s[j]);
+                        // The smallest row so far comes with the key: an old value costs at most an
+                        // atomicMin that changes nothing.
+                        ld_relaxed_pair(t.words + 2 * s[j], va[j], vb[j]);
                     }
                 }
             }
@@ -158,10 +175,15 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
                 } else if (!PAIR) {
                     if (va[j] == ka[j]) {
                         done = true;
+                        cur[j] = static_cast<unsigned>(vb[j]);
                     } else if (va[j] == GI_EMPTY) {
-                        const unsigned long long old = atomicCAS(t.words + 2 * s[j], GI_EMPTY, ka[j]);
-                        if (old == GI_EMPTY) ++fresh;
-                        done = old == GI_EMPTY || old == ka[j];
+                        // Claimed with the row as its smallest row.
+                        const unsigned long long row = static_cast<unsigned long long>(base + j * GI_THREADS + threadIdx.x);
+                        unsigned long long oa, ob;
+                        cas_pair(t.words + 2 * s[j], GI_EMPTY, ~0ull, ka[j], 0xffffffff00000000ull | row, oa, ob);
+                        if (oa == GI_EMPTY) ++fresh;
+                        done = oa == GI_EMPTY || oa == ka[j];
+                        cur[j] = oa == GI_EMPTY ? 0u : static_cast<unsigned>(ob);
                     }
                 } else if (va[j] != GI_EMPTY && vb[j] != GI_EMPTY) {
                     // A slot is written once, from (EMPTY, EMPTY): a pair with no EMPTY half is whole.
@@ -181,12 +203,12 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
             }
         }
         if (gave_up) {
-            if (SMALL) atomicExch(flags + 1, 1u);
+            if (SMALL && gives_up) atomicExch(flags + 1, 1u);
             else set_timeout(st);
         }
         if (SMALL) {
             const unsigned c = __reduce_add_sync(FULL, fresh);
-            if (lane == 0 && c && atomicAdd(flags, c) + c > max_keys) atomicExch(flags + 1, 1u);
+            if (lane == 0 && c && atomicAdd(flags, c) + c > max_keys && gives_up) atomicExch(flags + 1, 1u);
         }
         if (gave_up) continue;
 #pragma unroll
@@ -194,7 +216,7 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
             if (!(in & (1u << j))) continue;
             const unsigned row = static_cast<unsigned>(base + j * GI_THREADS + threadIdx.x);
             unsigned *m = &t.meta(s[j])->x;
-            if ((CAS_FIRST && s[j] != 0 ? cur[j] : ld_relaxed32(m)) > row) atomicMin(m, row);
+            if ((!PAIR && s[j] != 0 ? cur[j] : ld_relaxed32(m)) > row) atomicMin(m, row);
             slot_of[row] = static_cast<unsigned>(s[j]);
         }
     }
@@ -288,6 +310,63 @@ __global__ void __launch_bounds__(GI_THREADS, 4) gi_number_kernel(const unsigned
     release_ticket(counters, tiles);
 }
 
+// ------------------------------------------------------------------ numbering by ranks
+//
+// bits[w] marks the first occurrences among rows 32 w .. 32 w + 31, and rank[w] = {first occurrences
+// before row 32 w, bits[w]}, so that the id of the group whose first row is m is one 8-byte read.
+__device__ __forceinline__ unsigned gn_id(const uint2 *__restrict__ rank, unsigned m) {
+    const uint2 r = __ldg(rank + (m >> 5));
+    return r.x + __popc(r.y & ((1u << (m & 31u)) - 1u));
+}
+
+// The first occurrences of a table, and (IDS) the slots' ids once they are ranked.
+template <bool IDS>
+__global__ void __launch_bounds__(256) gn_slots_kernel(GroupTable t, unsigned *__restrict__ bits, const uint2 *__restrict__ rank) {
+    const unsigned long long stride = static_cast<unsigned long long>(gridDim.x) * blockDim.x;
+    for (unsigned long long s = static_cast<unsigned long long>(blockIdx.x) * blockDim.x + threadIdx.x; s <= t.mask; s += stride) {
+        uint2 *m = t.meta(s);
+        const unsigned row = m->x;
+        if (row == 0xffffffffu) continue;
+        if (IDS) m->y = gn_id(rank, row);
+        else atomicOr(bits + (row >> 5), 1u << (row & 31u));
+    }
+}
+
+__global__ void __launch_bounds__(256) gn_counts_kernel(const unsigned *__restrict__ bits, int64_t words, unsigned *__restrict__ counts) {
+    const int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (w < words) counts[w] = __popc(bits[w]);
+}
+
+__global__ void __launch_bounds__(256) gn_rank_kernel(const unsigned *__restrict__ bits, const unsigned *__restrict__ before,
+                                                      int64_t words, uint2 *__restrict__ rank) {
+    const int64_t w = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (w < words) rank[w] = make_uint2(before[w], bits[w]);
+}
+
+// Every row's id: from its slot (of = slots), or by its smallest row's rank (ROWS: of = those rows).
+// Four rows a thread, their reads in flight together.
+template <bool ROWS>
+__global__ void __launch_bounds__(256) gn_write_kernel(const unsigned *__restrict__ of, int64_t n, GroupTable t,
+                                                       const uint2 *__restrict__ rank, long long *__restrict__ out) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
+    auto id = [&](unsigned v) { return static_cast<long long>(ROWS ? gn_id(rank, v) : t.meta(v)->y); };
+    if (i + 4 <= n) {  // both arrays are allocations of their own
+        const uint4 v = __ldcs(reinterpret_cast<const uint4 *>(of + i));
+        const long long a = id(v.x), b = id(v.y), c = id(v.z), d = id(v.w);
+        __stcs(reinterpret_cast<longlong2 *>(out + i), make_longlong2(a, b));
+        __stcs(reinterpret_cast<longlong2 *>(out + i) + 1, make_longlong2(c, d));
+    } else {
+        for (int64_t r = i; r < n; ++r) out[r] = id(of[r]);
+    }
+}
+
+// The marks of rows whose smallest row is known.
+__global__ void __launch_bounds__(256) gn_marks_kernel(const unsigned *__restrict__ minrow, int64_t n, unsigned *__restrict__ bits) {
+    const int64_t r = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const unsigned m = __ballot_sync(FULL, r < n && minrow[r] == static_cast<unsigned>(r));
+    if ((threadIdx.x & 31) == 0 && r < n) bits[r >> 5] = m;
+}
+
 // Every slot free: keys GI_EMPTY, smallest row and id all ones.
 __global__ void __launch_bounds__(256) gi_clear_kernel(ulonglong2 *__restrict__ p, int64_t pairs, int w) {
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -307,13 +386,15 @@ __global__ void __launch_bounds__(256) gi_clear_kernel(ulonglong2 *__restrict__ 
 // through three sub-tables in rotation that stay in L2, one launch per region: a region's
 // sub-table is cleared, filled (claim by 128-bit CAS, smallest row by atomicMin) and read back
 // (each pair's smallest row of its key) in three consecutive launches, each of which also does
-// the other two jobs for the neighbouring regions. The launches are bound by the L2's 128-bit
+// the other two jobs for the neighbouring regions. (Neighbouring regions are taken together up to
+// GR_STEP_ROWS rows: a launch of a few rows takes 10 us all the same, so 256 of them took 2.6 ms
+// whatever the rows.) The launches are bound by the L2's 128-bit
 // CAS operations, not by DRAM: tables at load up to 2/3 (fitting L2 better) made probes longer
 // and the call slower, and so did slots tagged with the region instead of cleared (a read
 // before each CAS). The smallest rows go back to row order
-// through the tiles' staged runs, and the numbering runs in row order as in gi_number_kernel,
-// except that a row whose key first occurs in an earlier tile reads its id from the output row
-// of that first occurrence (written by then, or awaited with a bounded wait).
+// through the tiles' staged runs, and are ranked (above). (Numbered in one lookback kernel, whose rows
+// waited for the output row of their first occurrence, tiles waited for tiles that waited in turn: 4.8
+// ms of the 8.1 that 20 M rows of 15 M keys took.)
 constexpr int GR_BITS = 8, GR_NB = 1 << GR_BITS;
 constexpr int GR_THREADS = 256, GR_ITEMS = 16, GR_TILE = GR_THREADS * GR_ITEMS;
 
@@ -511,86 +592,6 @@ __global__ void __launch_bounds__(GR_THREADS) gr_restore_kernel(const unsigned *
     }
 }
 
-// The numbering of gi_number_kernel from each row's smallest row of its key: first occurrences
-// (smallest row = the row) are ranked in row order by a decoupled lookback; a repeat takes the
-// id of its first occurrence, from the tile's bitmap when that is in the same tile, else from
-// the output row of the first occurrence (out starts as all ones; a bounded wait).
-__global__ void __launch_bounds__(GI_THREADS, 4) gr_number_kernel(const unsigned *__restrict__ minrow, int64_t n,
-                                                                  int tiles, unsigned long long *words, unsigned epoch,
-                                                                  unsigned *counters, long long *out, DevStatus *st) {
-    __shared__ unsigned long long s_prefix;
-    __shared__ unsigned s_keep[GI_TILE / 32];
-    __shared__ unsigned s_wpre[GI_TILE / 32];
-    __shared__ long long s_out[GI_THREADS * GI_OUT_STRIDE];
-    const int tile = take_ticket(counters);
-    const int64_t t0 = static_cast<int64_t>(tile) * GI_TILE;
-    const int64_t row0 = t0 + threadIdx.x * GI_ITEMS;
-    unsigned mr[GI_ITEMS];
-    if (row0 + GI_ITEMS <= n) {
-        const uint4 *v = reinterpret_cast<const uint4 *>(minrow + row0);
-#pragma unroll
-        for (int q = 0; q < GI_ITEMS / 4; ++q) {
-            const uint4 w = __ldcs(v + q);
-            mr[4 * q] = w.x;
-            mr[4 * q + 1] = w.y;
-            mr[4 * q + 2] = w.z;
-            mr[4 * q + 3] = w.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < GI_ITEMS; ++j) mr[j] = row0 + j < n ? minrow[row0 + j] : 0u;
-    }
-    int rel[GI_ITEMS];
-    unsigned keep = 0;
-#pragma unroll
-    for (int j = 0; j < GI_ITEMS; ++j) {
-        const int64_t r = row0 + j;
-        rel[j] = -1;
-        if (r < n) {
-            rel[j] = static_cast<int>(static_cast<int64_t>(mr[j]) - t0);
-            if (mr[j] == static_cast<unsigned>(r)) keep |= 1u << j;
-        }
-    }
-    const unsigned odd = __shfl_down_sync(FULL, keep, 1);
-    if (!(threadIdx.x & 1)) s_keep[threadIdx.x >> 1] = keep | (odd << 16);
-    unsigned long long c = __popc(keep), tile_count;
-    const unsigned long long off = block_exclusive_sum<unsigned long long>(c, &tile_count);
-    if (!(threadIdx.x & 1)) s_wpre[threadIdx.x >> 1] = static_cast<unsigned>(off);
-    if (threadIdx.x < 32) {
-        unsigned long long pre = lookback_publish<4, CountRec>(words, tile, tile_count, 0ull, epoch, st);
-        if (threadIdx.x == 0) s_prefix = pre;
-    }
-    __syncthreads();
-    const unsigned prefix = static_cast<unsigned>(s_prefix);
-#pragma unroll
-    for (int j = 0; j < GI_ITEMS; ++j) {
-        if (row0 + j >= n) continue;
-        unsigned long long g;
-        if (rel[j] >= 0) {
-            const int w = rel[j] >> 5, bit = rel[j] & 31;
-            g = prefix + s_wpre[w] + __popc(s_keep[w] & ((1u << bit) - 1u));
-        } else {
-            const unsigned long long *p = reinterpret_cast<const unsigned long long *>(out + mr[j]);
-            unsigned it = 0;
-            const unsigned limit = wait_limit(st);
-            while ((g = ld_relaxed64(p)) == ~0ull) {
-                if (++it > limit) {
-                    set_timeout(st);
-                    break;
-                }
-                backoff(it);
-            }
-        }
-        s_out[threadIdx.x * GI_OUT_STRIDE + j] = static_cast<long long>(g);
-    }
-    __syncthreads();
-    const int rows = static_cast<int>(n - t0 < GI_TILE ? n - t0 : GI_TILE);
-    for (int i = threadIdx.x; i < rows; i += GI_THREADS)
-        st_relaxed64(reinterpret_cast<unsigned long long *>(out + t0 + i),
-                     static_cast<unsigned long long>(s_out[(i / GI_ITEMS) * GI_OUT_STRIDE + (i % GI_ITEMS)]));
-    release_ticket(counters, tiles);
-}
-
 struct GroupScratch {
     vkc_array *words = nullptr;
     void release() {
@@ -612,22 +613,57 @@ static vkc_status new_table(vkc_ctx *ctx, uint64_t slots, bool pair, GroupScratc
 
 // One wave of resident blocks (the grid-stride loop gives every block the same share, so a
 // second, partial wave would run at a fraction of the occupancy).
-template <bool PAIR>
-static void launch_insert(vkc_ctx *ctx, bool small, const long long *a, const long long *b, int64_t n,
-                          const GroupTable &t, unsigned *slot_of, unsigned *flags) {
-    static int resident[2] = {0, 0};
-    auto kern = small ? gi_insert_kernel<PAIR, true> : gi_insert_kernel<PAIR, false>;
-    int &per_sm = resident[small ? 1 : 0];
+template <bool PAIR, bool SMALL>
+static void launch_insert(vkc_ctx *ctx, bool gives_up, const long long *a, const long long *b, int64_t n, const GroupTable &t,
+                          unsigned *slot_of, unsigned *flags) {
+    static int per_sm = 0;
+    auto kern = gi_insert_kernel<PAIR, SMALL>;
     if (per_sm == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GI_THREADS, 0) != cudaSuccess ||
                         per_sm < 1))
         per_sm = 1;
     const int grid = stream_grid(ctx, n, GI_THREADS, per_sm, GI_THREADS * GI_ROWS);
-    kern<<<grid, GI_THREADS, 0, ctx->stream>>>(a, b, n, t, slot_of, flags, ctx->status);
+    kern<<<grid, GI_THREADS, 0, ctx->stream>>>(a, b, n, gives_up, t, slot_of, flags, ctx->status);
 }
 
-
-// Single keys, many distinct, at least GR_MIN_ROWS rows: the region-partitioned path above.
+// Single keys, many distinct, at least GR_MIN_ROWS rows: the region-partitioned path above. A step
+// takes regions of GR_STEP_ROWS rows together: sub-tables of 16 MiB, three of which stay in L2.
 constexpr int64_t GR_MIN_ROWS = int64_t(1) << 22;
+constexpr int64_t GR_STEP_ROWS = int64_t(1) << 19;
+
+// From this many rows on the table's numbering goes by ranks.
+constexpr int64_t GN_MIN_ROWS = int64_t(1) << 22;
+
+// Ranks the marked first occurrences (bits, one word per 32 of n rows) into rank[]; counts, before and
+// sums are scratch. Then every row's id.
+struct Ranking {
+    vkc_array *arr[5] = {};
+    unsigned *bits = nullptr, *counts = nullptr, *before = nullptr, *sums = nullptr;
+    uint2 *rank = nullptr;
+    int64_t words = 0;
+    vkc_status alloc(vkc_ctx *ctx, int64_t n, bool zero) {
+        words = (n + 31) / 32;
+        const int64_t sizes[5] = {words, words, words, scan_counts_sum_words(words), words};
+        for (int i = 0; i < 5; ++i)
+            if (new_array(ctx, i == 4 ? VKC_U64 : VKC_I32, sizes[i], zero && i == 0, &arr[i])) return VKC_ALLOC;
+        bits = static_cast<unsigned *>(arr[0]->data());
+        counts = static_cast<unsigned *>(arr[1]->data());
+        before = static_cast<unsigned *>(arr[2]->data());
+        sums = static_cast<unsigned *>(arr[3]->data());
+        rank = static_cast<uint2 *>(arr[4]->data());
+        return VKC_OK;
+    }
+    void ranks(vkc_ctx *ctx) {
+        const int g = static_cast<int>((words + 255) / 256);
+        gn_counts_kernel<<<g, 256, 0, ctx->stream>>>(bits, words, counts);
+        scan_counts(ctx, counts, words, sums, before);
+        gn_rank_kernel<<<g, 256, 0, ctx->stream>>>(bits, before, words, rank);
+    }
+    ~Ranking() {
+        for (vkc_array *a : arr)
+            if (a) vkc_array_release(a);
+    }
+};
+static int gn_write_grid(int64_t n) { return static_cast<int>((n + 1023) / 1024); }
 
 static vkc_status run_group_partitioned(vkc_ctx *ctx, const long long *keys, int64_t n, vkc_array *o) {
     const int tiles = static_cast<int>((n + GR_TILE - 1) / GR_TILE);
@@ -662,10 +698,18 @@ static vkc_status run_group_partitioned(vkc_ctx *ctx, const long long *keys, int
     VKC_CUDA(ctx, cudaMemcpy2DAsync(starts, sizeof(unsigned), offs, static_cast<size_t>(tiles) * sizeof(unsigned),
                                     sizeof(unsigned), GR_NB, cudaMemcpyDeviceToHost, ctx->stream));
     VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    std::vector<unsigned> start(starts, starts + GR_NB);
+    // The steps' regions: neighbouring ones together.
+    std::vector<unsigned> start;
+    for (int r = 0; r < GR_NB;) {
+        start.push_back(starts[r]);
+        int e = r + 1;
+        while (e < GR_NB && (e + 1 < GR_NB ? starts[e + 1] : static_cast<unsigned>(n)) - starts[r] <= GR_STEP_ROWS) ++e;
+        r = e;
+    }
+    const int steps = static_cast<int>(start.size());
     start.push_back(static_cast<unsigned>(n));
     unsigned most = 1;
-    for (int r = 0; r < GR_NB; ++r) most = std::max(most, start[r + 1] - start[r]);
+    for (int r = 0; r < steps; ++r) most = std::max(most, start[r + 1] - start[r]);
     uint64_t slots = 2;
     while (slots < 2ull * most) slots <<= 1;
     if ((st = new_array(ctx, VKC_U64, static_cast<int64_t>(6 * slots), false, &arr[9]))) return done(st);
@@ -673,9 +717,9 @@ static vkc_status run_group_partitioned(vkc_ctx *ctx, const long long *keys, int
     auto table = [&](int k) { return GroupTable{words + 2 * slots * static_cast<uint64_t>(k % 3), slots - 1, 2}; };
     gi_clear_kernel<<<stream_grid(ctx, static_cast<int64_t>(slots), 256, 8, 2048), 256, 0, ctx->stream>>>(
         reinterpret_cast<ulonglong2 *>(table(0).words), static_cast<int64_t>(slots), 2);
-    for (int k = 0; k <= GR_NB; ++k) {
+    for (int k = 0; k <= steps; ++k) {
         GrStep s{};
-        if (k < GR_NB) {
+        if (k < steps) {
             s.ins0 = start[k];
             s.ins1 = start[k + 1];
         }
@@ -686,20 +730,20 @@ static vkc_status run_group_partitioned(vkc_ctx *ctx, const long long *keys, int
         s.ins = table(k);
         s.min = table(k + 2);  // (k - 1) % 3
         s.clr = table(k + 1);
-        s.clr_slots = k + 1 < GR_NB ? static_cast<int64_t>(slots) : 0;
+        s.clr_slots = k + 1 < steps ? static_cast<int64_t>(slots) : 0;
         const unsigned rows = std::max(s.ins1 - s.ins0, s.min1 - s.min0);
         const unsigned grid = std::max(1u, (rows + 255) / 256);
         gr_step_kernel<<<grid, 256, 0, ctx->stream>>>(keys_p, rows_p, slot_p, min_p, s, ctx->status);
     }
     if ((st = launched(ctx, "gr_regions"))) return done(st);
     gr_restore_kernel<<<tiles, GR_THREADS, 0, ctx->stream>>>(min_p, loc, counts, offs, n, tiles, minrow);
-    VKC_CUDA(ctx, cudaMemsetAsync(o->data(), 0xff, static_cast<size_t>(n) * 8, ctx->stream));
-    const int gtiles = static_cast<int>((n + GI_TILE - 1) / GI_TILE);
-    unsigned long long *recs;
-    if ((st = rec_arena(ctx, gtiles, &recs))) return done(st);
-    gr_number_kernel<<<gtiles, GI_THREADS, 0, ctx->stream>>>(minrow, n, gtiles, recs, next_epoch(ctx), ctx->counters,
-                                                            static_cast<long long *>(o->data()), ctx->status);
-    return done(launched(ctx, "gr_number"));
+    Ranking rk;
+    if ((st = rk.alloc(ctx, n, false))) return done(st);
+    gn_marks_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, ctx->stream>>>(minrow, n, rk.bits);
+    rk.ranks(ctx);
+    gn_write_kernel<true><<<gn_write_grid(n), 256, 0, ctx->stream>>>(minrow, n, GroupTable{}, rk.rank,
+                                                                     static_cast<long long *>(o->data()));
+    return done(launched(ctx, "gn_write"));
 }
 
 static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *xb, vkc_value *out) {
@@ -745,8 +789,8 @@ static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *
             vkc_array_release(o);
             return st;
         }
-        if (xb) launch_insert<true>(ctx, true, a, b, n, t, slot_of, flags);
-        else launch_insert<false>(ctx, true, a, b, n, t, slot_of, flags);
+        if (xb) launch_insert<true, true>(ctx, true, a, b, n, t, slot_of, flags);
+        else launch_insert<false, true>(ctx, true, a, b, n, t, slot_of, flags);
         if ((st = launched(ctx, "gi_insert"))) {
             cleanup();
             vkc_array_release(o);
@@ -786,24 +830,39 @@ static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *
             vkc_array_release(o);
             return st;
         }
-        if (xb) launch_insert<true>(ctx, false, a, b, n, t, slot_of, flags);
-        else launch_insert<false>(ctx, false, a, b, n, t, slot_of, flags);
+        // Many distinct keys are only known of inputs whose first table gave up.
+        const bool many = slots > first_slots;
+        if (xb && many) launch_insert<true, false>(ctx, false, a, b, n, t, slot_of, flags);
+        else if (xb) launch_insert<true, true>(ctx, false, a, b, n, t, slot_of, flags);
+        else if (many) launch_insert<false, false>(ctx, false, a, b, n, t, slot_of, flags);
+        else launch_insert<false, true>(ctx, false, a, b, n, t, slot_of, flags);
         if ((st = launched(ctx, "gi_insert"))) {
             cleanup();
             vkc_array_release(o);
             return st;
         }
     }
-    int tiles = static_cast<int>((n + GI_TILE - 1) / GI_TILE);
-    unsigned long long *recs;
-    if ((st = rec_arena(ctx, tiles, &recs))) {
-        cleanup();
-        vkc_array_release(o);
-        return st;
+    Ranking rk;
+    if (n >= GN_MIN_ROWS) {
+        if (rk.alloc(ctx, n, true)) return alloc_fail();
+        const int g = stream_grid(ctx, static_cast<int64_t>(t.mask + 1), 256, 8, 1024);
+        gn_slots_kernel<false><<<g, 256, 0, ctx->stream>>>(t, rk.bits, nullptr);
+        rk.ranks(ctx);
+        gn_slots_kernel<true><<<g, 256, 0, ctx->stream>>>(t, nullptr, rk.rank);
+        gn_write_kernel<false><<<gn_write_grid(n), 256, 0, ctx->stream>>>(slot_of, n, t, nullptr,
+                                                                          static_cast<long long *>(o->data()));
+    } else {
+        const int tiles = static_cast<int>((n + GI_TILE - 1) / GI_TILE);
+        unsigned long long *recs;
+        if ((st = rec_arena(ctx, tiles, &recs))) {
+            cleanup();
+            vkc_array_release(o);
+            return st;
+        }
+        gi_number_kernel<<<tiles, GI_THREADS, 0, ctx->stream>>>(slot_of, n, t, tiles, recs, next_epoch(ctx), ctx->counters,
+                                                               static_cast<long long *>(o->data()), ctx->status);
     }
-    gi_number_kernel<<<tiles, GI_THREADS, 0, ctx->stream>>>(slot_of, n, t, tiles, recs, next_epoch(ctx), ctx->counters,
-                                                           static_cast<long long *>(o->data()), ctx->status);
-    if ((st = launched(ctx, "gi_number"))) {
+    if ((st = launched(ctx, "group_number"))) {
         cleanup();
         vkc_array_release(o);
         return st;

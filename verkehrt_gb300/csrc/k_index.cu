@@ -432,11 +432,14 @@ __global__ void __launch_bounds__(256) keys_check_kernel(const long long *__rest
 
 // Per-bucket wrapping sums (vals) or counts (vals == nullptr). Every warp walks chunks of
 // BK_ITEMS groups of 32 consecutive rows (one coalesced load per group and array, all groups of
-// a chunk loaded before any is added). Within a group, runs of equal keys in consecutive lanes
-// are summed by a segmented warp scan, so only the lane that ends a run adds it to a bucket; the
-// run that ends a group is carried into the next group while the key stays the same. Sorted
-// keys (run numbers, sorted group keys) thus cost about one addition per run instead of one per
-// row, which removes the contention of long runs on one bucket. Buckets below SMEM_BINS are
+// a chunk loaded before any is added). A group with no two equal neighbours, nearly every one of
+// unsorted keys, adds its rows as they are (the runs' machinery below, thirty shuffles a group, bound
+// this kernel: calls on 30 M rows in 10 / 1000 / 2^16 buckets took 450 / 252 / 240 us, now 224 / 125 /
+// 225, the last ones bound by the L2's atomics). In the others, runs of equal keys
+// in consecutive lanes are summed by a segmented warp scan, so only the lane that ends a run adds it to
+// a bucket; the run that ends a group is carried into the next group while the key stays the same:
+// sorted keys (run numbers, sorted group keys) cost about one addition per run instead of one per row,
+// which removes the contention of long runs on one bucket. Buckets below SMEM_BINS are
 // added in shared memory per block and to the output once per block; the others go to global
 // atomics. Small keys are where random contention is: group ids number groups by first
 // occurrence, so frequent groups get small ids (under a Zipf(1.1) key distribution the first
@@ -449,9 +452,15 @@ __global__ void __launch_bounds__(256) bucket_kernel(const long long *__restrict
                                                      const unsigned long long *__restrict__ vals, int64_t n,
                                                      uint64_t nb, unsigned long long *__restrict__ out,
                                                      DevStatus *status) {
-    __shared__ unsigned long long bins[SMEM_BINS];
+    // Shared bins in 32-bit words, whose atomics the SM executes itself (64-bit ones are a loop of
+    // compare-and-swaps, as long as a warp's most frequent key): the low words, and the high ones with
+    // the carries. A block counts below 2^32 rows.
+    __shared__ unsigned bins[COUNT ? 1 : 2][SMEM_BINS];
     const int sb = nb < static_cast<uint64_t>(SMEM_BINS) ? static_cast<int>(nb) : SMEM_BINS;
-    for (int b = threadIdx.x; b < sb; b += blockDim.x) bins[b] = 0;
+    for (int b = threadIdx.x; b < sb; b += blockDim.x) {
+        bins[0][b] = 0;
+        if (!COUNT) bins[COUNT ? 0 : 1][b] = 0;
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -459,8 +468,15 @@ __global__ void __launch_bounds__(256) bucket_kernel(const long long *__restrict
     const int64_t chunks = (n + chunk_rows - 1) / chunk_rows;
     const unsigned below = (1u << lane) - 1u;
     auto add = [&](long long k, unsigned long long v) {
-        if (k < SMEM_BINS) atomicAdd(&bins[k], v);
-        else atomicAdd(out + k, v);
+        if (k >= SMEM_BINS) {
+            atomicAdd(out + k, v);
+        } else if (COUNT) {
+            atomicAdd(&bins[0][k], static_cast<unsigned>(v));
+        } else {
+            const unsigned lo = static_cast<unsigned>(v), old = atomicAdd(&bins[0][k], lo);
+            const unsigned hi = static_cast<unsigned>(v >> 32) + (old + lo < lo ? 1u : 0u);
+            if (hi) atomicAdd(&bins[COUNT ? 0 : 1][k], hi);
+        }
     };
     constexpr long long NONE = -1;  // a lane with no row in range: never added
     unsigned long long bad = ~0ull;
@@ -484,6 +500,15 @@ __global__ void __launch_bounds__(256) bucket_kernel(const long long *__restrict
             if (i < n && static_cast<uint64_t>(key) >= nb) {
                 if (static_cast<unsigned long long>(i) < bad) bad = static_cast<unsigned long long>(i);
                 key = NONE;
+            }
+            // The low halves decide most groups: two different ones are two different keys.
+            const unsigned low = static_cast<unsigned>(key);
+            const unsigned before = __shfl_up_sync(FULL, low, 1);  // every lane takes part
+            if (!__any_sync(FULL, lane != 0 && before == low)) {
+                if (lane == 0 && ckey != NONE) add(ckey, csum);
+                ckey = NONE;
+                if (key != NONE) add(key, v[r]);
+                continue;
             }
             unsigned long long x = key == NONE ? 0ull : v[r];
             // Runs of equal keys: a lane heads a run when its key differs from the lane before.
@@ -514,8 +539,10 @@ __global__ void __launch_bounds__(256) bucket_kernel(const long long *__restrict
     if (lane == 0 && ckey != NONE) add(ckey, csum);
     if (bad != ~0ull) atomicMin(&status->first_bad, bad);
     __syncthreads();
-    for (int b = threadIdx.x; b < sb; b += blockDim.x)
-        if (bins[b]) atomicAdd(out + b, bins[b]);
+    for (int b = threadIdx.x; b < sb; b += blockDim.x) {
+        const unsigned long long v = bins[0][b] | (COUNT ? 0ull : static_cast<unsigned long long>(bins[COUNT ? 0 : 1][b]) << 32);
+        if (v) atomicAdd(out + b, v);
+    }
 }
 
 // The reference's error for the first key outside [0, nb) (checked_keys, index.rs:116-130):
