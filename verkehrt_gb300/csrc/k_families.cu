@@ -6,7 +6,8 @@
 //               (src/kernels/scalar/reduce.rs:331-726)
 //   fused       dot/sumsq/count_<cmp>/filter_<cmp>/condsum_<cmp> on f32, i64, u64, i32
 //               (src/kernels/scalar/fused.rs:73-379)
-//   scans       scan_<fold>_T, scan_by_<fold>_T, reduce_into_<fold>_T, prev_T
+//   scans       scan_<fold>_T, scan_by_<fold>_T (their entries; the passes are fold_scan.cuh's),
+//               reduce_into_<fold>_T, prev_T
 //               (src/kernels/scalar/scan.rs:16-439)
 //   whole       group_id_T, group_id2_A_B (group.rs:259-363),
 //               fill_T, same_len_T (construct.rs:49-120), slice_T (index.rs:240-258)
@@ -14,13 +15,14 @@
 // Values travel as 64-bit words: i32 sign-extended, u8 and bool zero-extended, f32 as its 32
 // bits. Every fold except the canonical float sum and product is order-free (wrapping integer
 // arithmetic, the 754-2019 minimum/maximum, bit operations), so those reductions are a plain
-// grid fold and the scans a reduce-then-scan over 4096-row tiles. The canonical order of a float
+// grid fold. The canonical order of a float
 // product is sixteen chains of dependent IEEE multiplies: one block stages the rows in shared
 // memory while sixteen threads run the chains (the float sums have exact parallel paths, in
 // k_canon.cu and k_canon32.cu).
 #include <climits>
 #include <cstring>
 
+#include "folds.h"
 #include "kcommon.cuh"
 #include "reduce_common.h"
 
@@ -35,20 +37,8 @@ ReducerImpl *make_canon32_cond(vkc_ctx *ctx, int cmp);
 
 namespace {
 
-typedef unsigned long long u64;
-
-enum Fold { F_ADD = 0, F_MUL = 1, F_MIN = 2, F_MAX = 3, F_AND = 4, F_OR = 5, F_XOR = 6 };
 const char *FOLD_NAMES[7] = {"add", "mul", "min", "max", "and", "or", "xor"};
 const char *CMP_NAME[6] = {"eq", "ne", "lt", "le", "gt", "ge"};
-
-__host__ __device__ constexpr int width_of(vkc_type t) {
-    return t == VKC_F64 || t == VKC_I64 || t == VKC_U64 ? 8 : (t == VKC_F32 || t == VKC_I32 ? 4 : 1);
-}
-__host__ __device__ constexpr vkc_type sum_type(vkc_type t) {
-    return t == VKC_I32 ? VKC_I64 : (t == VKC_U8 ? VKC_U64 : t);
-}
-__host__ __device__ constexpr bool is_float(vkc_type t) { return t == VKC_F64 || t == VKC_F32; }
-__host__ __device__ constexpr bool is_signed_t(vkc_type t) { return t == VKC_I64 || t == VKC_I32; }
 
 // Element load and store as words.
 template <vkc_type T> __device__ __forceinline__ u64 ld_word(const void *p, int64_t i) {
@@ -61,12 +51,6 @@ template <int W> __device__ __forceinline__ void st_word(void *p, int64_t i, u64
     if (W == 8) static_cast<u64 *>(p)[i] = v;
     else if (W == 4) static_cast<unsigned *>(p)[i] = static_cast<unsigned>(v);
     else static_cast<unsigned char *>(p)[i] = static_cast<unsigned char>(v);
-}
-
-// Num::wrapping on the element type (elementwise.rs:386-400): truncate and widen back.
-template <vkc_type T> __host__ __device__ constexpr u64 wrap(u64 v) {
-    return T == VKC_I32 ? static_cast<u64>(static_cast<long long>(static_cast<int>(static_cast<unsigned>(v))))
-           : (T == VKC_U8 || T == VKC_BOOL) ? (v & 0xffull) : v;
 }
 
 __device__ __forceinline__ bool nan64(u64 b) { return (b & ~(1ull << 63)) > 0x7ff0000000000000ull; }
@@ -106,23 +90,6 @@ template <vkc_type T, int F> __device__ __forceinline__ u64 step(u64 acc, u64 x)
     if (F == F_AND) return acc & x;
     if (F == F_OR) return acc | x;
     return acc ^ x;
-}
-
-// scan.rs:99-120, :130-233 (identity): add/or/xor 0, mul 1, and all ones (bool: true), min the
-// highest value (+inf), max the lowest (-inf).
-template <vkc_type T, int F> __host__ __device__ constexpr u64 identity() {
-    return F == F_ADD || F == F_OR || F == F_XOR ? 0ull
-           : F == F_MUL ? 1ull
-           : F == F_AND ? (T == VKC_BOOL ? 1ull : wrap<T>(~0ull))
-           : F == F_MIN ? (T == VKC_F64 ? 0x7ff0000000000000ull
-                           : T == VKC_F32 ? 0x7f800000ull
-                           : T == VKC_I64 ? 0x7fffffffffffffffull
-                           : T == VKC_I32 ? 0x7fffffffull
-                           : T == VKC_U8 ? 0xffull : ~0ull)
-                        : (T == VKC_F64 ? 0xfff0000000000000ull
-                           : T == VKC_F32 ? 0xff800000ull
-                           : T == VKC_I64 ? 0x8000000000000000ull
-                           : T == VKC_I32 ? 0xffffffff80000000ull : 0ull);
 }
 
 // fused.rs:41-54: the comparison of the single-op kernels (IEEE for floats: NaN is unordered).
@@ -501,206 +468,7 @@ template <vkc_type T> ReducerImpl *make_product(vkc_ctx *ctx) {
     return r;
 }
 
-// ------------------------------------------------------------------ scans
-//
-// scan.rs:248-282: row 0 and every row whose start flag is set lift their value, every other
-// row steps the running value; state carries across updates. With the fold's identity as the
-// state before the first row (step(identity, x) = lift(x)), out[i] is the fold of the state and
-// the rows from the last start through i: an associative fold of (flag, value) pairs,
-// (f1, v1) then (f2, v2) = (f1 | f2, f2 ? v2 : v1 op v2). Three kernels: tile aggregates, one
-// block's exclusive scan of them from the carried state, and each tile's rows from its prefix.
-constexpr int SC_T = 256, SC_I = 16, SC_ROWS = SC_T * SC_I;
-
-struct SegVal {
-    u64 v;
-    unsigned f;
-};
-
-template <vkc_type T, int F> __device__ __forceinline__ SegVal seg_op(SegVal a, SegVal b) {
-    return SegVal{b.f ? b.v : step<T, F>(a.v, b.v), a.f | b.f};
-}
-
-// Inclusive block scan of one pair per thread, in thread order; *total gets the block's pair.
-template <vkc_type T, int F> __device__ SegVal block_scan(SegVal x, SegVal *total) {
-    __shared__ u64 wv[SC_T / 32];
-    __shared__ unsigned wf[SC_T / 32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        SegVal y{__shfl_up_sync(FULL, x.v, o), __shfl_up_sync(FULL, x.f, o)};
-        if (lane >= o) x = seg_op<T, F>(y, x);
-    }
-    if (lane == 31) {
-        wv[w] = x.v;
-        wf[w] = x.f;
-    }
-    __syncthreads();
-    SegVal before{identity<T, F>(), 0};
-    for (int i = 0; i < w; ++i) before = seg_op<T, F>(before, SegVal{wv[i], wf[i]});
-    SegVal t{identity<T, F>(), 0};
-    for (int i = 0; i < SC_T / 32; ++i) t = seg_op<T, F>(t, SegVal{wv[i], wf[i]});
-    *total = t;
-    __syncthreads();
-    return w ? seg_op<T, F>(before, x) : x;
-}
-
-// IT: the element type; OT: the word domain of the fold (the sum type for add).
-template <vkc_type IT, vkc_type OT, int F, bool BY>
-__device__ __forceinline__ SegVal thread_rows(const void *x, const unsigned char *s, int64_t r0, int64_t n, u64 *v) {
-    SegVal acc{identity<OT, F>(), 0};
-#pragma unroll
-    for (int j = 0; j < SC_I; ++j) {
-        const int64_t r = r0 + j;
-        v[j] = r < n ? ld_word<IT>(x, r) : identity<OT, F>();
-        const unsigned f = (BY && r < n) ? (s[r] != 0) : 0u;
-        acc = f ? SegVal{v[j], 1u} : SegVal{step<OT, F>(acc.v, v[j]), acc.f};
-    }
-    return acc;
-}
-
-template <vkc_type IT, vkc_type OT, int F, bool BY>
-__global__ void __launch_bounds__(SC_T) fam_scan_agg(const void *x, const unsigned char *s, int64_t n, u64 *aggv,
-                                                     unsigned *aggf) {
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * SC_ROWS + threadIdx.x * SC_I;
-    u64 v[SC_I];
-    SegVal mine = thread_rows<IT, OT, F, BY>(x, s, r0, n, v);
-    SegVal tot;
-    block_scan<OT, F>(mine, &tot);
-    if (threadIdx.x == 0) {
-        aggv[blockIdx.x] = tot.v;
-        aggf[blockIdx.x] = tot.f;
-    }
-}
-
-// One block: the exclusive prefix of every tile from the carried state (carry[0]).
-template <vkc_type OT, int F>
-__global__ void __launch_bounds__(1024) fam_scan_prefix(u64 *aggv, const unsigned *aggf, int tiles, const u64 *carry) {
-    __shared__ u64 tv[1024];
-    __shared__ unsigned tf[1024];
-    const int per = (tiles + 1023) / 1024;
-    const int t0 = threadIdx.x * per, t1 = min(tiles, t0 + per);
-    SegVal acc{identity<OT, F>(), 0};
-    for (int t = t0; t < t1; ++t) acc = seg_op<OT, F>(acc, SegVal{aggv[t], aggf[t]});
-    tv[threadIdx.x] = acc.v;
-    tf[threadIdx.x] = acc.f;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        SegVal run{carry[0], 0};
-        for (int i = 0; i < 1024; ++i) {
-            const SegVal mine{tv[i], tf[i]};
-            tv[i] = run.v;
-            run = seg_op<OT, F>(run, mine);
-        }
-    }
-    __syncthreads();
-    SegVal run{tv[threadIdx.x], 0};
-    for (int t = t0; t < t1; ++t) {
-        const SegVal mine{aggv[t], aggf[t]};
-        aggv[t] = run.v;  // exclusive prefix of tile t
-        run = seg_op<OT, F>(run, mine);
-    }
-}
-
-template <vkc_type IT, vkc_type OT, int F, bool BY>
-__global__ void __launch_bounds__(SC_T) fam_scan_apply(const void *x, const unsigned char *s, int64_t n,
-                                                       const u64 *prefix, void *out, u64 *carry) {
-    const int64_t r0 = static_cast<int64_t>(blockIdx.x) * SC_ROWS + threadIdx.x * SC_I;
-    u64 v[SC_I];
-    SegVal mine = thread_rows<IT, OT, F, BY>(x, s, r0, n, v);
-    SegVal tot;
-    const SegVal incl = block_scan<OT, F>(mine, &tot);
-    // The value before this thread's rows: the tile's prefix, then the earlier threads' rows (the
-    // inclusive scan of the thread before).
-    SegVal before{prefix[blockIdx.x], 0};
-    {
-        __shared__ u64 pv[SC_T];
-        __shared__ unsigned pf[SC_T];
-        pv[threadIdx.x] = incl.v;
-        pf[threadIdx.x] = incl.f;
-        __syncthreads();
-        if (threadIdx.x) before = seg_op<OT, F>(before, SegVal{pv[threadIdx.x - 1], pf[threadIdx.x - 1]});
-    }
-    u64 acc = before.v;
-#pragma unroll
-    for (int j = 0; j < SC_I; ++j) {
-        const int64_t r = r0 + j;
-        if (r >= n) break;
-        const bool f = BY && s[r] != 0;
-        acc = f ? v[j] : step<OT, F>(acc, v[j]);
-        if (F != F_ADD) acc = wrap<OT>(acc);
-        st_word<width_of(OT)>(out, r, acc);
-        if (r == n - 1) carry[0] = acc;
-    }
-}
-
-// Scanner of one fold. carry[0]: the output of the last row so far, the identity before any.
-struct FamScan : ScannerImpl {
-    vkc_type in, out;
-    bool by;
-    u64 *carry = nullptr;
-    DeviceMem mem;
-    using Launch = void (*)(vkc_ctx *, const void *, const unsigned char *, int64_t, void *, u64 *, u64 *, unsigned *);
-    Launch launch = nullptr;
-    vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs, vkc_array *o) override {
-        vkc_status st;
-        const int want = by ? 2 : 1;
-        if (nargs != want) return fail(ctx, VKC_RUNTIME, arity_error(want, nargs));
-        if (!rows_arg(ctx, args[0], in, &st)) return st;
-        if (by && !rows_arg(ctx, args[1], VKC_BOOL, &st)) return st;
-        if (o->type != out) return fail(ctx, VKC_RUNTIME, "bad destination");
-        const int64_t n = args[0].len();
-        if (o->len != n || (by && args[1].len() != n))
-            return fail(ctx, VKC_RUNTIME, "length mismatch: " + std::to_string(n) + " rows for a destination of " +
-                                              std::to_string(o->len) + " rows");
-        if (n == 0) return VKC_OK;
-        const int64_t tiles = (n + SC_ROWS - 1) / SC_ROWS;
-        void *p;
-        if ((st = scratch(ctx, static_cast<size_t>(tiles) * 12 + 256, &p))) return st;
-        launch(ctx, args[0].a->data(), by ? static_cast<const unsigned char *>(args[1].a->data()) : nullptr, n,
-               o->data(), carry, static_cast<u64 *>(p), reinterpret_cast<unsigned *>(static_cast<u64 *>(p) + tiles));
-        return launched(ctx, "family_scan");
-    }
-};
-
-template <vkc_type IT, vkc_type OT, int F, bool BY>
-void launch_scan_fam(vkc_ctx *ctx, const void *x, const unsigned char *s, int64_t n, void *out, u64 *carry,
-                     u64 *aggv, unsigned *aggf) {
-    const int tiles = static_cast<int>((n + SC_ROWS - 1) / SC_ROWS);
-    fam_scan_agg<IT, OT, F, BY><<<tiles, SC_T, 0, ctx->stream>>>(x, s, n, aggv, aggf);
-    fam_scan_prefix<OT, F><<<1, 1024, 0, ctx->stream>>>(aggv, aggf, tiles, carry);
-    fam_scan_apply<IT, OT, F, BY><<<tiles, SC_T, 0, ctx->stream>>>(x, s, n, aggv, out, carry);
-}
-
-template <vkc_type IT, int F, bool BY> ScannerImpl *make_scan_fam(vkc_ctx *ctx) {
-    constexpr vkc_type OT = F == F_ADD ? sum_type(IT) : IT;
-    auto *s = new FamScan;
-    s->in = IT;
-    s->out = OT;
-    s->by = BY;
-    s->launch = launch_scan_fam<IT, OT, F, BY>;
-    if (cudaMallocAsync(reinterpret_cast<void **>(&s->carry), 8, ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        delete s;
-        return nullptr;
-    }
-    s->mem.ptr = s->carry;
-    s->mem.box = ctx->box;
-    const u64 id = identity<OT, F>();
-    void *h;
-    if (pinned(ctx, 8, &h) || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        delete s;
-        return nullptr;
-    }
-    memcpy(h, &id, 8);
-    if (cudaMemcpyAsync(s->carry, h, 8, cudaMemcpyHostToDevice, ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-        cudaGetLastError();
-        delete s;
-        return nullptr;
-    }
-    return s;
-}
+// ------------------------------------------------------------------ prev
 
 // prev_T (scan.rs:16-73): out[0] is the fill on the first update, else the last row of the
 // previous update; out[i] = x[i - 1]. carry: [0] last row, [1] seen.
@@ -1139,14 +907,18 @@ template <vkc_type T> void reg_fused(std::vector<KernelDef> &t) {
     reg_cmp<T, 5>(t);
 }
 
+template <vkc_type T> ScanMake scan_make(int fold, bool by) {
+    return width_of(T) == 8 ? wide_scan(T, fold, by) : narrow_scan(T, fold, by);
+}
+
 // scan_<f>_T, scan_by_<f>_T, reduce_into_<f>_T (scan.rs:330-385): costs in+out widths, +1 for
 // scan_by, 8 + in + 2 out for reduce_into.
 template <vkc_type T, int F> void reg_fold(std::vector<KernelDef> &t) {
     constexpr vkc_type OT = F == F_ADD ? sum_type(T) : T;
     const std::string n = std::string(FOLD_NAMES[F]) + "_" + type_name(T);
     const uint64_t cost = width_of(T) + width_of(OT);
-    if (!has(t, "scan_" + n)) add_scan(t, "scan_" + n, {arr(T)}, OT, cost, make_scan_fam<T, F, false>);
-    if (!has(t, "scan_by_" + n)) add_scan(t, "scan_by_" + n, {arr(T), arr(VKC_BOOL)}, OT, cost + 1, make_scan_fam<T, F, true>);
+    if (!has(t, "scan_" + n)) add_scan(t, "scan_" + n, {arr(T)}, OT, cost, scan_make<T>(F, false));
+    if (!has(t, "scan_by_" + n)) add_scan(t, "scan_by_" + n, {arr(T), arr(VKC_BOOL)}, OT, cost + 1, scan_make<T>(F, true));
     if (!has(t, "reduce_into_" + n))
         add_whole(t, "reduce_into_" + n, {arr(VKC_I64), arr(T), sca(VKC_I64)}, OT, 8 + width_of(T) + 2 * width_of(OT),
                   reduce_into_fam<T, F>);

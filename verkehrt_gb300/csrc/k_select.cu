@@ -54,6 +54,7 @@ __device__ __forceinline__ unsigned nonzero_bytes(unsigned v) {
 // read from global memory instead of the slot.
 template <int KIND, int W, bool POS = false> struct SelectPass {
     static constexpr int THREADS = SEL_THREADS;
+    static constexpr bool ONE_READ = false;
     using R = CountRec;
     using V = unsigned long long;
     using T = typename Word<W>::T;

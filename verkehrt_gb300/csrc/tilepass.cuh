@@ -207,6 +207,16 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
 // Orders this thread's shared-memory accesses before later bulk copies into the same bytes.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// A bulk copy shared -> global (the same rules), as a group of its own of this thread, and the waits for
+// every such copy of the thread to have read its shared memory, and to be done.
+__device__ __forceinline__ void bulk_store(void *dst, const void *src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Waits for phase `parity` of `bar` to complete. On a wait that runs out it records a timeout
 // and waits once more, as long again, for the copy to land before the block goes on.
 __device__ __forceinline__ void mbar_wait(unsigned long long *bar, unsigned parity, DevStatus *status) {
@@ -240,6 +250,10 @@ __device__ __forceinline__ void mbar_wait(unsigned long long *bar, unsigned pari
 //   void flush(int tile, V pre, const Staged &, unsigned char *slot)
 //                                per compute warp: writes the slice given everything before it
 //   void last_tile(V inclusive)  run by one thread with the inclusive prefix of the last tile
+//   ONE_READ                     the tile is read once: V count(tile, slot, Staged &) stages it in
+//                                registers as well, the slot is free again after it, there is no
+//                                stage(), flush(tile, pre, const Staged &, after) gets the shared memory
+//                                behind the slots instead, and void finish() ends each compute warp
 // and the launch hands out `tiles` tiles. Returns true in every thread of the block that
 // finishes last (after a fence: it may read what every block wrote); that block has reset the
 // ticket counters for the next launch.
@@ -252,7 +266,7 @@ __device__ bool tile_pass(const Pass &p, typename Pass::R::W *recs, int tiles, u
     constexpr int NB = Pass::THREADS + 32;     // threads at each named barrier: compute + one warp
     constexpr int S = Pass::SLOTS;
     static_assert(WARPS <= 30, "one warp combines the slices of a tile");
-    static_assert(S >= 3 && S <= 8, "slots: one counted, one staged, at least one in flight");
+    static_assert(S >= (Pass::ONE_READ ? 2 : 3) && S <= 8, "slots: one counted, one staged, at least one in flight");
     static_assert(Pass::SLOT_BYTES % 16 == 0, "slots hold whole 16-byte units");
     constexpr int BAR_AGG = 1, BAR_PRE = 3, BAR_CNT = 5, BAR_FREE = 6;  // 2, 2, 1 and S ids
     extern __shared__ __align__(128) unsigned char tp_smem[];
@@ -260,6 +274,7 @@ __device__ bool tile_pass(const Pass &p, typename Pass::R::W *recs, int tiles, u
     __shared__ V s_agg[2][WARPS];             // slice aggregates (tile k in [k & 1])
     __shared__ V s_pre[2][WARPS];             // slice prefixes (everything before the slice)
     __shared__ int s_tile[S];                 // the tile in each slot (tile k in k % S), or `tiles`
+    __shared__ int s_id[2];                   // ONE_READ, whose slots are refilled early: tile k, or `tiles`
     __shared__ int s_last;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     auto slot_ptr = [&](int i) { return tp_smem + i * Pass::SLOT_BYTES; };
@@ -298,7 +313,7 @@ __device__ bool tile_pass(const Pass &p, typename Pass::R::W *recs, int tiles, u
         // starts on tile k, so each lookback overlaps the compute warps' stage, flush and next
         // count.
         named_sync_i<BAR_AGG, 2, NB>(0);
-        int cur = s_tile[0];
+        int cur = Pass::ONE_READ ? s_id[0] : s_tile[0];
         for (int k = 0; cur < tiles; ++k) {
             const V inc = warp_inclusive<R>(lane < WARPS ? s_agg[k & 1][lane] : R::ident());
             V ex = R::shfl_up(inc, 1);
@@ -313,7 +328,7 @@ __device__ bool tile_pass(const Pass &p, typename Pass::R::W *recs, int tiles, u
             if (lane < WARPS) s_pre[k & 1][lane] = R::op(pre, ex);
             named_arrive_i<BAR_PRE, 2, NB>(k & 1);
             named_sync_i<BAR_AGG, 2, NB>((k + 1) & 1);
-            cur = s_tile[(k + 1) % S];
+            cur = Pass::ONE_READ ? s_id[(k + 1) & 1] : s_tile[(k + 1) % S];
         }
     } else {
         // Compute warps. After each count, warp 0 publishes the tile's aggregate.
@@ -327,30 +342,58 @@ __device__ bool tile_pass(const Pass &p, typename Pass::R::W *recs, int tiles, u
             named_arrive_i<BAR_AGG, 2, NB>(k);
         };
         unsigned phase = 0;  // parity of the next wait, per slot
-        mbar_wait(&s_full[0], 0, status);
-        phase ^= 1u;
-        int cur = s_tile[0];
-        if (cur < tiles) {
-            const V a = p.count(cur, slot_ptr(0));
-            if (lane == 0) s_agg[0][w] = a;
-        }
-        counted(cur, 0);
-        for (int k = 0; cur < tiles; ++k) {
-            const int sc = k % S, sn = (k + 1) % S;
-            mbar_wait(&s_full[sn], (phase >> sn) & 1u, status);
-            phase ^= 1u << sn;
-            const int nxt = s_tile[sn];
-            if (nxt < tiles) {
-                const V a = p.count(nxt, slot_ptr(sn));
-                if (lane == 0) s_agg[(k + 1) & 1][w] = a;
+        if constexpr (Pass::ONE_READ) {
+            // Tile k is flushed after the count of tile k + 1.
+            typename Pass::Staged st, nst;
+            int cur = tiles;
+            for (int k = 0;; ++k) {
+                const int sn = k % S;
+                mbar_wait(&s_full[sn], (phase >> sn) & 1u, status);
+                phase ^= 1u << sn;
+                const int nxt = s_tile[sn];
+                if (nxt < tiles) {
+                    const V a = p.count(nxt, slot_ptr(sn), nst);
+                    if (lane == 0) s_agg[k & 1][w] = a;
+                    fence_proxy_async();
+                    named_arrive_i<BAR_FREE, S, NB>(sn);
+                }
+                if (threadIdx.x == 0) s_id[k & 1] = nxt;
+                counted(nxt, k & 1);
+                if (k > 0) {
+                    named_sync_i<BAR_PRE, 2, NB>((k - 1) & 1);
+                    p.flush(cur, s_pre[(k - 1) & 1][w], st, slot_ptr(S));
+                }
+                if (nxt >= tiles) break;
+                cur = nxt;
+                st = nst;
             }
-            counted(nxt, (k + 1) & 1);
-            const typename Pass::Staged st = p.stage(cur, slot_ptr(sc));
-            named_sync_i<BAR_PRE, 2, NB>(k & 1);
-            p.flush(cur, s_pre[k & 1][w], st, slot_ptr(sc));
-            fence_proxy_async();
-            named_arrive_i<BAR_FREE, S, NB>(sc);
-            cur = nxt;
+            p.finish();
+        } else {
+            mbar_wait(&s_full[0], 0, status);
+            phase ^= 1u;
+            int cur = s_tile[0];
+            if (cur < tiles) {
+                const V a = p.count(cur, slot_ptr(0));
+                if (lane == 0) s_agg[0][w] = a;
+            }
+            counted(cur, 0);
+            for (int k = 0; cur < tiles; ++k) {
+                const int sc = k % S, sn = (k + 1) % S;
+                mbar_wait(&s_full[sn], (phase >> sn) & 1u, status);
+                phase ^= 1u << sn;
+                const int nxt = s_tile[sn];
+                if (nxt < tiles) {
+                    const V a = p.count(nxt, slot_ptr(sn));
+                    if (lane == 0) s_agg[(k + 1) & 1][w] = a;
+                }
+                counted(nxt, (k + 1) & 1);
+                const typename Pass::Staged st = p.stage(cur, slot_ptr(sc));
+                named_sync_i<BAR_PRE, 2, NB>(k & 1);
+                p.flush(cur, s_pre[k & 1][w], st, slot_ptr(sc));
+                fence_proxy_async();
+                named_arrive_i<BAR_FREE, S, NB>(sc);
+                cur = nxt;
+            }
         }
     }
     __syncthreads();
