@@ -904,75 +904,23 @@ __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long lon
     return m;
 }
 
-// Resolves tile `tp` for lane L from the state s: the warp recomputes the tile's 32 segment
-// transfer functions from the rows (lane j = segment j) for the state's binade and the next,
-// applies them in order, and adds the rows of any segment they do not carry one by one. `held`: the
-// row values in shared memory (WalkSmem), or nullptr.
-template <int OP, bool SIGNED>
-__device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int tp, int L, unsigned long long s,
-                                           const unsigned long long *held) {
-    const int lane = threadIdx.x & 31;
-    unsigned long long v[CT_SEG_BLOCKS][2];
-    const int64_t blk0 = static_cast<int64_t>(tp) * CT_BLOCKS + lane * CT_SEG_BLOCKS;
-#pragma unroll
-    for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
-        if (held) {
-            v[i][0] = held[i * 32 + lane];
-            v[i][1] = 0;
-            continue;
-        }
-        int64_t b = blk0 + i;
-        unsigned long long xv = 0, yv = 0;
-        if (b < nb) {
-            xv = args.x[b * 16 + L];
-            if (OP == ROW_DOT) yv = args.y[b * 16 + L];
-            v[i][0] = row_value<OP>(args, xv, yv);
-        } else {
-            v[i][0] = 0;
-        }
-        v[i][1] = 0;
-    }
-    int seg = 0;
-    while (seg < CT_SEGS) {
-        const int E = state_binade(s);
-        if (E != NO_E && E >= -959) {
-            TF f{0, 0};
-            bool ok = lane >= seg && seg_tf<SIGNED>(v, 0, 1023 + E, &f);
-            if (lane < seg) {
-                f = TF{0, 0};
-                ok = true;  // already consumed: identity
-            }
-            unsigned long long r = s;
-            int m = apply_prefix<SIGNED>(f, ok, s, E, &r);
-            if (m > seg) {
-                s = r;
-                seg = m;
-                continue;
-            }
-        }
-        // Segment `seg` is not carried: its owner adds its rows one by one.
-        unsigned long long r = 0;
-        if (lane == seg) {
-            double d = as_f64(s);
-#pragma unroll
-            for (int i = 0; i < CT_SEG_BLOCKS; ++i) d = __dadd_rn(d, as_f64(v[i][0]));
-            r = as_bits(d);
-        }
-        s = __shfl_sync(FULL, r, seg);
-        ++seg;
-    }
-    return s;
-}
-
 // K4b: one block per lane. The block first copies the lane's chunk records, and the tile
 // records of the chunks without one ("mixed"), into shared memory; then warp 0 walks the tiles
 // from the lane's exact state: whole 32-tile chunks while their transfer function holds, single
 // tiles inside mixed chunks, and resolves from the rows the tiles that none carries (binade
 // crossings, negative or special rows, the first rows of the lane).
-constexpr int WK_THREADS = 256;
+//
+// One warp's chain of dependent steps bounds it, so that what can be made ahead is made by the other
+// warps: the segment functions of the tiles whose rows are held (made when the walk came to a crossing,
+// 2400 cycles each time, they were 36,000 of the 90,000 cycles of 2^20 rows; now 45,000 and 6000 ahead).
+// The rows, a sector each, cost the block's SM a cycle each; more loads in flight do not help.
+constexpr int WK_THREADS = 512;
 constexpr int WK_MAX_CHUNKS = 2048;  // chunk records held in shared memory (2^28 rows)
 constexpr int WK_MAX_MIXED = 48;     // mixed chunks whose tile records are held there
-constexpr int WK_MAX_ROWS = 40;      // tiles whose rows are held there: those likely to be resolved
+constexpr int WK_MAX_ROWS = 32;      // tiles whose rows are held there: those likely to be resolved
+constexpr int WK_FIRST_FN = 8;       // functions of a lane's first tile: its last eight binades
+constexpr int WK_MAX_FN = 2 * WK_MAX_ROWS + WK_FIRST_FN;
+constexpr unsigned long long FN_NONE = 1ull << 62;  // a segment without a function
 
 // The walk's progress over windows of the SM clock: a window in which it advanced fewer tiles
 // than the lane chain would (WALK_MIN_TILES in WALK_WINDOW cycles, about 2 tiles a microsecond)
@@ -1003,9 +951,112 @@ struct WalkSmem {
     TF mD[WK_MAX_MIXED][32][2];
     unsigned long long rows[WK_MAX_ROWS][CT_BLOCKS];  // row values, row r at (r % 8) * 32 + r / 8
     int tile_of[WK_MAX_ROWS];
+    // The functions of tile q's segments in binade fn_E[q] + i, at fn_at[q] + i: where each adds one
+    // increment whatever the parity (fn_plain) the sums of the increments through each, otherwise the
+    // functions as they are, d0 and d1 (halfway rows are common in the first binades: a row of 53 bits is
+    // one with probability 2^-k when k bits are rounded off).
+    unsigned long long fn[WK_MAX_FN][CT_SEGS], fn1[WK_MAX_FN][CT_SEGS];
+    bool fn_plain[WK_MAX_FN];
+    int fn_E[WK_MAX_ROWS], fn_n[WK_MAX_ROWS], fn_at[WK_MAX_ROWS];
     short rows_of[WK_MAX_MIXED][32];
     int nmixed, nrows;
 };
+
+// Resolves tile `tp` for lane L from the state s: the warp recomputes the tile's 32 segment
+// transfer functions from the rows (lane j = segment j) for the state's binade and the next,
+// applies them in order, and adds the rows of any segment they do not carry one by one. q >= 0: the
+// tile's rows are in sm.rows[q]. Their functions may be in sm.fn too (not SIGNED): then a run of
+// segments costs a few reads and a vote, or a composition, against the 2400 cycles of functions made and
+// composed here, and the segment of a crossing some 600, eight dependent additions.
+template <int OP, bool SIGNED>
+__device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int tp, int L, unsigned long long s,
+                                           const WalkSmem *sm, int q) {
+    const int lane = threadIdx.x & 31;
+    const unsigned long long *held = q >= 0 ? sm->rows[q] : nullptr;
+    int seg = 0;
+    if (!SIGNED && held && sm->fn_n[q] > 0) {
+        const int E0 = sm->fn_E[q], fn_n = sm->fn_n[q], at = sm->fn_at[q];
+        while (seg < CT_SEGS) {
+            const int E = state_binade(s);
+            if (E != NO_E) {
+                if (E < E0 || E >= E0 + fn_n) break;
+                const int e = at + E - E0;
+                int m;
+                if (sm->fn_plain[e]) {
+                    const unsigned long long *P = sm->fn[e];
+                    const unsigned long long before = seg ? P[seg - 1] : 0ull, S = (s & MANT) | ONE52;
+                    const unsigned out = __ballot_sync(FULL, lane >= seg && S + (P[lane] - before) >= (ONE52 << 1));
+                    m = out ? __ffs(out) - 1 : CT_SEGS;
+                    if (m > seg) s = (static_cast<unsigned long long>(E + 1023) << 52) | ((S + (P[m - 1] - before)) & MANT);
+                } else {
+                    const TF f = lane < seg ? TF{0, 0} : TF{sm->fn[e][lane], sm->fn1[e][lane]};
+                    unsigned long long r = s;
+                    m = apply_prefix<false>(f, f.d0 < FN_NONE, s, E, &r);
+                    if (m > seg) s = r;
+                }
+                if (m > seg) {
+                    seg = m;
+                    if (seg == CT_SEGS) break;
+                }
+            }
+            double d = as_f64(s);
+#pragma unroll
+            for (int i = 0; i < CT_SEG_BLOCKS; ++i) d = __dadd_rn(d, as_f64(held[i * 32 + seg]));
+            s = as_bits(d);
+            ++seg;
+        }
+        if (seg == CT_SEGS) return s;
+    }
+    unsigned long long v[CT_SEG_BLOCKS][2];
+    const int64_t blk0 = static_cast<int64_t>(tp) * CT_BLOCKS + lane * CT_SEG_BLOCKS;
+#pragma unroll
+    for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
+        if (held) {
+            v[i][0] = held[i * 32 + lane];
+            v[i][1] = 0;
+            continue;
+        }
+        int64_t b = blk0 + i;
+        unsigned long long xv = 0, yv = 0;
+        if (b < nb) {
+            xv = args.x[b * 16 + L];
+            if (OP == ROW_DOT) yv = args.y[b * 16 + L];
+            v[i][0] = row_value<OP>(args, xv, yv);
+        } else {
+            v[i][0] = 0;
+        }
+        v[i][1] = 0;
+    }
+    while (seg < CT_SEGS) {
+        const int E = state_binade(s);
+        if (E != NO_E && E >= -959) {
+            TF f{0, 0};
+            bool ok = lane >= seg && seg_tf<SIGNED>(v, 0, 1023 + E, &f);
+            if (lane < seg) {
+                f = TF{0, 0};
+                ok = true;  // already consumed: identity
+            }
+            unsigned long long r = s;
+            int m = apply_prefix<SIGNED>(f, ok, s, E, &r);
+            if (m > seg) {
+                s = r;
+                seg = m;
+                continue;
+            }
+        }
+        // Segment `seg` is not carried: its owner adds its rows one by one.
+        unsigned long long r = 0;
+        if (lane == seg) {
+            double d = as_f64(s);
+#pragma unroll
+            for (int i = 0; i < CT_SEG_BLOCKS; ++i) d = __dadd_rn(d, as_f64(v[i][0]));
+            r = as_bits(d);
+        }
+        s = __shfl_sync(FULL, r, seg);
+        ++seg;
+    }
+    return s;
+}
 
 // Chunk k of lane L tile by tile from state s (one warp): runs of tiles whose transfer
 // functions hold, and the tiles none carries resolved from the rows. RECORD (scans) stores the
@@ -1049,16 +1100,18 @@ __device__ __forceinline__ unsigned long long walk_chunk_tiles(const RowArgs &ar
             }
         }
         unsigned long long r = s, mine = 0;
-        const int mt = Et == NO_E ? 0 : apply_prefix<SIGNED>(g, usable, s, Et, &r, RECORD ? &mine : nullptr);
+        const int mt = __shfl_sync(FULL, usable, 0) ? apply_prefix<SIGNED>(g, usable, s, Et, &r, RECORD ? &mine : nullptr) : 0;
         if (mt > 0) {
             if (RECORD && lane + 1 < mt) rec[tp + lane + 1] = mine;
             s = r;
             tp += mt;
-        } else {
-            const int q = slot >= 0 ? sm->rows_of[slot][tp - k * 32] : -1;
-            s = resolve_tile<OP, SIGNED>(args, nb, tp, L, s, q >= 0 ? sm->rows[q] : nullptr);
-            ++tp;
+            if (tp >= end) break;
+            if (RECORD && lane == 0) rec[tp] = s;
         }
+        // The tile at which the run ended would end the next one too.
+        const int q = slot >= 0 ? sm->rows_of[slot][tp - k * 32] : -1;
+        s = resolve_tile<OP, SIGNED>(args, nb, tp, L, s, sm, q);
+        ++tp;
     }
     return s;
 }
@@ -1090,9 +1143,8 @@ __device__ __forceinline__ unsigned long long walk_lane(const RowArgs &args, int
             if (ce != NO_E && ce == E) f = held ? sm.chunkD[kc] : gD[kc];
         }
         unsigned long long r = s, mine = 0;
-        int m = E == NO_E ? 0
-                          : apply_prefix<SIGNED>(f, kc < C && ce != NO_E && ce == E, s, E, &r,
-                                                 RECORD ? &mine : nullptr);
+        const bool usable = kc < C && ce != NO_E && ce == E;
+        const int m = __shfl_sync(FULL, usable, 0) ? apply_prefix<SIGNED>(f, usable, s, E, &r, RECORD ? &mine : nullptr) : 0;
         if (m > 0) {
             if (RECORD) {
                 unsigned long long *rec = wk.tstate + static_cast<int64_t>(L) * (T + 1);
@@ -1102,9 +1154,9 @@ __device__ __forceinline__ unsigned long long walk_lane(const RowArgs &args, int
             }
             s = r;
             k += m;
-            continue;
+            if (m == 32 || k >= C) continue;
         }
-        // Chunk k, tile by tile.
+        // Chunk k, which ended the run, tile by tile.
         s = walk_chunk_tiles<OP, SIGNED, RECORD>(args, nb, T, wk, &sm, held ? sm.mixed_of[k] : -1, L, k, s,
                                                  &clk, RECORD ? nullptr : stop);
         if (*stop >= 0) return s;
@@ -1130,7 +1182,8 @@ __global__ void __launch_bounds__(WK_THREADS) canon_walk_kernel(RowArgs args, in
             sm.chunkE[c] = e;
             sm.chunkD[c] = gD[c];
             short slot = -1;
-            if (e == NO_E) {
+            // Without a function, or followed by a chunk of another binade: the sum may cross in its last tiles.
+            if (e == NO_E || (c + 1 < C && gE[c + 1] != e)) {
                 int k = atomicAdd(&sm.nmixed, 1);
                 if (k < WK_MAX_MIXED) {
                     slot = static_cast<short>(k);
@@ -1172,14 +1225,66 @@ __global__ void __launch_bounds__(WK_THREADS) canon_walk_kernel(RowArgs args, in
         __syncthreads();
         // The rows of those tiles, all in flight at once (a walk that loaded each tile's when it came
         // to it waited a DRAM round trip per crossing).
-        static_assert(WK_THREADS == CT_BLOCKS, "a thread per row of a lane's tile");
-        const int nr = min(sm.nrows, WK_MAX_ROWS);
+        static_assert(WK_THREADS % CT_BLOCKS == 0, "a thread per row of a lane's tile");
+        const int nr = min(sm.nrows, WK_MAX_ROWS), row = t % CT_BLOCKS;
 #pragma unroll 8
-        for (int k = 0; k < nr; ++k) {
-            const int64_t b = static_cast<int64_t>(sm.tile_of[k]) * CT_BLOCKS + t;
+        for (int k = t / CT_BLOCKS; k < nr; k += WK_THREADS / CT_BLOCKS) {
+            const int64_t b = static_cast<int64_t>(sm.tile_of[k]) * CT_BLOCKS + row;
             unsigned long long v = 0;
             if (b < nb) v = row_value<OP>(args, args.x[b * 16 + L], OP == ROW_DOT ? args.y[b * 16 + L] : 0ull);
-            sm.rows[k][(t % CT_SEG_BLOCKS) * 32 + t / CT_SEG_BLOCKS] = v;
+            sm.rows[k][(row % CT_SEG_BLOCKS) * 32 + row / CT_SEG_BLOCKS] = v;
+        }
+        // The binades whose functions are made ahead: the tile's candidates, or the last ones of the lane's
+        // first tile, which rises through many.
+        if (t < nr) {
+            const int tp = sm.tile_of[t];
+            const int2 c = *reinterpret_cast<const int2 *>(&wk.cand[(static_cast<int64_t>(tp) * 16 + L) * 2]);
+            int E0 = c.x, fns = c.x == NO_E ? 0 : (c.y == c.x + 1 ? 2 : 1), at = 2 * t;
+            if (tp == 0 && c.x == NO_E) {
+                const int E = binade(((fresh ? 0.0 : as_f64(state->lanes[L])) + static_cast<double>(wk.apx[static_cast<int64_t>(L) * T])) *
+                                     (1.0 + 0x1p-12));
+                if (E != NO_E && E - (WK_FIRST_FN - 1) >= -959) {
+                    E0 = E - (WK_FIRST_FN - 1);
+                    fns = WK_FIRST_FN;
+                    at = 2 * WK_MAX_ROWS;
+                }
+            }
+            sm.fn_E[t] = E0;
+            sm.fn_n[t] = fns;
+            sm.fn_at[t] = at;
+        }
+        __syncthreads();
+        // A warp each: the tile's segments in the lanes, as K3 makes them, and their sums.
+        if (wk.flags[T] == 0) {
+            const int lane = t & 31;
+            for (int e = t >> 5; e < WK_MAX_FN; e += WK_THREADS / 32) {
+                int q = e >> 1, i = e & 1;
+                if (e >= 2 * WK_MAX_ROWS) {
+                    i = e - 2 * WK_MAX_ROWS;
+                    for (q = 0; q < nr && sm.fn_at[q] != 2 * WK_MAX_ROWS;) ++q;
+                }
+                if (q >= nr || i >= sm.fn_n[q] || sm.fn_at[q] + i != e) continue;
+                unsigned long long v[CT_SEG_BLOCKS][2];
+#pragma unroll
+                for (int j = 0; j < CT_SEG_BLOCKS; ++j) {
+                    v[j][0] = sm.rows[q][j * 32 + lane];
+                    v[j][1] = 0;
+                }
+                TF f{0, 0};
+                const bool ok = seg_tf<false>(v, 0, 1023 + sm.fn_E[q] + i, &f);
+                unsigned long long d = ok ? f.d0 : FN_NONE;
+                const bool plain = __all_sync(FULL, ok && f.d0 == f.d1);
+                if (plain) {
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const unsigned long long y = __shfl_up_sync(FULL, d, o);
+                        if (lane >= o) d += y;
+                    }
+                }
+                sm.fn[e][lane] = d;
+                sm.fn1[e][lane] = f.d1;
+                if (lane == 0) sm.fn_plain[e] = plain;
+            }
         }
     }
     __syncthreads();
