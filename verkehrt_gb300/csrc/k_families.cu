@@ -4,8 +4,8 @@
 //
 //   reductions  reduce_add/mul/min/max_T, reduce_and/or/xor_T, argmin/argmax_T, any, all
 //               (src/kernels/scalar/reduce.rs:331-726)
-//   fused       dot/sumsq/count_<cmp>/filter_<cmp>/condsum_<cmp> on f32, i64, u64, i32
-//               (src/kernels/scalar/fused.rs:73-379)
+//   fused       dot/sumsq/count_<cmp>/condsum_<cmp> on f32, i64, u64, i32, and the entries of
+//               filter_<cmp> (k_select.cu's) (src/kernels/scalar/fused.rs:73-379)
 //   scans       scan_<fold>_T, scan_by_<fold>_T (their entries; the passes are fold_scan.cuh's),
 //               reduce_into_<fold>_T, prev_T
 //               (src/kernels/scalar/scan.rs:16-439)
@@ -638,41 +638,6 @@ vkc_status reduce_into_fam(vkc_ctx *ctx, const vkc_value *args, int nargs, vkc_v
     return VKC_OK;
 }
 
-// ------------------------------------------------------------------ filter on other types
-
-// filter_<cmp>_T (fused.rs:214-236): the rows with x <cmp> c, in order, through compress_T with
-// the comparison's mask.
-template <vkc_type T>
-__global__ void fam_mask_kernel(const void *x, int64_t n, int cmp, u64 c, unsigned char *m) {
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-        m[i] = cmp_test<T>(cmp, ld_word<T>(x, i), c) ? 1 : 0;
-}
-
-template <vkc_type T, int C>
-vkc_status filter_fam(vkc_ctx *ctx, const Arg *args, int nargs, int64_t base, Builder *out) {
-    vkc_status st;
-    if (nargs != 2) return fail(ctx, VKC_RUNTIME, arity_error(2, nargs));
-    if (!rows_arg(ctx, args[0], T, &st) || !splat_arg(ctx, args[1], T, &st)) return st;
-    const int64_t n = args[0].len();
-    if (n == 0) return VKC_OK;
-    vkc_array *m;
-    if ((st = new_array(ctx, VKC_BOOL, n, false, &m))) return st;
-    const int g = stream_grid(ctx, n, 256, 8, 2048);
-    fam_mask_kernel<T><<<g, 256, 0, ctx->stream>>>(args[0].a->data(), n, C, scalar_word(T, args[1].s),
-                                                   static_cast<unsigned char *>(m->data()));
-    if ((st = launched(ctx, "family_mask"))) {
-        vkc_array_release(m);
-        return st;
-    }
-    static const KernelDef *comp = nullptr;
-    if (!comp) comp = kernel_def((std::string("compress_") + type_name(T)).c_str());
-    Arg ca[2] = {args[0], Arg{true, m, vkc_scalar{}}};
-    st = comp->sel(ctx, ca, 2, base, out);
-    vkc_array_release(m);
-    return st;
-}
-
 // ------------------------------------------------------------------ whole kernels
 
 // Widens keys to i64 for the i64 group ids (any one-to-one image serves).
@@ -877,7 +842,7 @@ template <vkc_type T, int C> void reg_cmp(std::vector<KernelDef> &t) {
     add_red(t, "count_" + c + "_" + n, {arr(T), sca(T)}, VKC_I64, w,
             [](vkc_ctx *x) { return make_fold<T, F_ADD, R_PRED, 2>(x, VKC_I64, C, false, ""); });
     KernelDef f{"filter_" + c + "_" + n, VKC_SELECTION, {arr(T), sca(T)}, true, T, 2 * w};
-    f.sel = filter_fam<T, C>;
+    f.sel = filter_fn(T, C);
     t.push_back(f);
     if (T == VKC_F32)
         add_red(t, "condsum_" + c + "_" + n, {arr(T), sca(T), sca(T)}, T, w,

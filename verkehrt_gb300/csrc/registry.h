@@ -87,6 +87,9 @@ struct KernelDef {
 // The table's entry of that name (for entries built from other entries), or nullptr.
 const KernelDef *kernel_def(const char *name);
 
+// The entry of filter_<cmp>_T (eq, ne, lt, le, gt, ge) of a 4- or 8-byte type (k_select.cu).
+SelectFn filter_fn(vkc_type t, int cmp);
+
 // Registration by family (called once, in this order, to build the table).
 void register_construct(std::vector<KernelDef> &t);
 void register_reduce(std::vector<KernelDef> &t);

@@ -214,7 +214,9 @@ __device__ __forceinline__ void bulk_store(void *dst, const void *src, unsigned 
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
-__device__ __forceinline__ void bulk_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+template <int PENDING = 0> __device__ __forceinline__ void bulk_store_wait_read() {  // but the last PENDING
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory");
+}
 __device__ __forceinline__ void bulk_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Waits for phase `parity` of `bar` to complete. On a wait that runs out it records a timeout
