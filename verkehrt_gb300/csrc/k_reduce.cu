@@ -254,6 +254,8 @@ __global__ void __launch_bounds__(256) extreme_kernel(const long long *__restric
     };
     unsigned long long bi = ~0ull, nan = ~0ull;
     if (ARG) {
+        // Integer rows that are all the worst value better none: the first of them.
+        if (!F64 && any && bpos == ~0u) bpos = 0;
         if (bpos != ~0u) bi = row_of(bpos);
         if (npos != ~0u) nan = row_of(npos);
     } else {
