@@ -142,20 +142,41 @@ struct RowArgs {
     int cmp;
     u64 c, e;
 };
-template <vkc_type T, int ROW> __device__ __forceinline__ u64 row_value(const RowArgs &a, int64_t i) {
-    const u64 v = ld_word<T>(a.x, i);
-    if (ROW == R_DOT) return mul_t<T>(v, ld_word<T>(a.y, i));
+template <vkc_type T, int ROW> __device__ __forceinline__ u64 row_value(const RowArgs &a, u64 v, u64 y) {
+    if (ROW == R_DOT) return mul_t<T>(v, y);
     if (ROW == R_SUMSQ) return mul_t<T>(v, v);
     if (ROW == R_COND) return cmp_test<T>(a.cmp, v, a.c) ? v : a.e;
     if (ROW == R_PRED) return cmp_test<T>(a.cmp, v, a.c) ? 1ull : 0ull;
     return v;
 }
 
+template <vkc_type T, int ROW> __device__ __forceinline__ u64 row_at(const RowArgs &a, int64_t i) {
+    return row_value<T, ROW>(a, ld_word<T>(a.x, i), ROW == R_DOT ? ld_word<T>(a.y, i) : 0ull);
+}
+
+// Element k of a 16-byte unit, as a word.
+template <vkc_type T> __device__ __forceinline__ u64 unit_word(const uint4 &q, int k) {
+    const unsigned w[4] = {q.x, q.y, q.z, q.w};
+    if (width_of(T) == 8) return w[2 * k] | static_cast<u64>(w[2 * k + 1]) << 32;
+    if (T == VKC_F32) return w[k];
+    if (T == VKC_I32) return static_cast<u64>(static_cast<long long>(static_cast<int>(w[k])));
+    return (w[k >> 2] >> (8 * (k & 3))) & 0xffu;
+}
+
+// Rows before the first 16-byte unit of `p`, at most n.
+template <vkc_type T> __device__ __forceinline__ int64_t unit_head(const void *p, int64_t n) {
+    const int64_t h = static_cast<int64_t>((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15) / width_of(T);
+    return h < n ? h : n;
+}
+
 // ------------------------------------------------------------------ order-free folds
 
-// Every block folds its rows (grid-stride, four rows in flight per thread), the warps and the
-// block combine (the fold is commutative), and the last block to finish folds the block
-// partials into the reducer's state word.
+// Every block folds its rows (grid-stride, four 16-byte loads in flight per thread; the rows outside
+// the 16-byte grid, and all of a dot product whose columns lie differently on it, one by one), the warps
+// and the block combine (the fold is commutative), and the last block to finish folds the block
+// partials into the reducer's state word. (Loads of one element,
+// 2^26 rows: reduce_max_i32 316 us a call, now 75, reduce_add_i32 317 and 56, dot_i32 230 and 91, count_gt_f32
+// 217 and 58.)
 template <vkc_type T, int F, int ROW>
 __global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64 *partials, unsigned *done, bool fresh, u64 *state,
                                                        u64 *host) {
@@ -163,13 +184,32 @@ __global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64
     u64 acc = identity<AT, F>();
     const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = tid; i < n; i += 4 * stride) {
-        u64 v[4];
+    constexpr int E = 16 / width_of(T);  // rows of a unit
+    constexpr int U = ROW == R_DOT ? 2 : 4;
+    const bool alike = ROW != R_DOT || ((reinterpret_cast<uintptr_t>(a.x) ^ reinterpret_cast<uintptr_t>(a.y)) & 15) == 0;
+    const int64_t head = alike ? unit_head<T>(a.x, n) : n;
+    const int64_t units = (n - head) / E;
+    const auto *x = reinterpret_cast<const uint4 *>(static_cast<const unsigned char *>(a.x) + head * width_of(T));
+    const auto *y = reinterpret_cast<const uint4 *>(static_cast<const unsigned char *>(a.y) + head * width_of(T));
+    auto unit = [&](const uint4 &p, const uint4 &q) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = i + u * stride < n ? row_value<T, ROW>(a, i + u * stride) : identity<AT, F>();
+        for (int k = 0; k < E; ++k)
+            acc = step<AT, F>(acc, row_value<T, ROW>(a, unit_word<T>(p, k), ROW == R_DOT ? unit_word<T>(q, k) : 0ull));
+    };
+    int64_t i = tid;
+    for (; i + (U - 1) * stride < units; i += U * stride) {
+        uint4 p[U], q[U];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) acc = step<AT, F>(acc, v[u]);
+        for (int u = 0; u < U; ++u) {
+            p[u] = __ldcs(x + i + u * stride);
+            q[u] = ROW == R_DOT ? __ldcs(y + i + u * stride) : uint4{};
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) unit(p[u], q[u]);
     }
+    for (; i < units; i += stride) unit(x[i], ROW == R_DOT ? y[i] : uint4{});
+    for (int64_t r = tid; r < head; r += stride) acc = step<AT, F>(acc, row_at<T, ROW>(a, r));
+    for (int64_t r = head + units * E + tid; r < n; r += stride) acc = step<AT, F>(acc, row_at<T, ROW>(a, r));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc = step<AT, F>(acc, __shfl_xor_sync(FULL, acc, o));
     __shared__ u64 ws[8];
@@ -219,7 +259,39 @@ __global__ void __launch_bounds__(256) fam_arg_kernel(const void *x, int64_t n, 
     u64 h = ~0ull, r = ~0ull;
     const int64_t tid = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-    for (int64_t i = tid; i < n; i += stride) arg_better(h, r, arg_key<T, MAX>(ld_word<T>(x, i)), base + static_cast<u64>(i));
+    // Four 16-byte loads in flight a thread, as in the folds; a thread's units come in row order, so that a
+    // strict comparison keeps the first row, as a position (unit of the thread, element) until the end.
+    constexpr int E = 16 / width_of(T);
+    const int64_t head = unit_head<T>(x, n), units = (n - head) / E;
+    const auto *xu = reinterpret_cast<const uint4 *>(static_cast<const unsigned char *>(x) + head * width_of(T));
+    int64_t at = -1;  // the best's unit
+    unsigned k_at = 0;
+    auto unit = [&](const uint4 &p, int64_t u) {
+        const u64 before = h;
+        if (at < 0) at = u;  // element 0 unless another is better (all may have the key ~0)
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            const u64 key = arg_key<T, MAX>(unit_word<T>(p, k));
+            if (key < h) {
+                h = key;
+                k_at = k;
+            }
+        }
+        if (h != before) at = u;
+    };
+    int64_t i = tid;
+    for (; i + 3 * stride < units; i += 4 * stride) {
+        uint4 p[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) p[u] = __ldcs(xu + i + u * stride);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) unit(p[u], i + u * stride);
+    }
+    for (; i < units; i += stride) unit(xu[i], i);
+    if (at >= 0) r = base + static_cast<u64>(head + at * E + k_at);
+    auto one = [&](int64_t q) { arg_better(h, r, arg_key<T, MAX>(ld_word<T>(x, q)), base + static_cast<u64>(q)); };
+    for (int64_t q = tid; q < head; q += stride) one(q);
+    for (int64_t q = head + units * E + tid; q < n; q += stride) one(q);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) arg_better(h, r, __shfl_xor_sync(FULL, h, o), __shfl_xor_sync(FULL, r, o));
     __shared__ u64 wh[8], wr[8];
