@@ -22,6 +22,7 @@
 //    arrays' numbers, found again from the positions.)
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <type_traits>
 #include <vector>
@@ -56,7 +57,9 @@ struct vkc_batch {
     void *img[2] = {nullptr, nullptr};  // 64-bit images of `total` rows each
     unsigned *pos[2] = {nullptr, nullptr};
     unsigned *counts = nullptr, *offs = nullptr, *sums = nullptr;
-    const vkc_batch *out_batch = nullptr;  // the batch whose pointers `outs` holds
+    const vkc_batch *out_batch = nullptr;  // the batch whose pointers `outs` and `segs` hold
+    std::unique_ptr<vkc::DeviceMem> segs;  // SortSeg[n] and each tile's array, when arrays are sorted for themselves
+    int seg_tiles = 0, seg_tile = 0;       // their tiles, or 0, and a tile's rows
 };
 
 namespace vkc {
@@ -250,10 +253,6 @@ __device__ __forceinline__ int batch_chunk_array(const int64_t *__restrict__ chu
 // sign-flipped image (NUMBER = false: the digits alone). One block per chunk: a search a block, not
 // one a row, and 12 bytes moved a row (the former pass wrote 64-bit images and positions from a grid
 // over the arrays: 326 us for 63 M rows).
-struct BatchDigits {
-    int n;
-    int shift[8];
-};
 template <class IMG, bool NUMBER>
 __global__ void __launch_bounds__(256) batch_images_kernel(const BSeg *__restrict__ segs, int nseg,
                                                            const int64_t *__restrict__ chunks, BatchDigits d,
@@ -448,6 +447,52 @@ extern "C" VKC_API vkc_status vkc_batch_dot_f64(vkc_ctx *ctx, vkc_batch *xs, vkc
     return launched(ctx, "batch_dot");
 }
 
+namespace vkc {
+
+// Whether each array is sorted for itself, in how many tiles of how many rows. A pass for each key digit
+// and none for the array's number, no images made before the first, one output array a tile; but a tile
+// holds rows of one array, so that short arrays leave it mostly empty: from half-full tiles of 2048 rows on
+// it is the faster way for any number of digits (4096 arrays of 1387 rows on average, 1 / 2 / 4 / 8 digits:
+// 119 / 190 / 340 / 672 us a call against 227 / 285 / 437 / 731 with the number in the image; of 967 rows,
+// 47% full, 8 digits 629 against 595). Tiles of 3072 rows are the better ones for longer arrays (4096 of
+// 15.5 K rows, 2 digits: 866 us, 921 in 2048, 857 in 4096, 1663 with the number; of 2774 rows 267 and 250).
+static void plan_segs(vkc_batch *b) {
+    b->seg_tile = b->total >= 4096 * static_cast<int64_t>(b->host.size()) ? 3072 : 2048;
+    int64_t tiles = 0;
+    for (const BSeg &g : b->host) tiles += (g.n + b->seg_tile - 1) / b->seg_tile;
+    b->seg_tiles = b->total >= tiles * (b->seg_tile / 2) ? static_cast<int>(tiles) : 0;
+}
+
+// The table of the arrays in the concatenation's order and of their tiles.
+static vkc_status upload_segs(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *outs) {
+    const size_t n = keys->arrays.size(), bytes = sizeof(SortSeg) * n + sizeof(int) * keys->seg_tiles;
+    std::vector<unsigned char> table(bytes);
+    auto *segs = reinterpret_cast<SortSeg *>(table.data());
+    int *tile = reinterpret_cast<int *>(segs + n);
+    int64_t base = 0, t = 0;
+    for (size_t i = 0; i < n; ++i) {
+        const vkc_array *a = keys->arrays[i];
+        segs[i] = SortSeg{static_cast<const unsigned long long *>(a->data()), static_cast<long long *>(outs->arrays[i]->data()), base,
+                          a->len, t};
+        for (int64_t j = 0; j < a->len; j += keys->seg_tile) tile[t++] = static_cast<int>(i);
+        base += a->len;
+    }
+    void *p = nullptr, *h;
+    VKC_CUDA(ctx, cudaMallocAsync(&p, bytes, ctx->stream));
+    keys->segs = std::make_unique<DeviceMem>();
+    keys->segs->ptr = p;
+    keys->segs->box = ctx->box;
+    vkc_status st;
+    if ((st = pinned(ctx, bytes, &h))) return st;
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    memcpy(h, table.data(), bytes);
+    VKC_CUDA(ctx, cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return VKC_OK;
+}
+
+}  // namespace vkc
+
 extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *outs,
                                                     unsigned key_digits) {
     if (!ctx || !keys || !outs) return VKC_USAGE;
@@ -471,6 +516,11 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
         keys->scratch.clear();
         int64_t cw, sw;
         radix_table_words(total, &cw, &sw);
+        plan_segs(keys);
+        if (keys->seg_tiles) {
+            cw = std::max(cw, int64_t(256) * keys->seg_tiles);
+            sw = std::max(sw, scan_counts_sum_words(cw));
+        }
         vkc_array *a[7];
         const vkc_type ty[7] = {VKC_U64, VKC_U64, VKC_I32, VKC_I32, VKC_I32, VKC_I32, VKC_I32};
         const int64_t len[7] = {total, total, total, total, cw, cw, sw};
@@ -497,6 +547,7 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
         memcpy(h, optr.data(), sizeof(long long *) * n);
         VKC_CUDA(ctx, cudaMemcpyAsync(p, h, sizeof(long long *) * n, cudaMemcpyHostToDevice, ctx->stream));
         VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        if (keys->seg_tiles && (st = upload_segs(ctx, keys, outs))) return st;
         keys->out_batch = outs;
     }
     if (n > 65536) return fail(ctx, VKC_USAGE, "batch argsort of more than 65536 arrays");
@@ -510,6 +561,12 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
     BatchDigits d{};
     for (int k = 0; k < 8; ++k)
         if ((key_digits >> k) & 1u) d.shift[d.n++] = 8 * k;
+    d.run = d.shift[d.n - 1] - d.shift[0] == 8 * (d.n - 1);
+    if (keys->seg_tiles) {
+        const auto *segs = static_cast<const SortSeg *>(keys->segs->ptr);
+        return radix_segs(ctx, BatchSegs{segs, reinterpret_cast<const int *>(segs + n), keys->seg_tiles, keys->seg_tile, d}, keys->img,
+                          keys->pos, total, RadixTables{keys->counts, keys->offs, keys->sums});
+    }
     const int numbers = n > 256 ? 2 : 1, digits = d.n + numbers;
     int shifts[8];
     for (int k = 0; k < 8; ++k) shifts[k] = 8 * k;

@@ -109,22 +109,88 @@ __global__ void __launch_bounds__(256) rs_range_kernel(KeySource k, int64_t n, u
     }
 }
 
+// Where a pass reads and writes. W (template): keys of W bytes with the row numbers as payloads
+// (the first pass of a sort), or 0: images and payloads. OUT (template): images and payloads, the
+// payloads alone as i64 rows (the last pass of an argsort), or each array's rows to its own output
+// (the last pass of a batched argsort, whose images hold the array's number above `index_shift`).
+enum RsOut { OUT_PAIRS = 0, OUT_ROWS = 1, OUT_BATCH = 2 };
+template <class IMG, class PAY> struct RsArgs {
+    KeySource k;
+    const IMG *img_in;
+    const PAY *pay_in;
+    IMG *img_out;
+    PAY *pay_out;
+    long long *out;
+    BatchOut batch;
+    // SEG passes: the arrays, and each tile's; the digits of the images.
+    const SortSeg *segs;
+    const int *tile_seg;
+    BatchDigits digits;
+};
+
+// What a block works on. SEG (template): every tile belongs to one array, whose rows are sorted among
+// themselves: the counts lie array-major, in an array digit-major, so that their one exclusive scan gives
+// each (array, digit, tile) its first row of the concatenation.
+struct RsTile {
+    int64_t row0, end;   // its rows
+    int64_t at, stride;  // digit d's count is number at + d * stride
+};
+template <bool SEG, int TILE> __device__ __forceinline__ RsTile rs_tile(const SortSeg &seg, int64_t n, int tiles, int tile) {
+    if constexpr (SEG) {
+        const int64_t j = tile - seg.tile0, r = j * TILE;
+        return RsTile{seg.base + r, min(seg.base + r + TILE, seg.base + seg.n), static_cast<int64_t>(RADIX) * seg.tile0 + j,
+                      (seg.n + TILE - 1) / TILE};
+    } else {
+        const int64_t r = static_cast<int64_t>(tile) * TILE;
+        return RsTile{r, min(r + TILE, n), tile, tiles};
+    }
+}
+// The images of rows r0 + 32 j of array `seg` (those below `end`): the chosen digits of the key side by
+// side, with `run` as many above the last one as the image holds, which no pass looks at. The loads are all
+// in flight together (a choice of digits between them took the first pass from 580 to 300 us, 63 M rows).
+template <int ITEMS, bool WHOLE, class IMG>
+__device__ __forceinline__ void seg_images(const SortSeg &seg, const BatchDigits &d, int64_t r0, int64_t end, IMG (&img)[ITEMS]) {
+    const unsigned long long *k = seg.keys + (r0 - seg.base);
+    const int sh = d.shift[0];
+    if (d.run) {
+#pragma unroll
+        for (int j = 0; j < ITEMS; ++j)
+            img[j] = WHOLE || r0 + j * 32 < end ? static_cast<IMG>((__ldcs(k + j * 32) ^ 0x8000000000000000ull) >> sh) : IMG(0);
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+        const unsigned long long key = WHOLE || r0 + j * 32 < end ? __ldcs(k + j * 32) ^ 0x8000000000000000ull : 0ull;
+        unsigned long long im = 0;
+        for (int i = 0; i < d.n; ++i) im |= ((key >> d.shift[i]) & 0xffull) << (8 * i);
+        img[j] = static_cast<IMG>(im);
+    }
+}
+
 // Up: the digit counts of every tile, digit-major: counts[d * tiles + tile]. Shared-memory
 // atomics into one histogram per warp (the order of the increments does not matter here). W: the
 // first pass, from keys of W bytes; 0: from images.
-template <int RS_ITEMS, int W, class IMG>
+template <int RS_ITEMS, int W, bool SEG, class IMG>
 __global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IMG *__restrict__ img_in, int64_t n,
-                                                           int shift, int tiles, unsigned *__restrict__ counts) {
+                                                           int shift, int tiles, unsigned *__restrict__ counts,
+                                                           const SortSeg *segs, const int *tile_seg, BatchDigits digits) {
     constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     __shared__ unsigned s_cnt[RS_WARPS][RADIX];
     const int tile = blockIdx.x;
+    const SortSeg seg = SEG ? segs[tile_seg[tile]] : SortSeg{};
+    const RsTile tl = rs_tile<SEG, RS_TILE>(seg, n, tiles, tile);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (int i = threadIdx.x; i < RS_WARPS * RADIX; i += RS_THREADS) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
-    const int64_t base = static_cast<int64_t>(tile) * RS_TILE + static_cast<int64_t>(w) * (32 * RS_ITEMS);
-    if (base + 32 * RS_ITEMS <= n) {
+    const int64_t base = tl.row0 + static_cast<int64_t>(w) * (32 * RS_ITEMS);
+    if (base + 32 * RS_ITEMS <= tl.end) {
         IMG img[RS_ITEMS];
-        if constexpr (W != 0) {
+        if constexpr (SEG && W != 0) {
+            seg_images<RS_ITEMS, true>(seg, digits, base + lane, tl.end, img);
+        } else if constexpr (SEG) {
+#pragma unroll
+            for (int j = 0; j < RS_ITEMS; ++j) img[j] = __ldcs(img_in + base + j * 32 + lane);
+        } else if constexpr (W != 0) {
 #pragma unroll
             for (int j = 0; j < RS_ITEMS; ++j) img[j] = static_cast<IMG>(key_image<W>(k, base + j * 32 + lane));
         } else {
@@ -145,11 +211,22 @@ __global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IM
         }
 #pragma unroll
         for (int j = 0; j < RS_ITEMS; ++j) atomicAdd(&s_cnt[w][static_cast<unsigned>(img[j] >> shift) & 0xffu], 1u);
+    } else if constexpr (SEG) {
+        IMG img[RS_ITEMS];
+        if constexpr (W != 0) {
+            seg_images<RS_ITEMS, false>(seg, digits, base + lane, tl.end, img);
+        } else {
+#pragma unroll
+            for (int j = 0; j < RS_ITEMS; ++j) img[j] = base + j * 32 + lane < tl.end ? __ldcs(img_in + base + j * 32 + lane) : IMG(0);
+        }
+#pragma unroll
+        for (int j = 0; j < RS_ITEMS; ++j)
+            if (base + j * 32 + lane < tl.end) atomicAdd(&s_cnt[w][static_cast<unsigned>(img[j] >> shift) & 0xffu], 1u);
     } else {
         for (int j = 0; j < RS_ITEMS; ++j) {
             const int64_t r = base + j * 32 + lane;
-            if (r < n) {
-                const IMG im = W != 0 ? static_cast<IMG>(key_image<W ? W : 8>(k, r)) : img_in[r];
+            if (r < tl.end) {
+                const IMG im = W == 0 ? img_in[r] : static_cast<IMG>(key_image<W ? W : 8>(k, r));
                 atomicAdd(&s_cnt[w][static_cast<unsigned>(im >> shift) & 0xffu], 1u);
             }
         }
@@ -159,7 +236,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IM
     unsigned total = 0;
 #pragma unroll
     for (int ww = 0; ww < RS_WARPS; ++ww) total += s_cnt[ww][d];
-    counts[static_cast<int64_t>(d) * tiles + tile] = total;
+    counts[tl.at + d * tl.stride] = total;
 }
 
 // The lanes of the warp whose 8-bit digit equals this lane's, among the lanes of `valid`: one
@@ -270,21 +347,6 @@ void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, uns
         rs_scan_apply<false><<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
 }
 
-// Where a pass reads and writes. W (template): keys of W bytes with the row numbers as payloads
-// (the first pass of a sort), or 0: images and payloads. OUT (template): images and payloads, the
-// payloads alone as i64 rows (the last pass of an argsort), or each array's rows to its own output
-// (the last pass of a batched argsort, whose images hold the array's number above `index_shift`).
-enum RsOut { OUT_PAIRS = 0, OUT_ROWS = 1, OUT_BATCH = 2 };
-template <class IMG, class PAY> struct RsArgs {
-    KeySource k;
-    const IMG *img_in;
-    const PAY *pay_in;
-    IMG *img_out;
-    PAY *pay_out;
-    long long *out;
-    BatchOut batch;
-};
-
 // Down: one pass over digit `shift` with the tile's first output row per digit in
 // offsets[d * tiles + tile]. Bound by issue and by its shared-memory wavefronts: 40 M rows of 32-bit
 // images take about 170 us (190 with two table lookups a row and three blocks an SM) against 95 us
@@ -298,22 +360,24 @@ struct __align__(16) RsShared {
 
 // The body of a down tile; WHOLE when every row of the tile is below n (all but the last
 // tile), which drops the per-row bounds checks.
-template <int RS_ITEMS, int W, int OUT, class IMG, class PAY, bool WHOLE>
-__device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, int64_t n, int shift, int tile, RsShared &sm,
-                                             unsigned char *smem) {
+template <int RS_ITEMS, int W, int OUT, bool SEG, class IMG, class PAY, bool WHOLE>
+__device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, const SortSeg &seg, const RsTile &tl, int shift,
+                                             RsShared &sm, unsigned char *smem) {
     constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     // Rows of this warp: warp-striped, row = base + j*32 + lane, so (j, lane) is row order.
-    const int64_t base = static_cast<int64_t>(tile) * RS_TILE + static_cast<int64_t>(w) * (32 * RS_ITEMS);
+    const int64_t base = tl.row0 + static_cast<int64_t>(w) * (32 * RS_ITEMS);
     IMG img[RS_ITEMS];
     PAY pay[W ? 1 : RS_ITEMS];
     unsigned rank2[RS_ITEMS / 2];  // two 16-bit ranks per word
     const unsigned lt = (1u << lane) - 1;
+    if constexpr (SEG && W != 0) seg_images<RS_ITEMS, WHOLE>(seg, a.digits, base + lane, tl.end, img);
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j) {
         const int64_t r = base + j * 32 + lane;
-        const bool in = WHOLE || r < n;
-        if constexpr (W != 0) {
+        const bool in = WHOLE || r < tl.end;
+        if constexpr (SEG && W != 0) {
+        } else if constexpr (W != 0) {
             img[j] = in ? static_cast<IMG>(key_image<W>(a.k, r)) : IMG(0);
         } else {
             img[j] = in ? __ldcs(a.img_in + r) : IMG(0);
@@ -322,7 +386,7 @@ __device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, int64_t 
     }
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j) {
-        const bool in = WHOLE || base + j * 32 + lane < n;
+        const bool in = WHOLE || base + j * 32 + lane < tl.end;
         const unsigned d = static_cast<unsigned>(img[j] >> shift) & 0xffu;
         // Rank among this warp's earlier rows with the same digit.
         const unsigned peers = digit_peers(d, WHOLE ? FULL : __ballot_sync(FULL, in));
@@ -361,20 +425,23 @@ __device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, int64_t 
     IMG *s_img = reinterpret_cast<IMG *>(smem + sizeof(PAY) * RS_TILE);
 #pragma unroll
     for (int j = 0; j < RS_ITEMS; ++j) {
-        if (WHOLE || base + j * 32 + lane < n) {
+        if (WHOLE || base + j * 32 + lane < tl.end) {
             const unsigned l = sm.w[w][static_cast<unsigned>(img[j] >> shift) & 0xffu] +
                                ((rank2[j / 2] >> (16 * (j & 1))) & 0xffffu);
             s_img[l] = img[j];
-            if constexpr (W != 0) s_pay[l] = static_cast<PAY>(base + j * 32 + lane);
+            if constexpr (W != 0) s_pay[l] = static_cast<PAY>(base + j * 32 + lane - (SEG ? seg.base : 0));
             else s_pay[l] = pay[j];
         }
     }
     __syncthreads();
+    long long *const out = seg.out - seg.base;
     auto put = [&](int l) {
         const IMG im = s_img[l];
         const unsigned dst = sm.excl[static_cast<unsigned>(im >> shift) & 0xffu] + static_cast<unsigned>(l);
         if constexpr (OUT == OUT_ROWS) {
             a.out[dst] = static_cast<long long>(s_pay[l]);
+        } else if constexpr (OUT == OUT_BATCH && SEG) {
+            out[dst] = static_cast<long long>(s_pay[l]);
         } else if constexpr (OUT == OUT_BATCH) {
             const unsigned i = static_cast<unsigned>(im >> a.batch.index_shift);
             const int64_t first = __ldg(a.batch.bases + i);
@@ -388,39 +455,42 @@ __device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, int64_t 
 #pragma unroll
         for (int i = 0; i < RS_ITEMS; ++i) put(static_cast<int>(threadIdx.x) + i * RS_THREADS);
     } else {
-        const int rows = static_cast<int>(n - static_cast<int64_t>(tile) * RS_TILE);
+        const int rows = static_cast<int>(tl.end - tl.row0);
         for (int l = threadIdx.x; l < rows; l += RS_THREADS) put(l);
     }
 }
 
-template <int RS_ITEMS, int W, int OUT, class IMG, class PAY>
+template <int RS_ITEMS, int W, int OUT, bool SEG, class IMG, class PAY>
 __global__ void __launch_bounds__(RS_THREADS, (RsShape<RS_ITEMS, sizeof(IMG) + sizeof(PAY)>::MIN_BLOCKS))
     rs_down_kernel(RsArgs<IMG, PAY> a, int64_t n, int shift, int tiles, const unsigned *__restrict__ offsets) {
     __shared__ RsShared sm;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     const int tile = blockIdx.x;
+    const SortSeg seg = SEG ? a.segs[a.tile_seg[tile]] : SortSeg{};
+    const RsTile tl = rs_tile<SEG, RS_THREADS * RS_ITEMS>(seg, n, tiles, tile);
     for (int i = threadIdx.x; i < RS_WARPS * RADIX / 2; i += RS_THREADS) reinterpret_cast<unsigned *>(&sm.w[0][0])[i] = 0u;
-    sm.excl[threadIdx.x] = offsets[static_cast<int64_t>(threadIdx.x) * tiles + tile];  // RS_THREADS == RADIX
+    sm.excl[threadIdx.x] = offsets[tl.at + threadIdx.x * tl.stride];  // RS_THREADS == RADIX
     __syncthreads();
-    if (static_cast<int64_t>(tile + 1) * (RS_THREADS * RS_ITEMS) <= n)
-        rs_down_tile<RS_ITEMS, W, OUT, IMG, PAY, true>(a, n, shift, tile, sm, rs_smem);
+    if (tl.row0 + RS_THREADS * RS_ITEMS <= tl.end)
+        rs_down_tile<RS_ITEMS, W, OUT, SEG, IMG, PAY, true>(a, seg, tl, shift, sm, rs_smem);
     else
-        rs_down_tile<RS_ITEMS, W, OUT, IMG, PAY, false>(a, n, shift, tile, sm, rs_smem);
+        rs_down_tile<RS_ITEMS, W, OUT, SEG, IMG, PAY, false>(a, seg, tl, shift, sm, rs_smem);
 }
 
 // One pass in the tuned shape: up, the scan, down.
-template <int ITEMS, int W, int OUT, class IMG, class PAY>
-static void radix_pass_shape(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t) {
+template <int ITEMS, int W, int OUT, class IMG, class PAY, bool SEG = false>
+static void radix_pass_shape(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t, int seg_tiles = 0) {
     using S = RsShape<ITEMS, sizeof(IMG) + sizeof(PAY)>;
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {
-        cudaFuncSetAttribute(rs_down_kernel<ITEMS, W, OUT, IMG, PAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(rs_down_kernel<ITEMS, W, OUT, SEG, IMG, PAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(S::DOWN_SMEM));
     });
-    const int tiles = static_cast<int>((n + S::TILE - 1) / S::TILE);
-    rs_up_kernel<ITEMS, W, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(a.k, a.img_in, n, shift, tiles, t.counts);
+    const int tiles = SEG ? seg_tiles : static_cast<int>((n + S::TILE - 1) / S::TILE);
+    rs_up_kernel<ITEMS, W, SEG, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(a.k, a.img_in, n, shift, tiles, t.counts, a.segs,
+                                                                            a.tile_seg, a.digits);
     scan_counts(ctx, t.counts, static_cast<int64_t>(RADIX) * tiles, t.sums, t.offs);
-    rs_down_kernel<ITEMS, W, OUT, IMG, PAY><<<tiles, RS_THREADS, S::DOWN_SMEM, ctx->stream>>>(a, n, shift, tiles, t.offs);
+    rs_down_kernel<ITEMS, W, OUT, SEG, IMG, PAY><<<tiles, RS_THREADS, S::DOWN_SMEM, ctx->stream>>>(a, n, shift, tiles, t.offs);
 }
 template <int W, int OUT, class IMG, class PAY>
 static vkc_status radix_pass(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t) {
@@ -486,6 +556,41 @@ static vkc_status radix_argsort(vkc_ctx *ctx, const KeySource &k, IMG *const img
         cur = to;
     }
     return VKC_OK;
+}
+
+template <int ITEMS, class IMG>
+static vkc_status segs_argsort(vkc_ctx *ctx, const BatchSegs &b, IMG *const img[2], unsigned *const pos[2], int64_t n,
+                               const RadixTables &t) {
+    int cur = 0;
+    for (int i = 0; i < b.digits.n; ++i) {
+        RsArgs<IMG, unsigned> a{};
+        a.segs = b.segs;
+        a.tile_seg = b.tile_seg;
+        a.digits = b.digits;
+        a.img_in = img[cur];
+        a.pay_in = pos[cur];
+        const int to = i ? 1 - cur : 0, shift = 8 * i;
+        a.img_out = img[to];
+        a.pay_out = pos[to];
+        const bool last = i == b.digits.n - 1;
+        if (i == 0 && last) radix_pass_shape<ITEMS, 8, OUT_BATCH, IMG, unsigned, true>(ctx, a, n, shift, t, b.tiles);
+        else if (i == 0) radix_pass_shape<ITEMS, 8, OUT_PAIRS, IMG, unsigned, true>(ctx, a, n, shift, t, b.tiles);
+        else if (last) radix_pass_shape<ITEMS, 0, OUT_BATCH, IMG, unsigned, true>(ctx, a, n, shift, t, b.tiles);
+        else radix_pass_shape<ITEMS, 0, OUT_PAIRS, IMG, unsigned, true>(ctx, a, n, shift, t, b.tiles);
+        const vkc_status st = launched(ctx, "radix_segs");
+        if (st) return st;
+        cur = to;
+    }
+    return VKC_OK;
+}
+vkc_status radix_segs(vkc_ctx *ctx, const BatchSegs &b, void *const img[2], unsigned *const pos[2], int64_t n,
+                      const RadixTables &t) {
+    if (b.digits.n > 4) {
+        unsigned long long *w[2] = {static_cast<unsigned long long *>(img[0]), static_cast<unsigned long long *>(img[1])};
+        return b.tile == RS_THREADS * 8 ? segs_argsort<8>(ctx, b, w, pos, n, t) : segs_argsort<12>(ctx, b, w, pos, n, t);
+    }
+    unsigned *w[2] = {static_cast<unsigned *>(img[0]), static_cast<unsigned *>(img[1])};
+    return b.tile == RS_THREADS * 8 ? segs_argsort<8>(ctx, b, w, pos, n, t) : segs_argsort<12>(ctx, b, w, pos, n, t);
 }
 
 vkc_status radix_batch(vkc_ctx *ctx, bool wide, const void *images, void *const img[2], unsigned *const pos[2],

@@ -30,6 +30,30 @@ template <class IMG, class PAY>
 vkc_status radix_pairs(vkc_ctx *ctx, const RadixPairs<IMG, PAY> &p, int64_t n, const int *shifts, int passes,
                        const RadixTables &t, int *which);
 
+// The key digits of a batched argsort, least first: bit offsets of bytes (run: one after the other).
+struct BatchDigits {
+    int n, run;
+    int shift[8];
+};
+
+// Batched argsort, each array for itself: tiles of `tile` rows of one array each (2048 or 3072), a pass per key digit, from
+// the keys to the outputs' positions. img[] and pos[] are two buffers of n rows each (images of 32 bits
+// for up to four digits, else 64); the tables hold 256 counts a tile. Enqueue only.
+struct SortSeg {
+    const unsigned long long *keys;
+    long long *out;
+    int64_t base, n;  // its rows of the concatenation
+    int64_t tile0;    // its first tile
+};
+struct BatchSegs {
+    const SortSeg *segs;   // in the concatenation's order
+    const int *tile_seg;   // each tile's array
+    int tiles, tile;
+    BatchDigits digits;
+};
+vkc_status radix_segs(vkc_ctx *ctx, const BatchSegs &b, void *const img[2], unsigned *const pos[2], int64_t n,
+                      const RadixTables &t);
+
 // Batched argsort over n rows of all the arrays, concatenated: row i has the image (array number <<
 // index_shift) + key digits in images[] (64 bits when `wide`, else 32); the passes over `shifts` sort
 // the rows by it, and the last one writes every row's position in its array to that array's output.
