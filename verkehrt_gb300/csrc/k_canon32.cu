@@ -386,7 +386,8 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
         sm.ccode[c] = k;
         sm.crun[c] = gcrun[c];
         short slot = -1;
-        if (k == C32_NONE) {
+        // Without a function, or followed by a chunk of another binade: the sum may cross in its last tiles.
+        if (k == C32_NONE || (c + 1 < C && gccode[c + 1] != k)) {
             const int m = atomicAdd(&sm.nmixed, 1);
             if (m < W32_MIXED) {
                 slot = static_cast<short>(m);
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
     int tile = 0;
     while (tile < T && s == s) {  // a NaN stays one
         const unsigned code = code32(s);
-        const int c = tile / C32_CHUNK;
+        int c = tile / C32_CHUNK;
         if (code != C32_NONE && tile % C32_CHUNK == 0) {
             const int k = c + lane;
             unsigned kc = C32_NONE;
@@ -437,13 +438,15 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
                 kc = k < W32_CHUNKS ? sm.ccode[k] : gccode[k];
                 if (kc == code) f = k < W32_CHUNKS ? sm.crun[k] : gcrun[k];
             }
-            const int m = advance32(f, kc == code, &s);
+            const int m = __shfl_sync(FULL, kc == code, 0) ? advance32(f, kc == code, &s) : 0;
             if (m > 0) {
-                tile = (c + m) * C32_CHUNK;
-                continue;
+                c += m;
+                tile = c * C32_CHUNK;
+                if (m == 32 || tile >= T) continue;  // else the chunk that ended the run, tile by tile
             }
         }
-        const int slot = c < W32_CHUNKS ? sm.mixed_of[c] : -1, j0 = tile % C32_CHUNK;
+        const int slot = c < W32_CHUNKS ? sm.mixed_of[c] : -1;
+        int j0 = tile % C32_CHUNK;
         if (code != C32_NONE) {
             const int j = j0 + lane, k = tile + lane;
             unsigned kc = C32_NONE;
@@ -452,10 +455,11 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
                 kc = slot >= 0 ? sm.code[slot][j] : gcode[k];
                 if (kc == code) f = slot >= 0 ? sm.run[slot][j] : grun[k];
             }
-            const int m = advance32(f, kc == code, &s);
+            const int m = __shfl_sync(FULL, kc == code, 0) ? advance32(f, kc == code, &s) : 0;
             if (m > 0) {
                 tile += m;
-                continue;
+                j0 += m;
+                if (j0 >= C32_CHUNK || tile >= T) continue;  // else the tile that ended the run
             }
         }
         // The tile's rows, sixteen a thread.
