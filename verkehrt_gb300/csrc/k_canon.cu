@@ -426,6 +426,7 @@ constexpr int FULL_TILES = 4096;
 
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(CT_THREADS) canon_sums_kernel(RowArgs args, int64_t nb, int T, CanonWork wk) {
+    chain_enter();
     __shared__ float part[CT_THREADS / 32][16];
     const int t = threadIdx.x, lp = t & 7, seg = t >> 3, tile = blockIdx.x;
     if (tile == 0 && t < 2) wk.flags[T + t] = 0;  // no negative row yet, no tile listed
@@ -506,6 +507,7 @@ constexpr int CAND_PER = CAND_GROUP / CAND_THREADS;
 // groups): the groups before this one are summed here, not by K2a.
 template <bool CHECK, bool FULL_SUMS>
 __global__ void __launch_bounds__(CAND_THREADS) canon_cand_kernel(int T, int G, CanonWork wk, bool fresh, const CanonState *state) {
+    chain_enter();
     __shared__ double s_base;
     __shared__ double s_before[CAND_THREADS / 32];
     const int L = blockIdx.x / G, g = blockIdx.x % G, t = threadIdx.x;
@@ -758,6 +760,7 @@ __device__ __forceinline__ void tf_tile(const RowArgs &args, int64_t nb, int T, 
 
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(CT_THREADS, 4) canon_tf_kernel(RowArgs args, int64_t nb, int T, CanonWork wk) {
+    chain_enter();
     tf_tile<OP, ALIGNED, false>(args, nb, T, wk, blockIdx.x);
 }
 
@@ -772,6 +775,7 @@ __global__ void __launch_bounds__(256) canon_flag_list_kernel(int T, CanonWork w
 // K3c: persistent blocks over the list of flagged tiles.
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(CT_THREADS, 4) canon_tf_flagged_kernel(RowArgs args, int64_t nb, int T, CanonWork wk) {
+    chain_enter();
     const int count = wk.flags[T + 1];
     for (int i = blockIdx.x; i < count; i += gridDim.x) {
         __syncthreads();  // the previous tile's shared arrays are free
@@ -799,6 +803,7 @@ __device__ __forceinline__ bool tile_tf(const CanonWork &wk, int T, int L, int t
 // tile of the chunk has one in the same binade (the binade of candidate 0 of the chunk's
 // first tile).
 __global__ void __launch_bounds__(256) canon_chunk_kernel(int T, int C, CanonWork wk) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int64_t gw = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (gw >= static_cast<int64_t>(16) * C) return;
@@ -1168,6 +1173,7 @@ __device__ __forceinline__ unsigned long long walk_lane(const RowArgs &args, int
 template <int OP, bool RECORD>
 __global__ void __launch_bounds__(WK_THREADS) canon_walk_kernel(RowArgs args, int64_t nb, int T, int C, CanonWork wk,
                                                                 bool fresh, CanonState *state) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char walk_smem[];
     WalkSmem &sm = *reinterpret_cast<WalkSmem *>(walk_smem);
     const int L = blockIdx.x, t = threadIdx.x;
@@ -1588,6 +1594,7 @@ __device__ __forceinline__ void chain_lane(const RowArgs &args, int64_t nb, int 
 template <int OP, int ROWS>
 __global__ void __launch_bounds__(32) canon_chain_kernel(RowArgs args, int64_t nb, int T, CanonWork wk, CanonState *state,
                                                          int rest, unsigned *done, unsigned long long *result) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned long long chain_smem_buf[];
     chain_lane<OP, ROWS>(args, nb, T, wk, state, chain_smem_buf);
     if (!result || !last_block(done)) return;
@@ -1614,9 +1621,9 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
     if (wk.listed) {
         canon_sums_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
         if ((st = launched(ctx, "canon_sums"))) return st;
-        canon_cand_kernel<false, true><<<16 * G, CAND_THREADS, 0, ctx->stream>>>(T, G, wk, fresh, state);
+        launch_next(canon_cand_kernel<false, true>, 16 * G, CAND_THREADS, 0, ctx->stream, T, G, wk, fresh, state);
         if ((st = launched(ctx, "canon_cand"))) return st;
-        canon_tf_kernel<OP, ALIGNED><<<T, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+        launch_next(canon_tf_kernel<OP, ALIGNED>, T, CT_THREADS, 0, ctx->stream, a, nb, T, wk);
         if ((st = launched(ctx, "canon_tf"))) return st;
     } else {
         canon_apx_kernel<OP, ALIGNED><<<(T + APX_TILES - 1) / APX_TILES, CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
@@ -1636,10 +1643,10 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
         canon_flag_list_kernel<<<std::min(T / 256 + 1, 1024), 256, 0, ctx->stream>>>(T, wk);
         if ((st = launched(ctx, "canon_check"))) return st;
     }
-    canon_tf_flagged_kernel<OP, ALIGNED><<<std::min(T, 4 * ctx->sms), CT_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+    launch_next(canon_tf_flagged_kernel<OP, ALIGNED>, std::min(T, 4 * ctx->sms), CT_THREADS, 0, ctx->stream, a, nb, T, wk);
     if ((st = launched(ctx, "canon_tf_flagged"))) return st;
     int warps = 16 * C;
-    canon_chunk_kernel<<<(warps + 7) / 8, 256, 0, ctx->stream>>>(T, C, wk);
+    launch_next(canon_chunk_kernel, (warps + 7) / 8, 256, 0, ctx->stream, T, C, wk);
     if ((st = launched(ctx, "canon_chunk"))) return st;
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {
@@ -1647,7 +1654,7 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
                              static_cast<int>(sizeof(WalkSmem)));
     });
     if constexpr (RECORD) VKC_CUDA(ctx, cudaMemsetAsync(wk.whole, 0, static_cast<size_t>(C) * 16 * sizeof(int), ctx->stream));
-    canon_walk_kernel<OP, RECORD><<<16, WK_THREADS, sizeof(WalkSmem), ctx->stream>>>(a, nb, T, C, wk, fresh, state);
+    launch_next(canon_walk_kernel<OP, RECORD>, 16, WK_THREADS, sizeof(WalkSmem), ctx->stream, a, nb, T, C, wk, fresh, state);
     if ((st = launched(ctx, "canon_walk"))) return st;
     if constexpr (!RECORD) {
         static std::atomic<unsigned long long> chain_configured{0};
@@ -1661,9 +1668,9 @@ static vkc_status launch_canon(vkc_ctx *ctx, const RowArgs &a, int64_t nb, int T
         });
         unsigned *done = ctx->counters + 1;
         switch (tune(ctx, TK_CHAIN_ROWS, nb * 16)) {
-        case 4: canon_chain_kernel<OP, 4><<<16, 32, chain_smem<OP, 4>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
-        case 16: canon_chain_kernel<OP, 16><<<16, 32, chain_smem<OP, 16>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
-        default: canon_chain_kernel<OP, 8><<<16, 32, chain_smem<OP, 8>(), ctx->stream>>>(a, nb, T, wk, state, rest, done, result); break;
+        case 4: launch_next(canon_chain_kernel<OP, 4>, 16, 32, chain_smem<OP, 4>(), ctx->stream, a, nb, T, wk, state, rest, done, result); break;
+        case 16: launch_next(canon_chain_kernel<OP, 16>, 16, 32, chain_smem<OP, 16>(), ctx->stream, a, nb, T, wk, state, rest, done, result); break;
+        default: launch_next(canon_chain_kernel<OP, 8>, 16, 32, chain_smem<OP, 8>(), ctx->stream, a, nb, T, wk, state, rest, done, result); break;
         }
         if ((st = launched(ctx, "canon_chain"))) return st;
     }
