@@ -190,6 +190,7 @@ __device__ __forceinline__ void load32(const Args32 &a, int64_t nb, int tile, fl
 // C1. Bound by the read.
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(C32_THREADS) c32_sums(Args32 a, int64_t nb, int T, Work32 wk) {
+    chain_enter();
     __shared__ float part[C32_THREADS / 32][16];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     float v[4][C32_RUN];
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(C32_THREADS) c32_sums(Args32 a, int64_t nb, in
 
 // C2: one block per lane; a thread takes a run of consecutive tiles.
 __global__ void __launch_bounds__(1024) c32_binades(int T, Work32 wk, const State32 *state) {
+    chain_enter();
     __shared__ double warp_tot[32];
     const int L = blockIdx.x, t = threadIdx.x, lane = t & 31, w = t >> 5;
     const float *apx = wk.apx + static_cast<int64_t>(L) * T;
@@ -241,6 +243,7 @@ __global__ void __launch_bounds__(1024) c32_binades(int T, Work32 wk, const Stat
 // memory. Runs that only move up and meet no tie (d0 == d1) compose by adding.
 template <int OP, bool ALIGNED>
 __global__ void __launch_bounds__(C32_THREADS) c32_runs(Args32 a, int64_t nb, int T, Work32 wk) {
+    chain_enter();
     __shared__ Run32 part[C32_THREADS / 32][16];
     __shared__ unsigned bad[C32_THREADS / 32];
     __shared__ unsigned s_code[16];
@@ -305,6 +308,7 @@ __global__ void __launch_bounds__(C32_THREADS) c32_runs(Args32 a, int64_t nb, in
 
 // C4: one warp per lane and chunk.
 __global__ void __launch_bounds__(256) c32_chunks(int T, int C, Work32 wk) {
+    chain_enter();
     const int lane = threadIdx.x & 31;
     const int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (g >= static_cast<int64_t>(16) * C) return;
@@ -372,6 +376,7 @@ template <int OP> __device__ __forceinline__ float row_of(const Args32 &a, int64
 
 template <int OP>
 __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int C, Work32 wk, State32 *state) {
+    chain_enter();
     extern __shared__ __align__(16) unsigned char walk32_smem[];
     Walk32 &sm = *reinterpret_cast<Walk32 *>(walk32_smem);
     const int L = blockIdx.x, t = threadIdx.x;
@@ -581,12 +586,14 @@ __global__ void __launch_bounds__(512) c32_chain(Args32 a, int nb, int rest, boo
 
 // The rest rows (fewer than 16), kept as row values until finish.
 template <int OP> __global__ void c32_tail(Args32 a, int64_t first, int rest, State32 *state) {
+    chain_enter();
     const int j = threadIdx.x;
     if (j < rest) state->tail[j] = value32<OP>(a, a.x[first + j], OP == R32_DOT ? a.y[first + j] : 0.f);
 }
 
 // reduce.rs:77-91 (finish_lanes).
 __global__ void c32_finish(State32 *state, int tail_len, float *host) {
+    chain_enter();
     float acc[16];
     for (int j = 0; j < 16; ++j) acc[j] = state->lanes[j];
     for (int step = 8; step > 0; step >>= 1)
@@ -638,14 +645,14 @@ template <int OP> vkc_status launch_canon32(vkc_ctx *ctx, const Args32 &a, int64
     if (aligned) c32_sums<OP, true><<<T, C32_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
     else c32_sums<OP, false><<<T, C32_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
     if ((st = launched(ctx, "canon32_sums"))) return st;
-    c32_binades<<<16, 1024, 0, ctx->stream>>>(T, wk, state);
+    launch_next(c32_binades, 16, 1024, 0, ctx->stream, T, wk, state);
     if ((st = launched(ctx, "canon32_binades"))) return st;
-    if (aligned) c32_runs<OP, true><<<T, C32_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
-    else c32_runs<OP, false><<<T, C32_THREADS, 0, ctx->stream>>>(a, nb, T, wk);
+    if (aligned) launch_next(c32_runs<OP, true>, T, C32_THREADS, 0, ctx->stream, a, nb, T, wk);
+    else launch_next(c32_runs<OP, false>, T, C32_THREADS, 0, ctx->stream, a, nb, T, wk);
     if ((st = launched(ctx, "canon32_runs"))) return st;
-    c32_chunks<<<static_cast<int>((static_cast<int64_t>(16) * C + 7) / 8), 256, 0, ctx->stream>>>(T, C, wk);
+    launch_next(c32_chunks, static_cast<unsigned>((static_cast<int64_t>(16) * C + 7) / 8), 256, 0, ctx->stream, T, C, wk);
     if ((st = launched(ctx, "canon32_chunks"))) return st;
-    c32_walk<OP><<<16, 256, sizeof(Walk32), ctx->stream>>>(a, nb, T, C, wk, state);
+    launch_next(c32_walk<OP>, 16, 256, sizeof(Walk32), ctx->stream, a, nb, T, C, wk, state);
     return launched(ctx, "canon32_walk");
 }
 
@@ -697,7 +704,7 @@ template <int OP> struct Canon32Reducer : DevReducer {
             if (fresh && (st = zero(ctx))) return st;
             st = launch_canon32<OP>(ctx, a, nb, s);
             if (!st && rest > 0) {
-                c32_tail<OP><<<1, 16, 0, ctx->stream>>>(a, nb * 16, rest, s);
+                launch_next(c32_tail<OP>, 1, 16, 0, ctx->stream, a, nb * 16, rest, s);
                 st = launched(ctx, "canon32_tail");
             }
         }
@@ -728,7 +735,7 @@ template <int OP> struct Canon32Reducer : DevReducer {
     vkc_status combine(vkc_ctx *ctx) {
         vkc_status st;
         if (fresh && (st = zero(ctx))) return st;
-        c32_finish<<<1, 1, 0, ctx->stream>>>(static_cast<State32 *>(state), tail_len, static_cast<float *>(host));
+        launch_next(c32_finish, 1, 1, 0, ctx->stream, static_cast<State32 *>(state), tail_len, static_cast<float *>(host));
         updated(ctx);
         return launched(ctx, "canon32_finish");
     }
