@@ -171,9 +171,12 @@ __device__ __forceinline__ void seg_images(const SortSeg &seg, const BatchDigits
 // atomics into one histogram per warp (the order of the increments does not matter here). W: the
 // first pass, from keys of W bytes; 0: from images.
 template <int RS_ITEMS, int W, bool SEG, class IMG>
-__global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IMG *__restrict__ img_in, int64_t n,
-                                                           int shift, int tiles, unsigned *__restrict__ counts,
+__global__ void __launch_bounds__(RS_THREADS) rs_up_kernel(KeySource k, const IMG *img_in, int64_t n,
+                                                           int shift, int tiles, unsigned *counts,
                                                            const SortSeg *segs, const int *tile_seg, BatchDigits digits) {
+    chain_enter();
+    img_in = chained(img_in);
+    k.keys = chained(k.keys);
     constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
     __shared__ unsigned s_cnt[RS_WARPS][RADIX];
     const int tile = blockIdx.x;
@@ -258,8 +261,8 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 
-__global__ void __launch_bounds__(SCAN_THREADS) rs_scan_sums(const unsigned *__restrict__ c, int64_t m,
-                                                              unsigned *__restrict__ sums) {
+__global__ void __launch_bounds__(SCAN_THREADS) rs_scan_sums(const unsigned *c, int64_t m, unsigned *sums) {
+    chain_enter();
     const int64_t b0 = static_cast<int64_t>(blockIdx.x) * SCAN_CHUNK;
     unsigned t = 0;
 #pragma unroll
@@ -274,6 +277,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) rs_scan_sums(const unsigned *__r
 
 // One block: exclusive scan of `k` block sums in place.
 __global__ void __launch_bounds__(1024) rs_scan_top(unsigned *sums, int k) {
+    chain_enter();
     __shared__ unsigned carry;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
@@ -294,9 +298,8 @@ __global__ void __launch_bounds__(1024) rs_scan_top(unsigned *sums, int k) {
 // thread's rows move as four 16-byte accesses (one word at a time, each warp access touched 32
 // sectors: 17 us for 2.5 M counts).
 template <bool VEC>
-__global__ void __launch_bounds__(SCAN_THREADS) rs_scan_apply(const unsigned *__restrict__ c, int64_t m,
-                                                               const unsigned *__restrict__ sums,
-                                                               unsigned *__restrict__ out) {
+__global__ void __launch_bounds__(SCAN_THREADS) rs_scan_apply(const unsigned *c, int64_t m, const unsigned *sums, unsigned *out) {
+    chain_enter();
     const int64_t b0 = static_cast<int64_t>(blockIdx.x) * SCAN_CHUNK + static_cast<int64_t>(threadIdx.x) * SCAN_ITEMS;
     const bool whole = VEC && b0 + SCAN_ITEMS <= m;
     unsigned v[SCAN_ITEMS], t = 0;
@@ -336,9 +339,11 @@ __global__ void __launch_bounds__(SCAN_THREADS) rs_scan_apply(const unsigned *__
 
 // A short table in one block: every 16-byte unit of it in a register, the warps' sums of its eight pieces
 // scanned by one warp. (A pass over up to 2^18 rows spends most of its time in launches: with the three
-// kernels above a sort of 2^18 32-bit keys took about 135 us a call, now 105.)
+// kernels above a sort of 2^18 32-bit keys took about 135 us a call, then 105, and 84 since the passes'
+// kernels are launched as a chain.)
 constexpr int SCAN_ONE = 32768;
-__global__ void __launch_bounds__(1024) rs_scan_one(const unsigned *__restrict__ c, int m, unsigned *__restrict__ out) {
+__global__ void __launch_bounds__(1024) rs_scan_one(const unsigned *c, int m, unsigned *out) {
+    chain_enter();
     __shared__ unsigned s_sum[8 * 32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     uint4 v[8];
@@ -399,16 +404,16 @@ int64_t scan_counts_sum_words(int64_t m) { return (m + SCAN_CHUNK - 1) / SCAN_CH
 void scan_counts(vkc_ctx *ctx, const unsigned *c, int64_t m, unsigned *sums, unsigned *out) {
     const bool vec = ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     if (vec && m <= SCAN_ONE && m % 4 == 0) {
-        rs_scan_one<<<1, 1024, 0, ctx->stream>>>(c, static_cast<int>(m), out);
+        launch_next(rs_scan_one, 1, 1024, 0, ctx->stream, c, static_cast<int>(m), out);
         return;
     }
     const int chunks = static_cast<int>(scan_counts_sum_words(m));
-    rs_scan_sums<<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums);
-    rs_scan_top<<<1, 1024, 0, ctx->stream>>>(sums, chunks);
+    launch_next(rs_scan_sums, chunks, SCAN_THREADS, 0, ctx->stream, c, m, sums);
+    launch_next(rs_scan_top, 1, 1024, 0, ctx->stream, sums, chunks);
     if (vec)
-        rs_scan_apply<true><<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
+        launch_next(rs_scan_apply<true>, chunks, SCAN_THREADS, 0, ctx->stream, c, m, sums, out);
     else
-        rs_scan_apply<false><<<chunks, SCAN_THREADS, 0, ctx->stream>>>(c, m, sums, out);
+        launch_next(rs_scan_apply<false>, chunks, SCAN_THREADS, 0, ctx->stream, c, m, sums, out);
 }
 
 // Down: one pass over digit `shift` with the tile's first output row per digit in
@@ -526,7 +531,11 @@ __device__ __forceinline__ void rs_down_tile(const RsArgs<IMG, PAY> &a, const So
 
 template <int RS_ITEMS, int W, int OUT, bool SEG, class IMG, class PAY>
 __global__ void __launch_bounds__(RS_THREADS, (RsShape<RS_ITEMS, sizeof(IMG) + sizeof(PAY)>::MIN_BLOCKS))
-    rs_down_kernel(RsArgs<IMG, PAY> a, int64_t n, int shift, int tiles, const unsigned *__restrict__ offsets) {
+    rs_down_kernel(RsArgs<IMG, PAY> a, int64_t n, int shift, int tiles, const unsigned *offsets) {
+    chain_enter();
+    a.img_in = chained(a.img_in);
+    a.pay_in = chained(a.pay_in);
+    a.k.keys = chained(a.k.keys);
     __shared__ RsShared sm;
     extern __shared__ __align__(16) unsigned char rs_smem[];
     const int tile = blockIdx.x;
@@ -551,10 +560,10 @@ static void radix_pass_shape(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n,
                              static_cast<int>(S::DOWN_SMEM));
     });
     const int tiles = SEG ? seg_tiles : static_cast<int>((n + S::TILE - 1) / S::TILE);
-    rs_up_kernel<ITEMS, W, SEG, IMG><<<tiles, RS_THREADS, 0, ctx->stream>>>(a.k, a.img_in, n, shift, tiles, t.counts, a.segs,
-                                                                            a.tile_seg, a.digits);
+    launch_next(rs_up_kernel<ITEMS, W, SEG, IMG>, tiles, RS_THREADS, 0, ctx->stream, a.k, a.img_in, n, shift, tiles, t.counts, a.segs,
+                a.tile_seg, a.digits);
     scan_counts(ctx, t.counts, static_cast<int64_t>(RADIX) * tiles, t.sums, t.offs);
-    rs_down_kernel<ITEMS, W, OUT, SEG, IMG, PAY><<<tiles, RS_THREADS, S::DOWN_SMEM, ctx->stream>>>(a, n, shift, tiles, t.offs);
+    launch_next(rs_down_kernel<ITEMS, W, OUT, SEG, IMG, PAY>, tiles, RS_THREADS, S::DOWN_SMEM, ctx->stream, a, n, shift, tiles, t.offs);
 }
 template <int W, int OUT, class IMG, class PAY>
 static vkc_status radix_pass(vkc_ctx *ctx, const RsArgs<IMG, PAY> &a, int64_t n, int shift, const RadixTables &t) {

@@ -145,6 +145,12 @@ __device__ __forceinline__ void chain_enter() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// A pointer to what the kernel before wrote, for loads with a cache hint: known only after the wait.
+template <class T> __device__ __forceinline__ T *chained(T *p) {
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 template <class... P, class... A>
 inline void launch_next(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, A... args) {
     cudaLaunchAttribute attr{};
