@@ -9,15 +9,16 @@
 // synchronisation, and no allocation once a batch's scratch exists, so a sequence of them can
 // be captured in a CUDA graph (vkc_graph_begin / vkc_graph_end) and replayed.
 //
-//  * filter -> sum (vkc_batch_filter_sum_f64): one persistent kernel; a block takes an array,
-//    counts its survivors, then compacts them in row order chunk by chunk and feeds them to the
+//  * filter -> sum (vkc_batch_filter_sum_f64): one persistent kernel; a block takes an array and
+//    compacts its survivors in row order chunk by chunk, feeding the whole blocks of 16 to the
 //    reference's 16 lanes (lane j takes survivors j, j+16, ... below the last whole block of 16,
 //    with IEEE adds in that order), combines the lanes +8, +4, +2, +1 and adds the tail
 //    (src/kernels/scalar/reduce.rs:45-91): the bits of filter then reduce_add_f64.
-//  * argsort (vkc_batch_argsort_i64): every row of every array gets one image, its array's number
-//    above the key digits given (all eight when none are), in 32 bits where they fit; stable radix
-//    passes over the image sort all rows by (array, key), and the last one writes each array's
-//    positions to its output relative to its first row. Stability makes every output the array's
+//  * argsort (vkc_batch_argsort_i64): each array sorted for itself by stable radix passes over the key
+//    digits given (all eight when none are), in tiles of one array each (radix.h, radix_segs). In
+//    batches of short arrays (plan_segs) every row gets one image instead, its array's number above
+//    the key digits, in 32 bits where they fit; the passes sort all rows by (array, key), and the last
+//    one writes each array's positions to its output. Stability makes every output the array's
 //    own argsort. (Key digits and number beyond 64 bits: the order by the keys first, then by the
 //    arrays' numbers, found again from the positions.)
 #include <algorithm>

@@ -4,11 +4,12 @@
 // The ids depend only on the order in which distinct keys first appear (group.rs:1-5), so any
 // correct table gives the reference's output. Two kernels:
 //  1. insert: open addressing with linear probing. A free slot holds the key EMPTY (the byte
-//     0x80 repeated) and is claimed by a CAS on the key itself (a 128-bit CAS for key pairs),
-//     so a probe that reads its key needs no further synchronisation. Slot 0 is never probed:
+//     0x80 repeated) and is claimed, with the row, by one 128-bit CAS (for key pairs by a CAS on the
+//     keys), so a probe that reads its key needs no further synchronisation. Slot 0 is never probed:
 //     it belongs to the key EMPTY (or the pair (EMPTY, EMPTY)), whose rows go there directly.
-//     Each slot keeps the smallest row that holds its key (atomicMin, skipped when the stored
-//     row is already smaller), and each row records its slot. A thread probes four rows at once.
+//     Each slot keeps the smallest row that holds its key (atomicMin, skipped when the stored row,
+//     read with the key, is already smaller), and each row records its slot. A thread probes four
+//     rows at once.
 //  2. number: the smallest rows of the slots are the first occurrences, and a group's id is the rank
 //     of its first row among them. They are marked in a bitmap of the rows, whose words' counts are
 //     scanned; each occupied slot takes its id from there, and every row reads its slot's. Short
