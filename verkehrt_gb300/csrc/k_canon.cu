@@ -194,7 +194,7 @@ __device__ __forceinline__ bool seg_tf(const unsigned long long (&v)[CT_SEG_BLOC
 #pragma unroll
     for (int i = 0; i < CT_SEG_BLOCKS; ++i) {
         exmax = max(exmax, static_cast<unsigned>(v[i][h] >> 52) & (SIGNED ? 0x7ffu : 0xfffu));
-        if (SIGNED) sgn |= static_cast<unsigned>(v[i][h] >> 63);
+        if (SIGNED) sgn |= v[i][h] > (1ull << 63);  // -0.0 moves no state
     }
     if (exmax >= static_cast<unsigned>(KE)) return false;
     if (SIGNED && sgn) return seg_tf_signed(v, h, KE, exmax, out);
@@ -838,13 +838,19 @@ __device__ __forceinline__ int state_binade(unsigned long long s) {
 // leading lanes whose prefix applies to state s (usable and inside the binade). Returns that
 // count and, in *out, the state after them.
 //
-// SIGNED: every function as the move of the state's magnitude from an even and an odd start and the
-// bounds of the moves on the way, so that one composition without branches serves signed functions,
-// unsigned ones and ties (composing TFs as such, with both kinds in a warp, took about 4000 cycles a
-// call, and the walk of 2^27 rows of u - 1/4 1.0 ms, slow enough to hand some lanes to the chain).
+// SIGNED: every function as the move of the state's magnitude from an even and an odd start, the lowest
+// state within the functions that may move it down (NO_FALL when there is none) and the highest one on
+// the way, so that one composition without branches serves signed functions, unsigned ones and ties
+// (composing TFs as such, with both kinds in a warp, took about 4000 cycles a call, and the walk of 2^27
+// rows of u - 1/4 1.0 ms, slow enough to hand some lanes to the chain).
+//
+// The lowest state has to stay an ulp above 2^E whatever rose before it: a sum that rounds to 2^E may lie
+// below it, on the finer grid, and so may one whose fall rounds to no ulp at all. (A composed move from
+// 2^E up by k ulps and down by k again ends where it began, but the exact sum may round below.)
 struct Move {
     long long d0, d1, mn, mx;
 };
+constexpr long long NO_FALL = 1ll << 61;  // far above the moves of 32 functions
 
 template <bool SIGNED = true>
 __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long long s, int E,
@@ -857,12 +863,13 @@ __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long lon
         const unsigned long long up = f.d0, dn = (f.d1 & SIGNED_TF) ? f.d1 & ~SIGNED_TF : 0ull;
         const bool parity = !(f.d1 & SIGNED_TF) && f.d0 != f.d1;  // only for states as the rows: not negative
         ok = ok && max(up, parity ? f.d1 : dn) < (ONE52 << 1) && !(parity && neg);
-        Move m{0, 0, 0, 0};
+        Move m{0, 0, NO_FALL, 0};
         if (ok) {
             const long long u = static_cast<long long>(up), d = static_cast<long long>(dn);
             m.d0 = neg ? d - u : u - d;
             m.d1 = parity ? static_cast<long long>(f.d1) : m.d0;
-            m.mn = neg ? -u : -d;
+            // A positive row lowers a negative state's magnitude, and no function tells that it holds none.
+            m.mn = neg ? -u : ((f.d1 & SIGNED_TF) ? -d : NO_FALL);
             m.mx = neg ? d : max(u, parity ? m.d1 : 0ll);
         }
         const bool ties = __any_sync(FULL, m.d0 != m.d1);
@@ -881,7 +888,7 @@ __device__ __forceinline__ int apply_prefix(TF f, bool usable, unsigned long lon
         const unsigned long long ef = static_cast<unsigned long long>(E + 1023);
         const long long S = static_cast<long long>((s & MANT) | ONE52);
         ok = ok && ((s >> 52) & 0x7ff) == ef && S + m.mx < static_cast<long long>(ONE52 << 1) &&
-             (m.mn >= 0 || S + m.mn > static_cast<long long>(ONE52));
+             S + m.mn > static_cast<long long>(ONE52);
         r = (s & (1ull << 63)) | (ef << 52) | (static_cast<unsigned long long>(S + ((S & 1) ? m.d1 : m.d0)) & MANT);
     } else {
         if (!__any_sync(FULL, usable && f.d0 != f.d1)) {
@@ -1063,6 +1070,18 @@ __device__ unsigned long long resolve_tile(const RowArgs &args, int64_t nb, int 
     return s;
 }
 
+// A state of exactly 2^E has the finer grid below it, so that no function of a negative state and no signed
+// one applies to it. But rows that move nothing on that grid leave it as it is, and their function one
+// binade lower, recorded for a sum this close to it, says so. (Else the zeros behind a first row of -1 in
+// 2^24 rows, all resolved tile by tile, then by the lane chain, took 64 ms.)
+__device__ __forceinline__ bool moves_nothing(TF f) { return f.d0 == 0 && (f.d1 & ~SIGNED_TF) == 0; }
+
+// The leading threads of the warp for which `p` holds.
+__device__ __forceinline__ int leading(bool p) {
+    const unsigned no = __ballot_sync(FULL, !p);
+    return no ? __ffs(no) - 1 : 32;
+}
+
 // Chunk k of lane L tile by tile from state s (one warp): runs of tiles whose transfer
 // functions hold, and the tiles none carries resolved from the rows. RECORD (scans) stores the
 // exact state before each tile. sm and slot give the chunk's tile records when the walk holds
@@ -1112,6 +1131,14 @@ __device__ __forceinline__ unsigned long long walk_chunk_tiles(const RowArgs &ar
             tp += mt;
             if (tp >= end) break;
             if (RECORD && lane == 0) rec[tp] = s;
+        } else if (SIGNED && Et != NO_E && (s & MANT) == 0) {
+            TF z{0, 0};
+            const int m = leading(tl < end && tile_tf(wk, T, L, tl, Et - 1, &z) && moves_nothing(z));
+            if (m > 0) {
+                if (RECORD && lane + 1 < m) rec[tp + lane + 1] = s;
+                tp += m;
+                continue;
+            }
         }
         // The tile at which the run ended would end the next one too.
         const int q = slot >= 0 ? sm->rows_of[slot][tp - k * 32] : -1;
@@ -1160,6 +1187,12 @@ __device__ __forceinline__ unsigned long long walk_lane(const RowArgs &args, int
             s = r;
             k += m;
             if (m == 32 || k >= C) continue;
+        } else if (SIGNED && !RECORD && E != NO_E && (s & MANT) == 0) {
+            const int z = leading(kc < C && ce == E - 1 && moves_nothing(held ? sm.chunkD[kc] : gD[kc]));
+            if (z > 0) {
+                k += z;
+                continue;
+            }
         }
         // Chunk k, which ended the run, tile by tile.
         s = walk_chunk_tiles<OP, SIGNED, RECORD>(args, nb, T, wk, &sm, held ? sm.mixed_of[k] : -1, L, k, s,
