@@ -69,10 +69,16 @@ template <int OP> __device__ __forceinline__ float value32(const Args32 &a, floa
 }
 
 // The effect of a run of rows on a state of one binade: the magnitude's move in ulps from an even
-// (d0) and an odd (d1) start, and bounds of every move on the way.
+// (d0) and an odd (d1) start, a bound of the highest state on the way (mx) and of the lowest one within
+// the parts that may move it down (mn; NO_FALL32 when there is none).
+//
+// The lowest state has to stay an ulp above 2^E whatever rose before it: a sum that rounds to 2^E may lie
+// below it, on the finer grid. (A run up by k ulps and one down by k, composed, end where they began.)
 struct Run32 {
     int d0, d1, mn, mx;
 };
+constexpr int NO_FALL32 = 1 << 30;  // no composed move reaches 2^29 (c32_runs): sums with it do not wrap
+constexpr Run32 STILL32{0, 0, NO_FALL32, 0};
 
 __device__ __forceinline__ Run32 then32(Run32 a, Run32 b) {
     return Run32{a.d0 + ((a.d0 & 1) ? b.d1 : b.d0), a.d1 + ((a.d1 & 1) ? b.d0 : b.d1),
@@ -107,7 +113,7 @@ __device__ __forceinline__ Start32 start32(unsigned code) {
                    __uint_as_float(e | 0x7ffffdu)};
 }
 
-// The run of N row values from both starts. False (and the identity) when it leaves the binade or
+// The run of N row values from both starts. False (and no move) when it leaves the binade or
 // meets a NaN.
 template <int N> __device__ __forceinline__ bool run32(const float (&v)[N], unsigned code, Run32 *out) {
     const Start32 st = start32(code);
@@ -127,17 +133,17 @@ template <int N> __device__ __forceinline__ bool run32(const float (&v)[N], unsi
     const bool ok = lo >= st.lo && hi <= st.hi && a >= st.lo && b >= st.lo;
     // Offsets of the odd run differ from the even run's by at most one.
     *out = ok ? Run32{__float_as_int(a) - base, __float_as_int(b) - base - 1,
-                      (down >> 31) ? __float_as_int(lo) - base - 1 : 0, __float_as_int(hi) - base + 1}
-              : Run32{0, 0, 0, 0};
+                      (down >> 31) ? __float_as_int(lo) - base - 1 : NO_FALL32, __float_as_int(hi) - base + 1}
+              : STILL32;
     return ok;
 }
 
-// Applies f to state s, known to be of f's binade: false when a state on the way could leave it. A
-// run with a row that moves the magnitude down (mn < 0) keeps every state above 2^E by an ulp, so
-// that no exact sum falls into the finer grid below.
+// Applies f to state s, known to be of f's binade: false when a state on the way could leave it. Rows
+// that move the magnitude down keep every state above 2^E by an ulp, so that no exact sum falls into the
+// finer grid below.
 __device__ __forceinline__ bool apply32(float s, Run32 f, float *out) {
     const int bits = __float_as_int(s), S = (bits & 0x7fffff) | 0x800000;
-    if (S + f.mx >= C32_TOP || (f.mn < 0 && S + f.mn <= C32_TOP / 2)) return false;
+    if (S + f.mx >= C32_TOP || S + f.mn <= C32_TOP / 2) return false;
     *out = __int_as_float(bits + ((S & 1) ? f.d1 : f.d0));
     return true;
 }
@@ -258,9 +264,9 @@ __global__ void __launch_bounds__(C32_THREADS) c32_runs(Args32 a, int64_t nb, in
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
         const unsigned code = s_code[(lane & 3) * 4 + h];
-        f[h] = Run32{0, 0, 0, 0};
+        f[h] = STILL32;
         if (code == C32_NONE || !run32<C32_RUN>(v[h], code, &f[h])) fails |= 1u << h;
-        simple = simple && f[h].d0 == f[h].d1 && f[h].mn == 0 && f[h].mx == f[h].d0 + 1;
+        simple = simple && f[h].d0 == f[h].d1 && f[h].mn == NO_FALL32 && f[h].mx == f[h].d0 + 1;
     }
     if (__all_sync(FULL, simple)) {
 #pragma unroll
@@ -268,7 +274,7 @@ __global__ void __launch_bounds__(C32_THREADS) c32_runs(Args32 a, int64_t nb, in
             int d = f[h].d0;
 #pragma unroll
             for (int o = 4; o < 32; o <<= 1) d += __shfl_xor_sync(FULL, d, o);
-            f[h] = Run32{d, d, 0, d + 1};
+            f[h] = Run32{d, d, NO_FALL32, d + 1};
         }
     } else {
 #pragma unroll
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(256) c32_chunks(int T, int C, Work32 wk) {
     const int L = static_cast<int>(g / C), k = static_cast<int>(g % C), tile = k * C32_CHUNK + lane;
     const int64_t at = static_cast<int64_t>(L) * T + tile;
     const unsigned first = wk.code[static_cast<int64_t>(L) * T + k * C32_CHUNK];
-    Run32 f{0, 0, 0, 0};
+    Run32 f = STILL32;
     bool ok = first != C32_NONE;
     if (tile < T) {
         ok = ok && wk.code[at] == first;
@@ -438,7 +444,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
         if (code != C32_NONE && tile % C32_CHUNK == 0) {
             const int k = c + lane;
             unsigned kc = C32_NONE;
-            Run32 f{0, 0, 0, 0};
+            Run32 f = STILL32;
             if (k < C) {
                 kc = k < W32_CHUNKS ? sm.ccode[k] : gccode[k];
                 if (kc == code) f = k < W32_CHUNKS ? sm.crun[k] : gcrun[k];
@@ -455,7 +461,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
         if (code != C32_NONE) {
             const int j = j0 + lane, k = tile + lane;
             unsigned kc = C32_NONE;
-            Run32 f{0, 0, 0, 0};
+            Run32 f = STILL32;
             if (j < C32_CHUNK && k < T) {
                 kc = slot >= 0 ? sm.code[slot][j] : gcode[k];
                 if (kc == code) f = slot >= 0 ? sm.run[slot][j] : grun[k];
@@ -503,7 +509,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
             if (rest == 0) break;
             done = __ffs(rest) - 1;
             if (now != C32_NONE) {
-                Run32 f{0, 0, 0, 0};
+                Run32 f = STILL32;
                 const bool ok = lane < done || run32<R32_ROWS>(v, now, &f);
                 const int m = advance32(f, ok, &s);
                 if (m > done) {
