@@ -41,6 +41,14 @@ struct BSeg {
     int64_t index;  // position of the array in the caller's list
 };
 
+// A batched argsort's outputs: their rows' addresses, and the tables on the device that hold them.
+struct BatchOuts {
+    std::vector<void *> rows;
+    DeviceMem outs;         // output pointers [n], index order
+    DeviceMem segs;         // SortSeg[n] and each tile's array, when arrays are sorted for themselves
+    bool captured = false;  // a graph holds the tables: kept until the batch is freed
+};
+
 }  // namespace vkc
 
 struct vkc_batch {
@@ -51,16 +59,14 @@ struct vkc_batch {
     int64_t total = 0;
     vkc::DeviceMem table;             // BSeg[n] on the device, largest first
     vkc::DeviceMem bases;             // int64 first rows [n + 1], index order (for the argsort)
-    vkc::DeviceMem outs;              // argsort output pointers [n], index order
     vkc::DeviceMem chunks;            // int64 [n + 1]: first concat chunk of each array, table order
     // Argsort scratch, made on first use.
     std::vector<vkc_array *> scratch;
     void *img[2] = {nullptr, nullptr};  // 64-bit images of `total` rows each
     unsigned *pos[2] = {nullptr, nullptr};
     unsigned *counts = nullptr, *offs = nullptr, *sums = nullptr;
-    const vkc_batch *out_batch = nullptr;  // the batch whose pointers `outs` and `segs` hold
-    std::unique_ptr<vkc::DeviceMem> segs;  // SortSeg[n] and each tile's array, when arrays are sorted for themselves
-    int seg_tiles = 0, seg_tile = 0;       // their tiles, or 0, and a tile's rows
+    int seg_tiles = 0, seg_tile = 0;  // tiles of arrays sorted for themselves, or 0, and a tile's rows
+    std::vector<std::unique_ptr<vkc::BatchOuts>> outs;  // the last few outputs' tables, and captured ones
 };
 
 namespace vkc {
@@ -485,31 +491,87 @@ static void plan_segs(vkc_batch *b) {
     b->seg_tiles = b->total >= tiles * (b->seg_tile / 2) ? static_cast<int>(tiles) : 0;
 }
 
-// The table of the arrays in the concatenation's order and of their tiles.
-static vkc_status upload_segs(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *outs) {
-    const size_t n = keys->arrays.size(), bytes = sizeof(SortSeg) * n + sizeof(int) * keys->seg_tiles;
-    std::vector<unsigned char> table(bytes);
-    auto *segs = reinterpret_cast<SortSeg *>(table.data());
-    int *tile = reinterpret_cast<int *>(segs + n);
-    int64_t base = 0, t = 0;
-    for (size_t i = 0; i < n; ++i) {
-        const vkc_array *a = keys->arrays[i];
-        segs[i] = SortSeg{static_cast<const unsigned long long *>(a->data()), static_cast<long long *>(outs->arrays[i]->data()), base,
-                          a->len, t};
-        for (int64_t j = 0; j < a->len; j += keys->seg_tile) tile[t++] = static_cast<int>(i);
-        base += a->len;
+static vkc_status upload_table(vkc_ctx *ctx, DeviceMem &m, const void *src, size_t bytes) {
+    void *h;
+    m.box = ctx->box;
+    VKC_CUDA(ctx, cudaMallocAsync(&m.ptr, bytes, ctx->stream));
+    const vkc_status st = pinned(ctx, bytes, &h);
+    if (st) return st;
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    memcpy(h, src, bytes);
+    VKC_CUDA(ctx, cudaMemcpyAsync(m.ptr, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return VKC_OK;
+}
+
+// The sort's scratch (it depends on the keys alone): all of it or none.
+static vkc_status argsort_scratch(vkc_ctx *ctx, vkc_batch *keys) {
+    const int64_t total = keys->total;
+    int64_t cw, sw;
+    radix_table_words(total, &cw, &sw);
+    plan_segs(keys);
+    if (keys->seg_tiles) {
+        cw = std::max(cw, int64_t(256) * keys->seg_tiles);
+        sw = std::max(sw, scan_counts_sum_words(cw));
     }
-    void *p = nullptr, *h;
-    VKC_CUDA(ctx, cudaMallocAsync(&p, bytes, ctx->stream));
-    keys->segs = std::make_unique<DeviceMem>();
-    keys->segs->ptr = p;
-    keys->segs->box = ctx->box;
-    vkc_status st;
-    if ((st = pinned(ctx, bytes, &h))) return st;
-    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    memcpy(h, table.data(), bytes);
-    VKC_CUDA(ctx, cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
-    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    vkc_array *a[7] = {};
+    const vkc_type ty[7] = {VKC_U64, VKC_U64, VKC_I32, VKC_I32, VKC_I32, VKC_I32, VKC_I32};
+    const int64_t len[7] = {total, total, total, total, cw, cw, sw};
+    for (int i = 0; i < 7; ++i) {
+        const vkc_status st = new_array(ctx, ty[i], len[i], false, &a[i]);
+        if (st) {
+            for (int j = 0; j < i; ++j) vkc_array_release(a[j]);
+            return st;
+        }
+    }
+    keys->scratch.assign(a, a + 7);
+    keys->img[0] = a[0]->data();
+    keys->img[1] = a[1]->data();
+    keys->pos[0] = static_cast<unsigned *>(a[2]->data());
+    keys->pos[1] = static_cast<unsigned *>(a[3]->data());
+    keys->counts = static_cast<unsigned *>(a[4]->data());
+    keys->offs = static_cast<unsigned *>(a[5]->data());
+    keys->sums = static_cast<unsigned *>(a[6]->data());
+    return VKC_OK;
+}
+
+// The tables of these outputs, made on their first use. Outputs are told apart by their rows' addresses,
+// all that the tables hold of them: a batch's own address may be another one's after it is freed.
+constexpr int BATCH_OUTS = 4;  // outputs whose tables are kept beside the captured ones
+static vkc_status argsort_outs(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *outs, bool cap, const BatchOuts **found) {
+    const size_t n = keys->arrays.size();
+    for (auto &o : keys->outs) {
+        bool same = true;
+        for (size_t i = 0; i < n && same; ++i) same = o->rows[i] == outs->arrays[i]->data();
+        if (!same) continue;
+        o->captured = o->captured || cap;
+        *found = o.get();
+        return VKC_OK;
+    }
+    if (cap) return fail(ctx, VKC_USAGE, "batch argsort: make its first call before capturing");
+    auto o = std::make_unique<BatchOuts>();
+    for (const vkc_array *a : outs->arrays) o->rows.push_back(a->data());
+    vkc_status st = upload_table(ctx, o->outs, o->rows.data(), sizeof(void *) * n);
+    if (!st && keys->seg_tiles) {
+        // The arrays in the concatenation's order, and each tile's array.
+        std::vector<unsigned char> table(sizeof(SortSeg) * n + sizeof(int) * keys->seg_tiles);
+        auto *segs = reinterpret_cast<SortSeg *>(table.data());
+        int *tile = reinterpret_cast<int *>(segs + n);
+        int64_t base = 0, t = 0;
+        for (size_t i = 0; i < n; ++i) {
+            const vkc_array *a = keys->arrays[i];
+            segs[i] = SortSeg{static_cast<const unsigned long long *>(a->data()), static_cast<long long *>(o->rows[i]), base, a->len, t};
+            for (int64_t j = 0; j < a->len; j += keys->seg_tile) tile[t++] = static_cast<int>(i);
+            base += a->len;
+        }
+        st = upload_table(ctx, o->segs, table.data(), table.size());
+    }
+    if (st) return st;
+    const auto old = std::find_if(keys->outs.begin(), keys->outs.end(), [](const auto &p) { return !p->captured; });
+    if (std::count_if(keys->outs.begin(), keys->outs.end(), [](const auto &p) { return !p->captured; }) >= BATCH_OUTS)
+        keys->outs.erase(old);
+    keys->outs.push_back(std::move(o));
+    *found = keys->outs.back().get();
     return VKC_OK;
 }
 
@@ -530,48 +592,14 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
     for (int i = 0; i < n; ++i) await_write(ctx, outs->arrays[i]);
     if (total >= (int64_t(1) << 32)) return fail(ctx, VKC_USAGE, "batch argsort of 2^32 rows or more");
     const bool cap = capturing(ctx);
-    // Scratch (first use only, never during a capture).
-    if (keys->scratch.empty() || keys->out_batch != outs) {
+    vkc_status st;
+    // Scratch and the outputs' tables: on first use, never during a capture.
+    if (keys->scratch.empty()) {
         if (cap) return fail(ctx, VKC_USAGE, "batch argsort: make its first call before capturing");
-        vkc_status st;
-        for (vkc_array *a : keys->scratch) vkc_array_release(a);
-        keys->scratch.clear();
-        int64_t cw, sw;
-        radix_table_words(total, &cw, &sw);
-        plan_segs(keys);
-        if (keys->seg_tiles) {
-            cw = std::max(cw, int64_t(256) * keys->seg_tiles);
-            sw = std::max(sw, scan_counts_sum_words(cw));
-        }
-        vkc_array *a[7];
-        const vkc_type ty[7] = {VKC_U64, VKC_U64, VKC_I32, VKC_I32, VKC_I32, VKC_I32, VKC_I32};
-        const int64_t len[7] = {total, total, total, total, cw, cw, sw};
-        for (int i = 0; i < 7; ++i) {
-            if ((st = new_array(ctx, ty[i], len[i], false, &a[i]))) return st;
-            keys->scratch.push_back(a[i]);
-        }
-        keys->img[0] = a[0]->data();
-        keys->img[1] = a[1]->data();
-        keys->pos[0] = static_cast<unsigned *>(a[2]->data());
-        keys->pos[1] = static_cast<unsigned *>(a[3]->data());
-        keys->counts = static_cast<unsigned *>(a[4]->data());
-        keys->offs = static_cast<unsigned *>(a[5]->data());
-        keys->sums = static_cast<unsigned *>(a[6]->data());
-        std::vector<long long *> optr(n);
-        for (int i = 0; i < n; ++i) optr[i] = static_cast<long long *>(outs->arrays[i]->data());
-        void *p = nullptr;
-        VKC_CUDA(ctx, cudaMallocAsync(&p, sizeof(long long *) * n, ctx->stream));
-        keys->outs.ptr = p;
-        keys->outs.box = ctx->box;
-        void *h;
-        if ((st = pinned(ctx, sizeof(long long *) * n, &h))) return st;
-        VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        memcpy(h, optr.data(), sizeof(long long *) * n);
-        VKC_CUDA(ctx, cudaMemcpyAsync(p, h, sizeof(long long *) * n, cudaMemcpyHostToDevice, ctx->stream));
-        VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if (keys->seg_tiles && (st = upload_segs(ctx, keys, outs))) return st;
-        keys->out_batch = outs;
+        if ((st = argsort_scratch(ctx, keys))) return st;
     }
+    const BatchOuts *to;
+    if ((st = argsort_outs(ctx, keys, outs, cap, &to))) return st;
     if (n > 65536) return fail(ctx, VKC_USAGE, "batch argsort of more than 65536 arrays");
     const auto *tab = static_cast<const BSeg *>(keys->table.ptr);
     const auto *bases = static_cast<const int64_t *>(keys->bases.ptr);
@@ -585,7 +613,7 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
         if ((key_digits >> k) & 1u) d.shift[d.n++] = 8 * k;
     d.run = d.shift[d.n - 1] - d.shift[0] == 8 * (d.n - 1);
     if (keys->seg_tiles) {
-        const auto *segs = static_cast<const SortSeg *>(keys->segs->ptr);
+        const auto *segs = static_cast<const SortSeg *>(to->segs.ptr);
         return radix_segs(ctx, BatchSegs{segs, reinterpret_cast<const int *>(segs + n), keys->seg_tiles, keys->seg_tile, d}, keys->img,
                           keys->pos, total, RadixTables{keys->counts, keys->offs, keys->sums});
     }
@@ -593,9 +621,8 @@ extern "C" VKC_API vkc_status vkc_batch_argsort_i64(vkc_ctx *ctx, vkc_batch *key
     int shifts[8];
     for (int k = 0; k < 8; ++k) shifts[k] = 8 * k;
     const RadixTables t{keys->counts, keys->offs, keys->sums};
-    BatchOut batch{bases, static_cast<const unsigned long long *>(keys->outs.ptr), 8 * d.n};
+    BatchOut batch{bases, static_cast<const unsigned long long *>(to->outs.ptr), 8 * d.n};
     const int blocks = static_cast<int>(nchunks);
-    vkc_status st;
     if (digits <= 4) {
         batch_images_kernel<unsigned, true><<<blocks, 256, 0, ctx->stream>>>(tab, n, ch, d, static_cast<unsigned *>(keys->img[1]));
         if ((st = launched(ctx, "batch_images"))) return st;
