@@ -1853,18 +1853,19 @@ struct CanonReducer : DevReducer {
         vkc_status st = take(ctx, args, nargs, &a);
         if (st) return st;
         const int64_t n = args[0].len();
-        auto *to = static_cast<unsigned long long *>(dst ? dst : (host ? host : &static_cast<CanonState *>(state)->result));
+        if (!dst && !(dst = slot(ctx))) dst = &static_cast<CanonState *>(state)->result;
+        auto *to = static_cast<unsigned long long *>(dst);
         st = n / 16 <= CANON_SEQ_BLOCKS ? seq(ctx, a, n, to) : tiles(ctx, a, n / 16, static_cast<int>(n % 16), to);
-        if (st || dst) return st;
+        if (st || !out) return st;
         out->type = VKC_F64;
-        return host ? result(ctx, &out->bits, 8) : download(ctx, &out->bits, 8, offsetof(CanonState, result));
+        return result(ctx, &out->bits, 8, offsetof(CanonState, result));
     }
 
     // finish_lanes on the device; the result in the state and the slot.
     vkc_status combine(vkc_ctx *ctx) {
         vkc_status st;
         if (fresh && (st = zero(ctx))) return st;
-        canon_finish<<<1, 1, 0, ctx->stream>>>(static_cast<CanonState *>(state), tail_len, static_cast<unsigned long long *>(host));
+        canon_finish<<<1, 1, 0, ctx->stream>>>(static_cast<CanonState *>(state), tail_len, static_cast<unsigned long long *>(slot(ctx)));
         updated(ctx);
         return launched(ctx, "canon_finish");
     }
@@ -1872,7 +1873,7 @@ struct CanonReducer : DevReducer {
         const vkc_status st = combine(ctx);
         if (st) return st;
         out->type = VKC_F64;
-        return host ? result(ctx, &out->bits, 8) : download(ctx, &out->bits, 8, offsetof(CanonState, result));
+        return result(ctx, &out->bits, 8, offsetof(CanonState, result));
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
         const vkc_status st = combine(ctx);

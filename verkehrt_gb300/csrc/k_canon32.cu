@@ -720,7 +720,7 @@ template <int OP> struct Canon32Reducer : DevReducer {
     }
     vkc_status read(vkc_ctx *ctx, vkc_scalar *out) {
         unsigned b = 0;
-        const vkc_status st = host ? result(ctx, &b, 4) : download(ctx, &b, 4, offsetof(State32, result));
+        const vkc_status st = result(ctx, &b, 4, offsetof(State32, result));
         out->type = VKC_F32;
         out->bits = b;
         return st;
@@ -733,15 +733,16 @@ template <int OP> struct Canon32Reducer : DevReducer {
         if (st) return st;
         const int64_t n = args[0].len();
         auto *s = static_cast<State32 *>(state);
-        auto *to = static_cast<float *>(dst ? dst : (host ? host : &s->result));
+        if (!dst && !(dst = slot(ctx))) dst = &s->result;
+        auto *to = static_cast<float *>(dst);
         st = launch_chain32<OP>(ctx, a, static_cast<int>(n / 16), static_cast<int>(n % 16), fresh, s, to);
         updated(ctx);
-        return st || dst ? st : read(ctx, out);
+        return st || !out ? st : read(ctx, out);
     }
     vkc_status combine(vkc_ctx *ctx) {
         vkc_status st;
         if (fresh && (st = zero(ctx))) return st;
-        launch_next(c32_finish, 1, 1, 0, ctx->stream, static_cast<State32 *>(state), tail_len, static_cast<float *>(host));
+        launch_next(c32_finish, 1, 1, 0, ctx->stream, static_cast<State32 *>(state), tail_len, static_cast<float *>(slot(ctx)));
         updated(ctx);
         return launched(ctx, "canon32_finish");
     }

@@ -374,7 +374,7 @@ struct FamReducer : DevReducer {
         const int grid = stream_grid(ctx, n, 256, tune(ctx, TK_STREAM_BLOCKS, n), 4096);
         void *part;
         if ((st = scratch(ctx, 16 * static_cast<size_t>(grid), &part))) return st;
-        launch(ctx, a, n, grid, part, base, fresh, static_cast<u64 *>(state), static_cast<u64 *>(host));
+        launch(ctx, a, n, grid, part, base, fresh, static_cast<u64 *>(state), static_cast<u64 *>(slot(ctx)));
         updated(ctx);
         base += static_cast<u64>(n);
         return launched(ctx, "family_fold");
@@ -512,7 +512,7 @@ template <vkc_type T> struct ChainReducer : DevReducer {
         return launched(ctx, "family_chain");
     }
     vkc_status combine(vkc_ctx *ctx) {
-        fam_chain_finish<T><<<1, 1, 0, ctx->stream>>>(static_cast<u64 *>(state), tail_len, static_cast<u64 *>(host));
+        fam_chain_finish<T><<<1, 1, 0, ctx->stream>>>(static_cast<u64 *>(state), tail_len, static_cast<u64 *>(slot(ctx)));
         updated(ctx);
         return launched(ctx, "family_chain_finish");
     }
@@ -520,7 +520,7 @@ template <vkc_type T> struct ChainReducer : DevReducer {
         vkc_status st = combine(ctx);
         if (st) return st;
         u64 r = 0;
-        if ((st = host ? result(ctx, &r, 8) : download(ctx, &r, 8, 32 * 8))) return st;
+        if ((st = result(ctx, &r, 8, 32 * 8))) return st;
         *out = word_scalar(T, r);
         return VKC_OK;
     }

@@ -142,7 +142,7 @@ struct CountReducer : DevReducer {
         if ((st = scratch(ctx, sizeof(unsigned long long) * grid, &part))) return st;
         auto *s = static_cast<unsigned long long *>(state);
         auto *pp = static_cast<unsigned long long *>(part);
-        auto *hs = static_cast<unsigned long long *>(host);
+        auto *hs = static_cast<unsigned long long *>(slot(ctx));
         if (cmp < 0) {
             count_kernel<true, false><<<grid, 256, 0, ctx->stream>>>(args[0].a->data(), n, CmpRange{}, pp, ctx->counters + 1, fresh, s, hs);
         } else {
@@ -370,9 +370,10 @@ struct ExtremeReducer : DevReducer {
         if ((st = scratch(ctx, sizeof(ExtState) * grid, &part))) return st;
         auto *p = static_cast<ExtState *>(part);
         auto *s = static_cast<ExtState *>(state);
+        auto *hs = static_cast<ExtState *>(slot(ctx));
         const long long *x = static_cast<const long long *>(args[0].a->data());
         bool f = type == VKC_F64;
-#define EXT_LAUNCH(MX, F, A) extreme_kernel<MX, F, A><<<grid, 256, 0, ctx->stream>>>(x, n, consumed, p, ctx->counters + 1, fresh, s, static_cast<ExtState *>(host))
+#define EXT_LAUNCH(MX, F, A) extreme_kernel<MX, F, A><<<grid, 256, 0, ctx->stream>>>(x, n, consumed, p, ctx->counters + 1, fresh, s, hs)
         if (arg) {
             if (max && f) EXT_LAUNCH(true, true, true);
             else if (max) EXT_LAUNCH(true, false, true);
@@ -483,7 +484,7 @@ struct IntSumReducer : DevReducer {
         isum_kernel<<<grid, 256, 0, ctx->stream>>>(
             static_cast<const unsigned long long *>(args[0].a->data()), n,
             static_cast<unsigned long long *>(part), ctx->counters + 1, fresh,
-            static_cast<unsigned long long *>(state), static_cast<unsigned long long *>(host));
+            static_cast<unsigned long long *>(state), static_cast<unsigned long long *>(slot(ctx)));
         updated(ctx);
         return launched(ctx, "isum");
     }

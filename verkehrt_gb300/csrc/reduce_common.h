@@ -20,23 +20,33 @@ static __global__ void reducer_fill_kernel(unsigned long long *p, int n, Words4 
 }
 
 // A reducer whose running state is a small device buffer owned by the reducer, uninitialised until
-// the first update (`fresh`: its kernels then read no state, which saves a launch to clear it). The
-// kernel that ends an update also writes the state's result words to `host`, a pinned slot, so that
+// the first update (`fresh`: its kernels then read no state, which saves a launch to clear it).
+// The kernel that ends an update also writes the state's result words to a pinned slot, so that
 // finish only waits for the stream: a call of a few rows costs one launch and one wait (a cleared
 // state, a device-to-host copy and the pool's allocation and release around it made count_gt_f64 of
-// 4096 rows take 31 us a call, now 20). Without a slot (all taken, or a capture) finish copies.
+// 4096 rows take 31 us a call, now 20). Without a slot finish copies: where the result goes to a device
+// address, where all slots are taken, and once an update was captured, whose replays write no slot.
 struct DevReducer : ReducerImpl {
     void *state = nullptr;
     size_t bytes = 0;
     DeviceMem mem;  // gives `state` back on the context's stream, even after the context closed
-    void *host = nullptr;
+    void *host = nullptr;  // the slot, from the first update that writes one
+    bool copies = false;   // no update writes the slot from here on
     bool fresh = true;
     cudaStream_t used = nullptr;  // the stream of the updates since the last result was read
+    // The slot of a reducer dropped without finish may still be written: by the stream `used`.
     ~DevReducer() override {
-        if (!host) return;
-        // A reducer dropped without finish may still have a kernel that writes the slot.
-        if (used) cudaStreamSynchronize(used);
-        mem.box->give_slot(host);
+        if (host) mem.box->give_slot(host, used);
+    }
+    // Where an update that is about to be launched writes its result, or nullptr.
+    void *slot(vkc_ctx *ctx) {
+        if (copies) return nullptr;
+        copies = stream_capturing(ctx->stream);
+        if (!copies && !host) {
+            host = mem.box->take_slot(ctx->stream);
+            copies = !host;
+        }
+        return copies ? nullptr : host;
     }
     // After an update's launch.
     void updated(vkc_ctx *ctx) {
@@ -47,11 +57,10 @@ struct DevReducer : ReducerImpl {
         bytes = n;
         bool captured;
         const vkc_status st = state_block(ctx, n, &mem, &captured);
-        if (st) return st;
         state = mem.ptr;
-        if (!captured) host = ctx->box->take_slot();
-        return VKC_OK;
+        return st;
     }
+    void into_device() override { copies = true; }
     // The state's n bytes zeroed (before a first update whose kernels read it).
     vkc_status zero(vkc_ctx *ctx) {
         VKC_CUDA(ctx, cudaMemsetAsync(state, 0, bytes, ctx->stream));
@@ -65,9 +74,10 @@ struct DevReducer : ReducerImpl {
                                                        Words4{{w0, w1, w2, w3}});
         return launched(ctx, "reducer_fill");
     }
-    // What the updates left in the slot, once the stream is done; or the state's first n bytes.
-    vkc_status result(vkc_ctx *ctx, void *h, size_t n) {
-        if (!host) return download(ctx, h, n);
+    // What the updates left in the slot, once the stream is done; or the state's n bytes from byte `at`,
+    // where those words lie in it.
+    vkc_status result(vkc_ctx *ctx, void *h, size_t n, size_t at = 0) {
+        if (copies || !host) return download(ctx, h, n, at);
         VKC_CUDA(ctx, cudaStreamSynchronize(used));
         used = nullptr;
         memcpy(h, host, n);

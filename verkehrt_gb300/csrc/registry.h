@@ -47,6 +47,8 @@ struct ReducerImpl {
     // report, an empty input where that is an error, is decided by the rows the reducer was
     // given, which the host knows.
     virtual vkc_status finish_into(vkc_ctx *ctx, void *dst);
+    // The result will go to a device address (once with dst, finish_into): nothing for the host to read.
+    virtual void into_device() {}
     // One update with every row and finish, where a reducer can run both in one launch (*done): the
     // result goes to *out, or with `dst` its bits to that device address, enqueued only.
     virtual vkc_status once(vkc_ctx *, const Arg *, int, vkc_scalar *, void *, bool *done) {

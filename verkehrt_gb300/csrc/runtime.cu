@@ -57,24 +57,28 @@ void StreamBox::give(void *p, size_t cls) {
     cudaFreeAsync(p, stream);
 }
 
-void *StreamBox::take_slot() {
+void *StreamBox::take_slot(cudaStream_t s) {
     std::lock_guard<std::mutex> lock(mu);
     if (!slots && cudaMallocHost(reinterpret_cast<void **>(&slots), RESULT_SLOT * RESULT_SLOTS) != cudaSuccess) {
         cudaGetLastError();
         slots = nullptr;
         return nullptr;
     }
+    const uint64_t taken = s == stream ? slots_used : slots_used | slots_late;
     for (int i = 0; i < RESULT_SLOTS; ++i)
-        if (!((slots_used >> i) & 1)) {
+        if (!((taken >> i) & 1)) {
             slots_used |= uint64_t(1) << i;
             return slots + i * RESULT_SLOT;
         }
     return nullptr;
 }
 
-void StreamBox::give_slot(void *slot) {
+void StreamBox::give_slot(void *slot, cudaStream_t writer) {
+    if (writer && writer != stream) return;
     std::lock_guard<std::mutex> lock(mu);
-    slots_used &= ~(uint64_t(1) << ((static_cast<char *>(slot) - slots) / RESULT_SLOT));
+    const uint64_t bit = uint64_t(1) << ((static_cast<char *>(slot) - slots) / RESULT_SLOT);
+    slots_used &= ~bit;
+    slots_late = writer ? slots_late | bit : slots_late & ~bit;
 }
 
 DeviceMem::~DeviceMem() {
@@ -95,7 +99,6 @@ Buffer::~Buffer() {
 
 // Makes `stream` wait for *e (once), then drops the event. Under graph capture an event from
 // outside the capture cannot be waited on by the stream, so the host waits for it instead.
-static bool stream_capturing(cudaStream_t stream);
 // A host wait for an event, allowed during this thread's stream capture.
 static void host_wait(cudaEvent_t e) {
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -128,7 +131,7 @@ void await_values(vkc_ctx *ctx, const vkc_value *args, int nargs) {
         if (args[i].kind == VKC_VALUE_ARRAY && args[i].array) await_read(ctx, args[i].array);
 }
 
-static bool stream_capturing(cudaStream_t stream) {
+bool stream_capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
 }
@@ -978,6 +981,7 @@ vkc_status vkc_call_into(vkc_ctx *ctx, int id, const vkc_value *args, int nargs,
     await_write(ctx, out);
     ReducerImpl *r = d->red(ctx);
     if (!r) return ctx->err.empty() ? fail(ctx, VKC_ALLOC, "cannot allocate a reducer") : VKC_ALLOC;
+    r->into_device();
     // As vkc_call: one update with all rows, none on empty input.
     void *dst = static_cast<char *>(out->data()) + row * type_width(out->type);
     bool done = false;

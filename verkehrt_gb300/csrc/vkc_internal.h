@@ -53,7 +53,7 @@ struct StreamBox {
     // Pinned host slots of RESULT_SLOT bytes for results that kernels write themselves (made on
     // first use, freed with the box): bit i of slots_used is set while slot i is taken.
     char *slots = nullptr;
-    uint64_t slots_used = 0;
+    uint64_t slots_used = 0, slots_late = 0;
     ~StreamBox();
     // A block of at least `bytes` (its class size in *cls), or nullptr.
     void *take(size_t bytes, size_t *cls);
@@ -61,9 +61,12 @@ struct StreamBox {
     void give(void *p, size_t cls);
     // Frees every cached block.
     void release_all();
-    // A free result slot, or nullptr when all are taken.
-    void *take_slot();
-    void give_slot(void *slot);
+    // A free result slot for kernels of `s`, or nullptr when there is none.
+    void *take_slot(cudaStream_t s);
+    // Gives it back. writer: a stream that may still run a kernel that writes it, or nullptr. On the
+    // box's own stream the next taker's kernels, and its wait, come after that one (slots_late); a slot
+    // that another stream may still write is not handed out again.
+    void give_slot(void *slot, cudaStream_t writer);
 };
 constexpr int RESULT_SLOT = 64, RESULT_SLOTS = 64;
 
@@ -219,6 +222,7 @@ vkc_status launched(vkc_ctx *ctx, const char *what);
 // New array of `len` rows (uninitialised unless `zero`). Message texts follow
 // src/value.rs:285-307.
 vkc_status new_array(vkc_ctx *ctx, vkc_type t, int64_t len, bool zero, vkc_array **out);
+bool stream_capturing(cudaStream_t stream);
 // A device block for a small state (uninitialised), from the box's cache where that is possible: a
 // block taken while a graph is captured belongs to the graph's replays, so it is the graph's own
 // allocation then. *captured tells which.
