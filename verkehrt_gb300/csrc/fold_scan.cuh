@@ -42,7 +42,7 @@ template <vkc_type IT, int F> struct ScanOp {
     using SW = typename std::conditional<OW == 8, long long, int>::type;
     static constexpr int SIGN = 8 * sizeof(W) - 1;
 
-    __device__ static __forceinline__ W key(W b) { return b ^ (static_cast<W>(static_cast<SW>(b) >> SIGN) >> 1); }
+    __host__ __device__ static __forceinline__ W key(W b) { return b ^ (static_cast<W>(static_cast<SW>(b) >> SIGN) >> 1); }
     // The canonical NaN's bits; its key: above +inf's of a maximum, below -inf's of a minimum.
     static constexpr W QNAN = OW == 8 ? static_cast<W>(0x7ff8000000000000ull) : static_cast<W>(0x7fc00000u);
     static constexpr W NAN_KEY = F == F_MAX ? QNAN : static_cast<W>(~QNAN);
@@ -59,7 +59,7 @@ template <vkc_type IT, int F> struct ScanOp {
         if (!FLT) return k;
         return F == F_MIN && k == NAN_KEY ? QNAN : key(k);
     }
-    __device__ static __forceinline__ W ident() {
+    __host__ __device__ static __forceinline__ W ident() {
         constexpr u64 id = identity<OT, F>();
         return FLT ? key(static_cast<W>(id)) : static_cast<W>(id);
     }
@@ -409,9 +409,14 @@ void launch_scan(int device, int sms, cudaStream_t stream, const void *x, const 
 }
 
 template <vkc_type IT, int F, bool BY> struct ScanImpl : ScannerImpl {
-    ScanState *state = nullptr;  // uninitialised until the first update (fresh)
+    ScanState *state = nullptr;  // uninitialised until the first update (fresh) or begin
     bool fresh = true;
     DeviceMem mem;  // owns `state`
+    vkc_status begin(vkc_ctx *ctx) override {
+        fresh = false;
+        reducer_fill_kernel<<<1, 64, 0, ctx->stream>>>(&state->last, 1, Words4{{static_cast<u64>(ScanOp<IT, F>::ident())}});
+        return launched(ctx, "scan_begin");
+    }
     // scan.rs:228-282 (tile_rows): arity, kinds, then destination rows.
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs, vkc_array *out) override {
         vkc_status st;

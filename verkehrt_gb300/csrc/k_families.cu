@@ -228,7 +228,11 @@ __global__ void __launch_bounds__(256) fam_fold_kernel(RowArgs a, int64_t n, u64
         if (threadIdx.x == 0) {
             if (!fresh) s = step<AT, F>(state[0], s);
             state[0] = s;
-            if (host) host[0] = s;
+            state[2] = 1;  // rows seen
+            if (host) {
+                host[0] = s;
+                host[2] = 1;
+            }
         }
     }
 }
@@ -313,9 +317,11 @@ __global__ void __launch_bounds__(256) fam_arg_kernel(const void *x, int64_t n, 
             if (!fresh) arg_better(bh, br, state[0], state[1]);
             state[0] = bh;
             state[1] = br;
+            state[2] = 1;
             if (host) {
                 host[0] = bh;
                 host[1] = br;
+                host[2] = 1;
             }
         }
     }
@@ -337,7 +343,8 @@ u64 scalar_word(vkc_type t, const vkc_scalar &s) {
     return s.bits;
 }
 
-// Reducers of the order-free folds. State: [0] the folded word (argmin/argmax: [0] key, [1] row).
+// Reducers of the order-free folds. State: [0] the folded word (argmin/argmax: [0] key, [1] row), [2]
+// whether any row was seen.
 // `base` counts the rows of earlier updates.
 struct FamReducer : DevReducer {
     vkc_type in, out;
@@ -348,10 +355,14 @@ struct FamReducer : DevReducer {
     bool empty_error = false;  // min/max/argmin/argmax of no rows fail
     const char *what = "";
     u64 base = 0;
-    u64 empty = 0;  // the result word of no rows
+    u64 empty = ~0ull;  // the word of no rows: the result, or argmin/argmax's key
     using Launch = void (*)(vkc_ctx *, const RowArgs &, int64_t, int, void *, u64, bool, u64 *, u64 *);
     Launch launch = nullptr;
 
+    vkc_status begin(vkc_ctx *ctx) override {
+        fresh = false;
+        return fill(ctx, 3, empty, ~0ull, 0);
+    }
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != nargs_want) return fail(ctx, VKC_RUNTIME, arity_error(nargs_want, nargs));
@@ -380,15 +391,15 @@ struct FamReducer : DevReducer {
         return launched(ctx, "family_fold");
     }
     vkc_status finish(vkc_ctx *ctx, vkc_scalar *out_s) override {
-        if (empty_error && fresh) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
-        u64 h[2] = {empty, 0};
+        u64 h[3] = {empty, 0, 0};
         vkc_status st = fresh ? VKC_OK : result(ctx, h, sizeof h);
         if (st) return st;
+        if (empty_error && !h[2]) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
         *out_s = fold < 0 ? scalar_i64(static_cast<int64_t>(h[1])) : word_scalar(out, h[0]);
         return VKC_OK;
     }
     vkc_status finish_into(vkc_ctx *ctx, void *dst) override {
-        if (empty_error && fresh) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
+        if (empty_error && base == 0) return fail(ctx, VKC_RUNTIME, std::string(what) + " of an empty array");
         const vkc_status st = fresh ? fill(ctx, 1, empty) : VKC_OK;
         if (st) return st;
         // Words are little-endian: the result type's bytes are the word's low bytes.
@@ -409,7 +420,7 @@ void launch_arg(vkc_ctx *ctx, const RowArgs &a, int64_t n, int grid, void *part,
 template <vkc_type T, int F, int ROW, int NARGS>
 ReducerImpl *make_fold(vkc_ctx *ctx, vkc_type out, int cmp, bool empty_error, const char *what) {
     auto *r = new FamReducer;
-    if (r->alloc(ctx, 16)) {
+    if (r->alloc(ctx, 24)) {
         delete r;
         return nullptr;
     }
@@ -428,7 +439,7 @@ ReducerImpl *make_fold(vkc_ctx *ctx, vkc_type out, int cmp, bool empty_error, co
 
 template <vkc_type T, bool MAX> ReducerImpl *make_arg(vkc_ctx *ctx) {
     auto *r = new FamReducer;
-    if (r->alloc(ctx, 16)) {
+    if (r->alloc(ctx, 24)) {
         delete r;
         return nullptr;
     }
@@ -495,6 +506,8 @@ template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len, u6
 // CanonicalAcc (reduce.rs:253-323) on the device. State: [0..15] lanes, [16..31] tail, [32] result.
 template <vkc_type T> struct ChainReducer : DevReducer {
     int tail_len = 0;
+
+    vkc_status begin(vkc_ctx *) override { return VKC_OK; }  // made with its state
 
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;

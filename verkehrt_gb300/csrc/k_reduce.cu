@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(256) extreme_kernel(const long long *__restric
             for (int w = 1; w < 8; ++w) take(ws[w].key, ws[w].idx, ws[w].nan_idx);
             if (!fresh) {
                 const ExtState s = *state;
-                take(s.key, s.idx, s.nan_idx);
+                if (s.seen) take(s.key, s.idx, s.nan_idx);
             }
             *state = ExtState{k, i, nn, 1};
             if (host) *host = ExtState{k, i, nn, 1};
@@ -359,6 +359,10 @@ struct ExtremeReducer : DevReducer {
     bool max, arg;
     vkc_type type;
     unsigned long long consumed = 0;
+    vkc_status begin(vkc_ctx *ctx) override {
+        fresh = false;
+        return fill(ctx, 4, 0, ~0ull, ~0ull, 0);  // ExtState{0, ~0, ~0, 0}
+    }
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));

@@ -20,7 +20,7 @@ static __global__ void reducer_fill_kernel(unsigned long long *p, int n, Words4 
 }
 
 // A reducer whose running state is a small device buffer owned by the reducer, uninitialised until
-// the first update (`fresh`: its kernels then read no state, which saves a launch to clear it).
+// the first update (`fresh`: its kernels then read no state, which saves a launch to clear it) or begin.
 // The kernel that ends an update also writes the state's result words to a pinned slot, so that
 // finish only waits for the stream: a call of a few rows costs one launch and one wait (a cleared
 // state, a device-to-host copy and the pool's allocation and release around it made count_gt_f64 of
@@ -59,6 +59,10 @@ struct DevReducer : ReducerImpl {
         const vkc_status st = state_block(ctx, n, &mem, &captured);
         state = mem.ptr;
         return st;
+    }
+    vkc_status begin(vkc_ctx *ctx) override {
+        fresh = false;
+        return zero(ctx);
     }
     void into_device() override { copies = true; }
     // The state's n bytes zeroed (before a first update whose kernels read it).

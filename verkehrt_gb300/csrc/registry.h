@@ -47,6 +47,9 @@ struct ReducerImpl {
     // report, an empty input where that is an error, is decided by the rows the reducer was
     // given, which the host knows.
     virtual vkc_status finish_into(vkc_ctx *ctx, void *dst);
+    // The state of no rows set on the device, for a reducer that outlives the call that made it: its
+    // updates may be captured in a graph, whose replays go on from the state they find.
+    virtual vkc_status begin(vkc_ctx *) { return VKC_OK; }
     // The result will go to a device address (once with dst, finish_into): nothing for the host to read.
     virtual void into_device() {}
     // One update with every row and finish, where a reducer can run both in one launch (*done): the
@@ -60,6 +63,8 @@ struct ReducerImpl {
 // Scanner (src/kernels.rs:65-88): carried state on the device.
 struct ScannerImpl {
     virtual ~ScannerImpl() {}
+    // The state of no rows set on the device (as ReducerImpl::begin).
+    virtual vkc_status begin(vkc_ctx *) { return VKC_OK; }
     virtual vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs, vkc_array *out) = 0;
 };
 

@@ -926,6 +926,11 @@ vkc_status vkc_reducer_new(vkc_ctx *ctx, int id, vkc_reducer **out) {
     if (d->cls != VKC_REDUCTION) return fail(ctx, VKC_USAGE, d->name + " is not a reduction");
     ReducerImpl *r = d->red(ctx);
     if (!r) return VKC_ALLOC;
+    const vkc_status st = r->begin(ctx);
+    if (st) {
+        delete r;
+        return st;
+    }
     *out = new vkc_reducer{ctx, r};
     return VKC_OK;
 }
@@ -1007,6 +1012,11 @@ vkc_status vkc_scanner_new(vkc_ctx *ctx, int id, vkc_scanner **out) {
     if (d->cls != VKC_SCAN) return fail(ctx, VKC_USAGE, d->name + " is not a scan");
     ScannerImpl *s = d->scan(ctx);
     if (!s) return VKC_ALLOC;
+    const vkc_status st = s->begin(ctx);
+    if (st) {
+        delete s;
+        return st;
+    }
     *out = new vkc_scanner{ctx, s};
     return VKC_OK;
 }
