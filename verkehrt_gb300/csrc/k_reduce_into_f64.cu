@@ -15,7 +15,8 @@
 //  * otherwise the rows below b are sorted, stably, by (key, stripe), a 32-bit image whose radix
 //    passes carry the values; each stripe of each bucket is then a contiguous chain that one thread
 //    adds in index order, the sixteen of a bucket side by side, so that they combine by shuffles;
-//    one thread folds the tail rows in order. (Until now an argsort, two gathers by its order and a
+//    one thread folds the tail rows in order. Buckets with chains far longer than even keys give are
+//    masked instead (rif_limit). (Until now an argsort, two gathers by its order and a
 //    warp a chain whose 32 lanes all ran the chain: 4.36 ms against 0.72 for 33 M rows in 1024
 //    buckets, 2.26 ms of it FP64 adds that 31 lanes repeated.)
 //  * buckets so many that a table of their chains would dwarf the rows (rif_tables): the chains are
@@ -23,6 +24,7 @@
 // Arguments and errors follow reduce_into_add_i64 (index.rs:194-222): the values' kind first,
 // then the keys (checked_keys, index.rs:116-130), a length mismatch, the result's allocation.
 #include <algorithm>
+#include <vector>
 
 #include "add_bits.cuh"
 #include "radix.h"
@@ -33,12 +35,27 @@ namespace vkc {
 vkc_status bucket_key_error(vkc_ctx *ctx, const long long *k, int64_t n, int64_t nb, bool *found);
 
 // Measured: the masked path costs about 130 us a bucket and 7.2 us a bucket per million rows; the
-// sorted one 100 us, 16 us per million rows and its chains at 40 ns a row (n / (16 nb) rows each when
-// the buckets are even). Masked where that is less: up to 1 bucket of 2^17 rows, 4 of 2^20, 15 of 2^25.
+// sorted one 100 us, 16 us per million rows and its longest chain at 40 ns a row, n / (16 nb) rows when
+// the keys are even. Masked where that is less: up to 1 bucket of 2^17 rows, 4 of 2^20, 15 of 2^25.
+static double rif_mask_us(int64_t n) { return 130.0 + 7.2e-6 * static_cast<double>(n); }
+constexpr double RIF_CHAIN_US = 0.04;  // a row of a chain
 static bool rif_masks(int64_t n, int64_t nb) {
-    const double m = static_cast<double>(n) * 1e-6, k = static_cast<double>(nb);
-    return k * (130.0 + 7.2 * m) < 100.0 + 16.0 * m + 2500.0 * m / k;
+    const double rows = static_cast<double>(n), k = static_cast<double>(nb);
+    return k * rif_mask_us(n) < 100.0 + 16e-6 * rows + RIF_CHAIN_US * rows / (16.0 * k);
 }
+// Keys need not be even. A bucket with a chain of more rows than this is left out of the sorted path's
+// first sums, which note it (RifHeavy): masked sums of such buckets follow where they take less than the
+// longest chain, else the chains themselves. Twice the even chain, so that keys about even are summed at
+// once; and rows that take as long as a bucket's masked sum. (2^25 rows, 95% of them in one of 16 / 1024
+// buckets: 83.1 / 83.0 ms in chains, 0.95 / 0.88 ms so; 16 even ones 5.83 ms either way.)
+static unsigned rif_limit(int64_t n, int64_t nb) {
+    const double rows = std::max(rif_mask_us(n) / RIF_CHAIN_US, static_cast<double>(n) / (8.0 * static_cast<double>(nb)));
+    return static_cast<unsigned>(std::min(rows, 4e9));
+}
+struct RifHeavy {
+    static constexpr int MOST = 254;
+    unsigned count, longest, bucket[MOST];  // all zero before the sums
+};
 // Images (key * 16 + stripe) of 32 bits, and a table of every chain no larger than a few rows' worth.
 static bool rif_tables(int64_t n, int64_t nb) {
     return n < (int64_t(1) << 32) && nb <= (int64_t(1) << 28) && nb <= n + (int64_t(1) << 16);
@@ -152,6 +169,13 @@ __global__ void rif_tail_kernel(const long long *__restrict__ keys, const unsign
         if (static_cast<uint64_t>(keys[i]) < nb) out[keys[i]] = static_cast<unsigned long long>(__double_as_longlong(__dadd_rn(as_f64(out[keys[i]]), as_f64(x[i]))));
 }
 
+static vkc_status rif_tail(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t b, int64_t n, int64_t nb,
+                           unsigned long long *out) {
+    if (b == n) return VKC_OK;
+    rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(keys, x, b, n, static_cast<uint64_t>(nb), out);
+    return launched(ctx, "rif_tail");
+}
+
 // A whole entry of the table by name, on array arguments; the result array in *res.
 static vkc_status call_whole(vkc_ctx *ctx, const char *name, std::initializer_list<const vkc_array *> arrays,
                              vkc_array **res) {
@@ -210,22 +234,41 @@ __global__ void __launch_bounds__(256) rif_spans_kernel(const unsigned *__restri
     }
 }
 
+// Whether a bucket, whose sixteen chains lie in sixteen lanes from `lane` & 16 on, has a chain of more than
+// `limit` rows; noted, and *flag set for the host, when `heavy` is given.
+__device__ __forceinline__ bool rif_is_heavy(unsigned len, unsigned limit, int64_t bucket, RifHeavy *heavy, unsigned *flag) {
+    unsigned most = len;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(FULL, most, o));
+    if (most <= limit) return false;
+    if (heavy && (threadIdx.x & 15) == 0) {
+        const unsigned i = atomicAdd(&heavy->count, 1u);
+        if (i < RifHeavy::MOST) heavy->bucket[i] = static_cast<unsigned>(bucket);
+        atomicMax(&heavy->longest, most);
+        *reinterpret_cast<volatile unsigned *>(flag) = 1u;
+    }
+    return true;
+}
+
 // One block per two buckets: a warp adds, one thread per chain, and a second warp copies the next
 // RC_ROWS rows of each of the 32 chains into shared memory (each a coalesced run, RC_STAGES - 1
 // stages ahead; by the adding warp itself the copies' issue took half as long again as the adds). A
 // row of a chain costs 31 ns, the latency of an FP64 add. (add_bits, the adds as integer steps, took
-// 110 ns: it pays where a chain's neighbours fill the pipe, not here.)
+// 110 ns: it pays where a chain's neighbours fill the pipe, not here.) With `heavy` the buckets with a
+// chain beyond `limit` are noted there and left out.
 constexpr int RC_ROWS = 32, RC_STAGES = 3, RC_PITCH = RC_ROWS + 1;
 
 __global__ void __launch_bounds__(64) rif_sum_kernel(const uint2 *__restrict__ span, const unsigned long long *__restrict__ v,
-                                                     int64_t nb, unsigned long long *__restrict__ out) {
+                                                     int64_t nb, unsigned long long *__restrict__ out, unsigned limit,
+                                                     RifHeavy *heavy, unsigned *flag) {
     __shared__ unsigned long long buf[RC_STAGES][32][RC_PITCH];
     const int lane = threadIdx.x & 31;
     const bool copies = threadIdx.x >= 32;
     for (int64_t pair = blockIdx.x; pair * 2 < nb; pair += gridDim.x) {
         const int64_t c = pair * 32 + lane;
         const uint2 s = c < nb * 16 ? span[c] : make_uint2(0u, 0u);
-        const unsigned len = s.y - s.x, most = __reduce_max_sync(FULL, len);
+        const bool mine = !heavy || !rif_is_heavy(s.y - s.x, limit, c >> 4, copies ? nullptr : heavy, flag);
+        const unsigned len = mine ? s.y - s.x : 0u, most = __reduce_max_sync(FULL, len);
         const int steps = static_cast<int>((static_cast<int64_t>(most) + RC_ROWS - 1) / RC_ROWS);
         auto issue = [&](int k) {
             if (k < steps) {
@@ -273,7 +316,7 @@ __global__ void __launch_bounds__(64) rif_sum_kernel(const uint2 *__restrict__ s
                 const double other = __shfl_down_sync(FULL, acc, step, 16);
                 if ((lane & 15) < step) acc = __dadd_rn(acc, other);
             }
-            if ((lane & 15) == 0 && c < nb * 16) out[c >> 4] = as_bits(acc);
+            if ((lane & 15) == 0 && c < nb * 16 && mine) out[c >> 4] = as_bits(acc);
         }
         __syncthreads();  // the buffers are free for the next pair
     }
@@ -284,9 +327,12 @@ __global__ void __launch_bounds__(64) rif_sum_kernel(const uint2 *__restrict__ s
 // buckets of 2^20 rows took 883 us.)
 constexpr int64_t RIF_SHORT_ROWS = 4;  // average rows of a chain below which this form runs
 __global__ void __launch_bounds__(256) rif_short_kernel(const uint2 *__restrict__ span, const unsigned long long *__restrict__ v,
-                                                        int64_t nb, unsigned long long *__restrict__ out) {
+                                                        int64_t nb, unsigned long long *__restrict__ out, unsigned limit,
+                                                        RifHeavy *heavy, unsigned *flag) {
     const int64_t c = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint2 s = c < nb * 16 ? span[c] : make_uint2(0u, 0u);
+    uint2 s = c < nb * 16 ? span[c] : make_uint2(0u, 0u);
+    const bool left_out = rif_is_heavy(s.y - s.x, limit, c >> 4, heavy, flag);
+    if (left_out) s.y = s.x;
     double acc = 0.0;
     for (unsigned p = s.x; p < s.y; p += 4) {
         double t[4];
@@ -300,63 +346,17 @@ __global__ void __launch_bounds__(256) rif_short_kernel(const uint2 *__restrict_
         const double other = __shfl_down_sync(FULL, acc, step, 16);
         if ((threadIdx.x & 15) < step) acc = __dadd_rn(acc, other);
     }
-    if ((threadIdx.x & 15) == 0 && c < nb * 16) out[c >> 4] = as_bits(acc);
+    if ((threadIdx.x & 15) == 0 && c < nb * 16 && !left_out) out[c >> 4] = as_bits(acc);
 }
 
-static vkc_status rif_sorted(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t n, int64_t b,
-                             int64_t nb, unsigned long long *out) {
-    int passes = 1;  // of the image's bits: the largest is 16 nb - 1
-    while (passes < 4 && ((16 * static_cast<uint64_t>(nb) - 1) >> (8 * passes))) ++passes;
-    static const int shifts[4] = {0, 8, 16, 24};
-    vkc_array *ia = nullptr, *ib = nullptr, *va = nullptr, *vb = nullptr, *ca = nullptr, *oa = nullptr, *sa = nullptr,
-              *sp = nullptr;
-    auto done = [&](vkc_status st) {
-        for (vkc_array *a : {ia, ib, va, vb, ca, oa, sa, sp})
-            if (a) vkc_array_release(a);
-        return st;
-    };
-    int64_t cw, sw;
-    radix_table_words(b, &cw, &sw);
-    vkc_status st;
-    if ((st = new_array(ctx, VKC_I32, b, false, &ia)) || (st = new_array(ctx, VKC_I32, b, false, &ib)) ||
-        (st = new_array(ctx, VKC_F64, b, false, &va)) || (passes > 1 && (st = new_array(ctx, VKC_F64, b, false, &vb))) ||
-        (st = new_array(ctx, VKC_I32, cw, false, &ca)) || (st = new_array(ctx, VKC_I32, cw, false, &oa)) ||
-        (st = new_array(ctx, VKC_I32, sw, false, &sa)) || (st = new_array(ctx, VKC_U64, 16 * nb, true, &sp)))
-        return done(st);
-    auto *first = static_cast<unsigned *>(ib->data());
-    rif_images_kernel<<<stream_grid(ctx, n, 256, 8, 4096), 256, 0, ctx->stream>>>(keys, n, b, static_cast<uint64_t>(nb), first,
-                                                                                  ctx->status);
-    if ((st = launched(ctx, "rif_images"))) return done(st);
-    const RadixTables t{static_cast<unsigned *>(ca->data()), static_cast<unsigned *>(oa->data()),
-                        static_cast<unsigned *>(sa->data())};
-    const RadixPairs<unsigned, unsigned long long> p{
-        first, x, {static_cast<unsigned *>(ia->data()), first},
-        {static_cast<unsigned long long *>(va->data()), vb ? static_cast<unsigned long long *>(vb->data()) : nullptr}};
-    int at = 0;
-    if ((st = radix_pairs(ctx, p, b, shifts, passes, t, &at))) return done(st);
-    auto *span = static_cast<uint2 *>(sp->data());
-    rif_spans_kernel<<<stream_grid(ctx, b / 4, 256, 8, 1024), 256, 0, ctx->stream>>>(p.img[at], b, span);
-    if (b < RIF_SHORT_ROWS * 16 * nb) {
-        rif_short_kernel<<<static_cast<int>((16 * nb + 255) / 256), 256, 0, ctx->stream>>>(span, p.pay[at], nb, out);
-    } else {
-        // Every pair of buckets that fits a wave of resident blocks, then further ones by stride.
-        const int64_t pairs = (nb + 1) / 2;
-        const int grid = static_cast<int>(std::min<int64_t>(pairs, static_cast<int64_t>(ctx->sms) * 8));
-        rif_sum_kernel<<<grid, 64, 0, ctx->stream>>>(span, p.pay[at], nb, out);
-    }
-    return done(launched(ctx, "rif_sums"));
-}
-
-// ------------------------------------------------------------------ the other paths
-
-// The masked path: for each bucket, reduce_add_f64 of the rows with the others read as +0.0.
+// The masked path: for each of the buckets, reduce_add_f64 of the rows with the others read as +0.0.
 static vkc_status rif_masked(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t n,
-                             int64_t nb, unsigned long long *out) {
+                             const std::vector<unsigned> &buckets, unsigned long long *out) {
     vkc_array *v;
     vkc_status st = new_array(ctx, VKC_F64, n, false, &v);
     if (st) return st;
     const KernelDef *sum = kernel_def("reduce_add_f64");
-    for (int64_t k = 0; k < nb && !st; ++k) {
+    for (const unsigned k : buckets) {
         rif_mask_kernel<<<stream_grid(ctx, n, 256, 8, 4096), 256, 0, ctx->stream>>>(
             keys, x, n, k, static_cast<unsigned long long *>(v->data()));
         if ((st = launched(ctx, "rif_mask"))) break;
@@ -372,11 +372,83 @@ static vkc_status rif_masked(vkc_ctx *ctx, const long long *keys, const unsigned
         delete r;
         if (st) break;
         rif_store_kernel<<<1, 1, 0, ctx->stream>>>(out, k, s.bits);
-        st = launched(ctx, "rif_store");
+        if ((st = launched(ctx, "rif_store"))) break;
     }
     vkc_array_release(v);
     return st;
 }
+
+// The sorted path and the rows from b on, waited for; *bad: some key is out of range (and no sum holds).
+static vkc_status rif_sorted(vkc_ctx *ctx, const long long *keys, const unsigned long long *x, int64_t n, int64_t b,
+                             int64_t nb, unsigned long long *out, bool *bad) {
+    int passes = 1;  // of the image's bits: the largest is 16 nb - 1
+    while (passes < 4 && ((16 * static_cast<uint64_t>(nb) - 1) >> (8 * passes))) ++passes;
+    static const int shifts[4] = {0, 8, 16, 24};
+    vkc_array *ia = nullptr, *ib = nullptr, *va = nullptr, *vb = nullptr, *ca = nullptr, *oa = nullptr, *sa = nullptr,
+              *sp = nullptr;
+    auto done = [&](vkc_status st) {
+        for (vkc_array *a : {ia, ib, va, vb, ca, oa, sa, sp})
+            if (a) vkc_array_release(a);
+        return st;
+    };
+    int64_t cw, sw;
+    radix_table_words(b, &cw, &sw);
+    vkc_status st;
+    void *h;
+    if ((st = new_array(ctx, VKC_I32, b, false, &ia)) || (st = new_array(ctx, VKC_I32, b, false, &ib)) ||
+        (st = new_array(ctx, VKC_F64, b, false, &va)) || (passes > 1 && (st = new_array(ctx, VKC_F64, b, false, &vb))) ||
+        (st = new_array(ctx, VKC_I32, cw, false, &ca)) || (st = new_array(ctx, VKC_I32, cw, false, &oa)) ||
+        (st = new_array(ctx, VKC_I32, sw, false, &sa)) ||
+        (st = new_array(ctx, VKC_U64, 16 * nb + static_cast<int64_t>(sizeof(RifHeavy) / 8), true, &sp)) ||
+        (st = pinned(ctx, sizeof(RifHeavy), &h)))
+        return done(st);
+    auto *first = static_cast<unsigned *>(ib->data());
+    rif_images_kernel<<<stream_grid(ctx, n, 256, 8, 4096), 256, 0, ctx->stream>>>(keys, n, b, static_cast<uint64_t>(nb), first,
+                                                                                  ctx->status);
+    if ((st = launched(ctx, "rif_images"))) return done(st);
+    const RadixTables t{static_cast<unsigned *>(ca->data()), static_cast<unsigned *>(oa->data()),
+                        static_cast<unsigned *>(sa->data())};
+    const RadixPairs<unsigned, unsigned long long> p{
+        first, x, {static_cast<unsigned *>(ia->data()), first},
+        {static_cast<unsigned long long *>(va->data()), vb ? static_cast<unsigned long long *>(vb->data()) : nullptr}};
+    int at = 0;
+    if ((st = radix_pairs(ctx, p, b, shifts, passes, t, &at))) return done(st);
+    auto *span = static_cast<uint2 *>(sp->data());
+    auto *heavy = reinterpret_cast<RifHeavy *>(span + 16 * nb);
+    auto *flag = static_cast<unsigned *>(h);
+    *flag = 0;
+    const unsigned limit = rif_limit(n, nb);
+    rif_spans_kernel<<<stream_grid(ctx, b / 4, 256, 8, 1024), 256, 0, ctx->stream>>>(p.img[at], b, span);
+    // Every pair of buckets that fits a wave of resident blocks, then further ones by stride.
+    const int pairs = static_cast<int>(std::min<int64_t>((nb + 1) / 2, static_cast<int64_t>(ctx->sms) * 8));
+    if (b < RIF_SHORT_ROWS * 16 * nb)
+        rif_short_kernel<<<static_cast<int>((16 * nb + 255) / 256), 256, 0, ctx->stream>>>(span, p.pay[at], nb, out, limit, heavy, flag);
+    else
+        rif_sum_kernel<<<pairs, 64, 0, ctx->stream>>>(span, p.pay[at], nb, out, limit, heavy, flag);
+    if ((st = launched(ctx, "rif_sums"))) return done(st);
+    if ((st = rif_tail(ctx, keys, x, b, n, nb, out))) return done(st);
+    DevStatus ds;
+    if ((st = read_status(ctx, &ds))) return done(st);
+    *bad = ds.first_bad != ~0ull;
+    if (*bad || !*flag) return done(VKC_OK);
+    // Buckets with long chains: masked, the rows from b on among them, or their chains and then those rows.
+    RifHeavy hv;
+    VKC_CUDA(ctx, cudaMemcpyAsync(h, heavy, sizeof hv, cudaMemcpyDeviceToHost, ctx->stream));
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    memcpy(&hv, h, sizeof hv);
+    if (hv.count <= RifHeavy::MOST && hv.count * rif_mask_us(n) < RIF_CHAIN_US * hv.longest) {
+        st = rif_masked(ctx, keys, x, n, std::vector<unsigned>(hv.bucket, hv.bucket + hv.count), out);
+        if (st != VKC_ALLOC) return done(st);
+    }
+    // (Every sum again: the others have their tail rows already.)
+    rif_sum_kernel<<<pairs, 64, 0, ctx->stream>>>(span, p.pay[at], nb, out, 0u, nullptr, nullptr);
+    if ((st = launched(ctx, "rif_sums"))) return done(st);
+    if ((st = rif_tail(ctx, keys, x, b, n, nb, out))) return done(st);
+    VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return done(VKC_OK);
+}
+
+// ------------------------------------------------------------------ the other paths
 
 // Without a table of the chains, over the rows below b (b > 0).
 static vkc_status rif_scanned(vkc_ctx *ctx, const vkc_array *keys, const vkc_array *vals, int64_t b,
@@ -446,23 +518,17 @@ static vkc_status reduce_into_add_f64(vkc_ctx *ctx, const vkc_value *args, int n
     const int64_t b = n - n % 16;
     if (b > 0 && nb > 0 && !rif_masks(n, nb) && rif_tables(n, nb)) {
         // The keys are checked with their images; an error is found once the sums are done.
-        st = rif_sorted(ctx, k, x, n, b, nb, ov);
-        if (!st && b < n) {
-            rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(k, x, b, n, static_cast<uint64_t>(nb), ov);
-            st = launched(ctx, "rif_tail");
-        }
-        DevStatus ds;
-        if (!st) st = read_status(ctx, &ds);
-        if (!st && ds.first_bad != ~0ull) st = bucket_key_error(ctx, k, n, nb, &found);
+        bool bad = false;
+        st = rif_sorted(ctx, k, x, n, b, nb, ov, &bad);
+        if (!st && bad) st = bucket_key_error(ctx, k, n, nb, &found);
     } else if (!(st = bucket_key_error(ctx, k, n, nb, &found)) && n > 0) {
         if (rif_masks(n, nb)) {
-            st = rif_masked(ctx, k, x, n, nb, ov);
+            std::vector<unsigned> all(static_cast<size_t>(nb));
+            for (int64_t i = 0; i < nb; ++i) all[static_cast<size_t>(i)] = static_cast<unsigned>(i);
+            st = rif_masked(ctx, k, x, n, all, ov);
         } else {
             if (b > 0) st = rif_scanned(ctx, keys, vals, b, ov);
-            if (!st && b < n) {
-                rif_tail_kernel<<<1, 1, 0, ctx->stream>>>(k, x, b, n, static_cast<uint64_t>(nb), ov);
-                st = launched(ctx, "rif_tail");
-            }
+            if (!st) st = rif_tail(ctx, k, x, b, n, nb, ov);
         }
     }
     if (st) {
