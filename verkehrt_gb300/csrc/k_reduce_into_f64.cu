@@ -516,12 +516,17 @@ static vkc_status reduce_into_add_f64(vkc_ctx *ctx, const vkc_value *args, int n
     auto *ov = static_cast<unsigned long long *>(o->data());
     const auto *x = static_cast<const unsigned long long *>(vals->data());
     const int64_t b = n - n % 16;
-    if (b > 0 && nb > 0 && !rif_masks(n, nb) && rif_tables(n, nb)) {
+    bool sorted = b > 0 && nb > 0 && !rif_masks(n, nb) && rif_tables(n, nb);
+    if (sorted) {
         // The keys are checked with their images; an error is found once the sums are done.
         bool bad = false;
         st = rif_sorted(ctx, k, x, n, b, nb, ov, &bad);
         if (!st && bad) st = bucket_key_error(ctx, k, n, nb, &found);
-    } else if (!(st = bucket_key_error(ctx, k, n, nb, &found)) && n > 0) {
+        // Its table takes 128 bytes a bucket: without room for it, the chains by a scan.
+        sorted = st != VKC_ALLOC;
+        if (!sorted) VKC_CUDA(ctx, cudaMemsetAsync(ov, 0, static_cast<size_t>(nb) * 8, ctx->stream));
+    }
+    if (!sorted && !(st = bucket_key_error(ctx, k, n, nb, &found)) && n > 0) {
         if (rif_masks(n, nb)) {
             std::vector<unsigned> all(static_cast<size_t>(nb));
             for (int64_t i = 0; i < nb; ++i) all[static_cast<size_t>(i)] = static_cast<unsigned>(i);
