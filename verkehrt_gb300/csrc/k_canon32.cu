@@ -370,6 +370,7 @@ struct Walk32 {
     int chunk_of[W32_MIXED];
     int tile_of[W32_TILES];
     short rows_of[W32_MIXED][C32_CHUNK];
+    alignas(16) float chain[C32_BLOCKS];
     int nmixed, ntiles;
 };
 
@@ -379,6 +380,31 @@ template <int OP> __device__ __forceinline__ float row_of(const Args32 &a, int64
     if (b >= nb) return 0.f;
     return value32<OP>(a, __ldg(a.x + b * 16 + L), OP == R32_DOT ? __ldg(a.y + b * 16 + L) : 0.f);
 }
+
+// The rows of threads `first` on (sixteen each, of the whole warp in v) added one after another.
+__device__ __forceinline__ float chain_rows(float (&buf)[C32_BLOCKS], const float (&v)[R32_ROWS], int first, float s) {
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < R32_ROWS; i += 4)
+        *reinterpret_cast<float4 *>(&buf[(threadIdx.x & 31) * R32_ROWS + i]) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    __syncwarp();
+    for (int r = first * R32_ROWS; r < C32_BLOCKS; r += R32_ROWS) {
+        float4 x[R32_ROWS / 4];
+#pragma unroll
+        for (int i = 0; i < R32_ROWS / 4; ++i) x[i] = *reinterpret_cast<const float4 *>(&buf[r + 4 * i]);
+#pragma unroll
+        for (int i = 0; i < R32_ROWS / 4; ++i)
+            s = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(s, x[i].x), x[i].y), x[i].z), x[i].w);
+    }
+    return s;
+}
+
+// A thread whose rows no run carries costs a failed run, a composition and its sixteen adds, some 800
+// cycles, where a chain adds the sixteen rows in 70. So after this many of them the rest of the tile is a
+// chain, and sooner in the tiles after one that was. (Lanes whose rows leave their binade all the time took
+// 26,000 cycles a tile: reduce_add_f32 of 2^20 rows that alternate between about -1e6 and 1e6 1690 us a call, now
+// 377, one block of sixteen chains 920; of 2^17 such rows 290 / 86 / 149.)
+constexpr int W32_FAILS = 2;
 
 template <int OP>
 __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int C, Work32 wk, State32 *state) {
@@ -437,7 +463,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
     float s = state->lanes[L];
     int ahead = -1;  // the tile whose rows `next` holds
     float next[R32_ROWS];
-    int tile = 0;
+    int tile = 0, chained = 0;  // chained: resolved tiles in a row that ended as chains
     while (tile < T && s == s) {  // a NaN stays one
         const unsigned code = code32(s);
         int c = tile / C32_CHUNK;
@@ -451,6 +477,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
             }
             const int m = __shfl_sync(FULL, kc == code, 0) ? advance32(f, kc == code, &s) : 0;
             if (m > 0) {
+                chained = 0;
                 c += m;
                 tile = c * C32_CHUNK;
                 if (m == 32 || tile >= T) continue;  // else the chunk that ended the run, tile by tile
@@ -468,6 +495,7 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
             }
             const int m = __shfl_sync(FULL, kc == code, 0) ? advance32(f, kc == code, &s) : 0;
             if (m > 0) {
+                chained = 0;
                 tile += m;
                 j0 += m;
                 if (j0 >= C32_CHUNK || tile >= T) continue;  // else the tile that ended the run
@@ -504,10 +532,15 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
             for (int i = 0; i < R32_ROWS; ++i) any |= __float_as_uint(v[i]) << 1;
             live = __ballot_sync(FULL, any != 0);
         }
+        int fails = W32_FAILS - chained;
         for (int done = 0; done < 32;) {
             const unsigned now = code32(s), rest = live & (FULL << done);
             if (rest == 0) break;
             done = __ffs(rest) - 1;
+            if (fails <= 0) {
+                s = chain_rows(sm.chain, v, done, s);
+                break;
+            }
             if (now != C32_NONE) {
                 Run32 f = STILL32;
                 const bool ok = lane < done || run32<R32_ROWS>(v, now, &f);
@@ -524,7 +557,9 @@ __global__ void __launch_bounds__(256) c32_walk(Args32 a, int64_t nb, int T, int
             }
             s = __shfl_sync(FULL, r, done);
             ++done;
+            --fails;
         }
+        chained = fails <= 0 ? min(chained + 1, W32_FAILS) : 0;
         ++tile;
     }
     if (lane == 0) state->lanes[L] = s;
