@@ -541,8 +541,12 @@ __device__ __forceinline__ RgFold rg_fold_block(int kind, RgFold v) {
     return v;
 }
 
+__device__ __forceinline__ RgResult rg_result(const RgFold &v, const DevStatus *status) {
+    return RgResult{v, *reinterpret_cast<const volatile unsigned *>(&status->timeout)};
+}
+
 __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionProg P, int64_t n, int kind, bool f64,
-                                                                 RgFold *partials, unsigned *done, RgFold *result) {
+                                                                 RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     extern __shared__ unsigned long long s_w[];
     const int t = threadIdx.x;
     RgFold me{0, ~0ull, ~0ull, 0};
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionPro
         RgFold v{0, ~0ull, ~0ull, 0};
         for (unsigned q = t; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
         v = rg_fold_block(kind, v);
-        if (t == 0) *result = v;
+        if (t == 0) *result = rg_result(v, status);
     }
 }
 
@@ -713,7 +717,7 @@ __device__ __forceinline__ void rf_values(const RegionProg &P, int64_t b0, int64
 // by their order keys, as region_fold_kernel's (kind RF_MIN .. RF_ARGMAX).
 template <int NARR, int MODE>
 __global__ void __launch_bounds__(RG_THREADS, 4) region_f64_kernel(const RegionProg P, int64_t n, bool aligned, void *__restrict__ out,
-                                                                   int kind, RgFold *partials, unsigned *done, RgFold *result) {
+                                                                   int kind, RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     constexpr int RF_ROWS = rf_rows<NARR>(), RF_BLOCK_ROWS = RG_THREADS * RF_ROWS;
     extern __shared__ double s_d[];
     unsigned long long count = 0;
@@ -787,14 +791,14 @@ __global__ void __launch_bounds__(RG_THREADS, 4) region_f64_kernel(const RegionP
             RgFold v{0, ~0ull, ~0ull, 0};
             for (unsigned q = threadIdx.x; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
             v = rg_fold_block(kind, v);
-            if (threadIdx.x == 0) *result = v;
+            if (threadIdx.x == 0) *result = rg_result(v, status);
         }
     }
 }
 
 template <int NARR, int MODE>
 static vkc_status launch_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *partials, unsigned *done,
-                             RgFold *result) {
+                             RgResult *result) {
     constexpr int RF_BLOCK_ROWS = RG_THREADS * rf_rows<NARR>();
     const size_t smem = static_cast<size_t>(p.nslots) * RF_BLOCK_ROWS * sizeof(double);
     static std::atomic<unsigned long long> configured{0};
@@ -809,13 +813,13 @@ static vkc_status launch_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void 
     const int64_t blocks = (n + RF_BLOCK_ROWS - 1) / RF_BLOCK_ROWS;
     const int64_t most = std::min<int64_t>(static_cast<int64_t>(ctx->sms) * std::max(1, per_sm), RG_FOLD_MAX_GRID);
     const int grid = static_cast<int>(std::min<int64_t>(blocks, most));
-    region_f64_kernel<NARR, MODE><<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, aligned, out, kind, partials, done, result);
+    region_f64_kernel<NARR, MODE><<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, aligned, out, kind, partials, done, ctx->status, result);
     return launched(ctx, "region_f64");
 }
 
 template <int MODE>
 static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *out, int kind, RgFold *partials, unsigned *done,
-                          RgFold *result) {
+                          RgResult *result) {
     switch (p.narr) {
     case 1: return launch_f64<1, MODE>(ctx, p, n, out, kind, partials, done, result);
     case 2: return launch_f64<2, MODE>(ctx, p, n, out, kind, partials, done, result);
@@ -825,7 +829,7 @@ static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *ou
 }
 
 vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *partials,
-                              unsigned *done, RgFold *result) {
+                              unsigned *done, RgResult *result) {
     if (n <= 0) return VKC_OK;
     if (p.f64only && f64) return run_f64<RF_FOLD>(ctx, p, n, nullptr, kind, partials, done, result);
     const size_t smem = static_cast<size_t>(p.nslots) * RG_BLOCK_ROWS * sizeof(unsigned long long);
@@ -839,7 +843,7 @@ vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int 
     const int64_t blocks = (n + RG_BLOCK_ROWS - 1) / RG_BLOCK_ROWS;
     int64_t g = std::min<int64_t>(blocks, static_cast<int64_t>(ctx->sms) * std::max(1, per_sm));
     const int grid = static_cast<int>(std::min<int64_t>(g, RG_FOLD_MAX_GRID));
-    region_fold_kernel<<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, kind, f64, partials, done, result);
+    region_fold_kernel<<<grid, RG_THREADS, smem, ctx->stream>>>(p, n, kind, f64, partials, done, ctx->status, result);
     return launched(ctx, "region_fold");
 }
 

@@ -360,12 +360,17 @@ vkc_status vkc_region_reduce(vkc_ctx *ctx, int root, const int32_t *root_args, i
         // The last block writes the fold into pinned memory, so the call is one launch and one wait.
         void *partials, *host;
         if ((st = scratch(ctx, sizeof(RgFold) * RG_FOLD_MAX_GRID, &partials))) return st;
-        if ((st = pinned(ctx, sizeof(RgFold), &host))) return st;
+        if ((st = pinned(ctx, sizeof(RgResult), &host))) return st;
         st = launch_region_fold(ctx, p, n, f.kind, f.f64, static_cast<RgFold *>(partials), ctx->counters + 1,
-                                static_cast<RgFold *>(host));
+                                static_cast<RgResult *>(host));
         if (st) return st;
         VKC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        const RgFold r = *static_cast<const RgFold *>(host);
+        const RgResult res = *static_cast<const RgResult *>(host);
+        if (res.timeout) {  // a wait of earlier enqueued work ran out: clear the status word
+            DevStatus ds;
+            if ((st = read_status(ctx, &ds))) return st;
+        }
+        const RgFold &r = res.fold;
         out->kind = VKC_VALUE_SCALAR;
         const bool arg = f.kind == RF_ARGMIN || f.kind == RF_ARGMAX;
         if (f.kind == RF_SUM) {

@@ -66,11 +66,16 @@ struct RgFold {
     unsigned long long nan_idx;   // the first NaN row (~0: none)
     unsigned long long sum;       // RF_SUM: the wrapping sum
 };
+// What the host reads of a fold: the status word's timeout too, of work enqueued before it.
+struct RgResult {
+    RgFold fold;
+    unsigned timeout;
+};
 constexpr int RG_FOLD_MAX_GRID = 4096;
 // Folds `p`'s value over n > 0 rows into the pinned `result`, through one partial per block
 // (RG_FOLD_MAX_GRID at most); *done is a counter that is zero between launches.
 vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *partials,
-                              unsigned *done, RgFold *result);
+                              unsigned *done, RgResult *result);
 
 // Runs `p` over n rows into `out` (the last kernel's rows) on the context's stream; with
 // `count`, adds the number of nonzero result rows to the u64 at `out` instead.
