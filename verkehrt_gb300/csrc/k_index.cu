@@ -312,13 +312,15 @@ __global__ void __launch_bounds__(GP_THREADS, 6) gp_restore_kernel(const unsigne
 
 // The partitioned path pays when the source is beyond L2 (7 * 2^22 rows, 224 MiB; smaller ones hit
 // L2 often enough) and the index rows are at least half the source rows, so that each region line
-// fetched into L2 is read about twice (with fewer, the one-pass gather moves fewer DRAM bytes).
-// Measured on GB300 with as many index rows as source rows, one pass against four: 20 M rows 260
-// against 312 us, 28 M 421 / 410, 40 M 667 / 545, 2^28 45 against 68 G rows/s. Positions are u32:
-// fewer than 2^32 index rows.
+// fetched into L2 is read about twice (with fewer, the one-pass gather moves fewer DRAM bytes); three
+// quarters for the smallest sources, of which L2 holds more. Measured on GB300, one pass against four, with
+// as many index rows as source rows: 20 M rows 260 against 312 us, 29.4 M 444 / 412, 40 M 667 / 545, 2^28
+// 45 against 68 G rows/s; with half as many: 29.4 M 236 / 252, 34 M 283 / 283, 40 M 346 / 321, 50 M 449 /
+// 380; 29.4 M source rows with 5/8 of them 288 / 291, with 3/4 345 / 335. Positions are u32: fewer than 2^32
+// index rows.
 static bool gather_partitions(uint64_t nsrc, int64_t n) {
     return nsrc >= (uint64_t(7) << 22) && nsrc <= (uint64_t(1) << 38) && n >= (int64_t(1) << 22) &&
-           2 * static_cast<uint64_t>(n) >= nsrc && n < (int64_t(1) << 32);
+           4 * static_cast<uint64_t>(n) >= (nsrc < (uint64_t(1) << 25) ? 3 : 2) * nsrc && n < (int64_t(1) << 32);
 }
 
 static vkc_status gather_partitioned(vkc_ctx *ctx, const unsigned long long *src, uint64_t nsrc, const long long *idx,
