@@ -105,17 +105,15 @@ constexpr unsigned GI_AHEAD = 4, GI_STAGGER_NS = 4000;
 // one lookback kernel and the regions 256 launches; now 445 / 385 / 485 us / 1.79 / 2.06 ms.
 
 template <bool PAIR, bool SMALL>
-__global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *__restrict__ a,
-                                                               const long long *__restrict__ b, int64_t n,
-                                                               bool gives_up, GroupTable t, unsigned *__restrict__ slot_of,
-                                                               unsigned *flags, DevStatus *st) {
+__device__ __forceinline__ void gi_insert_rows(const long long *__restrict__ a, const long long *__restrict__ b, int64_t n,
+                                               bool gives_up, const GroupTable &t, unsigned *__restrict__ slot_of,
+                                               unsigned *flags, DevStatus *st) {
     constexpr bool CAS_FIRST = !SMALL && !PAIR;
     const int lane = threadIdx.x & 31;
     const int64_t step = static_cast<int64_t>(gridDim.x) * GI_THREADS * GI_ROWS;
     // The full table always has a free slot, so a probe ends within `mask` steps.
     const unsigned long long limit = SMALL && gives_up ? GI_SMALL_PROBES : t.mask;
     const unsigned max_keys = static_cast<unsigned>((t.mask + 1) / 2);
-    if (SMALL && blockIdx.x >= GI_AHEAD && gridDim.x >= 8 * GI_AHEAD) __nanosleep(GI_STAGGER_NS);
     for (int64_t base = static_cast<int64_t>(blockIdx.x) * GI_THREADS * GI_ROWS; base < n; base += step) {
         if (SMALL && gives_up) {
             const unsigned ov = lane == 0 ? ld_relaxed32(flags + 1) : 0u;
@@ -221,6 +219,40 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
             slot_of[row] = static_cast<unsigned>(s[j]);
         }
     }
+}
+
+template <bool PAIR, bool SMALL>
+__global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *__restrict__ a,
+                                                               const long long *__restrict__ b, int64_t n,
+                                                               bool gives_up, GroupTable t, unsigned *__restrict__ slot_of,
+                                                               unsigned *flags, DevStatus *st) {
+    if (SMALL && blockIdx.x >= GI_AHEAD && gridDim.x >= 8 * GI_AHEAD) __nanosleep(GI_STAGGER_NS);
+    gi_insert_rows<PAIR, SMALL>(a, b, n, gives_up, t, slot_of, flags, st);
+}
+
+// Short inputs, whose first table is the full one: nobody knows whether their keys are few, and the way of
+// few keys costs many distinct ones a read and the late start. So each block decides by its first rows:
+// where a warp's 32 share a key it takes the way of few keys, else of many. A call on 10^6 rows of 10 / 1000 /
+// 2^16 / all distinct keys with every block the way of few keys 79 / 69 / 89 / 112 us, of many 265 / 80 / 91 /
+// 102, so 80 / 68 / 88 / 101.
+constexpr unsigned GI_SHORT_STAGGER_NS = 2500;  // the first rows' read comes before it
+template <bool PAIR>
+__global__ void __launch_bounds__(GI_THREADS) gi_insert_short_kernel(const long long *__restrict__ a,
+                                                                     const long long *__restrict__ b, int64_t n, bool,
+                                                                     GroupTable t, unsigned *__restrict__ slot_of,
+                                                                     unsigned *flags, DevStatus *st) {
+    const int64_t r = static_cast<int64_t>(blockIdx.x) * GI_THREADS * GI_ROWS + threadIdx.x;
+    unsigned h = threadIdx.x;
+    if (r < n) {
+        const unsigned long long k = gmix(static_cast<unsigned long long>(a[r]));
+        h = static_cast<unsigned>((PAIR ? gmix(k ^ static_cast<unsigned long long>(b[r])) : k) >> 32);
+    }
+    if (!__syncthreads_or(__popc(__match_any_sync(FULL, h)) > 1)) {
+        gi_insert_rows<PAIR, false>(a, b, n, false, t, slot_of, flags, st);
+        return;
+    }
+    if (blockIdx.x >= GI_AHEAD && gridDim.x >= 8 * GI_AHEAD) __nanosleep(GI_SHORT_STAGGER_NS);
+    gi_insert_rows<PAIR, true>(a, b, n, false, t, slot_of, flags, st);
 }
 
 // Numbers the first occurrences in row order (a compaction of the rows whose slot's smallest
@@ -614,16 +646,18 @@ static vkc_status new_table(vkc_ctx *ctx, uint64_t slots, bool pair, GroupScratc
 
 // One wave of resident blocks (the grid-stride loop gives every block the same share, so a
 // second, partial wave would run at a fraction of the occupancy).
-template <bool PAIR, bool SMALL>
-static void launch_insert(vkc_ctx *ctx, bool gives_up, const long long *a, const long long *b, int64_t n, const GroupTable &t,
-                          unsigned *slot_of, unsigned *flags) {
+enum GiWay { GI_FIRST, GI_MANY, GI_SHORT };  // the first table, the full one after it, the full one at once
+template <bool PAIR, GiWay WAY>
+static void launch_insert(vkc_ctx *ctx, const long long *a, const long long *b, int64_t n, const GroupTable &t, unsigned *slot_of,
+                          unsigned *flags) {
     static int per_sm = 0;
-    auto kern = gi_insert_kernel<PAIR, SMALL>;
+    auto kern = gi_insert_kernel<PAIR, WAY == GI_FIRST>;
+    if (WAY == GI_SHORT) kern = gi_insert_short_kernel<PAIR>;
     if (per_sm == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GI_THREADS, 0) != cudaSuccess ||
                         per_sm < 1))
         per_sm = 1;
     const int grid = stream_grid(ctx, n, GI_THREADS, per_sm, GI_THREADS * GI_ROWS);
-    kern<<<grid, GI_THREADS, 0, ctx->stream>>>(a, b, n, gives_up, t, slot_of, flags, ctx->status);
+    kern<<<grid, GI_THREADS, 0, ctx->stream>>>(a, b, n, WAY == GI_FIRST, t, slot_of, flags, ctx->status);
 }
 
 // Single keys, many distinct, at least GR_MIN_ROWS rows: the region-partitioned path above. A step
@@ -790,8 +824,8 @@ static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *
             vkc_array_release(o);
             return st;
         }
-        if (xb) launch_insert<true, true>(ctx, true, a, b, n, t, slot_of, flags);
-        else launch_insert<false, true>(ctx, true, a, b, n, t, slot_of, flags);
+        if (xb) launch_insert<true, GI_FIRST>(ctx, a, b, n, t, slot_of, flags);
+        else launch_insert<false, GI_FIRST>(ctx, a, b, n, t, slot_of, flags);
         if ((st = launched(ctx, "gi_insert"))) {
             cleanup();
             vkc_array_release(o);
@@ -833,10 +867,10 @@ static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *
         }
         // Many distinct keys are only known of inputs whose first table gave up.
         const bool many = slots > first_slots;
-        if (xb && many) launch_insert<true, false>(ctx, false, a, b, n, t, slot_of, flags);
-        else if (xb) launch_insert<true, true>(ctx, false, a, b, n, t, slot_of, flags);
-        else if (many) launch_insert<false, false>(ctx, false, a, b, n, t, slot_of, flags);
-        else launch_insert<false, true>(ctx, false, a, b, n, t, slot_of, flags);
+        if (xb && many) launch_insert<true, GI_MANY>(ctx, a, b, n, t, slot_of, flags);
+        else if (xb) launch_insert<true, GI_SHORT>(ctx, a, b, n, t, slot_of, flags);
+        else if (many) launch_insert<false, GI_MANY>(ctx, a, b, n, t, slot_of, flags);
+        else launch_insert<false, GI_SHORT>(ctx, a, b, n, t, slot_of, flags);
         if ((st = launched(ctx, "gi_insert"))) {
             cleanup();
             vkc_array_release(o);
