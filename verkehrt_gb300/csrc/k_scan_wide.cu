@@ -6,7 +6,7 @@ namespace vkc {
 
 template <vkc_type T> static FoldScanMake int_scan(int fold, bool by) {
     switch (fold) {
-    case F_ADD: return scan_of<VKC_U64, F_ADD>(by);
+    case F_ADD: return scan_of<T, F_ADD>(by);
     case F_MUL: return scan_of<T, F_MUL>(by);
     case F_MIN: return scan_of<T, F_MIN>(by);
     case F_MAX: return scan_of<T, F_MAX>(by);
