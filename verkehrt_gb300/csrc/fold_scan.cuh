@@ -18,7 +18,10 @@
 namespace vkc {
 
 constexpr int SC_THREADS = 512;  // compute threads (+ 2 warps)
-constexpr int SC_WINDOW = 4;
+// The lookback's step: 32 tiles, one a lane. Wider ones find the prefix in one step too, but their polls,
+// four records a lane, slow the copies they wait for: calls on 2^27 / 2^28 i64 rows plain with 4 records a
+// lane 404 / 814 us, with 2 374 / 732, with 1 360 / 700; with segments 399 / 773, 395 / 753, 392 / 753.
+constexpr int SC_WINDOW = 1;
 constexpr int SC_SMEM = 224 * 1024;  // of the slots and the output rows
 
 // The carried state of a scanner: the last output (as a word of the fold) and, of prev, whether any
@@ -130,8 +133,8 @@ template <class Op> struct SegRec {
 // reach are the slice's rows before its first start. (Counted first, then scanned in
 // place with the starts beside the values and stored from there, the slot was read three times and written
 // once, and the segmented scan was bound by its instructions: calls on 2^27 i64 rows took 403 us plain
-// and 584 with segments, the other types' reduce, scan and apply kernels 1.1 to 2.6 ms. Now 400 to 420,
-// 402, i32 sums 385, f64 extremes 421 plain and 570 with segments, f32 202, u8 165; 2.15 GB take 317 us at
+// and 584 with segments, the other types' reduce, scan and apply kernels 1.1 to 2.6 ms. Now 360,
+// 392, i32 sums 347, f64 extremes 410 plain and 543 with segments, f32 199, u8 158; 2.15 GB take 317 us at
 // the copy's rate. Evict-first hints on the loads and stores change nothing.)
 //
 // Segments need no flags beside the values in the warp's scan: with the lanes that hold a start as a
