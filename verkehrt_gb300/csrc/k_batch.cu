@@ -22,6 +22,7 @@
 //    own argsort. (Key digits and number beyond 64 bits: the order by the keys first, then by the
 //    arrays' numbers, found again from the positions.)
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <memory>
 #include <numeric>
@@ -41,9 +42,10 @@ struct BSeg {
     int64_t index;  // position of the array in the caller's list
 };
 
-// A batched argsort's outputs: their rows' addresses, and the tables on the device that hold them.
+// A batched argsort's outputs: the number of their batch, and the tables on the device that hold their rows'
+// addresses.
 struct BatchOuts {
-    std::vector<void *> rows;
+    uint64_t serial = 0;
     DeviceMem outs;         // output pointers [n], index order
     DeviceMem segs;         // SortSeg[n] and each tile's array, when arrays are sorted for themselves
     bool captured = false;  // a graph holds the tables: kept until the batch is freed
@@ -53,6 +55,7 @@ struct BatchOuts {
 
 struct vkc_batch {
     vkc_ctx *ctx = nullptr;
+    uint64_t serial = 0;  // no other batch's, also after this one is freed
     vkc_type type = VKC_F64;
     std::vector<vkc_array *> arrays;  // retained, caller's order
     std::vector<vkc::BSeg> host;      // largest first
@@ -359,8 +362,10 @@ extern "C" VKC_API vkc_status vkc_batch_new(vkc_ctx *ctx, int n, vkc_array *cons
     if (!ctx || !out || n < 0 || (n > 0 && !arrays)) return VKC_USAGE;
     *out = nullptr;
     if (capturing(ctx)) return fail(ctx, VKC_USAGE, "vkc_batch_new during a stream capture");
+    static std::atomic<uint64_t> serials{0};
     auto *b = new vkc_batch;
     b->ctx = ctx;
+    b->serial = ++serials;
     b->type = n > 0 ? arrays[0]->type : VKC_F64;
     std::vector<int64_t> base(static_cast<size_t>(n) + 1, 0);
     for (int i = 0; i < n; ++i) {
@@ -535,23 +540,23 @@ static vkc_status argsort_scratch(vkc_ctx *ctx, vkc_batch *keys) {
     return VKC_OK;
 }
 
-// The tables of these outputs, made on their first use. Outputs are told apart by their rows' addresses,
-// all that the tables hold of them: a batch's own address may be another one's after it is freed.
+// The tables of these outputs, made on their first use. Batches are told apart by their numbers (a batch's
+// address may be another one's after it is freed), and a batch's arrays are the same all its life.
 constexpr int BATCH_OUTS = 4;  // outputs whose tables are kept beside the captured ones
 static vkc_status argsort_outs(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *outs, bool cap, const BatchOuts **found) {
     const size_t n = keys->arrays.size();
     for (auto &o : keys->outs) {
-        bool same = true;
-        for (size_t i = 0; i < n && same; ++i) same = o->rows[i] == outs->arrays[i]->data();
-        if (!same) continue;
+        if (o->serial != outs->serial) continue;
         o->captured = o->captured || cap;
         *found = o.get();
         return VKC_OK;
     }
     if (cap) return fail(ctx, VKC_USAGE, "batch argsort: make its first call before capturing");
     auto o = std::make_unique<BatchOuts>();
-    for (const vkc_array *a : outs->arrays) o->rows.push_back(a->data());
-    vkc_status st = upload_table(ctx, o->outs, o->rows.data(), sizeof(void *) * n);
+    o->serial = outs->serial;
+    std::vector<void *> rows;
+    for (const vkc_array *a : outs->arrays) rows.push_back(a->data());
+    vkc_status st = upload_table(ctx, o->outs, rows.data(), sizeof(void *) * n);
     if (!st && keys->seg_tiles) {
         // The arrays in the concatenation's order, and each tile's array.
         std::vector<unsigned char> table(sizeof(SortSeg) * n + sizeof(int) * keys->seg_tiles);
@@ -560,7 +565,7 @@ static vkc_status argsort_outs(vkc_ctx *ctx, vkc_batch *keys, const vkc_batch *o
         int64_t base = 0, t = 0;
         for (size_t i = 0; i < n; ++i) {
             const vkc_array *a = keys->arrays[i];
-            segs[i] = SortSeg{static_cast<const unsigned long long *>(a->data()), static_cast<long long *>(o->rows[i]), base, a->len, t};
+            segs[i] = SortSeg{static_cast<const unsigned long long *>(a->data()), static_cast<long long *>(rows[i]), base, a->len, t};
             for (int64_t j = 0; j < a->len; j += keys->seg_tile) tile[t++] = static_cast<int>(i);
             base += a->len;
         }
