@@ -715,8 +715,10 @@ __device__ __forceinline__ void rf_values(const RegionProg &P, int64_t b0, int64
 
 // RF_STORE: the rows into out. RF_COUNT: the true rows added to the u64 at out. RF_FOLD: the extremes
 // by their order keys, as region_fold_kernel's (kind RF_MIN .. RF_ARGMAX).
+// (Five blocks an SM for folds of four arrays: (a*b + c) - d of 50 M rows 427 us, 451 with four blocks; no
+// other form gains from it.)
 template <int NARR, int MODE>
-__global__ void __launch_bounds__(RG_THREADS, 4) region_f64_kernel(const RegionProg P, int64_t n, bool aligned, void *__restrict__ out,
+__global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 : 4) region_f64_kernel(const RegionProg P, int64_t n, bool aligned, void *__restrict__ out,
                                                                    int kind, RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     constexpr int RF_ROWS = rf_rows<NARR>(), RF_BLOCK_ROWS = RG_THREADS * RF_ROWS;
     extern __shared__ double s_d[];
@@ -828,10 +830,28 @@ static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *ou
     }
 }
 
+// Folds of one array through two or more FP64 operations and nothing else run faster in the word evaluator
+// from a few million rows on: the FP64 unit bounds both, and its steps of four rows keep more of it busy.
+// max of x*c + d, times x, + d, of 50 / 268 M rows 469 us / 2.33 ms there, 542 / 2.74 in the f64 one; x*c + x
+// 309 / 338 us of 50 M rows, 64 / 65 of 5 M, 41 / 39 of one. (With one operation 247 / 230 us of 50 M, with
+// min and max 864 / 516, with a selection 308 / 187.)
+static bool folds_as_words(const RegionProg &p, int64_t n) {
+    if (p.narr != 1 || n < (int64_t(1) << 22)) return false;
+    int ops = 0;
+    for (int k = 0; k < p.nk; ++k) {
+        switch (p.op[k].fn) {
+        case EF_ADD: case EF_SUB: case EF_MUL: case EF_DIV: case EF_NEG: case EF_SQRT: ++ops; break;
+        case EF_ABS: break;
+        default: return false;
+        }
+    }
+    return ops >= 2;
+}
+
 vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *partials,
                               unsigned *done, RgResult *result) {
     if (n <= 0) return VKC_OK;
-    if (p.f64only && f64) return run_f64<RF_FOLD>(ctx, p, n, nullptr, kind, partials, done, result);
+    if (p.f64only && f64 && !folds_as_words(p, n)) return run_f64<RF_FOLD>(ctx, p, n, nullptr, kind, partials, done, result);
     const size_t smem = static_cast<size_t>(p.nslots) * RG_BLOCK_ROWS * sizeof(unsigned long long);
     static std::atomic<unsigned long long> configured{0};
     once_per_device(configured, ctx->device, [] {
