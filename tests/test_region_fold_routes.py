@@ -40,6 +40,34 @@ def test_one_array(ctx, n, special):
                 assert got[2] == ctx.call(root, want, raw=True)[2], (kernels, root)
 
 
+def test_two_and_three_arrays(ctx):
+    import verkehrt_gb300 as vk
+
+    k = vk.region_kernel
+    n = TURN + 77
+    columns = [ctx.upload(oracle.rand_f64(n, s) - 0.5) for s in range(3)]
+    for inputs in (columns[:2], columns):
+        last = len(inputs) - 1
+        for count in (2, 3, 5):
+            kernels = [("mul_f64", (0, 1)), ("sub_f64", (k(0), last)), ("mul_f64", (k(1), 0)), ("neg_f64", (k(2),)),
+                       ("add_f64", (k(3), last))][:count]
+            want = whole(ctx, kernels, inputs)
+            for root in ("reduce_max_f64", "argmin_f64"):
+                got = ctx.region_reduce(root, [k(count - 1)], kernels, inputs, raw=True)
+                assert got[2] == ctx.call(root, want, raw=True)[2], (count, root)
+
+
+def test_negation(ctx):
+    import verkehrt_gb300 as vk
+
+    k = vk.region_kernel
+    x = np.concatenate([oracle.rand_f64(5000, 1) - 0.5, [0.0, -0.0, np.inf, -np.inf, 5e-324, -5e-324]])
+    dx = ctx.upload(x)
+    got = ctx.region([("neg_f64", (0,)), ("neg_f64", (k(0),)), ("neg_f64", (k(1),))], [dx]).numpy()
+    assert np.array_equal(got.view(np.uint64), (-x).view(np.uint64))
+    assert ctx.region_reduce("count", [k(1)], [("neg_f64", (0,)), ("gt_f64", (k(0), 0))], [dx]) == int((-x > x).sum())
+
+
 def test_four_arrays(ctx):
     import verkehrt_gb300 as vk
 

@@ -595,6 +595,10 @@ __device__ __forceinline__ double rg_max(double x, double y) {
     if (f64_nan_v(x) || f64_nan_v(y)) return ew_max(x, y);
     return f64_key(__double_as_longlong(x)) >= f64_key(__double_as_longlong(y)) ? x : y;
 }
+// ew_neg as an integer operation on the high word (on the whole value it is compiled to an FP64 add).
+__device__ __forceinline__ double rg_neg(double v) {
+    return __hiloint2double(static_cast<int>(static_cast<unsigned>(__double2hiint(v)) ^ 0x80000000u), __double2loint(v));
+}
 __device__ __forceinline__ double rg_one(bool c) { return __longlong_as_double(c ? 0x3ff0000000000000ll : 0ll); }
 __device__ __forceinline__ bool rg_true(double v) { return __double_as_longlong(v) != 0; }
 
@@ -693,7 +697,7 @@ __device__ __forceinline__ void rf_values(const RegionProg &P, int64_t b0, int64
             case EF_DIV: RF_OP(ew_div(x, y[r]))
             case EF_MIN: RF_OP(rg_min(x, y[r]))
             case EF_MAX: RF_OP(rg_max(x, y[r]))
-            case EF_NEG: RF_OP(ew_neg(x))
+            case EF_NEG: RF_OP(rg_neg(x))
             case EF_ABS: RF_OP(ew_abs(x))
             case EF_SQRT: RF_OP(ew_sqrt(x))
             case EF_LT: RF_OP(rg_one(x < y[r]))
@@ -715,8 +719,8 @@ __device__ __forceinline__ void rf_values(const RegionProg &P, int64_t b0, int64
 
 // RF_STORE: the rows into out. RF_COUNT: the true rows added to the u64 at out. RF_FOLD: the extremes
 // by their order keys, as region_fold_kernel's (kind RF_MIN .. RF_ARGMAX).
-// (Five blocks an SM for folds of four arrays: (a*b + c) - d of 50 M rows 427 us, 451 with four blocks; no
-// other form gains from it.)
+// (Five blocks an SM for folds of four arrays: a selection between two of their sums, 50 M rows, 452 us a
+// call, 515 with four blocks; no other form gains from it.)
 template <int NARR, int MODE>
 __global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 : 4) region_f64_kernel(const RegionProg P, int64_t n, bool aligned, void *__restrict__ out,
                                                                    int kind, RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
@@ -830,22 +834,23 @@ static vkc_status run_f64(vkc_ctx *ctx, const RegionProg &p, int64_t n, void *ou
     }
 }
 
-// Folds of one array through two or more FP64 operations and nothing else run faster in the word evaluator
-// from a few million rows on: the FP64 unit bounds both, and its steps of four rows keep more of it busy.
-// max of x*c + d, times x, + d, of 50 / 268 M rows 469 us / 2.33 ms there, 542 / 2.74 in the f64 one; x*c + x
-// 309 / 338 us of 50 M rows, 64 / 65 of 5 M, 41 / 39 of one. (With one operation 247 / 230 us of 50 M, with
-// min and max 864 / 516, with a selection 308 / 187.)
+// Folds of several FP64 operations and nothing else run faster in the word evaluator from a few million rows
+// on: the FP64 unit bounds both, and its steps of four rows keep more of it busy. Measured, words against
+// the f64 evaluator: one array, x*c + x of 5 / 50 M rows 64 / 309 us against 65 / 338 (1 M 41 / 39; one
+// operation 247 / 230 of 50 M, with a min and a max 864 / 516, with a selection 308 / 187); two arrays, three
+// and five operations of 50 M rows 402 / 567 us against 420 / 613 (two 349 / 327); three arrays 411 / 574
+// against 432 / 626 (two 360 / 340); four arrays 421 / 582 against 427 / 614.
 static bool folds_as_words(const RegionProg &p, int64_t n) {
-    if (p.narr != 1 || n < (int64_t(1) << 22)) return false;
+    if (n < (int64_t(1) << 22)) return false;
     int ops = 0;
     for (int k = 0; k < p.nk; ++k) {
         switch (p.op[k].fn) {
-        case EF_ADD: case EF_SUB: case EF_MUL: case EF_DIV: case EF_NEG: case EF_SQRT: ++ops; break;
-        case EF_ABS: break;
+        case EF_ADD: case EF_SUB: case EF_MUL: case EF_DIV: case EF_SQRT: ++ops; break;
+        case EF_NEG: case EF_ABS: break;  // on the sign bit
         default: return false;
         }
     }
-    return ops >= 2;
+    return ops >= (p.narr == 1 ? 2 : 3);
 }
 
 vkc_status launch_region_fold(vkc_ctx *ctx, const RegionProg &p, int64_t n, int kind, bool f64, RgFold *partials,
