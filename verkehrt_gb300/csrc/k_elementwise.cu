@@ -541,14 +541,17 @@ __device__ __forceinline__ RgFold rg_fold_block(int kind, RgFold v) {
     return v;
 }
 
-__device__ __forceinline__ RgResult rg_result(const RgFold &v, const DevStatus *status) {
-    return RgResult{v, *reinterpret_cast<const volatile unsigned *>(&status->timeout)};
+// The host has cleared result->timeout; `timeout` was read as the kernel began, off the end's path.
+__device__ __forceinline__ void rg_write(RgResult *result, const RgFold &v, unsigned timeout) {
+    result->fold = v;
+    if (timeout) result->timeout = timeout;
 }
 
 __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionProg P, int64_t n, int kind, bool f64,
                                                                  RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     extern __shared__ unsigned long long s_w[];
     const int t = threadIdx.x;
+    const unsigned timeout = t == 0 ? *reinterpret_cast<const volatile unsigned *>(&status->timeout) : 0u;
     RgFold me{0, ~0ull, ~0ull, 0};
     for (int64_t b0 = static_cast<int64_t>(blockIdx.x) * RG_BLOCK_ROWS; b0 < n;
          b0 += static_cast<int64_t>(gridDim.x) * RG_BLOCK_ROWS) {
@@ -576,7 +579,7 @@ __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionPro
         RgFold v{0, ~0ull, ~0ull, 0};
         for (unsigned q = t; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
         v = rg_fold_block(kind, v);
-        if (t == 0) *result = rg_result(v, status);
+        if (t == 0) rg_write(result, v, timeout);
     }
 }
 
@@ -726,6 +729,8 @@ __global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 :
                                                                    int kind, RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     constexpr int RF_ROWS = rf_rows<NARR>(), RF_BLOCK_ROWS = RG_THREADS * RF_ROWS;
     extern __shared__ double s_d[];
+    const unsigned timeout =
+        MODE == RF_FOLD && threadIdx.x == 0 ? *reinterpret_cast<const volatile unsigned *>(&status->timeout) : 0u;
     unsigned long long count = 0;
     // Extremes: keys compared as if for a minimum (a maximum's are complemented).
     const bool arg = kind == RF_ARGMIN || kind == RF_ARGMAX;
@@ -797,7 +802,7 @@ __global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 :
             RgFold v{0, ~0ull, ~0ull, 0};
             for (unsigned q = threadIdx.x; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
             v = rg_fold_block(kind, v);
-            if (threadIdx.x == 0) *result = rg_result(v, status);
+            if (threadIdx.x == 0) rg_write(result, v, timeout);
         }
     }
 }

@@ -359,10 +359,7 @@ struct FamReducer : DevReducer {
     using Launch = void (*)(vkc_ctx *, const RowArgs &, int64_t, int, void *, u64, bool, u64 *, u64 *);
     Launch launch = nullptr;
 
-    vkc_status begin(vkc_ctx *ctx) override {
-        fresh = false;
-        return fill(ctx, 3, empty, ~0ull, 0);
-    }
+    vkc_status clear(vkc_ctx *ctx) override { return fill(ctx, 3, empty, ~0ull, 0); }
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != nargs_want) return fail(ctx, VKC_RUNTIME, arity_error(nargs_want, nargs));
@@ -507,7 +504,7 @@ template <vkc_type T> __global__ void fam_chain_finish(u64 *st, int tail_len, u6
 template <vkc_type T> struct ChainReducer : DevReducer {
     int tail_len = 0;
 
-    vkc_status begin(vkc_ctx *) override { return VKC_OK; }  // made with its state
+    vkc_status clear(vkc_ctx *) override { return VKC_OK; }  // made with its state
 
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;

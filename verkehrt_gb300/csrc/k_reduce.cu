@@ -359,10 +359,7 @@ struct ExtremeReducer : DevReducer {
     bool max, arg;
     vkc_type type;
     unsigned long long consumed = 0;
-    vkc_status begin(vkc_ctx *ctx) override {
-        fresh = false;
-        return fill(ctx, 4, 0, ~0ull, ~0ull, 0);  // ExtState{0, ~0, ~0, 0}
-    }
+    vkc_status clear(vkc_ctx *ctx) override { return fill(ctx, 4, 0, ~0ull, ~0ull, 0); }  // ExtState{0, ~0, ~0, 0}
     vkc_status update(vkc_ctx *ctx, const Arg *args, int nargs) override {
         vkc_status st;
         if (nargs != 1) return fail(ctx, VKC_RUNTIME, arity_error(1, nargs));

@@ -361,6 +361,7 @@ vkc_status vkc_region_reduce(vkc_ctx *ctx, int root, const int32_t *root_args, i
         void *partials, *host;
         if ((st = scratch(ctx, sizeof(RgFold) * RG_FOLD_MAX_GRID, &partials))) return st;
         if ((st = pinned(ctx, sizeof(RgResult), &host))) return st;
+        static_cast<RgResult *>(host)->timeout = 0;
         st = launch_region_fold(ctx, p, n, f.kind, f.f64, static_cast<RgFold *>(partials), ctx->counters + 1,
                                 static_cast<RgResult *>(host));
         if (st) return st;

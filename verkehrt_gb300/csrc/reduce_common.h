@@ -32,6 +32,7 @@ struct DevReducer : ReducerImpl {
     DeviceMem mem;  // gives `state` back on the context's stream, even after the context closed
     void *host = nullptr;  // the slot, from the first update that writes one
     bool copies = false;   // no update writes the slot from here on
+    bool captured = false, lasts = false;  // made in a capture; used by later calls too (begin)
     bool fresh = true;
     cudaStream_t used = nullptr;  // the stream of the updates since the last result was read
     // The slot of a reducer dropped without finish may still be written: by the stream `used`.
@@ -41,7 +42,7 @@ struct DevReducer : ReducerImpl {
     // Where an update that is about to be launched writes its result, or nullptr.
     void *slot(vkc_ctx *ctx) {
         if (copies) return nullptr;
-        copies = stream_capturing(ctx->stream);
+        copies = lasts ? stream_capturing(ctx->stream) : captured;
         if (!copies && !host) {
             host = mem.box->take_slot(ctx->stream);
             copies = !host;
@@ -55,15 +56,17 @@ struct DevReducer : ReducerImpl {
     }
     vkc_status alloc(vkc_ctx *ctx, size_t n) {
         bytes = n;
-        bool captured;
         const vkc_status st = state_block(ctx, n, &mem, &captured);
         state = mem.ptr;
         return st;
     }
     vkc_status begin(vkc_ctx *ctx) override {
+        lasts = true;
         fresh = false;
-        return zero(ctx);
+        return clear(ctx);
     }
+    // The state of no rows.
+    virtual vkc_status clear(vkc_ctx *ctx) { return zero(ctx); }
     void into_device() override { copies = true; }
     // The state's n bytes zeroed (before a first update whose kernels read it).
     vkc_status zero(vkc_ctx *ctx) {
