@@ -541,7 +541,11 @@ __device__ __forceinline__ RgFold rg_fold_block(int kind, RgFold v) {
     return v;
 }
 
-// The host has cleared result->timeout; `timeout` was read as the kernel began, off the end's path.
+// The status word's timeout, read beside the partials (as the kernel begins it costs the loop a register: min of
+// x*y + z, 50 M rows, 20 us), and written with the fold: the host has cleared result->timeout.
+__device__ __forceinline__ unsigned rg_timeout(const DevStatus *status) {
+    return threadIdx.x == 0 ? *reinterpret_cast<const volatile unsigned *>(&status->timeout) : 0u;
+}
 __device__ __forceinline__ void rg_write(RgResult *result, const RgFold &v, unsigned timeout) {
     result->fold = v;
     if (timeout) result->timeout = timeout;
@@ -551,7 +555,6 @@ __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionPro
                                                                  RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     extern __shared__ unsigned long long s_w[];
     const int t = threadIdx.x;
-    const unsigned timeout = t == 0 ? *reinterpret_cast<const volatile unsigned *>(&status->timeout) : 0u;
     RgFold me{0, ~0ull, ~0ull, 0};
     for (int64_t b0 = static_cast<int64_t>(blockIdx.x) * RG_BLOCK_ROWS; b0 < n;
          b0 += static_cast<int64_t>(gridDim.x) * RG_BLOCK_ROWS) {
@@ -576,6 +579,7 @@ __global__ void __launch_bounds__(RG_THREADS) region_fold_kernel(const RegionPro
     const RgFold b = rg_fold_block(kind, me);
     if (t == 0) partials[blockIdx.x] = b;
     if (last_block(done)) {
+        const unsigned timeout = rg_timeout(status);
         RgFold v{0, ~0ull, ~0ull, 0};
         for (unsigned q = t; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
         v = rg_fold_block(kind, v);
@@ -729,8 +733,6 @@ __global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 :
                                                                    int kind, RgFold *partials, unsigned *done, const DevStatus *status, RgResult *result) {
     constexpr int RF_ROWS = rf_rows<NARR>(), RF_BLOCK_ROWS = RG_THREADS * RF_ROWS;
     extern __shared__ double s_d[];
-    const unsigned timeout =
-        MODE == RF_FOLD && threadIdx.x == 0 ? *reinterpret_cast<const volatile unsigned *>(&status->timeout) : 0u;
     unsigned long long count = 0;
     // Extremes: keys compared as if for a minimum (a maximum's are complemented).
     const bool arg = kind == RF_ARGMIN || kind == RF_ARGMAX;
@@ -799,6 +801,7 @@ __global__ void __launch_bounds__(RG_THREADS, NARR == 4 && MODE == RF_FOLD ? 5 :
         const RgFold b = rg_fold_block(kind, me);
         if (threadIdx.x == 0) partials[blockIdx.x] = b;
         if (last_block(done)) {
+            const unsigned timeout = rg_timeout(status);
             RgFold v{0, ~0ull, ~0ull, 0};
             for (unsigned q = threadIdx.x; q < gridDim.x; q += RG_THREADS) rg_fold_take(kind, v, partials[q]);
             v = rg_fold_block(kind, v);
