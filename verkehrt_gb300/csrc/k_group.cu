@@ -231,29 +231,33 @@ __global__ void __launch_bounds__(GI_THREADS) gi_insert_kernel(const long long *
 }
 
 // Short inputs, whose first table is the full one: nobody knows whether their keys are few, and the way of
-// few keys costs many distinct ones a read and the late start. So each block decides by its first rows:
-// where a warp's 32 share a key it takes the way of few keys, else of many. (Not with few blocks, whose
-// atomics hardly meet.) A call on 10^6 rows of 10 / 1000 /
-// 2^16 / all distinct keys with every block the way of few keys 79 / 69 / 89 / 112 us, of many 265 / 80 / 91 /
-// 102, so 80 / 68 / 88 / 101.
-constexpr unsigned GI_SHORT_STAGGER_NS = 2500;  // the first rows' read comes before it
+// few keys costs many distinct ones a read and the late start. So each block but the first GI_AHEAD decides by
+// its first rows: where a warp's 32 share a key it takes the way of few keys, else of many; and where many
+// share one, the few keys' atomics take turns for longer, and it starts later. (Not with few blocks, whose
+// atomics hardly meet.) A call on 10^6 rows of 2 / 10 / 1000 / 2^16 / all distinct keys with every block the
+// way of few keys 80 / 71 / 68 / 88 / 104 us, so 78 / 68 / 68 / 82 / 95 (of many, 10 keys took 265); without
+// the later start 86 / 70 / 68 / 82 / 96. Four blocks an SM: pairs would take 67 registers and three, 142 us
+// for distinct ones instead of 124.
+constexpr unsigned GI_SHORT_STAGGER_NS = 2500, GI_ALIKE_STAGGER_NS = 6000;  // the first rows' read comes before
+constexpr int GI_ALIKE = 7;  // rows of a warp that share a key: about ten keys or fewer
 template <bool PAIR>
-__global__ void __launch_bounds__(GI_THREADS) gi_insert_short_kernel(const long long *__restrict__ a,
-                                                                     const long long *__restrict__ b, int64_t n, bool,
-                                                                     GroupTable t, unsigned *__restrict__ slot_of,
-                                                                     unsigned *flags, DevStatus *st) {
-    if (gridDim.x >= 8 * GI_AHEAD) {
+__global__ void __launch_bounds__(GI_THREADS, 4) gi_insert_short_kernel(const long long *__restrict__ a,
+                                                                        const long long *__restrict__ b, int64_t n, bool,
+                                                                        GroupTable t, unsigned *__restrict__ slot_of,
+                                                                        unsigned *flags, DevStatus *st) {
+    if (gridDim.x >= 8 * GI_AHEAD && blockIdx.x >= GI_AHEAD) {
         const int64_t r = static_cast<int64_t>(blockIdx.x) * GI_THREADS * GI_ROWS + threadIdx.x;
         unsigned h = threadIdx.x;
         if (r < n) {
             const unsigned long long k = gmix(static_cast<unsigned long long>(a[r]));
             h = static_cast<unsigned>((PAIR ? gmix(k ^ static_cast<unsigned long long>(b[r])) : k) >> 32);
         }
-        if (!__syncthreads_or(__popc(__match_any_sync(FULL, h)) > 1)) {
+        const int alike = __popc(__match_any_sync(FULL, h));
+        if (!__syncthreads_or(alike > 1)) {
             gi_insert_rows<PAIR, false>(a, b, n, false, t, slot_of, flags, st);
             return;
         }
-        if (blockIdx.x >= GI_AHEAD) __nanosleep(GI_SHORT_STAGGER_NS);
+        __nanosleep(__syncthreads_or(alike >= GI_ALIKE) ? GI_ALIKE_STAGGER_NS : GI_SHORT_STAGGER_NS);
     }
     gi_insert_rows<PAIR, true>(a, b, n, false, t, slot_of, flags, st);
 }
