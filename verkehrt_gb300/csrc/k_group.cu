@@ -13,7 +13,8 @@
 //  2. number: the smallest rows of the slots are the first occurrences, and a group's id is the rank
 //     of its first row among them. They are marked in a bitmap of the rows, whose words' counts are
 //     scanned; each occupied slot takes its id from there, and every row reads its slot's. Short
-//     inputs (GN_MIN_ROWS) do it in one kernel instead, a decoupled-lookback compaction over rows.
+//     inputs (GN_MIN_ROWS) and full tables, whose slots are several times the rows, do it in one kernel
+//     instead, a decoupled-lookback compaction over rows.
 // Table size: the reference's maximum is nextpow2(2n) slots (group.rs:226-229). When that is
 // above the first table's size (2^group_first_table_log2 slots from the autotuner's table,
 // 2^21 by default, which stays in L2), the insert first runs on that table; it gives up (an
@@ -672,7 +673,9 @@ static void launch_insert(vkc_ctx *ctx, const long long *a, const long long *b, 
 constexpr int64_t GR_MIN_ROWS = int64_t(1) << 22;
 constexpr int64_t GR_STEP_ROWS = int64_t(1) << 19;
 
-// From this many rows on the table's numbering goes by ranks.
+// From this many rows on the first table's numbering goes by ranks. (The full table's reads its slots twice,
+// 32 bytes each: key pairs of 10 M rows, 1.5 M of them distinct, 1443 us a call by ranks, 1332 by the lookback;
+// all distinct 1996 / 1958.)
 constexpr int64_t GN_MIN_ROWS = int64_t(1) << 22;
 
 // Ranks the marked first occurrences (bits, one word per 32 of n rows) into rank[]; counts, before and
@@ -885,7 +888,7 @@ static vkc_status run_group(vkc_ctx *ctx, const vkc_array *xa, const vkc_array *
         }
     }
     Ranking rk;
-    if (n >= GN_MIN_ROWS) {
+    if (done && n >= GN_MIN_ROWS) {
         if (rk.alloc(ctx, n, true)) return alloc_fail();
         const int g = stream_grid(ctx, static_cast<int64_t>(t.mask + 1), 256, 8, 1024);
         gn_slots_kernel<false><<<g, 256, 0, ctx->stream>>>(t, rk.bits, nullptr);
